@@ -621,7 +621,8 @@ static int union_sssp(grus_batch *b, const grus_query *queries, const std::vecto
       grus_graph *g = b->graphs[p.graph];
       if (p.q.size() == 1) {
         const grus_query &q = queries[p.q[0]];
-        rc = grus_sssp(g, q.src, out + q.out_offset, nullptr, s);
+        rc = sssp_run(g, q.src, out + q.out_offset, nullptr, s, sssp_lane_tail(g));
+        *nlaunch += sssp_lane_tail(g);
         cv = sssp_ctrl(g);
       } else {
         uint32_t srcs[32];

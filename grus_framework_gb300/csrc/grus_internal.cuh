@@ -100,6 +100,16 @@ int msbfs_run(grus_graph *g, const uint32_t *hsrc, int k, uint32_t *const *outs,
 int msssp_run(grus_graph *g, const uint32_t *hsrc, int k, uint32_t *const *outs,
               grus_stats *stats, cudaStream_t s);
 
+// Single-source SSSP (sssp.cu).  tail: launch the cluster kernel behind the
+// persistent one (2 kernels, else 1); grus_sssp does where sssp_tail says so.
+// The batch and the server, whose lanes queue launches back to back, do on
+// graphs without hubs (sssp_lane_tail): on scale-free graphs the cluster
+// takes over the last few levels only (0-9 % of a query).
+int sssp_run(grus_graph *g, uint32_t src, uint32_t *dist, grus_stats *stats, cudaStream_t s,
+             bool tail);
+bool sssp_tail(const grus_graph *g);
+bool sssp_lane_tail(const grus_graph *g);
+
 // Fewest BFS queries on one graph of m edges for which one multi-source
 // launch (msbfs_run) beats as many single launches.  Measured on RMAT graphs
 // with random sources: a 16-source pack costs 2.2-5.3 single launches' time

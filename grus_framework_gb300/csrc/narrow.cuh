@@ -1,0 +1,638 @@
+// narrow.cuh -- a traversal with a small frontier, run by ONE thread-block
+// cluster (up to 16 CTAs): BFS (every edge counts 1) and SSSP (uint32 weights).
+//
+// A level of a few thousand edges costs a whole-GPU persistent kernel 9-14 us
+// of grid barriers and dependent loads whatever its size.  Here a step's cost
+// is one chain of loads inside one CTA, and what is small is kept on chip:
+//   * Work entries {v, begin, end, d} -- up to kPiece out-edges of v, reached
+//     at distance d -- sit in shared memory.  Vertex v has a home CTA
+//     (contiguous ranges of ids); a vertex improved by its home goes to that
+//     CTA's next list, one improved elsewhere to its home's inbox through
+//     distributed shared memory.
+//   * A CTA runs up to kRounds rounds over what its own rounds produce, with
+//     block barriers only, before the cluster barrier that makes the inboxes
+//     readable: graphs whose ids follow their geometry (grids, road networks,
+//     chains) cross the cluster barrier once per kRounds levels.
+//   * Distances are lowered by atomicMin in L2 (the one L2 round trip that a
+//     round waits for besides its adjacency loads); an entry whose d is no
+//     longer v's distance is skipped.  Rounds of different CTAs may run at
+//     different depths, so a vertex can be expanded again when a shorter path
+//     arrives later; distances below the threshold T bound how far ahead a
+//     CTA can get.  Whatever the schedule, the fixpoint -- the shortest
+//     distances -- is the same.
+//   * Distances of T and above wait in a far list per CTA (global memory);
+//     when no CTA has near work, T advances to the smallest far distance plus
+//     Delta (one cluster barrier), so all distances below the old T are final.
+// A full list never loses work: its overflow goes to the near or far bitmap,
+// which the next step (split) scans.
+//
+// Bound by latency: a round with one entry takes 1.0-1.3 us (a path of 4,001
+// vertices), of which the atomic's round trip is about a third, and a cluster
+// barrier with its stamps about 1 us more.  Measured for SSSP (a 1,021 x
+// 1,531 grid / a 40 x 3,000 grid / RMAT-12, ms): 512 threads and 8 rounds per
+// step 13.6 / 18.5 / 0.18, 4 rounds 12.7 / 14.8 / 0.18, 16 rounds 16.7 / 20.8
+// / 0.18; 1,024 threads and 4 rounds 11.8 / 14.5 / 0.17, which is kept: more
+// threads cost the narrowest frontiers 10 % and gain 10-20 % on wider ones.
+// Prefetching the lines after a target's (adjacency, offsets, distance) as
+// well as its own: 14.6 against 13.3 ms on the first grid.
+#pragma once
+
+#include <cooperative_groups.h>
+
+#include "device_util.cuh"
+
+namespace grus {
+namespace narrow {
+
+namespace cg = cooperative_groups;
+
+constexpr int kBlock = 1024;
+constexpr int kWarps = kBlock / 32;
+constexpr int kMaxCluster = 16;
+constexpr uint32_t kCap = 2048;      // entries of one list
+constexpr uint32_t kPiece = 64;      // edges per entry
+// Low-degree graphs, few entries: kLanes lanes per entry instead of a scan
+// over the entries' degrees (the path's round 1.57 -> 1.04 us with 512
+// threads; entries of up to 64 edges would take 8 serial steps instead:
+// RMAT-12 0.19 -> 0.25 ms).
+constexpr uint32_t kLanes = 8;
+constexpr uint32_t kFew = 32 / kLanes;       // entries per warp
+constexpr uint32_t kLowDegree = 2 * kLanes;  // largest out-degree of the graph
+constexpr int kRounds = 4;           // rounds between cluster barriers
+constexpr int kIlp = 2;              // 32-edge steps whose loads are in flight together
+constexpr uint32_t kFarCap = 8192;   // far entries per CTA and buffer
+constexpr uint32_t kInf = 4294967294u;
+constexpr uint32_t kRing = 128;      // BFS: depth counts, by depth modulo kRing
+constexpr uint32_t kUnitDelta = 32;  // BFS: levels per threshold step (<= kRing / 2)
+
+// Far lists of one cluster: 2 buffers per CTA.
+constexpr size_t kFarBytes = (size_t)kMaxCluster * 2 * kFarCap * sizeof(uint2);
+
+// Per-step record (SSSP) or per-level record (BFS), the layout of the
+// persistent kernels' traces.
+struct Trace {
+  unsigned long long t_ns, edges;
+  uint32_t count, tag;
+};
+
+struct View {
+  const uint32_t *__restrict__ offs;
+  const uint32_t *__restrict__ cols;
+  const uint32_t *__restrict__ wts;  // unused by BFS
+  uint32_t n, W;
+  uint32_t *dist;
+  uint32_t *nearbm;  // W words, all zero at the start
+  uint32_t *farbm;   // W words, zero but for what farbm_used announces
+  uint2 *far;        // kFarBytes
+  uint32_t delta;
+  bool adapt;        // SSSP: delta may grow while threshold steps do little
+  bool low_degree;   // every vertex has at most kLowDegree out-edges
+  uint32_t *err;
+  // null: none.  SSSP: record i is the i-th step's (from 1); BFS: record d
+  // counts the vertices of depth d.  Records to be written start out zero.
+  Trace *trace;
+  uint32_t trace_cap;
+  uint32_t tag;      // SSSP: threshold steps taken before
+};
+
+// Starts filling this SM's L1 with the line holding p (no wait).
+__device__ __forceinline__ void prefetch_l1(const void *p) {
+  asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+}
+
+struct Shared {
+  uint4 loc[2][kCap];
+  uint4 inb[2][kCap];
+  uint32_t cnt[3];                      // local list lengths, rotating by round
+  uint32_t incnt[2], farcnt[2];
+  // the last step in which this CTA pushed to an inbox, spilled to the near
+  // bitmap, put bits in the far bitmap (0: never), ...
+  uint32_t pushed, spilled, farbm;
+  // ... and rank 0: the last step in which any CTA had work left or spilled,
+  // and the last that put bits in the far bitmap
+  uint32_t g_farbm;
+  uint2 g_work;
+  uint32_t min_far;                     // smallest distance of this CTA's far vertices
+  uint32_t red[kWarps];
+  unsigned long long red64[kWarps];
+  int ring[kRing];                      // BFS: labels given minus labels replaced, by depth
+  int ring_sum[kRing];                  // rank 0: summed over the cluster
+};
+
+struct Result {
+  uint32_t steps = 0, splits = 0;
+  uint32_t last = 0;                    // BFS: largest depth (valid in rank 0)
+  unsigned long long visits = 0, nr = 0, mr = 0;  // this thread's share
+};
+
+template <bool kUnit>
+struct Engine {
+  const View &a;
+  Shared *s;
+  cg::cluster_group cl;
+  uint32_t rank, C, lane, warp;
+  uint32_t scale;             // home of v: umulhi(v, scale)
+  uint32_t T, step;           // steps count from 1 (0 = never)
+  uint32_t delta, last_split; // current threshold step and the last one's step number
+  uint32_t scanned;           // far bitmap bits up to this step have been taken
+  uint32_t cq, lb, ip, fb;    // read: cnt[cq], loc[lb], inb[ip], far buffer fb
+  Result res;
+
+  __device__ __forceinline__ Engine(const View &view, Shared *sh)
+      : a(view), s(sh), cl(cg::this_cluster()) {
+    rank = cl.block_rank();
+    C = cl.num_blocks();
+    lane = lane_id();
+    warp = threadIdx.x >> 5;
+    const unsigned long long q = ((unsigned long long)C << 32) / max(a.n, 1u);
+    scale = q > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)q;
+    T = 0;
+    step = 1;
+    scanned = last_split = 0;
+    delta = a.delta;
+    cq = lb = ip = fb = 0;
+    if (threadIdx.x < 3) s->cnt[threadIdx.x] = 0u;
+    if (threadIdx.x < 2) s->incnt[threadIdx.x] = s->farcnt[threadIdx.x] = 0u;
+    if (threadIdx.x < kRing) s->ring[threadIdx.x] = s->ring_sum[threadIdx.x] = 0;
+    if (threadIdx.x == 0) {
+      s->pushed = s->spilled = s->farbm = s->g_farbm = 0u;
+      s->g_work = make_uint2(0u, 0u);
+    }
+  }
+
+  __device__ __forceinline__ uint32_t home(uint32_t v) const { return __umulhi(v, scale); }
+
+  __device__ __forceinline__ void spill(uint32_t v) {
+    atomicOr(a.nearbm + (v >> 5), 1u << (v & 31u));
+    s->spilled = step;
+  }
+
+  // Queues the vertices u (edges [b,e), distance d) of the lanes with `want`:
+  // one entry at its home, or pieces of kPiece edges dealt over the cluster.
+  // Called by whole warps.
+  __device__ __forceinline__ void push(bool want, uint32_t u, uint32_t b, uint32_t e, uint32_t d) {
+    want = want && e > b;
+    const uint32_t nq = cq == 2 ? 0 : cq + 1;
+    const uint32_t o = home(u);
+    const bool big = want && e - b > kPiece;
+    const bool here = want && !big && o == rank;
+    if (here) {
+      const uint32_t pos = atomicAdd(&s->cnt[nq], 1u);
+      if (pos < kCap) s->loc[lb ^ 1u][pos] = make_uint4(u, b, e, d);
+      else spill(u);
+    }
+    if (__all_sync(0xffffffffu, here == want)) return;
+    const bool far_home = want && !big && o != rank;
+    const uint32_t mr = __ballot_sync(0xffffffffu, far_home);
+    if (far_home) {
+      const uint32_t peers = __match_any_sync(mr, o);
+      const int leader = __ffs(peers) - 1;
+      Shared *r = cl.map_shared_rank(s, o);
+      uint32_t base = 0;
+      if ((int)lane == leader) base = atomicAdd(&r->incnt[ip ^ 1u], __popc(peers));
+      base = __shfl_sync(peers, base, leader);
+      const uint32_t pos = base + __popc(peers & ((1u << lane) - 1u));
+      if (pos < kCap) r->inb[ip ^ 1u][pos] = make_uint4(u, b, e, d);
+      else spill(u);
+      s->pushed = step;
+    }
+    __syncwarp();
+    for (uint32_t mb = __ballot_sync(0xffffffffu, big); mb; mb &= mb - 1) {
+      const int j = __ffs(mb) - 1;
+      const uint32_t pu = __shfl_sync(0xffffffffu, u, j), pb = __shfl_sync(0xffffffffu, b, j);
+      const uint32_t pe = __shfl_sync(0xffffffffu, e, j), pd = __shfl_sync(0xffffffffu, d, j);
+      const uint32_t po = __shfl_sync(0xffffffffu, o, j);
+      const uint32_t np = (pe - pb + kPiece - 1) / kPiece;
+      for (uint32_t k = lane; k < np; k += 32) {
+        const uint32_t t = (po + k) % C;
+        const uint32_t xb = pb + k * kPiece;
+        const uint4 en = make_uint4(pu, xb, min(pe, xb + kPiece), pd);
+        if (t == rank) {
+          const uint32_t pos = atomicAdd(&s->cnt[nq], 1u);
+          if (pos < kCap) s->loc[lb ^ 1u][pos] = en;
+          else spill(pu);
+        } else {
+          Shared *r = cl.map_shared_rank(s, t);
+          const uint32_t pos = atomicAdd(&r->incnt[ip ^ 1u], 1u);
+          if (pos < kCap) r->inb[ip ^ 1u][pos] = en;
+          else spill(pu);
+          s->pushed = step;
+        }
+      }
+      __syncwarp();
+    }
+  }
+
+  // Puts (u, d) of the lanes with `want` on this CTA's far list `buf`.
+  __device__ __forceinline__ void push_far(bool want, uint32_t u, uint32_t d, uint32_t buf) {
+    const uint32_t m = __ballot_sync(0xffffffffu, want);
+    if (!m) return;
+    uint32_t base = 0;
+    const int leader = __ffs(m) - 1;
+    if ((int)lane == leader) base = atomicAdd(&s->farcnt[buf], __popc(m));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    if (want) {
+      const uint32_t pos = base + __popc(m & ((1u << lane) - 1u));
+      if (pos < kFarCap) {
+        a.far[(size_t)(rank * 2 + buf) * kFarCap + pos] = make_uint2(u, d);
+      } else {
+        atomicOr(a.farbm + (u >> 5), 1u << (u & 31u));
+        s->farbm = step;
+      }
+    }
+  }
+
+  // Relaxes the entries of a warp's lanes (v, [beg,end), d; the lanes with
+  // `has` are the first ones and their ranges are not empty): their edges are
+  // laid end to end, one per lane.  A target's offsets are loaded beside the
+  // atomic that lowers its distance, so pushing it waits for nothing more.
+  // Called by whole warps.
+  __device__ __forceinline__ void relax(uint4 en, bool has) {
+    const uint32_t deg = has ? en.z - en.y : 0u;
+    const uint32_t cur = has ? __ldcg(a.dist + en.x) : 0u;
+    uint32_t incl = deg;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+      if ((int)lane >= o) incl += t;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31), excl = incl - deg;
+    const bool fresh = cur == en.w;
+    for (uint32_t k0 = 0; k0 < total; k0 += 32 * kIlp) {
+      uint32_t u[kIlp], nd[kIlp], b[kIlp], e[kIlp], old[kIlp];
+      bool act[kIlp];
+#pragma unroll
+      for (int i = 0; i < kIlp; ++i) {
+        if (i && k0 + 32 * i >= total) {
+          u[i] = nd[i] = 0u;
+          act[i] = false;
+          continue;
+        }
+        // edge k0 + 32 i + lane's entry: the entries that begin before this
+        // step, and those that begin in it up to this lane
+        const uint32_t k1 = k0 + 32 * i, k = k1 + lane;
+        const uint32_t before = __popc(__ballot_sync(0xffffffffu, has && excl < k1));
+        const uint32_t heads =
+            __reduce_or_sync(0xffffffffu, has && excl >= k1 && excl < k1 + 32 ? 1u << (excl - k1) : 0u);
+        const uint32_t j = before + __popc(heads & (0xFFFFFFFFu >> (31u - lane))) - 1u;
+        const uint32_t ob = __shfl_sync(0xffffffffu, en.y, j);
+        const uint32_t of = __shfl_sync(0xffffffffu, excl, j);
+        const uint32_t od = __shfl_sync(0xffffffffu, en.w, j);
+        act[i] = k < total;
+        const uint32_t x = ob + (k - of);
+        u[i] = act[i] ? __ldg(a.cols + x) : 0u;
+        nd[i] = od + (kUnit ? 1u : (act[i] ? __ldg(a.wts + x) : 0u));
+        act[i] = __shfl_sync(0xffffffffu, (int)fresh, j) && act[i];
+      }
+      // a plain read first: most edges into a dense part of the graph improve
+      // nothing, and their atomics would queue up on its hubs
+#pragma unroll
+      for (int i = 0; i < kIlp; ++i) old[i] = act[i] ? __ldcg(a.dist + u[i]) : 0u;
+#pragma unroll
+      for (int i = 0; i < kIlp; ++i) {
+        res.visits += act[i];
+        act[i] = act[i] && nd[i] < old[i];
+      }
+#pragma unroll
+      for (int i = 0; i < kIlp; ++i) {
+        b[i] = act[i] ? __ldg(a.offs + u[i]) : 0u;
+        e[i] = act[i] ? __ldg(a.offs + u[i] + 1) : 0u;
+        old[i] = act[i] ? atomicMin(a.dist + u[i], nd[i]) : 0u;
+      }
+      // the edges of the targets that improve and stay on this SM: started
+      // before the atomics' answers arrive
+#pragma unroll
+      for (int i = 0; i < kIlp; ++i)
+        if (act[i]) prefetch_edges(b[i]);
+#pragma unroll
+      for (int i = 0; i < kIlp; ++i) {
+        if (i && k0 + 32 * i >= total) break;
+        settle(act[i] && nd[i] < old[i], true, u[i], nd[i], old[i], b[i], e[i]);
+      }
+    }
+  }
+
+  __device__ __forceinline__ void prefetch_edges(uint32_t b) {
+    prefetch_l1(a.cols + b);
+    if (!kUnit) prefetch_l1(a.wts + b);
+  }
+
+  // The lanes with `imp` lowered vertex u (edges [b,e)) from `old` to nd; the
+  // ones with `queue` too push it.  Called by whole warps.
+  __device__ __forceinline__ void settle(bool imp, bool queue, uint32_t u, uint32_t nd,
+                                         uint32_t old, uint32_t b, uint32_t e) {
+    if (!__any_sync(0xffffffffu, imp)) return;
+    if (imp) {
+      if (old == kInf) {
+        res.nr += 1;
+        res.mr += e - b;
+      }
+      if (kUnit) count_depth(nd, old, e - b);
+    }
+    push(imp && queue && nd < T, u, b, e, nd);
+    push_far(imp && queue && nd >= T && e > b, u, nd, fb);
+  }
+
+  // Few entries (at most kFew per warp): kLanes lanes per entry, no scan, and
+  // nothing waits for the check that an entry is still current.  A stale
+  // entry may lower a distance, but does not push: the entry that made it
+  // stale relaxes the same edge with a smaller candidate, before (then this
+  // one lowers nothing) or after (then that one lowers and pushes).
+  // Called by whole warps.
+  __device__ __forceinline__ void relax_few(uint4 en, bool has) {
+    const uint32_t cur = has ? __ldcg(a.dist + en.x) : 0u;
+    for (uint32_t x = en.y + (lane & (kLanes - 1)); __any_sync(0xffffffffu, has && x < en.z);
+         x += kLanes) {
+      const bool act = has && x < en.z;
+      const uint32_t u = act ? __ldg(a.cols + x) : 0u;
+      const uint32_t nd = en.w + (kUnit ? 1u : (act ? __ldg(a.wts + x) : 0u));
+      const uint32_t b = act ? __ldg(a.offs + u) : 0u, e = act ? __ldg(a.offs + u + 1) : 0u;
+      const uint32_t old = act ? atomicMin(a.dist + u, nd) : 0u;
+      if (act) prefetch_edges(b);
+      res.visits += act;
+      settle(act && nd < old, cur == en.w, u, nd, old, b, e);
+    }
+  }
+
+  // BFS: a vertex of degree `deg` got label nd in place of old.
+  __device__ __forceinline__ void count_depth(uint32_t nd, uint32_t old, uint32_t deg) {
+    atomicAdd(&s->ring[nd % kRing], 1);
+    if (old != kInf) atomicAdd(&s->ring[old % kRing], -1);
+    if (a.trace && nd < a.trace_cap) {
+      atomicAdd(&a.trace[nd].count, 1u);
+      atomicAdd(&a.trace[nd].edges, (unsigned long long)deg);
+    }
+    if (a.trace && old < a.trace_cap) {
+      atomicAdd(&a.trace[old].count, 0xFFFFFFFFu);
+      atomicAdd(&a.trace[old].edges, 0ull - deg);
+    }
+  }
+
+  // Vertices spilled to the near bitmap in the previous step: this CTA's
+  // share of the words, a word per warp at a time.
+  __device__ __forceinline__ void relax_spilled() {
+    const uint32_t per = (a.W + C - 1) / C;
+    const uint32_t w0 = min(a.W, rank * per), w1 = min(a.W, w0 + per);
+    for (uint32_t w = w0 + warp; w < w1; w += kWarps) {
+      uint32_t bits = 0;
+      if (lane == 0 && __ldcg(a.nearbm + w)) bits = atomicExch(a.nearbm + w, 0u);
+      bits = __shfl_sync(0xffffffffu, bits, 0);
+      if (!bits) continue;
+      const bool has = lane < __popc(bits);
+      const uint32_t v = w * 32 + (has ? __fns(bits, 0, lane + 1) : 0u);
+      uint4 en = make_uint4(v, 0u, 0u, 0u);
+      if (has) {
+        en.y = __ldg(a.offs + v);
+        en.z = __ldg(a.offs + v + 1);
+        en.w = __ldcg(a.dist + v);
+      }
+      relax(en, has);
+    }
+  }
+
+  __device__ __forceinline__ uint32_t block_min(uint32_t x) {
+    x = __reduce_min_sync(0xffffffffu, x);
+    if (lane == 0) s->red[warp] = x;
+    __syncthreads();
+    uint32_t m = 0xFFFFFFFFu;
+#pragma unroll
+    for (int i = 0; i < kWarps; ++i) m = min(m, s->red[i]);
+    return m;
+  }
+
+  // No CTA has near work: T advances past the smallest far distance and the
+  // far vertices below it are pushed (this CTA's list and, if any CTA put
+  // bits there, its share of the far bitmap).  False when nothing is far.
+  __device__ __forceinline__ bool split() {
+    const uint2 *cur = a.far + (size_t)(rank * 2 + fb) * kFarCap;
+    const uint32_t fc = min(s->farcnt[fb], kFarCap);
+    const bool bm = *(volatile uint32_t *)&cl.map_shared_rank(s, 0)->g_farbm > scanned;
+    scanned = step - 1;
+    const uint32_t per = (a.W + C - 1) / C;
+    const uint32_t w0 = min(a.W, rank * per), w1 = min(a.W, w0 + per);
+    uint32_t m = 0xFFFFFFFFu;
+    for (uint32_t i = threadIdx.x; i < fc; i += kBlock) {
+      const uint2 f = __ldcg(cur + i);
+      if (__ldcg(a.dist + f.x) == f.y) m = min(m, f.y);
+    }
+    if (bm) {
+      for (uint32_t w = w0 + threadIdx.x; w < w1; w += kBlock)
+        for (uint32_t bits = __ldcg(a.farbm + w); bits; bits &= bits - 1) {
+          const uint32_t d = __ldcg(a.dist + w * 32 + (__ffs(bits) - 1));
+          if (d >= T) m = min(m, d);  // below T: expanded as near since
+        }
+    }
+    m = block_min(m);
+    if (threadIdx.x == 0) s->min_far = m;
+    cl.sync();
+    const uint32_t gm = __reduce_min_sync(
+        0xffffffffu, *(volatile uint32_t *)&cl.map_shared_rank(s, lane % C)->min_far);
+    if (gm == 0xFFFFFFFFu) return false;
+    if (kUnit) {
+      // every depth below T is final; the labels of depth T stay counted
+      if (threadIdx.x < kRing && threadIdx.x != T % kRing) s->ring[threadIdx.x] = 0;
+      if (a.trace && rank == 0 && threadIdx.x == 0)
+        for (uint32_t d = T; d > 0 && d < a.trace_cap && a.trace[d].t_ns == 0; --d)
+          a.trace[d].t_ns = global_timer_ns();
+    }
+    const uint32_t Told = T;
+    // weights far above delta: a threshold step should last a few steps
+    if (a.adapt && step - last_split <= 3 && delta < 1u << 30) delta *= 2;
+    last_split = step;
+    T = gm > 0xFFFFFFFFu - delta ? 0xFFFFFFFFu : gm + delta;
+    const uint32_t rounds = (fc + kBlock - 1) / kBlock;
+    for (uint32_t r = 0; r < rounds; ++r) {
+      const uint32_t i = r * kBlock + threadIdx.x;
+      const uint2 f = i < fc ? __ldcg(cur + i) : make_uint2(0u, 0u);
+      const bool live = i < fc && __ldcg(a.dist + f.x) == f.y;
+      const uint32_t b = live ? __ldg(a.offs + f.x) : 0u, e = live ? __ldg(a.offs + f.x + 1) : 0u;
+      push(live && f.y < T, f.x, b, e, f.y);
+      push_far(live && f.y >= T, f.x, f.y, fb ^ 1u);
+    }
+    if (bm) {
+      for (uint32_t w = w0 + warp; w < w1; w += kWarps) {
+        // other CTAs may be setting bits of far vertices they cannot list
+        uint32_t bits = 0;
+        if (lane == 0 && __ldcg(a.farbm + w)) bits = atomicExch(a.farbm + w, 0u);
+        bits = __shfl_sync(0xffffffffu, bits, 0);
+        if (!bits) continue;
+        const uint32_t v = w * 32 + lane;
+        const bool has = (bits >> lane) & 1u;
+        const uint32_t d = has ? __ldcg(a.dist + v) : 0u;
+        const bool live = has && d >= Told;
+        const uint32_t b = live ? __ldg(a.offs + v) : 0u, e = live ? __ldg(a.offs + v + 1) : 0u;
+        push(live && d < T, v, b, e, d);
+        push_far(live && d >= T, v, d, fb ^ 1u);
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      s->farcnt[fb] = 0u;
+      s->cnt[cq == 0 ? 2 : cq - 1] = 0u;  // the list of the rounds to come
+    }
+    fb ^= 1u;
+    __syncthreads();
+    ++res.splits;
+    return true;
+  }
+
+  // After a round: the pushes made before the call become readable by their
+  // readers; true if any CTA has near work.
+  __device__ __forceinline__ bool end_step(bool &spilled) {
+    if (threadIdx.x == 0) {
+      // stamps only grow, so nobody clears them: a CTA already in the next
+      // step got there because this step had work, which every CTA saw
+      Shared *r = cl.map_shared_rank(s, 0);
+      if (s->cnt[cq] || s->pushed == step) *(volatile uint32_t *)&r->g_work.x = step;
+      if (s->spilled == step) *(volatile uint32_t *)&r->g_work.y = step;
+      if (s->farbm == step) *(volatile uint32_t *)&r->g_farbm = step;
+    }
+    cl.sync();
+    const Shared *r = cl.map_shared_rank(s, 0);
+    const uint32_t gw = *(const volatile uint32_t *)&r->g_work.x;
+    const uint32_t gs = *(const volatile uint32_t *)&r->g_work.y;
+    spilled = gs >= step;
+    ip ^= 1u;
+    ++step;
+    return gw >= step - 1 || spilled;
+  }
+
+  __device__ __forceinline__ void next_round() {
+    __syncthreads();
+    cq = cq == 2 ? 0 : cq + 1;
+    lb ^= 1u;
+  }
+
+  // Runs the traversal to its end.  Before the call the caller has
+  // synchronised the cluster after construction and then pushed the starting
+  // entries (all below T).
+  __device__ __forceinline__ void run() {
+    next_round();
+    while (true) {
+      bool spilled = false;
+      const bool work = end_step(spilled);
+      if (!work) {
+        if (!split()) break;
+        next_round();
+      }
+      const unsigned long long v0 = res.visits;
+      uint32_t taken = 0;
+#pragma unroll 1
+      for (int r = 0; r < kRounds; ++r) {
+        const uint32_t nc = min(s->cnt[cq], kCap);
+        const uint32_t ni = r == 0 ? min(s->incnt[ip], kCap) : 0u;
+        const uint32_t total = nc + ni;
+        const bool scan = r == 0 && spilled;
+        if (total == 0 && !scan) break;
+        // the list after next was read in the round before this one
+        if (threadIdx.x == 0) s->cnt[cq == 0 ? 2 : cq - 1] = 0u;
+        taken += total;
+        if (a.low_degree && total <= kWarps * kFew) {
+          const uint32_t i = warp * kFew + lane / kLanes;
+          const bool has = i < total;
+          uint4 en = make_uint4(0u, 0u, 0u, 0u);
+          if (has) en = i < nc ? s->loc[lb][i] : s->inb[ip][i - nc];
+          relax_few(en, has);
+        } else {
+          const uint32_t epw = min(32u, (total + kWarps - 1) / kWarps);
+          for (uint32_t base = warp * epw; base < total; base += kWarps * epw) {
+            const uint32_t i = base + lane;
+            const bool has = lane < epw && i < total;
+            uint4 en = make_uint4(0u, 0u, 0u, 0u);
+            if (has) en = i < nc ? s->loc[lb][i] : s->inb[ip][i - nc];
+            relax(en, has);
+          }
+        }
+        if (scan) relax_spilled();
+        next_round();
+        if (r == 0 && threadIdx.x == 0) s->incnt[ip] = 0u;
+      }
+      ++res.steps;
+      if (!kUnit && a.trace && res.steps < a.trace_cap) {
+        Trace *t = a.trace + res.steps;
+        atomicAdd(&t->edges, res.visits - v0);
+        if (threadIdx.x == 0) {
+          atomicAdd(&t->count, taken);
+          if (rank == 0) {
+            t->t_ns = global_timer_ns();
+            t->tag = a.tag + res.splits;
+          }
+        }
+      }
+      if ((unsigned long long)step > 16ull * a.n + 1024ull) {
+        if (rank == 0 && threadIdx.x == 0) atomicOr(a.err, kErrLevels);
+        break;
+      }
+    }
+    if (kUnit) {
+      // the largest depth still held by a vertex, among the last threshold's
+      __syncthreads();
+      if (threadIdx.x < kRing && s->ring[threadIdx.x])
+        atomicAdd(&cl.map_shared_rank(s, 0)->ring_sum[threadIdx.x], s->ring[threadIdx.x]);
+      cl.sync();
+      if (rank == 0 && threadIdx.x == 0) {
+        uint32_t d = T;  // the labels of [T - Delta, T] are counted
+        while (d > T - a.delta && s->ring_sum[d % kRing] <= 0) --d;
+        res.last = d;
+      }
+    }
+    cl.sync();  // no CTA leaves while another may still write its shared memory
+  }
+
+  // Sum over the block of a per-thread count; valid in thread 0.
+  __device__ __forceinline__ unsigned long long block_sum(unsigned long long x) {
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    __syncthreads();
+    if (lane == 0) s->red64[warp] = x;
+    __syncthreads();
+    unsigned long long t = 0;
+    if (threadIdx.x == 0)
+      for (int i = 0; i < kWarps; ++i) t += s->red64[i];
+    return t;
+  }
+};
+
+// Launch attributes of a one-cluster kernel using Engine: the largest cluster
+// (16, 8, 4, 2 or 1 CTAs) the device can co-schedule.
+template <class Kernel>
+int cluster_size(Kernel kern) {
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Shared));
+  cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  for (int k = kMaxCluster; k > 1; k /= 2) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)k;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)k);
+    cfg.blockDim = dim3(kBlock);
+    cfg.dynamicSmemBytes = sizeof(Shared);
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int nc = 0;
+    if (cudaOccupancyMaxActiveClusters(&nc, kern, &cfg) == cudaSuccess && nc >= 1) return k;
+    cudaGetLastError();
+  }
+  return 1;
+}
+
+template <class Kernel, class Args>
+cudaError_t launch(Kernel kern, int cluster, const Args &a, cudaStream_t s) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)cluster;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)cluster);
+  cfg.blockDim = dim3(kBlock);
+  cfg.dynamicSmemBytes = sizeof(Shared);
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, a);
+}
+
+}  // namespace narrow
+}  // namespace grus

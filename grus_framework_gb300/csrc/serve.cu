@@ -229,7 +229,8 @@ size_t big_workspace_bytes(const grus_graph *g, uint32_t algo, bool multi) {
   const size_t n = g->n, m = g->m;
   if (algo == GRUS_ALGO_SSSP && multi) return 128 * n + 16 * n + m / 8 + (1u << 20);
   // a BFS pack also keeps 64 depth bytes per vertex
-  return (algo == GRUS_ALGO_SSSP ? 20 * n : (multi ? 104 * n : 40 * n)) + m / 32 + (1u << 20);
+  // ... and a single query 2 MB of far lists
+  return (algo == GRUS_ALGO_SSSP ? 20 * n : (multi ? 104 * n : 40 * n)) + m / 32 + (4u << 20);
 }
 
 bool big_workspace_ready(const grus_graph *g, uint32_t algo, bool multi) {
@@ -271,8 +272,9 @@ int big_launch(grus_server *s, BigJob &j) {
   }
   int rc;
   if (!multi) {
-    rc = r.algo == GRUS_ALGO_SSSP ? grus_sssp(g, r.src, r.out, nullptr, s->big_stream)
-                                  : grus_bfs(g, r.src, r.out, nullptr, s->big_stream);
+    rc = r.algo == GRUS_ALGO_SSSP
+             ? sssp_run(g, r.src, r.out, nullptr, s->big_stream, sssp_lane_tail(g))
+             : grus_bfs(g, r.src, r.out, nullptr, s->big_stream);
   } else {
     uint32_t srcs[64];
     uint32_t *outs[64];
@@ -285,8 +287,9 @@ int big_launch(grus_server *s, BigJob &j) {
              : msbfs_run(g, srcs, (int)j.group.size(), outs, nullptr, s->big_stream);
   }
   if (rc) return rc;
-  // a single BFS is the persistent kernel and its narrow-tail kernel
-  s->kernel_launches += (!multi && r.algo != GRUS_ALGO_SSSP) ? 2 : 1;
+  // a single query is one kernel and, for BFS and where sssp_lane_tail says
+  // so, the narrow one behind it; a pack is one kernel
+  s->kernel_launches += !multi && (r.algo != GRUS_ALGO_SSSP || sssp_lane_tail(g)) ? 2 : 1;
   j.ctrl = r.algo == GRUS_ALGO_SSSP ? (multi ? msssp_ctrl(g) : sssp_ctrl(g))
                                     : (multi ? msbfs_ctrl(g) : bfs_ctrl(g));
   *j.h_err = 0;

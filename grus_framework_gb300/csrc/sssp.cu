@@ -24,11 +24,16 @@
 // bucket of the smallest far distance) and F is scanned: vertices below the
 // old T were expanded as near since and are dropped, vertices below the new T
 // move to N[L & 1], the rest stay.  Every wait is a bounded grid barrier.
+//
+// A level costs the grid at least 13 us, so levels that stay small are handed
+// to one thread-block cluster (sssp_narrow, narrow.cuh), which also runs small
+// graphs from the start.
 #include <algorithm>
 #include <cstring>
 
 #include "expand.cuh"
 #include "grus_internal.cuh"
+#include "narrow.cuh"
 
 namespace grus {
 namespace {
@@ -36,6 +41,29 @@ namespace {
 constexpr int kBlock = 256;
 constexpr uint32_t kDefHuge = 1024;
 constexpr uint32_t kDefDelta = 640;
+// Hand-over to the cluster kernel (sssp_narrow): levels of at most
+// kNarrowNf near vertices per cluster CTA, one after another.  While they
+// shrink (the end of a traversal) with at most 2^kNarrowBits unreached
+// out-edges left; or after kNarrowSteady of them with a frontier no larger
+// than a plane's circle would be (4 s^2 at level s: a random graph's frontier
+// grows past it) -- high diameter, where every level costs the whole grid
+// 13-19 us however small it is.  The edge bound caps what a cluster, a tenth
+// of the chip, can be left with; levels that stay small three times longer
+// raise it.
+constexpr uint32_t kNarrowNf = 128;
+constexpr uint32_t kNarrowSteady = 8;
+constexpr uint32_t kNarrowBits = 22, kNarrowBitsLong = 26;
+// Delta of the cluster kernel unless the caller set one: its levels are
+// short, so more distance per threshold step pays (grid 1021 x 1531: Delta
+// 640 11.8 ms, 1,280 11.1 ms, 2,560 12.6 ms).
+constexpr uint32_t kNarrowDelta = 1280;
+// Graphs whose whole traversal runs in the cluster kernel, one launch without
+// grid barriers: up to 2^17 edges, or 2^19 when no vertex has more than 64
+// out-edges.  Times against the grid kernel: RMAT-10 0.079 / 0.213 ms, RMAT-12
+// (97 K edges) 0.167 / 0.279; RMAT-13 (204 K, hubs) 0.27-0.43 / 0.35-0.38;
+// uniform degree 8, 160 K edges 0.224 / 0.440, 400 K edges 0.38 / 0.57.
+constexpr uint64_t kWholeM = 1u << 17, kWholeMLow = 1u << 19;
+constexpr uint32_t kWholeDegree = 64;
 
 struct Slot {
   uint32_t qcount, ccount;
@@ -64,11 +92,22 @@ struct LevelTrace {
   uint32_t frontier, splits;
 };
 
+// Hand-over from the persistent kernel to sssp_narrow.
+constexpr int kMaxTries = 4;
+struct Handover {
+  uint32_t flag;                     // 1: sssp_narrow continues the traversal
+  uint32_t qcount;                   // vertices of the near set (Args::queue)
+  uint32_t T, sel;                   // threshold; near[sel] is all zero
+  unsigned long long mu[kMaxTries];  // unreached out-edges and vertices, by
+  uint32_t nu[kMaxTries];            // attempt
+};
+
 struct Args {
   const uint32_t *__restrict__ offs;
   const uint32_t *__restrict__ cols;
   const uint32_t *__restrict__ wts;
   uint32_t n, W;
+  uint64_t m;
   uint32_t src;
   uint32_t *dist;
   uint32_t *near[2];      // W words each
@@ -84,6 +123,13 @@ struct Args {
   LevelTrace *trace;
   uint32_t delta, huge;
   uint64_t timeout_ns;
+  Handover *ho;
+  uint32_t narrow_nf;     // near vertices sssp_narrow may be handed (0: never)
+  uint32_t narrow_delta;
+  bool narrow_adapt;      // no Delta set by the caller
+  uint2 *far;             // its far lists
+  bool whole;             // sssp_narrow runs the whole traversal
+  bool low_degree;        // max out-degree <= narrow::kLowDegree
 };
 
 struct Workspace {
@@ -94,16 +140,18 @@ struct Workspace {
   uint32_t *queues = nullptr;   // n
   uint4 *chunks = nullptr;
   uint32_t chunk_cap = 0;
+  uint2 *far = nullptr;         // far lists of sssp_narrow, behind the bitmaps
   char *ctrl = nullptr, *ctrl_host = nullptr;
   LevelTrace *trace = nullptr, *trace_host = nullptr;
   int trace_levels = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 };
 
-constexpr size_t kOffSlots = 0, kOffFar = 256, kOffBar = 384, kOffErr = 640,
+constexpr size_t kOffSlots = 0, kOffFar = 256, kOffHo = 288, kOffBar = 384, kOffErr = 640,
                  kOffSummary = 704, kCtrlBytes = 768;
 static_assert(kOffBar % 128 == 0 && kOffBar + sizeof(GridBarrier) <= kOffErr, "barrier layout");
-static_assert(4 * sizeof(Slot) <= kOffFar && sizeof(FarCtl) <= kOffBar - kOffFar &&
+static_assert(4 * sizeof(Slot) <= kOffFar && sizeof(FarCtl) <= kOffHo - kOffFar &&
+                  sizeof(Handover) <= kOffBar - kOffHo &&
                   sizeof(Summary) <= kCtrlBytes - kOffSummary,
               "control block layout");
 
@@ -137,7 +185,9 @@ int ws_get(grus_graph *g, Workspace **out) {
   const uint32_t huge = std::min(tune_or(g->tuning.huge_degree, kDefHuge), 256u);
   w->chunk_cap = (uint32_t)std::min<uint64_t>(g->m / kChunk + g->m / huge + 2, 0x7FFFFFFFull);
   const uint64_t n1 = std::max<uint64_t>(g->n, 1);
-  cudaError_t e = cudaMalloc(&w->bitmaps, w->bitmap_bytes);
+  // one allocation with the far lists: a first call pays for each
+  cudaError_t e = cudaMalloc(&w->bitmaps, w->bitmap_bytes + narrow::kFarBytes);
+  if (e == cudaSuccess) w->far = (uint2 *)((char *)w->bitmaps + w->bitmap_bytes);
   if (e == cudaSuccess) e = cudaMalloc(&w->queues, n1 * 4);
   if (e == cudaSuccess) e = cudaMalloc(&w->chunks, (uint64_t)w->chunk_cap * sizeof(uint4));
   if (e == cudaSuccess) e = cudaMalloc(&w->ctrl, kCtrlBytes);
@@ -181,7 +231,57 @@ struct RelaxVisitor {
   }
 };
 
-__global__ void __launch_bounds__(kBlock) sssp_persistent(Args a) {
+// Attempt to hand the traversal over at level L, whose near set is the queue
+// of qc vertices: kHandedOver when done, else the new `small` word.  Every
+// thread of the grid calls it; out of line, as it runs a few times per
+// traversal at most and must not cost the level loop registers.
+constexpr uint32_t kHandedOver = 0xFFFFFFFFu;
+__device__ __noinline__ uint32_t try_hand_over(const Args &a, uint32_t small, uint32_t L, uint32_t T,
+                                               uint32_t splits, uint32_t qc,
+                                               unsigned long long visits) {
+  const uint32_t run = small & 0xFFFFu;
+  // the previous level's list length: its slot is cleared two levels later
+  const bool shrinking = qc < __ldcg(&a.slots[(L + 3) & 3u].qcount);
+  const bool steady = run >= kNarrowSteady && qc <= 4 * run * run;
+  if (!(shrinking || steady)) return run == 0xFFFFu ? small - 1 : small;
+  const uint32_t gtid = blockIdx.x * kBlock + threadIdx.x, nthreads = gridDim.x * kBlock;
+  // one counter pair per attempt: the runs they need are 2, 8, 24, 72, ...
+  uint32_t k = 0;
+  for (uint32_t need = small >> 16; need > 2u; need = need > kNarrowSteady ? need / 3 : 2u) ++k;
+  if (k >= kMaxTries) return 0xFFFE0000u;  // no further attempt
+  unsigned long long mu = 0, nu = 0;
+  for (uint32_t v = gtid; v < a.n; v += nthreads)
+    if (__ldcg(a.dist + v) == kInfinit) {
+      ++nu;
+      mu += __ldg(a.offs + v + 1) - __ldg(a.offs + v);
+    }
+  const unsigned long long bmu = block_sum_u64<kBlock>(mu);
+  const unsigned long long bnu = block_sum_u64<kBlock>(nu);
+  if (threadIdx.x == 0 && bnu) {
+    atomicAdd(&a.ho->mu[k], bmu);
+    atomicAdd(&a.ho->nu[k], (uint32_t)bnu);
+  }
+  if (!grid_sync(a.bar, a.err, a.timeout_ns)) return kHandedOver;
+  mu = __ldcg(&a.ho->mu[k]);
+  if (mu <= 1ull << (run >= 3 * kNarrowSteady ? kNarrowBitsLong : kNarrowBits)) {
+    if (gtid == 0) {
+      a.ho->qcount = qc;
+      a.ho->T = T;
+      a.ho->sel = (L + 1) & 1u;
+      a.summary->levels = L;
+      a.summary->splits = splits;
+      a.summary->visits = visits;
+      a.summary->nr = a.n - __ldcg(&a.ho->nu[k]);
+      a.summary->mr = a.m - mu;
+      a.ho->flag = 1u;
+    }
+    return kHandedOver;
+  }
+  const uint32_t need = small >> 16 ? small >> 16 : 2u;
+  return run | (need < kNarrowSteady ? kNarrowSteady : 3 * need) << 16;
+}
+
+__global__ void __launch_bounds__(kBlock, 8) sssp_persistent(Args a) {
   const uint32_t gtid = blockIdx.x * kBlock + threadIdx.x;
   const uint32_t nthreads = gridDim.x * kBlock;
   // prologue: distances to INFINIT, bitmaps and control words to zero
@@ -193,6 +293,7 @@ __global__ void __launch_bounds__(kBlock) sssp_persistent(Args a) {
   }
   if (gtid < 4 * sizeof(Slot) / 4) ((uint32_t *)a.slots)[gtid] = 0u;
   if (gtid < sizeof(FarCtl) / 4) ((uint32_t *)a.farctl)[gtid] = 0u;
+  if (gtid < sizeof(Handover) / 4) ((uint32_t *)a.ho)[gtid] = 0u;
   if (gtid == 0) {
     a.farctl->minfar[0] = 0xFFFFFFFFu;
     a.farctl->minfar[1] = 0xFFFFFFFFu;
@@ -205,6 +306,7 @@ __global__ void __launch_bounds__(kBlock) sssp_persistent(Args a) {
   if (!grid_sync(a.bar, a.err, a.timeout_ns)) return;
 
   uint32_t L = 0, T = a.delta, splits = 0;
+  uint32_t small = 0;  // small levels in a row, and from 2^16 on how many the next attempt needs
   unsigned long long visits = 0;
   if (gtid == 0 && a.trace) a.trace[0] = LevelTrace{global_timer_ns(), 0ull, 1u, 0u};
   while (true) {
@@ -268,6 +370,13 @@ __global__ void __launch_bounds__(kBlock) sssp_persistent(Args a) {
       if (mv_all == 0 && rem_all == 0) break;  // nothing near, nothing far: done
       continue;  // compact the moved vertices (or split again)
     }
+    // levels that are small one after another: the cluster kernel takes over
+    small = cc == 0 && qc <= a.narrow_nf ? small + 1 : small & ~0xFFFFu;
+    if ((small & 0xFFFFu) >= 2u && (small & 0xFFFFu) >= small >> 16) {
+      const uint32_t r = try_hand_over(a, small, L, T, splits, qc, visits);
+      if (r == kHandedOver) return;
+      small = r;
+    }
     RelaxVisitor vis{&a, T, nnext, 0ull};
     expand_binned<kBlock>(a.offs, a.queue, qc, a.chunks, cc, vis);
     const unsigned long long bv = block_sum_u64<kBlock>(vis.visits);
@@ -283,18 +392,21 @@ __global__ void __launch_bounds__(kBlock) sssp_persistent(Args a) {
       break;
     }
   }
-  // epilogue: reached vertices and their out-degree sum (m_r)
-  unsigned long long nr = 0, mr = 0;
-  for (uint32_t v = gtid; v < a.n; v += nthreads)
-    if (__ldcg(a.dist + v) != kInfinit) {
-      ++nr;
-      mr += __ldg(a.offs + v + 1) - __ldg(a.offs + v);
+  // epilogue, for a caller that asked for statistics: reached vertices and
+  // their out-degree sum (m_r)
+  if (a.trace) {
+    unsigned long long nr = 0, mr = 0;
+    for (uint32_t v = gtid; v < a.n; v += nthreads)
+      if (__ldcg(a.dist + v) != kInfinit) {
+        ++nr;
+        mr += __ldg(a.offs + v + 1) - __ldg(a.offs + v);
+      }
+    const unsigned long long bnr = block_sum_u64<kBlock>(nr);
+    const unsigned long long bmr = block_sum_u64<kBlock>(mr);
+    if (threadIdx.x == 0) {
+      atomicAdd(&a.summary->nr, bnr);
+      atomicAdd(&a.summary->mr, bmr);
     }
-  const unsigned long long bnr = block_sum_u64<kBlock>(nr);
-  const unsigned long long bmr = block_sum_u64<kBlock>(mr);
-  if (threadIdx.x == 0) {
-    atomicAdd(&a.summary->nr, bnr);
-    atomicAdd(&a.summary->mr, bmr);
   }
   if (gtid == 0) {
     a.summary->levels = L;
@@ -303,13 +415,104 @@ __global__ void __launch_bounds__(kBlock) sssp_persistent(Args a) {
   }
 }
 
+// One cluster: the rest of a traversal whose near set has become small
+// (handed over by sssp_persistent; returns at once otherwise), or all of a
+// traversal of a small graph.
+__global__ void __launch_bounds__(narrow::kBlock) sssp_narrow(Args a) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  if (!a.whole && __ldcg(&a.ho->flag) != 1u) return;  // the same answer in every CTA
+  narrow::View view;
+  view.offs = a.offs;
+  view.cols = a.cols;
+  view.wts = a.wts;
+  view.n = a.n;
+  view.W = a.W;
+  view.dist = a.dist;
+  view.farbm = a.farbm;
+  view.far = a.far;
+  view.delta = a.narrow_delta;
+  view.adapt = a.narrow_adapt;
+  view.low_degree = a.low_degree;
+  view.err = a.err;
+  const uint32_t L0 = a.whole ? 0u : __ldcg(&a.summary->levels);
+  view.tag = a.whole ? 0u : __ldcg(&a.summary->splits);
+  view.nearbm = a.near[a.whole ? 0u : __ldcg(&a.ho->sel)];
+  view.trace = a.trace && L0 < (uint32_t)kMaxTrace ? (narrow::Trace *)a.trace + L0 : nullptr;
+  view.trace_cap = L0 < (uint32_t)kMaxTrace ? kMaxTrace - L0 : 0u;
+  narrow::Engine<false> E(view, (narrow::Shared *)smem);
+  const uint32_t tid = E.rank * narrow::kBlock + threadIdx.x, nt = E.C * narrow::kBlock;
+  if (a.whole) {
+    for (uint32_t i = tid; i < a.n; i += nt) a.dist[i] = i == a.src ? 0u : kInfinit;
+    for (uint32_t i = tid; i < a.W; i += nt) {
+      view.nearbm[i] = 0u;
+      a.farbm[i] = 0u;
+    }
+    if (tid == 0) {
+      *a.summary = Summary{0u, 0u, 0u, 0u, 0ull, 1ull,
+                           (unsigned long long)(__ldg(a.offs + a.src + 1) - __ldg(a.offs + a.src))};
+      *a.err = 0u;
+    }
+  } else if (tid == 0) {
+    E.s->g_farbm = 1u;  // far vertices wait in the bitmap
+  }
+  if (view.trace) {
+    for (uint32_t i = tid; i < view.trace_cap; i += nt)
+      if (i || a.whole) view.trace[i] = narrow::Trace{i ? 0ull : global_timer_ns(), 0ull, 0u, 0u};
+  }
+  E.cl.sync();
+  if (a.whole) {
+    E.T = a.narrow_delta;
+    if (E.rank == 0 && E.warp == 0)
+      E.push(E.lane == 0, a.src, __ldg(a.offs + a.src), __ldg(a.offs + a.src + 1), 0u);
+  } else {
+    E.T = __ldcg(&a.ho->T);
+    const uint32_t qc = __ldcg(&a.ho->qcount);
+    for (uint32_t base = tid & ~31u; base < qc; base += nt) {
+      const uint32_t i = base + E.lane;
+      const bool has = i < qc;
+      const uint32_t v = has ? __ldcg(a.queue + i) : 0u;
+      E.push(has, v, has ? __ldg(a.offs + v) : 0u, has ? __ldg(a.offs + v + 1) : 0u,
+             has ? __ldcg(a.dist + v) : 0u);
+    }
+  }
+  E.run();
+  if (!a.trace) return;
+  const unsigned long long bv = E.block_sum(E.res.visits);
+  if (threadIdx.x == 0) {
+    atomicAdd(&a.summary->visits, bv);
+    if (E.rank == 0) {
+      a.summary->levels = L0 + E.res.steps;
+      a.summary->splits = view.tag + E.res.splits;
+    }
+  }
+  const unsigned long long bnr = E.block_sum(E.res.nr);
+  const unsigned long long bmr = E.block_sum(E.res.mr);
+  if (threadIdx.x == 0) {
+    atomicAdd(&a.summary->nr, bnr);
+    atomicAdd(&a.summary->mr, bmr);
+  }
+}
+
+int narrow_cluster() {
+  static const int c = narrow::cluster_size(sssp_narrow);
+  return c;
+}
+
+bool runs_whole(const grus_graph *g) {
+  return g->tuning.tail_cluster != 2 &&
+         (g->m <= kWholeM || (g->m <= kWholeMLow && g->max_deg <= kWholeDegree));
+}
+
 }  // namespace
-}  // namespace grus
 
-using namespace grus;
+bool sssp_tail(const grus_graph *g) {
+  return !runs_whole(g) && g->tuning.tail_cluster != 2;
+}
 
-extern "C" int grus_sssp(grus_graph *g, uint32_t src, uint32_t *dist,
-                         grus_stats *stats, void *stream) {
+bool sssp_lane_tail(const grus_graph *g) { return sssp_tail(g) && g->max_deg <= kWholeDegree; }
+
+int sssp_run(grus_graph *g, uint32_t src, uint32_t *dist, grus_stats *stats, cudaStream_t s,
+             bool tail) {
   if (!g || !dist) return GRUS_EINVAL;
   if (g->n == 0 || src >= g->n) {
     set_last_error("source vertex out of range");
@@ -319,7 +522,6 @@ extern "C" int grus_sssp(grus_graph *g, uint32_t src, uint32_t *dist,
     set_last_error("sssp needs edge weights (load with need_weights or generate weighted)");
     return GRUS_EINVAL;
   }
-  cudaStream_t s = (cudaStream_t)stream;
   std::lock_guard<std::mutex> lk(g->mu);
   Workspace *w = nullptr;
   int rc = ws_get(g, &w);
@@ -337,6 +539,7 @@ extern "C" int grus_sssp(grus_graph *g, uint32_t src, uint32_t *dist,
   a.wts = g->csr.wts;
   a.n = (uint32_t)g->n;
   a.W = w->W;
+  a.m = g->m;
   a.src = src;
   a.dist = dev_out ? dist : w->dist;
   const uint64_t Wp = ((uint64_t)w->W + 31) / 32 * 32;
@@ -357,17 +560,29 @@ extern "C" int grus_sssp(grus_graph *g, uint32_t src, uint32_t *dist,
   a.huge = tune_or(g->tuning.huge_degree, kDefHuge);
   a.timeout_ns = (uint64_t)tune_or(g->tuning.timeout_ms, 30000u) * 1000000ull;
 
+  a.ho = (Handover *)(w->ctrl + kOffHo);
+  a.far = w->far;
+  a.low_degree = g->max_deg <= narrow::kLowDegree;
+  const int ncl = narrow_cluster();
+  a.narrow_nf = tail ? kNarrowNf * (uint32_t)ncl : 0u;
+  a.narrow_delta = std::max(1u, tune_or(g->tuning.sssp_delta, kNarrowDelta));
+  a.narrow_adapt = g->tuning.sssp_delta == 0;
+  a.whole = runs_whole(g);
+
   const bool sync = stats != nullptr || !dev_out;
   // barrier, error word and summary: a timed-out launch leaves stale barrier state
-  GRUS_CUDA_TRY(cudaMemsetAsync(w->ctrl + kOffBar, 0, kCtrlBytes - kOffBar, s));
+  if (!a.whole) GRUS_CUDA_TRY(cudaMemsetAsync(w->ctrl + kOffBar, 0, kCtrlBytes - kOffBar, s));
   if (stats) GRUS_CUDA_TRY(cudaEventRecord(w->ev0, s));
   void *args[] = {&a};
   // the L2 window on the distances, which every relaxation reads and lowers
   // with an atomic: RMAT-22 1.99 -> 1.80-1.83 ms against the window on the
   // near/far bitmaps (small and hot enough to stay in L2 without it)
-  rc = launch_persistent((const void *)sssp_persistent, args, kBlock,
-                         (int)g->tuning.ctas_per_sm, occ, s, a.dist, (size_t)g->n * 4);
-  if (rc) return rc;
+  if (!a.whole) {
+    rc = launch_persistent((const void *)sssp_persistent, args, kBlock,
+                           (int)g->tuning.ctas_per_sm, occ, s, a.dist, (size_t)g->n * 4);
+    if (rc) return rc;
+  }
+  if (a.whole || a.narrow_nf) GRUS_CUDA_TRY(narrow::launch(sssp_narrow, ncl, a, s));
   if (stats) GRUS_CUDA_TRY(cudaEventRecord(w->ev1, s));
   if (!dev_out) GRUS_CUDA_TRY(cudaMemcpyAsync(dist, w->dist, g->n * 4, cudaMemcpyDeviceToHost, s));
   if (!sync) return GRUS_OK;
@@ -387,7 +602,7 @@ extern "C" int grus_sssp(grus_graph *g, uint32_t src, uint32_t *dist,
     std::memset(stats, 0, sizeof(*stats));
     stats->levels = sm->levels;
     stats->direction_switches = sm->splits;  // threshold advances
-    stats->kernel_launches = 1;
+    stats->kernel_launches = tail ? 2 : 1;
     stats->vertices_reached = sm->nr;
     stats->edges_reached = sm->mr;
     stats->edges_relaxed = sm->visits;
@@ -396,6 +611,15 @@ extern "C" int grus_sssp(grus_graph *g, uint32_t src, uint32_t *dist,
     stats->device_ms = ms;
   }
   return GRUS_OK;
+}
+
+}  // namespace grus
+
+using namespace grus;
+
+extern "C" int grus_sssp(grus_graph *g, uint32_t src, uint32_t *dist,
+                         grus_stats *stats, void *stream) {
+  return sssp_run(g, src, dist, stats, (cudaStream_t)stream, g && sssp_tail(g));
 }
 
 extern "C" int grus_sssp_trace(grus_graph *g, grus_level_trace *out, int max_levels) {
