@@ -933,7 +933,7 @@ int grus_batch_run(grus_batch *b, const grus_query *queries, int nq, uint32_t *o
       CtrlView cv;
       if (j - i == 1) {
         rc = q0.algo == GRUS_ALGO_SSSP ? grus_sssp(g, q0.src, out + q0.out_offset, nullptr, s)
-                                       : grus_bfs(g, q0.src, out + q0.out_offset, nullptr, s);
+                                       : bfs_run(g, q0.src, out + q0.out_offset, nullptr, s, false);
         // a single BFS is the persistent kernel and its narrow-tail kernel
         nlaunch += q0.algo == GRUS_ALGO_SSSP ? 1 : 2;
         cv = q0.algo == GRUS_ALGO_SSSP ? sssp_ctrl(g) : bfs_ctrl(g);

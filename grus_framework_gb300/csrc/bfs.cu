@@ -35,12 +35,9 @@
 //     the first push level after a pull level turns the frontier bitmap into
 //     the queue with one atomic per CTA per 256 words.
 //   * narrow tail: a long traversal (16+ levels) whose push frontier and
-//     remaining edges have become small is handed to bfs_narrow, a cluster of
-//     up to 16 CTAs of 1024 threads launched after the persistent kernel,
-//     which runs the remaining levels with one hardware cluster barrier each,
-//     frontiers in distributed shared memory and prefetches of the next
-//     level's adjacency (about 3.3 µs per level against 9-10 µs for a grid
-//     barrier level).
+//     remaining edges have become small is handed to bfs_narrow, one cluster
+//     of up to 16 CTAs launched after the persistent kernel (narrow.cuh); it
+//     also runs small graphs from the start.
 // Depths are order-independent (every writer stores level+1), so results are
 // bit-exact against the serial oracle whatever the schedule.
 #include <algorithm>
@@ -48,11 +45,10 @@
 
 #include "expand.cuh"
 #include "grus_internal.cuh"
+#include "narrow.cuh"
 
 namespace grus {
 namespace {
-
-namespace cg = cooperative_groups;
 
 constexpr int kBlock = 256;
 constexpr uint32_t kDefHuge = 8192;   // chunking threshold
@@ -65,14 +61,20 @@ constexpr float kDefAlpha = 15.f, kDefBeta = 18.f;
 // Narrow tail: a traversal still running after kNarrowAfter levels, with a
 // push frontier of at most kNarrowNf vertices per tail CTA and at most
 // kNarrowMu edges left whose source is undiscovered, is finished by one
-// thread-block cluster of up to 16 CTAs of 1024 threads.  The edge bound caps
-// the work the cluster may be left with.
+// thread-block cluster of up to 16 CTAs.  The edge bound caps the work the
+// cluster may be left with.  (Handing over the last one or two levels of a
+// shorter traversal costs what it saves: RMAT scales 16-20 0.072 -> 0.078 and
+// 0.086 -> 0.092 ms.)
 constexpr uint32_t kNarrowAfter = 16;
-constexpr uint32_t kNarrowNf = 4096;
+constexpr uint32_t kNarrowNf = 1024;
 constexpr uint64_t kNarrowMu = 1ull << 26;
-constexpr int kNarrowBlock = 1024;
-constexpr int kNarrowMaxCluster = 16;
-constexpr uint32_t kNarrowCap = 4096;   // shared-memory frontier entries per buffer per CTA
+// Graphs whose whole traversal runs in the cluster kernel, one launch without
+// grid barriers: up to 2^17 edges, or 2^18 when no vertex has more than 64
+// out-edges.  Times against the grid kernels: RMAT-10 0.036 / 0.059 ms,
+// RMAT-12 (97 K edges) 0.048 / 0.056, uniform degree 8, 160 K edges 0.077 /
+// 0.135, degree 4, 400 K edges 0.215 / 0.165.
+constexpr uint64_t kWholeM = 1u << 17, kWholeMLow = 1u << 18;
+constexpr uint32_t kWholeDegree = 64;
 
 struct LevelSlot {
   uint32_t qcount;         // queue entries of this level
@@ -97,7 +99,6 @@ struct Handover {
   uint32_t qsel;
   unsigned long long nr, mr;  // reach counts so far
   uint32_t bu_levels, switches;
-  uint32_t spill[3];          // spilled frontier entries, by depth mod 3
 };
 
 // Per-level record written by one thread after each level's barrier:
@@ -143,6 +144,10 @@ struct Args {
   uint32_t huge, bu_scan;
   uint32_t narrow_nf;     // hand over at most this many frontier vertices (0: never)
   Handover *ho;
+  uint2 *far;             // far lists of bfs_narrow
+  bool whole;             // bfs_narrow runs the whole traversal
+  uint32_t lanes;         // narrow::lanes_per_entry
+  bool ahead;             // narrow::View::ahead
   uint64_t timeout_ns;
 };
 
@@ -164,6 +169,7 @@ struct Workspace {
   uint32_t *planes = nullptr;    // P*Wp words: after the fronts from kPlanesMinN
   uint32_t *planes_own = nullptr;  // vertices on, else allocated when first asked for
   uint32_t *queues = nullptr;    // 2 * n
+  uint2 *far = nullptr;          // far lists of bfs_narrow, behind the bitmaps
   uint4 *chunks = nullptr;       // 2 * chunk_cap
   uint32_t chunk_cap = 0;
   char *ctrl = nullptr;          // slots, barrier, err, summary
@@ -220,7 +226,9 @@ int ws_get(grus_graph *g, Workspace **out) {
   const uint32_t huge = std::min(tune_or(g->tuning.huge_degree, kDefHuge), 256u);
   const uint64_t cap = g->m / kChunk + g->m / std::max(huge, 1u) + 2;
   w->chunk_cap = (uint32_t)std::min<uint64_t>(cap, 0x7FFFFFFFull);
-  cudaError_t e = cudaMalloc(&w->bitmaps, (5 + (with_planes ? (uint64_t)P : 0)) * Wp * 4);
+  const size_t map_bytes = (5 + (with_planes ? (uint64_t)P : 0)) * Wp * 4;
+  cudaError_t e = cudaMalloc(&w->bitmaps, map_bytes + narrow::far_bytes(g->n));
+  if (e == cudaSuccess) w->far = (uint2 *)((char *)w->bitmaps + map_bytes);
   if (e == cudaSuccess && with_planes) w->planes = w->bitmaps + 5 * Wp;
   if (e == cudaSuccess) e = cudaMalloc(&w->queues, 2 * std::max<uint64_t>(g->n, 1) * 4);
   if (e == cudaSuccess) e = cudaMalloc(&w->chunks, 2ull * w->chunk_cap * sizeof(uint4));
@@ -1023,303 +1031,103 @@ __global__ void __launch_bounds__(kBlock) bfs_persistent(Args a) {
   }
 }
 
-// Starts filling this SM's L1 (or only L2) with the line holding p (no wait).
-__device__ __forceinline__ void prefetch_l1(const void *p) {
-  asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
-}
-__device__ __forceinline__ void prefetch_l2(const void *p) {
-  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-}
-
-// Per-level state of the tail cluster.  Every frontier vertex has an owner
-// CTA (a hash of its id); the owner keeps it as the (begin, end) range of its
-// out-edges in shared memory, or -- beyond kNarrowCap entries -- the vertex id
-// goes to a global spill list shared by the cluster.
-struct Tail {
-  cg::cluster_group cl;
-  uint32_t rank, C;
-  uint2 *q;            // this CTA's 2 * kNarrowCap entries
-  uint32_t *cnt;       // this CTA's 2 entry counters
-  uint32_t *found;     // this CTA's flag: it found a vertex at this level
-};
-
-__device__ __forceinline__ uint32_t tail_owner(uint32_t v, uint32_t C) {
-  return __umulhi(v * 2654435761u, C);
-}
-
-// Claims up to kNarrowBatch targets at once.  The chain per batch is short:
-// the column ids come from L1 (their lines were prefetched), the claiming
-// atomicOr goes to L2 while the targets' offsets are prefetched, and a new
-// vertex's offsets then come from L1.  A new vertex gets depth d and, if it
-// has out-edges, a place in its owner's next frontier and a prefetch of its
-// first out-edges.
-constexpr int kNarrowBatch = 4;
-
-__device__ __forceinline__ void narrow_batch(const Args &a, Tail &t,
-                                             const uint32_t (&xs)[kNarrowBatch], int cnt,
-                                             uint32_t d, uint32_t nxt, unsigned long long &nr,
-                                             unsigned long long &mr) {
-  uint32_t c[kNarrowBatch], old[kNarrowBatch];
-#pragma unroll
-  for (int r = 0; r < kNarrowBatch; ++r) c[r] = r < cnt ? __ldg(a.cols + xs[r]) : 0u;
-#pragma unroll
-  for (int r = 0; r < kNarrowBatch; ++r)
-    if (r < cnt) prefetch_l1(a.offs + c[r]);
-#pragma unroll
-  for (int r = 0; r < kNarrowBatch; ++r) {
-    const uint32_t bit = 1u << (c[r] & 31u);
-    old[r] = r < cnt ? atomicOr(a.visited + (c[r] >> 5), bit) : bit;
+// One cluster (narrow.cuh): the rest of a traversal whose frontier has become
+// small, handed over by bfs_persistent (returns at once otherwise), or all of
+// a traversal of a small graph.  Depths are lowered in place, so a vertex may
+// get a depth too large before it gets its own; when it ends, all are final.
+__global__ void __launch_bounds__(narrow::kBlock) bfs_narrow(Args a) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  // flag, level, nf, qsel: the same in every CTA
+  static_assert(offsetof(Handover, qsel) == 12, "one 16-byte load");
+  const uint4 ho = a.whole ? make_uint4(1u, 0u, 0u, 0u) : __ldcg(reinterpret_cast<const uint4 *>(a.ho));
+  if (ho.x != 1u) return;
+  narrow::View view;
+  view.offs = a.offs;
+  view.cols = a.cols;
+  view.wts = nullptr;
+  view.n = a.n;
+  view.W = a.W;
+  view.m = (uint32_t)a.m;
+  view.dist = a.depth;
+  view.nearbm = a.front[0];
+  view.farbm = a.front[1];
+  view.far = a.far;
+  view.far_cap = narrow::far_cap(a.n);
+  view.delta = narrow::kUnitDelta;
+  view.adapt = false;
+  view.lanes = a.lanes;
+  view.ahead = a.ahead;
+  view.err = a.err;
+  view.trace = (narrow::Trace *)a.trace;
+  view.trace_cap = a.trace ? kMaxTrace : 0u;
+  view.tag = 0u;
+  narrow::Engine<true> E(view, (narrow::Shared *)smem);
+  const uint32_t tid = E.rank * narrow::kBlock + threadIdx.x, nt = E.C * narrow::kBlock;
+  const uint32_t d0 = ho.y;  // depth of the starting frontier
+  for (uint32_t d = d0 + 1 + tid; d < view.trace_cap; d += nt)
+    view.trace[d] = narrow::Trace{0ull, 0ull, 0u, 0u};
+  for (uint32_t i = tid; i < a.W; i += nt) {
+    view.nearbm[i] = 0u;
+    view.farbm[i] = 0u;
   }
-#pragma unroll
-  for (int r = 0; r < kNarrowBatch; ++r) {
-    if (old[r] & (1u << (c[r] & 31u))) continue;
-    const uint32_t v = c[r];
-    a.depth[v] = d;
-    const uint32_t cb = __ldg(a.offs + v), ce = __ldg(a.offs + v + 1);
-    ++nr;
-    mr += ce - cb;
-    *t.found = 1u;
-    if (ce == cb) continue;
-    const uint32_t o = tail_owner(v, t.C);
-    if (o == t.rank) {
-      prefetch_l1(a.cols + cb);
-      prefetch_l1(a.cols + ce - 1);
-    } else {
-      prefetch_l2(a.cols + cb);
-      prefetch_l2(a.cols + ce - 1);
-    }
-    // one reservation per owner among the lanes pushing together
-    cg::coalesced_group pg = cg::coalesced_threads();
-    cg::coalesced_group peers = cg::labeled_partition(pg, o);
-    uint32_t base = 0;
-    if (peers.thread_rank() == 0) base = atomicAdd(t.cl.map_shared_rank(t.cnt + nxt, o), peers.size());
-    const uint32_t pos = peers.shfl(base, 0) + peers.thread_rank();
-    if (pos < kNarrowCap) {
-      t.cl.map_shared_rank(t.q, o)[nxt * kNarrowCap + pos] = make_uint2(cb, ce);
-    } else {
-      const uint32_t g = atomicAdd(&a.ho->spill[d % 3], 1u);
-      if (g < a.queue_cap) a.queue[d & 1u][g] = v;
-      else atomicOr(a.err, kErrOverflow);  // cannot happen: spilled vertices are distinct
-    }
-  }
-}
-
-// The narrow tail of a long traversal: one cluster of C CTAs (1 <= C <= 16)
-// of 1024 threads takes the small frontier the persistent kernel handed over
-// and runs the remaining levels with one hardware cluster barrier per level.
-// Each CTA deals the edges of the frontier vertices it owns evenly to its
-// threads (a block scan of the degrees and a binary search for each thread's
-// first entry), so a wide vertex is shared by many threads, and each thread
-// claims its edges in batches; spilled entries are dealt over the whole
-// cluster one vertex per thread.  A CTA that found a vertex writes the new
-// depth into every CTA's stamp before the level's barrier, so after it each
-// CTA reads its own stamp; stamps only grow, so no CTA has to clear them.
-// Returns at once when the persistent kernel finished the traversal itself.
-__global__ void __launch_bounds__(kNarrowBlock) bfs_narrow(Args a) {
-  extern __shared__ uint2 s_q[];  // 2 * kNarrowCap entries
-  __shared__ uint32_t s_pref[kNarrowCap + 1];
-  __shared__ uint32_t s_cnt[2], s_found, s_stamp;
-  __shared__ unsigned long long s_red[kNarrowBlock / 32];
-  Handover *ho = a.ho;
-  if (__ldcg(&ho->flag) != 1u) return;  // the same answer in every CTA
-  Tail t{cg::this_cluster(), 0, 1, s_q, s_cnt, &s_found};
-  t.rank = t.cl.block_rank();
-  t.C = t.cl.num_blocks();
-  const uint32_t tid = threadIdx.x;
-  uint32_t d = __ldcg(&ho->level);  // depth of the current frontier
-  const uint32_t d0 = d;
-  const uint32_t nf0 = __ldcg(&ho->nf);
-  const uint32_t *q0 = a.queue[__ldcg(&ho->qsel)];
-  if (tid == 0) {
-    s_cnt[0] = 0;
-    s_cnt[1] = 0;
-    s_found = 0;
-    s_stamp = d;
-    if (t.rank == 0) {
-      ho->spill[d % 3] = 0u;  // the counters of depths d0 and d0 + 1
-      ho->spill[(d + 1) % 3] = 0u;
-      a.summary->nr = __ldcg(&ho->nr);
-      a.summary->mr = __ldcg(&ho->mr);
-      if (a.trace && d + 1 < (uint32_t)kMaxTrace) a.trace[d + 1] = LevelTrace{0ull, 0ull, 0u, 0u};
-    }
-  }
-  __syncthreads();
-  // this CTA's share of the handed-over queue (vertex ids) becomes ranges in
-  // buffer 0; vertices without out-edges are left out, so every entry has at
-  // least one edge, which the edge dealing relies on
-  for (uint32_t i = t.rank + t.C * tid; i < nf0; i += t.C * kNarrowBlock) {
-    const uint32_t v = __ldcg(q0 + i);
-    const uint2 r = make_uint2(__ldg(a.offs + v), __ldg(a.offs + v + 1));
-    if (r.x == r.y) continue;
-    const uint32_t pos = atomicAdd(&s_cnt[0], 1u);
-    if (pos < kNarrowCap) s_q[pos] = r;
-    else atomicOr(a.err, kErrOverflow);  // cannot happen: nf0 <= C * kNarrowCap
-  }
-  t.cl.sync();  // every CTA's counters are set before any remote push
-  unsigned long long nr = 0, mr = 0;
-  uint32_t cur = 0, levels = 0;
-  constexpr uint32_t kPer = (kNarrowCap + kNarrowBlock - 1) / kNarrowBlock;
-  while (true) {
-    const uint32_t nxt = cur ^ 1u;
-    const uint32_t in_smem = min(s_cnt[cur], kNarrowCap);
-    // entries spilled into the frontier at depth d
-    const uint32_t spilled = min(__ldcg(&ho->spill[d % 3]), a.queue_cap);
-    const uint2 *qc = s_q + cur * kNarrowCap;
-    // exclusive prefix of the entries' degrees; the first line of each
-    // entry's adjacency is pulled into L1 meanwhile
-    const uint32_t e0 = tid * kPer;
-    uint32_t sum = 0;
-#pragma unroll
-    for (uint32_t k = 0; k < kPer; ++k)
-      if (e0 + k < in_smem) {
-        const uint2 r = qc[e0 + k];
-        prefetch_l1(a.cols + r.x);
-        sum += r.y - r.x;
-      }
-    uint32_t E = 0;
-    uint32_t run = block_exclusive_scan<kNarrowBlock>(sum, &E);
-#pragma unroll
-    for (uint32_t k = 0; k < kPer; ++k)
-      if (e0 + k < in_smem) {
-        s_pref[e0 + k] = run;
-        run += qc[e0 + k].y - qc[e0 + k].x;
-      }
+  if (a.whole) {
+    for (uint32_t i = tid; i < a.n; i += nt) a.depth[i] = i == a.src ? 0u : kInfinit;
     if (tid == 0) {
-      s_pref[in_smem] = E;
-      // the spill counter for depth d + 2 is reused: its last readers
-      // finished before the previous cluster barrier
-      if (t.rank == 0) {
-        ho->spill[(d + 2) % 3] = 0u;
-        if (a.trace && d + 2 < (uint32_t)kMaxTrace) a.trace[d + 2] = LevelTrace{0ull, 0ull, 0u, 0u};
-      }
-      if (a.trace && d + 1 < (uint32_t)kMaxTrace) {
-        atomicAdd(&a.trace[d + 1].mf, (unsigned long long)E);
-        atomicAdd(&a.trace[d + 1].nf, in_smem);
-      }
+      *a.summary = Summary{0u, 0u, 0u, 0u, 1ull,
+                           (unsigned long long)(__ldg(a.offs + a.src + 1) - __ldg(a.offs + a.src))};
+      *a.err = 0u;
+      if (a.trace) a.trace[0] = LevelTrace{global_timer_ns(), 0ull, 1u, 0u};
     }
-    __syncthreads();
-    if (tid == 0) s_cnt[cur] = 0;  // read by every thread above; refilled next level
-    // this thread's edges [lo, hi) of the E in shared-memory entries
-    const uint32_t lo = (uint32_t)((unsigned long long)tid * E / kNarrowBlock);
-    const uint32_t hi = (uint32_t)((unsigned long long)(tid + 1) * E / kNarrowBlock);
-    if (lo < hi) {
-      uint32_t j = 0, span = in_smem;  // largest j with s_pref[j] <= lo
-      while (span > 1) {
-        const uint32_t half = span / 2;
-        if (s_pref[j + half] <= lo) j += half;
-        span -= half;
-      }
-      uint32_t x = qc[j].x + (lo - s_pref[j]);
-      uint32_t xe = qc[j].y;
-      for (uint32_t k = lo; k < hi; k += kNarrowBatch) {
-        const int cnt = (int)min(hi - k, (uint32_t)kNarrowBatch);
-        uint32_t xs[kNarrowBatch];
-#pragma unroll
-        for (int r = 0; r < kNarrowBatch; ++r) {
-          xs[r] = x;
-          if (r < cnt && ++x == xe && k + r + 1 < hi) {
-            ++j;
-            x = qc[j].x;
-            xe = qc[j].y;
-          }
-        }
-        narrow_batch(a, t, xs, cnt, d + 1, nxt, nr, mr);
-      }
-    }
-    // spilled entries (rare: a frontier beyond C * kNarrowCap), one vertex
-    // per thread over the whole cluster
-    if (spilled) {
-      const uint32_t *sp = a.queue[d & 1u];
-      for (uint32_t i = t.rank * kNarrowBlock + tid; i < spilled; i += t.C * kNarrowBlock) {
-        const uint32_t v = __ldcg(sp + i);
-        const uint32_t b = __ldg(a.offs + v), e = __ldg(a.offs + v + 1);
-        for (uint32_t x = b; x < e; x += kNarrowBatch) {
-          const int cnt = (int)min(e - x, (uint32_t)kNarrowBatch);
-          uint32_t xs[kNarrowBatch];
-#pragma unroll
-          for (int r = 0; r < kNarrowBatch; ++r) xs[r] = x + r;
-          narrow_batch(a, t, xs, cnt, d + 1, nxt, nr, mr);
-        }
-      }
-    }
-    __syncthreads();
-    if (tid < t.C && s_found) *t.cl.map_shared_rank(&s_stamp, tid) = d + 1;
-    // every push and stamp of this level is visible after the barrier
-    t.cl.sync();
-    if (tid == 0) s_found = 0;  // set again at the next level, after its scan barriers
-    const bool found = s_stamp > d;  // stamps only grow: a faster CTA may already write d + 2
-    if (t.rank == 0 && tid == 0 && a.trace && d + 1 < (uint32_t)kMaxTrace)
-      a.trace[d + 1].t_ns = global_timer_ns();
-    if (!found) {
-      levels = d + 1;  // nothing at depth d + 1
-      break;
-    }
-    ++d;
-    cur = nxt;
-    if (d > a.n + 1) {
-      if (t.rank == 0 && tid == 0) atomicOr(a.err, kErrLevels);
-      levels = d;
-      break;
+  } else if (tid == 0) {
+    *a.summary = Summary{0u, a.ho->bu_levels, a.ho->switches, 0u, a.ho->nr, a.ho->mr};
+  }
+  E.T = d0 + narrow::kUnitDelta;
+  E.cl.sync();
+  if (a.whole) {
+    if (E.rank == 0 && E.warp == 0)
+      E.push<true>(E.lane == 0, a.src, __ldg(a.offs + a.src), __ldg(a.offs + a.src + 1), 0u);
+  } else {
+    const uint32_t nf = ho.z;
+    const uint32_t *q = a.queue[ho.w];
+    for (uint32_t base = tid & ~31u; base < nf; base += nt) {
+      const uint32_t i = base + E.lane;
+      const bool has = i < nf;
+      const uint32_t v = has ? __ldcg(q + i) : 0u;
+      E.push<true>(has, v, has ? __ldg(a.offs + v) : 0u, has ? __ldg(a.offs + v + 1) : 0u, d0);
     }
   }
-  // reach counts: the persistent kernel's share (set above) plus each CTA's
-  for (int o = 16; o > 0; o >>= 1) {
-    nr += __shfl_down_sync(0xffffffffu, nr, o);
-    mr += __shfl_down_sync(0xffffffffu, mr, o);
-  }
-  if ((tid & 31u) == 0) s_red[tid >> 5] = nr;
-  __syncthreads();
-  if (tid == 0) {
-    unsigned long long v = 0;
-    for (int i = 0; i < kNarrowBlock / 32; ++i) v += s_red[i];
-    atomicAdd(&a.summary->nr, v);
-  }
-  __syncthreads();
-  if ((tid & 31u) == 0) s_red[tid >> 5] = mr;
-  __syncthreads();
-  if (tid == 0) {
-    unsigned long long v = 0;
-    for (int i = 0; i < kNarrowBlock / 32; ++i) v += s_red[i];
-    atomicAdd(&a.summary->mr, v);
-    if (t.rank == 0) {
-      a.summary->levels = levels;
-      a.summary->bu_levels = __ldcg(&ho->bu_levels);
-      a.summary->switches = __ldcg(&ho->switches);
-      a.summary->pad = d0;  // level of the hand-over
+  E.run();
+  const unsigned long long nr = E.block_sum(E.res.nr);
+  const unsigned long long mr = E.block_sum(E.res.mr);
+  if (threadIdx.x == 0) {
+    if (nr) {
+      atomicAdd(&a.summary->nr, nr);
+      atomicAdd(&a.summary->mr, mr);
+    }
+    if (E.rank == 0) {
+      a.summary->levels = E.res.last + 1;
+      if (!a.whole) a.ho->flag = 0u;
+      if (a.trace) {
+        const uint64_t t = global_timer_ns();
+        for (uint32_t d = min(E.res.last + 1, (uint32_t)kMaxTrace - 1); d > d0 && a.trace[d].t_ns == 0; --d)
+          a.trace[d].t_ns = t;
+      }
     }
   }
-  // no CTA leaves while another may still write its shared memory
-  t.cl.sync();
-  if (t.rank == 0 && tid == 0) ho->flag = 0u;
 }
 
-constexpr size_t kNarrowSmem = 2 * kNarrowCap * sizeof(uint2);
-
-// The largest cluster of bfs_narrow CTAs (16, 8, 4, 2 or 1) the device can
-// co-schedule, decided once per process; 1 needs no cluster launch.
 int narrow_cluster() {
-  static const int c = [] {
-    cudaFuncSetAttribute(bfs_narrow, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNarrowSmem);
-    cudaFuncSetAttribute(bfs_narrow, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    for (int k = kNarrowMaxCluster; k > 1; k /= 2) {
-      cudaLaunchAttribute attr;
-      attr.id = cudaLaunchAttributeClusterDimension;
-      attr.val.clusterDim.x = (unsigned)k;
-      attr.val.clusterDim.y = 1;
-      attr.val.clusterDim.z = 1;
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3((unsigned)k);
-      cfg.blockDim = dim3(kNarrowBlock);
-      cfg.dynamicSmemBytes = kNarrowSmem;
-      cfg.attrs = &attr;
-      cfg.numAttrs = 1;
-      int nc = 0;
-      if (cudaOccupancyMaxActiveClusters(&nc, bfs_narrow, &cfg) == cudaSuccess && nc >= 1) return k;
-      cudaGetLastError();
-    }
-    return 1;
-  }();
+  static const int c = narrow::cluster_size(bfs_narrow);
   return c;
+}
+
+// Small graphs run in the cluster kernel altogether, unless the caller set a
+// knob of the persistent kernel.
+bool runs_whole(const grus_graph *g) {
+  const grus_tuning &t = g->tuning;
+  return t.tail_cluster != 2 && t.alpha == 0.f && t.beta == 0.f && !t.ctas_per_sm &&
+         !t.huge_degree && !t.bu_scan && !t.bu_words && !t.depth_planes &&
+         (g->m <= kWholeM || (g->m <= kWholeMLow && g->max_deg <= kWholeDegree));
 }
 
 }  // namespace
@@ -1327,18 +1135,20 @@ int narrow_cluster() {
 
 using namespace grus;
 
-extern "C" int grus_bfs(grus_graph *g, uint32_t src, uint32_t *depth,
-                        grus_stats *stats, void *stream) {
+namespace grus {
+
+int bfs_run(grus_graph *g, uint32_t src, uint32_t *depth, grus_stats *stats, cudaStream_t s,
+            bool whole_ok) {
   if (!g || !depth) return GRUS_EINVAL;
   if (g->n == 0 || src >= g->n) {
     set_last_error("source vertex out of range");
     return GRUS_EINVAL;
   }
-  cudaStream_t s = (cudaStream_t)stream;
   std::lock_guard<std::mutex> lk(g->mu);
   Workspace *w = nullptr;
   int rc = ws_get(g, &w);
   if (rc) return rc;
+  const bool whole = whole_ok && runs_whole(g);
   const bool dev_out = is_device_pointer(depth);
   if (!dev_out && !w->depth) GRUS_CUDA_TRY(cudaMalloc(&w->depth, g->n * 4));
 
@@ -1374,7 +1184,7 @@ extern "C" int grus_bfs(grus_graph *g, uint32_t src, uint32_t *depth,
     a.icols = g->csr.cols;
   }
   a.allow_pull = a.ioffs != nullptr;
-  if (a.allow_pull) {
+  if (a.allow_pull && !whole) {
     rc = build_rep_locked(g);
     if (rc) return rc;
     a.rep = g->bfs_rep;
@@ -1417,6 +1227,10 @@ extern "C" int grus_bfs(grus_graph *g, uint32_t src, uint32_t *depth,
                       g->mem_mode == GRUS_MEM_MANAGED ? kDefBuScanManaged : kDefBuScan);
   const int ncl = narrow_cluster();
   a.narrow_nf = g->tuning.tail_cluster == 2 ? 0u : kNarrowNf * (uint32_t)ncl;
+  a.far = w->far;
+  a.whole = whole;
+  a.lanes = narrow::lanes_per_entry(g->max_deg);
+  a.ahead = a.lanes && narrow::beyond_l2(g->n, g->m, 4);
   a.ho = (Handover *)(w->ctrl + kOffHandover);
   a.timeout_ns = (uint64_t)tune_or(g->tuning.timeout_ms, 30000u) * 1000000ull;
 
@@ -1445,26 +1259,12 @@ extern "C" int grus_bfs(grus_graph *g, uint32_t src, uint32_t *depth,
 
   const bool sync = stats != nullptr || !dev_out;
   // barrier and error word: a timed-out launch leaves stale barrier state
-  GRUS_CUDA_TRY(cudaMemsetAsync(w->ctrl + kOffBar, 0, kOffSummary - kOffBar, s));
+  if (!whole) GRUS_CUDA_TRY(cudaMemsetAsync(w->ctrl + kOffBar, 0, kOffSummary - kOffBar, s));
   if (stats) GRUS_CUDA_TRY(cudaEventRecord(w->ev0, s));
-  GRUS_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, a));
-  // continues a long traversal the persistent kernel handed over; returns at
-  // once otherwise
-  {
-    cudaLaunchAttribute cattr;
-    cattr.id = cudaLaunchAttributeClusterDimension;
-    cattr.val.clusterDim.x = (unsigned)ncl;
-    cattr.val.clusterDim.y = 1;
-    cattr.val.clusterDim.z = 1;
-    cudaLaunchConfig_t ncfg = {};
-    ncfg.gridDim = dim3((unsigned)ncl);
-    ncfg.blockDim = dim3(kNarrowBlock);
-    ncfg.dynamicSmemBytes = kNarrowSmem;
-    ncfg.stream = s;
-    ncfg.attrs = &cattr;
-    ncfg.numAttrs = ncl > 1 ? 1 : 0;
-    GRUS_CUDA_TRY(cudaLaunchKernelEx(&ncfg, bfs_narrow, a));
-  }
+  if (!whole) GRUS_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, a));
+  // runs a small graph, or continues a traversal the persistent kernel handed
+  // over; returns at once otherwise
+  GRUS_CUDA_TRY(narrow::launch(bfs_narrow, ncl, a, s));
   if (stats) GRUS_CUDA_TRY(cudaEventRecord(w->ev1, s));
   if (!dev_out) GRUS_CUDA_TRY(cudaMemcpyAsync(depth, w->depth, g->n * 4, cudaMemcpyDeviceToHost, s));
   if (!sync) return GRUS_OK;
@@ -1486,7 +1286,7 @@ extern "C" int grus_bfs(grus_graph *g, uint32_t src, uint32_t *depth,
     stats->levels = sm->levels;
     stats->bottom_up_levels = sm->bu_levels;
     stats->direction_switches = sm->switches;
-    stats->kernel_launches = 2;
+    stats->kernel_launches = whole ? 1 : 2;
     stats->vertices_reached = sm->nr;
     stats->edges_reached = sm->mr;
     float ms = 0.f;
@@ -1494,6 +1294,13 @@ extern "C" int grus_bfs(grus_graph *g, uint32_t src, uint32_t *depth,
     stats->device_ms = ms;
   }
   return GRUS_OK;
+}
+
+}  // namespace grus
+
+extern "C" int grus_bfs(grus_graph *g, uint32_t src, uint32_t *depth,
+                        grus_stats *stats, void *stream) {
+  return bfs_run(g, src, depth, stats, (cudaStream_t)stream, true);
 }
 
 extern "C" int grus_bfs_trace(grus_graph *g, grus_level_trace *out, int max_levels) {

@@ -100,6 +100,11 @@ int msbfs_run(grus_graph *g, const uint32_t *hsrc, int k, uint32_t *const *outs,
 int msssp_run(grus_graph *g, const uint32_t *hsrc, int k, uint32_t *const *outs,
               grus_stats *stats, cudaStream_t s);
 
+// Single-source BFS (bfs.cu): two kernels, or one where whole_ok and the graph
+// is small.  grus_bfs allows it; the batch and the server, whose small graphs
+// run on cluster workers anyway, keep the two.
+int bfs_run(grus_graph *g, uint32_t src, uint32_t *depth, grus_stats *stats, cudaStream_t s,
+            bool whole_ok);
 // Single-source SSSP (sssp.cu).  tail: launch the cluster kernel behind the
 // persistent one (2 kernels, else 1); grus_sssp does where sssp_tail says so.
 // The batch and the server, whose lanes queue launches back to back, do on

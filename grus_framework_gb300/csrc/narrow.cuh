@@ -26,15 +26,15 @@
 // A full list never loses work: its overflow goes to the near or far bitmap,
 // which the next step (split) scans.
 //
-// Bound by latency: a round with one entry takes 1.0-1.3 us (a path of 4,001
+// Bound by latency: a round with one entry takes 1.4-1.6 us (a path of 4,001
 // vertices), of which the atomic's round trip is about a third, and a cluster
-// barrier with its stamps about 1 us more.  Measured for SSSP (a 1,021 x
-// 1,531 grid / a 40 x 3,000 grid / RMAT-12, ms): 512 threads and 8 rounds per
-// step 13.6 / 18.5 / 0.18, 4 rounds 12.7 / 14.8 / 0.18, 16 rounds 16.7 / 20.8
-// / 0.18; 1,024 threads and 4 rounds 11.8 / 14.5 / 0.17, which is kept: more
-// threads cost the narrowest frontiers 10 % and gain 10-20 % on wider ones.
-// Prefetching the lines after a target's (adjacency, offsets, distance) as
-// well as its own: 14.6 against 13.3 ms on the first grid.
+// barrier with its stamp about 0.8 us more.  Measured for SSSP (a 1,021 x
+// 1,531 grid / a 40 x 3,000 grid / RMAT-12, ms; the grid kernel 81 / 88 /
+// 0.29): 512 threads 13.5 / 11.4 / 0.17, 768 threads 10.9 / 11.7 / 0.14,
+// 1,024 threads 10.8 / 13.0 / 0.14.  1,024 are kept for the widest frontiers
+// (BFS on a 4,096 x 4,096 grid: 32.2, 30.2, 25.4 ms).  Rounds per step, with
+// an earlier form at 512 threads: 2 14.2 / 14.8, 4 12.7 / 14.8, 8 13.6 /
+// 18.5, 16 16.7 / 20.8.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -51,22 +51,32 @@ constexpr int kWarps = kBlock / 32;
 constexpr int kMaxCluster = 16;
 constexpr uint32_t kCap = 2048;      // entries of one list
 constexpr uint32_t kPiece = 64;      // edges per entry
-// Low-degree graphs, few entries: kLanes lanes per entry instead of a scan
-// over the entries' degrees (the path's round 1.57 -> 1.04 us with 512
-// threads; entries of up to 64 edges would take 8 serial steps instead:
-// RMAT-12 0.19 -> 0.25 ms).
-constexpr uint32_t kLanes = 8;
-constexpr uint32_t kFew = 32 / kLanes;       // entries per warp
-constexpr uint32_t kLowDegree = 2 * kLanes;  // largest out-degree of the graph
+// Low-degree graphs, few entries: 4 or 8 lanes per entry instead of a scan
+// over the entries' degrees (a path's round 1.57 -> 1.04 us with 512 threads;
+// entries of up to 64 edges would take 8 serial steps instead: RMAT-12 0.19
+// -> 0.25 ms).  0: the scan always.
+inline uint32_t lanes_per_entry(uint32_t max_degree) {
+  return max_degree <= 4 ? 4u : (max_degree <= 16 ? 8u : 0u);
+}
+// Whether a graph and its distances (`edge` bytes per edge) are beyond what L2
+// keeps: a wave over such a graph fetches the lines ahead of it (BFS on a
+// 4,096 x 4,096 grid 31.3 -> 29.1 ms; grids inside L2 lose 5 %).
+inline bool beyond_l2(uint64_t n, uint64_t m, uint32_t edge) {
+  return 8 * n + edge * m > (96ull << 20);
+}
 constexpr int kRounds = 4;           // rounds between cluster barriers
 constexpr int kIlp = 2;              // 32-edge steps whose loads are in flight together
-constexpr uint32_t kFarCap = 8192;   // far entries per CTA and buffer
+constexpr uint32_t kFarCap = 4096;   // most far entries per CTA and buffer
 constexpr uint32_t kInf = 4294967294u;
 constexpr uint32_t kRing = 128;      // BFS: depth counts, by depth modulo kRing
 constexpr uint32_t kUnitDelta = 32;  // BFS: levels per threshold step (<= kRing / 2)
 
-// Far lists of one cluster: 2 buffers per CTA.
-constexpr size_t kFarBytes = (size_t)kMaxCluster * 2 * kFarCap * sizeof(uint2);
+// Far lists of one cluster (2 buffers per CTA) for a graph of n vertices;
+// small graphs get short ones, so that a first call's allocation stays small.
+__host__ __device__ inline uint32_t far_cap(uint64_t n) {
+  return n >= 8ull * kFarCap ? kFarCap : (n < 512 ? 64u : (uint32_t)(n / 8));
+}
+inline size_t far_bytes(uint64_t n) { return (size_t)kMaxCluster * 2 * far_cap(n) * sizeof(uint2); }
 
 // Per-step record (SSSP) or per-level record (BFS), the layout of the
 // persistent kernels' traces.
@@ -79,14 +89,16 @@ struct View {
   const uint32_t *__restrict__ offs;
   const uint32_t *__restrict__ cols;
   const uint32_t *__restrict__ wts;  // unused by BFS
-  uint32_t n, W;
+  uint32_t n, W, m;
   uint32_t *dist;
   uint32_t *nearbm;  // W words, all zero at the start
   uint32_t *farbm;   // W words, zero but for what farbm_used announces
-  uint2 *far;        // kFarBytes
+  uint2 *far;        // far_bytes(n)
+  uint32_t far_cap;
   uint32_t delta;
   bool adapt;        // SSSP: delta may grow while threshold steps do little
-  bool low_degree;   // every vertex has at most kLowDegree out-edges
+  uint32_t lanes;    // lanes_per_entry of the graph
+  bool ahead;        // low degrees, and beyond_l2
   uint32_t *err;
   // null: none.  SSSP: record i is the i-th step's (from 1); BFS: record d
   // counts the vertices of depth d.  Records to be written start out zero.
@@ -100,11 +112,16 @@ __device__ __forceinline__ void prefetch_l1(const void *p) {
   asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
 }
 
+__device__ __forceinline__ void prefetch_l2(const void *p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
 struct Shared {
   uint4 loc[2][kCap];
   uint4 inb[2][kCap];
   uint32_t cnt[3];                      // local list lengths, rotating by round
   uint32_t incnt[2], farcnt[2];
+  uint32_t away[2];                     // entries pushed to other CTAs, by step parity
   // the last step in which this CTA pushed to an inbox, spilled to the near
   // bitmap, put bits in the far bitmap (0: never), ...
   uint32_t pushed, spilled, farbm;
@@ -112,6 +129,10 @@ struct Shared {
   // and the last that put bits in the far bitmap
   uint32_t g_farbm;
   uint2 g_work;
+  uint32_t g_far;                       // ... and had far vertices
+  // this CTA's copies: far bitmap bits up to this step have been taken; the
+  // last threshold step and its size
+  uint32_t scanned, last_split, delta;
   uint32_t min_far;                     // smallest distance of this CTA's far vertices
   uint32_t red[kWarps];
   unsigned long long red64[kWarps];
@@ -122,7 +143,7 @@ struct Shared {
 struct Result {
   uint32_t steps = 0, splits = 0;
   uint32_t last = 0;                    // BFS: largest depth (valid in rank 0)
-  unsigned long long visits = 0, nr = 0, mr = 0;  // this thread's share
+  uint32_t visits = 0, nr = 0, mr = 0;  // this thread's share (m < 2^32 bounds the last two)
 };
 
 template <bool kUnit>
@@ -131,11 +152,10 @@ struct Engine {
   Shared *s;
   cg::cluster_group cl;
   uint32_t rank, C, lane, warp;
+  uint32_t lane_shift;        // log2 of a.lanes
   uint32_t scale;             // home of v: umulhi(v, scale)
   uint32_t T, step;           // steps count from 1 (0 = never)
-  uint32_t delta, last_split; // current threshold step and the last one's step number
-  uint32_t scanned;           // far bitmap bits up to this step have been taken
-  uint32_t cq, lb, ip, fb;    // read: cnt[cq], loc[lb], inb[ip], far buffer fb
+  uint32_t cq, lb, fb;        // read: cnt[cq], loc[lb], far buffer fb
   Result res;
 
   __device__ __forceinline__ Engine(const View &view, Shared *sh)
@@ -144,22 +164,27 @@ struct Engine {
     C = cl.num_blocks();
     lane = lane_id();
     warp = threadIdx.x >> 5;
+    lane_shift = a.lanes ? 31 - __clz(a.lanes) : 0;
     const unsigned long long q = ((unsigned long long)C << 32) / max(a.n, 1u);
     scale = q > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)q;
     T = 0;
     step = 1;
-    scanned = last_split = 0;
-    delta = a.delta;
-    cq = lb = ip = fb = 0;
+    cq = lb = fb = 0;
     if (threadIdx.x < 3) s->cnt[threadIdx.x] = 0u;
-    if (threadIdx.x < 2) s->incnt[threadIdx.x] = s->farcnt[threadIdx.x] = 0u;
+    if (threadIdx.x < 2)
+      s->incnt[threadIdx.x] = s->farcnt[threadIdx.x] = s->away[threadIdx.x] = 0u;
     if (threadIdx.x < kRing) s->ring[threadIdx.x] = s->ring_sum[threadIdx.x] = 0;
     if (threadIdx.x == 0) {
       s->pushed = s->spilled = s->farbm = s->g_farbm = 0u;
       s->g_work = make_uint2(0u, 0u);
+      s->g_far = 0u;
+      s->scanned = s->last_split = 0u;
+      s->delta = a.delta;
     }
   }
 
+  // Which inbox is read in this step; the other one is written.
+  __device__ __forceinline__ uint32_t ip() const { return (step & 1u) ^ 1u; }
   __device__ __forceinline__ uint32_t home(uint32_t v) const { return __umulhi(v, scale); }
 
   __device__ __forceinline__ void spill(uint32_t v) {
@@ -168,13 +193,14 @@ struct Engine {
   }
 
   // Queues the vertices u (edges [b,e), distance d) of the lanes with `want`:
-  // one entry at its home, or pieces of kPiece edges dealt over the cluster.
-  // Called by whole warps.
+  // one entry at its home, or pieces of kPiece edges dealt over the cluster
+  // (kBig; without it no vertex has more).  Called by whole warps.
+  template <bool kBig>
   __device__ __forceinline__ void push(bool want, uint32_t u, uint32_t b, uint32_t e, uint32_t d) {
     want = want && e > b;
     const uint32_t nq = cq == 2 ? 0 : cq + 1;
     const uint32_t o = home(u);
-    const bool big = want && e - b > kPiece;
+    const bool big = kBig && want && e - b > kPiece;
     const bool here = want && !big && o == rank;
     if (here) {
       const uint32_t pos = atomicAdd(&s->cnt[nq], 1u);
@@ -189,23 +215,46 @@ struct Engine {
       const int leader = __ffs(peers) - 1;
       Shared *r = cl.map_shared_rank(s, o);
       uint32_t base = 0;
-      if ((int)lane == leader) base = atomicAdd(&r->incnt[ip ^ 1u], __popc(peers));
+      if ((int)lane == leader) {
+        base = atomicAdd(&r->incnt[ip() ^ 1u], __popc(peers));
+        atomicAdd(&s->away[ip()], __popc(peers));
+      }
       base = __shfl_sync(peers, base, leader);
       const uint32_t pos = base + __popc(peers & ((1u << lane) - 1u));
-      if (pos < kCap) r->inb[ip ^ 1u][pos] = make_uint4(u, b, e, d);
+      if (pos < kCap) r->inb[ip() ^ 1u][pos] = make_uint4(u, b, e, d);
       else spill(u);
       s->pushed = step;
     }
     __syncwarp();
-    for (uint32_t mb = __ballot_sync(0xffffffffu, big); mb; mb &= mb - 1) {
-      const int j = __ffs(mb) - 1;
+    if (kBig && __any_sync(0xffffffffu, big)) push_pieces(big, u, b, e, d);
+  }
+
+  // ... the vertices with more than kPiece edges: one piece per lane at a time.
+  __device__ __forceinline__ void push_pieces(bool big, uint32_t u, uint32_t b, uint32_t e, uint32_t d) {
+    const uint32_t nq = cq == 2 ? 0 : cq + 1;
+    const uint32_t np = big ? (e - b + kPiece - 1) / kPiece : 0u;
+    uint32_t incl = np;
+#pragma unroll
+    for (int o2 = 1; o2 < 32; o2 <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o2);
+      if ((int)lane >= o2) incl += t;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+    if (lane == 0) atomicAdd(&s->away[ip()], total - total / C);
+    for (uint32_t k0 = 0; k0 < total; k0 += 32) {
+      const uint32_t k = k0 + lane;
+      int j = 0;
+#pragma unroll
+      for (int st = 16; st >= 1; st >>= 1) {
+        const uint32_t pv = __shfl_sync(0xffffffffu, incl, j + st - 1);
+        if (pv <= k) j += st;
+      }
       const uint32_t pu = __shfl_sync(0xffffffffu, u, j), pb = __shfl_sync(0xffffffffu, b, j);
       const uint32_t pe = __shfl_sync(0xffffffffu, e, j), pd = __shfl_sync(0xffffffffu, d, j);
-      const uint32_t po = __shfl_sync(0xffffffffu, o, j);
-      const uint32_t np = (pe - pb + kPiece - 1) / kPiece;
-      for (uint32_t k = lane; k < np; k += 32) {
-        const uint32_t t = (po + k) % C;
-        const uint32_t xb = pb + k * kPiece;
+      const uint32_t at = k - __shfl_sync(0xffffffffu, incl - np, j);
+      if (k < total) {
+        const uint32_t t = (home(pu) + at) % C;
+        const uint32_t xb = pb + at * kPiece;
         const uint4 en = make_uint4(pu, xb, min(pe, xb + kPiece), pd);
         if (t == rank) {
           const uint32_t pos = atomicAdd(&s->cnt[nq], 1u);
@@ -213,13 +262,12 @@ struct Engine {
           else spill(pu);
         } else {
           Shared *r = cl.map_shared_rank(s, t);
-          const uint32_t pos = atomicAdd(&r->incnt[ip ^ 1u], 1u);
-          if (pos < kCap) r->inb[ip ^ 1u][pos] = en;
+          const uint32_t pos = atomicAdd(&r->incnt[ip() ^ 1u], 1u);
+          if (pos < kCap) r->inb[ip() ^ 1u][pos] = en;
           else spill(pu);
           s->pushed = step;
         }
       }
-      __syncwarp();
     }
   }
 
@@ -233,8 +281,8 @@ struct Engine {
     base = __shfl_sync(0xffffffffu, base, leader);
     if (want) {
       const uint32_t pos = base + __popc(m & ((1u << lane) - 1u));
-      if (pos < kFarCap) {
-        a.far[(size_t)(rank * 2 + buf) * kFarCap + pos] = make_uint2(u, d);
+      if (pos < a.far_cap) {
+        a.far[(size_t)(rank * 2 + buf) * a.far_cap + pos] = make_uint2(u, d);
       } else {
         atomicOr(a.farbm + (u >> 5), 1u << (u & 31u));
         s->farbm = step;
@@ -247,6 +295,10 @@ struct Engine {
   // laid end to end, one per lane.  A target's offsets are loaded beside the
   // atomic that lowers its distance, so pushing it waits for nothing more.
   // Called by whole warps.
+  // A stale entry's edges are not relaxed, and a plain read comes before each
+  // atomic: most edges into a dense part of the graph improve nothing, and
+  // their atomics would queue up on its hubs (without either, RMAT-12 SSSP
+  // 0.136 -> 0.167 ms).
   __device__ __forceinline__ void relax(uint4 en, bool has) {
     const uint32_t deg = has ? en.z - en.y : 0u;
     const uint32_t cur = has ? __ldcg(a.dist + en.x) : 0u;
@@ -284,8 +336,6 @@ struct Engine {
         nd[i] = od + (kUnit ? 1u : (act[i] ? __ldg(a.wts + x) : 0u));
         act[i] = __shfl_sync(0xffffffffu, (int)fresh, j) && act[i];
       }
-      // a plain read first: most edges into a dense part of the graph improve
-      // nothing, and their atomics would queue up on its hubs
 #pragma unroll
       for (int i = 0; i < kIlp; ++i) old[i] = act[i] ? __ldcg(a.dist + u[i]) : 0u;
 #pragma unroll
@@ -303,13 +353,23 @@ struct Engine {
       // before the atomics' answers arrive
 #pragma unroll
       for (int i = 0; i < kIlp; ++i)
-        if (act[i]) prefetch_edges(b[i]);
-#pragma unroll
-      for (int i = 0; i < kIlp; ++i) {
-        if (i && k0 + 32 * i >= total) break;
-        settle(act[i] && nd[i] < old[i], true, u[i], nd[i], old[i], b[i], e[i]);
+        if (e[i] > b[i]) prefetch_edges(b[i]);
+      // one copy of the code for both steps: the kernel's rounds are short
+      // enough to feel the instruction cache
+      static_assert(kIlp == 2, "two steps");
+#pragma unroll 1
+      for (int i = 0; i < kIlp && k0 + 32 * i < total; ++i) {
+        const bool imp = i ? act[1] && nd[1] < old[1] : act[0] && nd[0] < old[0];
+        settle<true>(imp, true, i ? u[1] : u[0], i ? nd[1] : nd[0], i ? old[1] : old[0],
+                     i ? b[1] : b[0], i ? e[1] : e[0]);
       }
     }
+  }
+
+  // The 128-byte lines behind and before word i's, within the array.
+  __device__ __forceinline__ void prefetch_near(const uint32_t *p, uint32_t i, uint32_t size) {
+    if (i + 32u < size) prefetch_l2(p + i + 32);
+    if (i >= 32u) prefetch_l2(p + i - 32);
   }
 
   __device__ __forceinline__ void prefetch_edges(uint32_t b) {
@@ -319,6 +379,7 @@ struct Engine {
 
   // The lanes with `imp` lowered vertex u (edges [b,e)) from `old` to nd; the
   // ones with `queue` too push it.  Called by whole warps.
+  template <bool kBig>
   __device__ __forceinline__ void settle(bool imp, bool queue, uint32_t u, uint32_t nd,
                                          uint32_t old, uint32_t b, uint32_t e) {
     if (!__any_sync(0xffffffffu, imp)) return;
@@ -329,28 +390,39 @@ struct Engine {
       }
       if (kUnit) count_depth(nd, old, e - b);
     }
-    push(imp && queue && nd < T, u, b, e, nd);
+    // a wave that reaches the start of a line goes on to the next one (or
+    // back to the one before): fetch both from HBM some levels ahead
+    if (imp && a.ahead) {
+      if ((u & 31u) == 16u) {
+        prefetch_near(a.offs, u, a.n);
+        prefetch_near(a.dist, u, a.n);
+      }
+      if ((b & 31u) < e - b) {
+        prefetch_near(a.cols, b, a.m);
+        if (!kUnit) prefetch_near(a.wts, b, a.m);
+      }
+    }
+    push<kBig>(imp && queue && nd < T, u, b, e, nd);
     push_far(imp && queue && nd >= T && e > b, u, nd, fb);
   }
 
-  // Few entries (at most kFew per warp): kLanes lanes per entry, no scan, and
-  // nothing waits for the check that an entry is still current.  A stale
-  // entry may lower a distance, but does not push: the entry that made it
-  // stale relaxes the same edge with a smaller candidate, before (then this
-  // one lowers nothing) or after (then that one lowers and pushes).
-  // Called by whole warps.
+  // Few entries: a.lanes lanes per entry, no scan, and nothing waits for the
+  // check that an entry is still current.  A stale entry may lower a distance,
+  // but does not push: the entry that made it stale relaxes the same edge with
+  // a smaller candidate, before (then this one lowers nothing) or after (then
+  // that one lowers and pushes).  Called by whole warps.
   __device__ __forceinline__ void relax_few(uint4 en, bool has) {
     const uint32_t cur = has ? __ldcg(a.dist + en.x) : 0u;
-    for (uint32_t x = en.y + (lane & (kLanes - 1)); __any_sync(0xffffffffu, has && x < en.z);
-         x += kLanes) {
+    for (uint32_t x = en.y + (lane & (a.lanes - 1)); __any_sync(0xffffffffu, has && x < en.z);
+         x += a.lanes) {
       const bool act = has && x < en.z;
       const uint32_t u = act ? __ldg(a.cols + x) : 0u;
       const uint32_t nd = en.w + (kUnit ? 1u : (act ? __ldg(a.wts + x) : 0u));
       const uint32_t b = act ? __ldg(a.offs + u) : 0u, e = act ? __ldg(a.offs + u + 1) : 0u;
       const uint32_t old = act ? atomicMin(a.dist + u, nd) : 0u;
-      if (act) prefetch_edges(b);
+      if (e > b) prefetch_edges(b);
       res.visits += act;
-      settle(act && nd < old, cur == en.w, u, nd, old, b, e);
+      settle<false>(act && nd < old, cur == en.w, u, nd, old, b, e);
     }
   }
 
@@ -369,8 +441,8 @@ struct Engine {
   }
 
   // Vertices spilled to the near bitmap in the previous step: this CTA's
-  // share of the words, a word per warp at a time.
-  __device__ __forceinline__ void relax_spilled() {
+  // share of the words goes back to the lists (what does not fit spills again).
+  __device__ __forceinline__ void take_spilled() {
     const uint32_t per = (a.W + C - 1) / C;
     const uint32_t w0 = min(a.W, rank * per), w1 = min(a.W, w0 + per);
     for (uint32_t w = w0 + warp; w < w1; w += kWarps) {
@@ -378,15 +450,10 @@ struct Engine {
       if (lane == 0 && __ldcg(a.nearbm + w)) bits = atomicExch(a.nearbm + w, 0u);
       bits = __shfl_sync(0xffffffffu, bits, 0);
       if (!bits) continue;
-      const bool has = lane < __popc(bits);
-      const uint32_t v = w * 32 + (has ? __fns(bits, 0, lane + 1) : 0u);
-      uint4 en = make_uint4(v, 0u, 0u, 0u);
-      if (has) {
-        en.y = __ldg(a.offs + v);
-        en.z = __ldg(a.offs + v + 1);
-        en.w = __ldcg(a.dist + v);
-      }
-      relax(en, has);
+      const bool has = (bits >> lane) & 1u;
+      const uint32_t v = w * 32 + lane;
+      push<true>(has, v, has ? __ldg(a.offs + v) : 0u, has ? __ldg(a.offs + v + 1) : 0u,
+                 has ? __ldcg(a.dist + v) : 0u);
     }
   }
 
@@ -404,10 +471,12 @@ struct Engine {
   // far vertices below it are pushed (this CTA's list and, if any CTA put
   // bits there, its share of the far bitmap).  False when nothing is far.
   __device__ __forceinline__ bool split() {
-    const uint2 *cur = a.far + (size_t)(rank * 2 + fb) * kFarCap;
-    const uint32_t fc = min(s->farcnt[fb], kFarCap);
-    const bool bm = *(volatile uint32_t *)&cl.map_shared_rank(s, 0)->g_farbm > scanned;
-    scanned = step - 1;
+    const uint2 *cur = a.far + (size_t)(rank * 2 + fb) * a.far_cap;
+    const uint32_t fc = min(s->farcnt[fb], a.far_cap);
+    const Shared *r0 = cl.map_shared_rank(s, 0);
+    const bool bm = *(const volatile uint32_t *)&r0->g_farbm > s->scanned;
+    // stamped in the step that just ended (no CTA is past this split)
+    if (!bm && *(const volatile uint32_t *)&r0->g_far < step - 1) return false;
     const uint32_t per = (a.W + C - 1) / C;
     const uint32_t w0 = min(a.W, rank * per), w1 = min(a.W, w0 + per);
     uint32_t m = 0xFFFFFFFFu;
@@ -437,37 +506,45 @@ struct Engine {
     }
     const uint32_t Told = T;
     // weights far above delta: a threshold step should last a few steps
-    if (a.adapt && step - last_split <= 3 && delta < 1u << 30) delta *= 2;
-    last_split = step;
+    uint32_t delta = s->delta;
+    if (a.adapt && step - s->last_split <= 3 && delta < 1u << 30) delta *= 2;
     T = gm > 0xFFFFFFFFu - delta ? 0xFFFFFFFFu : gm + delta;
-    const uint32_t rounds = (fc + kBlock - 1) / kBlock;
-    for (uint32_t r = 0; r < rounds; ++r) {
-      const uint32_t i = r * kBlock + threadIdx.x;
-      const uint2 f = i < fc ? __ldcg(cur + i) : make_uint2(0u, 0u);
-      const bool live = i < fc && __ldcg(a.dist + f.x) == f.y;
-      const uint32_t b = live ? __ldg(a.offs + f.x) : 0u, e = live ? __ldg(a.offs + f.x + 1) : 0u;
-      push(live && f.y < T, f.x, b, e, f.y);
-      push_far(live && f.y >= T, f.x, f.y, fb ^ 1u);
-    }
-    if (bm) {
-      for (uint32_t w = w0 + warp; w < w1; w += kWarps) {
+    const uint32_t lists = (fc + kBlock - 1) / kBlock;
+    const uint32_t words = bm ? (w1 - w0 + kWarps - 1) / kWarps : 0u;
+    for (uint32_t r = 0; r < lists + words; ++r) {
+      uint32_t v = 0, d = 0;
+      bool live = false;
+      if (r < lists) {
+        const uint32_t i = r * kBlock + threadIdx.x;
+        if (i < fc) {
+          const uint2 f = __ldcg(cur + i);
+          v = f.x;
+          d = f.y;
+          live = __ldcg(a.dist + v) == d;
+        }
+      } else {
+        const uint32_t w = w0 + (r - lists) * kWarps + warp;
         // other CTAs may be setting bits of far vertices they cannot list
         uint32_t bits = 0;
-        if (lane == 0 && __ldcg(a.farbm + w)) bits = atomicExch(a.farbm + w, 0u);
+        if (lane == 0 && w < w1 && __ldcg(a.farbm + w)) bits = atomicExch(a.farbm + w, 0u);
         bits = __shfl_sync(0xffffffffu, bits, 0);
         if (!bits) continue;
-        const uint32_t v = w * 32 + lane;
-        const bool has = (bits >> lane) & 1u;
-        const uint32_t d = has ? __ldcg(a.dist + v) : 0u;
-        const bool live = has && d >= Told;
-        const uint32_t b = live ? __ldg(a.offs + v) : 0u, e = live ? __ldg(a.offs + v + 1) : 0u;
-        push(live && d < T, v, b, e, d);
-        push_far(live && d >= T, v, d, fb ^ 1u);
+        v = w * 32 + lane;
+        if ((bits >> lane) & 1u) {
+          d = __ldcg(a.dist + v);
+          live = d >= Told;
+        }
       }
+      const uint32_t b = live ? __ldg(a.offs + v) : 0u, e = live ? __ldg(a.offs + v + 1) : 0u;
+      push<true>(live && d < T, v, b, e, d);
+      push_far(live && d >= T, v, d, fb ^ 1u);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
       s->farcnt[fb] = 0u;
+      s->scanned = step - 1;
+      s->last_split = step;
+      s->delta = delta;
       s->cnt[cq == 0 ? 2 : cq - 1] = 0u;  // the list of the rounds to come
     }
     fb ^= 1u;
@@ -486,13 +563,13 @@ struct Engine {
       if (s->cnt[cq] || s->pushed == step) *(volatile uint32_t *)&r->g_work.x = step;
       if (s->spilled == step) *(volatile uint32_t *)&r->g_work.y = step;
       if (s->farbm == step) *(volatile uint32_t *)&r->g_farbm = step;
+      if (s->farcnt[fb]) *(volatile uint32_t *)&r->g_far = step;
     }
     cl.sync();
     const Shared *r = cl.map_shared_rank(s, 0);
     const uint32_t gw = *(const volatile uint32_t *)&r->g_work.x;
     const uint32_t gs = *(const volatile uint32_t *)&r->g_work.y;
     spilled = gs >= step;
-    ip ^= 1u;
     ++step;
     return gw >= step - 1 || spilled;
   }
@@ -515,42 +592,50 @@ struct Engine {
         if (!split()) break;
         next_round();
       }
-      const unsigned long long v0 = res.visits;
+      const uint32_t v0 = res.visits;
       uint32_t taken = 0;
 #pragma unroll 1
       for (int r = 0; r < kRounds; ++r) {
         const uint32_t nc = min(s->cnt[cq], kCap);
-        const uint32_t ni = r == 0 ? min(s->incnt[ip], kCap) : 0u;
+        const uint32_t ni = r == 0 ? min(s->incnt[ip()], kCap) : 0u;
         const uint32_t total = nc + ni;
         const bool scan = r == 0 && spilled;
         if (total == 0 && !scan) break;
+        // ids that jump between homes: most of this step's pushes wait in
+        // other CTAs' inboxes, and further rounds over the rest only delay them
+        if (r && 4 * nc <= s->away[ip()]) break;
         // the list after next was read in the round before this one
         if (threadIdx.x == 0) s->cnt[cq == 0 ? 2 : cq - 1] = 0u;
         taken += total;
-        if (a.low_degree && total <= kWarps * kFew) {
-          const uint32_t i = warp * kFew + lane / kLanes;
-          const bool has = i < total;
-          uint4 en = make_uint4(0u, 0u, 0u, 0u);
-          if (has) en = i < nc ? s->loc[lb][i] : s->inb[ip][i - nc];
-          relax_few(en, has);
+        if (a.lanes && total * a.lanes <= 2 * kBlock) {
+          for (uint32_t base = threadIdx.x; base < total * a.lanes + lane; base += kBlock) {
+            const uint32_t i = base >> lane_shift;
+            const bool has = i < total;
+            uint4 en = make_uint4(0u, 0u, 0u, 0u);
+            if (has) en = i < nc ? s->loc[lb][i] : s->inb[ip()][i - nc];
+            relax_few(en, has);
+          }
         } else {
           const uint32_t epw = min(32u, (total + kWarps - 1) / kWarps);
           for (uint32_t base = warp * epw; base < total; base += kWarps * epw) {
             const uint32_t i = base + lane;
             const bool has = lane < epw && i < total;
             uint4 en = make_uint4(0u, 0u, 0u, 0u);
-            if (has) en = i < nc ? s->loc[lb][i] : s->inb[ip][i - nc];
+            if (has) en = i < nc ? s->loc[lb][i] : s->inb[ip()][i - nc];
             relax(en, has);
           }
         }
-        if (scan) relax_spilled();
+        if (scan) take_spilled();
         next_round();
-        if (r == 0 && threadIdx.x == 0) s->incnt[ip] = 0u;
+        if (r == 0 && threadIdx.x == 0) {
+          s->incnt[ip()] = 0u;
+          s->away[ip() ^ 1u] = 0u;
+        }
       }
       ++res.steps;
       if (!kUnit && a.trace && res.steps < a.trace_cap) {
         Trace *t = a.trace + res.steps;
-        atomicAdd(&t->edges, res.visits - v0);
+        atomicAdd(&t->edges, (unsigned long long)(res.visits - v0));
         if (threadIdx.x == 0) {
           atomicAdd(&t->count, taken);
           if (rank == 0) {
@@ -575,8 +660,9 @@ struct Engine {
         while (d > T - a.delta && s->ring_sum[d % kRing] <= 0) --d;
         res.last = d;
       }
+    } else {
+      cl.sync();  // no CTA leaves while another may still read its shared memory
     }
-    cl.sync();  // no CTA leaves while another may still write its shared memory
   }
 
   // Sum over the block of a per-thread count; valid in thread 0.

@@ -274,7 +274,7 @@ int big_launch(grus_server *s, BigJob &j) {
   if (!multi) {
     rc = r.algo == GRUS_ALGO_SSSP
              ? sssp_run(g, r.src, r.out, nullptr, s->big_stream, sssp_lane_tail(g))
-             : grus_bfs(g, r.src, r.out, nullptr, s->big_stream);
+             : bfs_run(g, r.src, r.out, nullptr, s->big_stream, false);
   } else {
     uint32_t srcs[64];
     uint32_t *outs[64];

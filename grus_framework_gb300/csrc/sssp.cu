@@ -41,18 +41,19 @@ namespace {
 constexpr int kBlock = 256;
 constexpr uint32_t kDefHuge = 1024;
 constexpr uint32_t kDefDelta = 640;
-// Hand-over to the cluster kernel (sssp_narrow): levels of at most
-// kNarrowNf near vertices per cluster CTA, one after another.  While they
-// shrink (the end of a traversal) with at most 2^kNarrowBits unreached
-// out-edges left; or after kNarrowSteady of them with a frontier no larger
-// than a plane's circle would be (4 s^2 at level s: a random graph's frontier
-// grows past it) -- high diameter, where every level costs the whole grid
-// 13-19 us however small it is.  The edge bound caps what a cluster, a tenth
-// of the chip, can be left with; levels that stay small three times longer
-// raise it.
+// Hand-over to the cluster kernel (sssp_narrow): kSteady levels in a row of at
+// most kNarrowNf near vertices per cluster CTA, and no more than a plane's
+// circle would have (4 s^2 at level s; a random graph's frontier grows past
+// it), if the unreached and far vertices have at most 2^kSteadyBits out-edges;
+// 2^kLongBits after 3 kSteady such levels of a graph without a vertex of more
+// than kLongDegree out-edges (grids, road networks).
+// The bounds cap what the cluster, a tenth of the chip, can be left with when
+// a long thin stretch ends in a dense part: uniform graphs of 2-9 M edges that
+// were handed over at 2^20 took 1.1-3.2 times the grid kernel's time.
 constexpr uint32_t kNarrowNf = 128;
-constexpr uint32_t kNarrowSteady = 8;
-constexpr uint32_t kNarrowBits = 22, kNarrowBitsLong = 26;
+constexpr uint32_t kSteady = 8;
+constexpr uint32_t kSteadyBits = 19, kLongBits = 26;
+constexpr uint32_t kLongDegree = 8;
 // Delta of the cluster kernel unless the caller set one: its levels are
 // short, so more distance per threshold step pays (grid 1021 x 1531: Delta
 // 640 11.8 ms, 1,280 11.1 ms, 2,560 12.6 ms).
@@ -98,8 +99,10 @@ struct Handover {
   uint32_t flag;                     // 1: sssp_narrow continues the traversal
   uint32_t qcount;                   // vertices of the near set (Args::queue)
   uint32_t T, sel;                   // threshold; near[sel] is all zero
-  unsigned long long mu[kMaxTries];  // unreached out-edges and vertices, by
-  uint32_t nu[kMaxTries];            // attempt
+  // by attempt: out-edges of the vertices that are not below the threshold,
+  // and the unreached vertices with their out-edges
+  unsigned long long left[kMaxTries], mu[kMaxTries];
+  uint32_t nu[kMaxTries];
 };
 
 struct Args {
@@ -129,7 +132,9 @@ struct Args {
   bool narrow_adapt;      // no Delta set by the caller
   uint2 *far;             // its far lists
   bool whole;             // sssp_narrow runs the whole traversal
-  bool low_degree;        // max out-degree <= narrow::kLowDegree
+  uint32_t max_deg;       // of the graph
+  uint32_t lanes;         // narrow::lanes_per_entry
+  bool ahead;             // narrow::View::ahead
 };
 
 struct Workspace {
@@ -186,7 +191,7 @@ int ws_get(grus_graph *g, Workspace **out) {
   w->chunk_cap = (uint32_t)std::min<uint64_t>(g->m / kChunk + g->m / huge + 2, 0x7FFFFFFFull);
   const uint64_t n1 = std::max<uint64_t>(g->n, 1);
   // one allocation with the far lists: a first call pays for each
-  cudaError_t e = cudaMalloc(&w->bitmaps, w->bitmap_bytes + narrow::kFarBytes);
+  cudaError_t e = cudaMalloc(&w->bitmaps, w->bitmap_bytes + narrow::far_bytes(g->n));
   if (e == cudaSuccess) w->far = (uint2 *)((char *)w->bitmaps + w->bitmap_bytes);
   if (e == cudaSuccess) e = cudaMalloc(&w->queues, n1 * 4);
   if (e == cudaSuccess) e = cudaMalloc(&w->chunks, (uint64_t)w->chunk_cap * sizeof(uint4));
@@ -232,56 +237,62 @@ struct RelaxVisitor {
 };
 
 // Attempt to hand the traversal over at level L, whose near set is the queue
-// of qc vertices: kHandedOver when done, else the new `small` word.  Every
-// thread of the grid calls it; out of line, as it runs a few times per
-// traversal at most and must not cost the level loop registers.
-constexpr uint32_t kHandedOver = 0xFFFFFFFFu;
-__device__ __noinline__ uint32_t try_hand_over(const Args &a, uint32_t small, uint32_t L, uint32_t T,
-                                               uint32_t splits, uint32_t qc,
-                                               unsigned long long visits) {
-  const uint32_t run = small & 0xFFFFu;
-  // the previous level's list length: its slot is cleared two levels later
-  const bool shrinking = qc < __ldcg(&a.slots[(L + 3) & 3u].qcount);
-  const bool steady = run >= kNarrowSteady && qc <= 4 * run * run;
-  if (!(shrinking || steady)) return run == 0xFFFFu ? small - 1 : small;
+// of qc vertices: kHandedOver when done, else how many small levels in a row
+// the next attempt needs.  Every thread of the grid calls it; out of line, as
+// it runs a few times per traversal at most and must not cost the level loop
+// registers.
+constexpr uint32_t kHandedOver = 0xFFFFFFFFu, kNever = 0xFFFFFFFEu;
+__device__ __noinline__ uint32_t try_hand_over(const Args &a, uint32_t run, uint32_t L, uint32_t T,
+                                               uint32_t splits, uint32_t qc) {
   const uint32_t gtid = blockIdx.x * kBlock + threadIdx.x, nthreads = gridDim.x * kBlock;
-  // one counter pair per attempt: the runs they need are 2, 8, 24, 72, ...
+  // one set of counters per attempt: the runs they need are 8, 24, 72, ...
   uint32_t k = 0;
-  for (uint32_t need = small >> 16; need > 2u; need = need > kNarrowSteady ? need / 3 : 2u) ++k;
-  if (k >= kMaxTries) return 0xFFFE0000u;  // no further attempt
-  unsigned long long mu = 0, nu = 0;
-  for (uint32_t v = gtid; v < a.n; v += nthreads)
-    if (__ldcg(a.dist + v) == kInfinit) {
+  for (uint32_t need = run; need > kSteady; need /= 3) ++k;
+  if (k >= kMaxTries) return kNever;
+  unsigned long long mu = 0, nu = 0, left = 0;
+  for (uint32_t v = gtid; v < a.n; v += nthreads) {
+    const uint32_t d = __ldcg(a.dist + v);
+    if (d < T) continue;
+    const uint32_t deg = __ldg(a.offs + v + 1) - __ldg(a.offs + v);
+    left += deg;
+    if (d == kInfinit) {
       ++nu;
-      mu += __ldg(a.offs + v + 1) - __ldg(a.offs + v);
+      mu += deg;
     }
+  }
   const unsigned long long bmu = block_sum_u64<kBlock>(mu);
   const unsigned long long bnu = block_sum_u64<kBlock>(nu);
-  if (threadIdx.x == 0 && bnu) {
+  const unsigned long long bleft = block_sum_u64<kBlock>(left);
+  if (threadIdx.x == 0 && (bnu || bleft)) {
+    atomicAdd(&a.ho->left[k], bleft);
     atomicAdd(&a.ho->mu[k], bmu);
     atomicAdd(&a.ho->nu[k], (uint32_t)bnu);
   }
   if (!grid_sync(a.bar, a.err, a.timeout_ns)) return kHandedOver;
   mu = __ldcg(&a.ho->mu[k]);
-  if (mu <= 1ull << (run >= 3 * kNarrowSteady ? kNarrowBitsLong : kNarrowBits)) {
-    if (gtid == 0) {
-      a.ho->qcount = qc;
-      a.ho->T = T;
-      a.ho->sel = (L + 1) & 1u;
-      a.summary->levels = L;
-      a.summary->splits = splits;
-      a.summary->visits = visits;
-      a.summary->nr = a.n - __ldcg(&a.ho->nu[k]);
-      a.summary->mr = a.m - mu;
-      a.ho->flag = 1u;
-    }
-    return kHandedOver;
+  const uint32_t bits = run >= 3 * kSteady && a.max_deg <= kLongDegree ? kLongBits : kSteadyBits;
+  if (__ldcg(&a.ho->left[k]) > 1ull << bits) return 3 * run;
+  if (gtid == 0) {
+    a.ho->qcount = qc;
+    a.ho->T = T;
+    a.ho->sel = (L + 1) & 1u;
+    a.summary->levels = L;
+    a.summary->splits = splits;
+    a.summary->nr = a.n - __ldcg(&a.ho->nu[k]);
+    a.summary->mr = a.m - mu;
+    a.ho->flag = 1u;
   }
-  const uint32_t need = small >> 16 ? small >> 16 : 2u;
-  return run | (need < kNarrowSteady ? kNarrowSteady : 3 * need) << 16;
+  return kHandedOver;
 }
 
 __global__ void __launch_bounds__(kBlock, 8) sssp_persistent(Args a) {
+  // small levels in a row, and how many the next attempt to hand over needs
+  // (in shared memory: the level loop has no register to spare at 8 CTAs/SM)
+  __shared__ uint32_t s_small, s_need;
+  if (threadIdx.x == 0) {
+    s_small = 0u;
+    s_need = a.narrow_nf ? kSteady : kNever;
+  }
   const uint32_t gtid = blockIdx.x * kBlock + threadIdx.x;
   const uint32_t nthreads = gridDim.x * kBlock;
   // prologue: distances to INFINIT, bitmaps and control words to zero
@@ -306,8 +317,6 @@ __global__ void __launch_bounds__(kBlock, 8) sssp_persistent(Args a) {
   if (!grid_sync(a.bar, a.err, a.timeout_ns)) return;
 
   uint32_t L = 0, T = a.delta, splits = 0;
-  uint32_t small = 0;  // small levels in a row, and from 2^16 on how many the next attempt needs
-  unsigned long long visits = 0;
   if (gtid == 0 && a.trace) a.trace[0] = LevelTrace{global_timer_ns(), 0ull, 1u, 0u};
   while (true) {
     Slot *sl = a.slots + (L & 3u);
@@ -371,11 +380,14 @@ __global__ void __launch_bounds__(kBlock, 8) sssp_persistent(Args a) {
       continue;  // compact the moved vertices (or split again)
     }
     // levels that are small one after another: the cluster kernel takes over
-    small = cc == 0 && qc <= a.narrow_nf ? small + 1 : small & ~0xFFFFu;
-    if ((small & 0xFFFFu) >= 2u && (small & 0xFFFFu) >= small >> 16) {
-      const uint32_t r = try_hand_over(a, small, L, T, splits, qc, visits);
+    if (threadIdx.x == 0) {
+      s_small = cc == 0 && qc <= a.narrow_nf && qc <= 4 * s_small * s_small + 64 ? s_small + 1 : 0u;
+    }
+    __syncthreads();
+    if (s_small == s_need) {
+      const uint32_t r = try_hand_over(a, s_small, L, T, splits, qc);
       if (r == kHandedOver) return;
-      small = r;
+      if (threadIdx.x == 0) s_need = r;
     }
     RelaxVisitor vis{&a, T, nnext, 0ull};
     expand_binned<kBlock>(a.offs, a.queue, qc, a.chunks, cc, vis);
@@ -383,10 +395,12 @@ __global__ void __launch_bounds__(kBlock, 8) sssp_persistent(Args a) {
     if (threadIdx.x == 0 && bv) atomicAdd(&sl->visits, bv);
     if (!grid_sync(a.bar, a.err, a.timeout_ns)) return;
     const unsigned long long lv = __ldcg(&sl->visits);
-    visits += lv;
     ++L;
-    if (gtid == 0 && a.trace && L < (uint32_t)kMaxTrace)
-      a.trace[L] = LevelTrace{global_timer_ns(), lv, qc + cc, splits};
+    if (gtid == 0) {
+      a.summary->visits += lv;
+      if (a.trace && L < (uint32_t)kMaxTrace)
+        a.trace[L] = LevelTrace{global_timer_ns(), lv, qc + cc, splits};
+    }
     if (L > 4u * a.n + 64u) {
       if (gtid == 0) atomicOr(a.err, kErrLevels);
       break;
@@ -411,7 +425,6 @@ __global__ void __launch_bounds__(kBlock, 8) sssp_persistent(Args a) {
   if (gtid == 0) {
     a.summary->levels = L;
     a.summary->splits = splits;
-    a.summary->visits = visits;
   }
 }
 
@@ -427,12 +440,15 @@ __global__ void __launch_bounds__(narrow::kBlock) sssp_narrow(Args a) {
   view.wts = a.wts;
   view.n = a.n;
   view.W = a.W;
+  view.m = (uint32_t)a.m;
   view.dist = a.dist;
   view.farbm = a.farbm;
   view.far = a.far;
+  view.far_cap = narrow::far_cap(a.n);
   view.delta = a.narrow_delta;
   view.adapt = a.narrow_adapt;
-  view.low_degree = a.low_degree;
+  view.lanes = a.lanes;
+  view.ahead = a.ahead;
   view.err = a.err;
   const uint32_t L0 = a.whole ? 0u : __ldcg(&a.summary->levels);
   view.tag = a.whole ? 0u : __ldcg(&a.summary->splits);
@@ -463,7 +479,7 @@ __global__ void __launch_bounds__(narrow::kBlock) sssp_narrow(Args a) {
   if (a.whole) {
     E.T = a.narrow_delta;
     if (E.rank == 0 && E.warp == 0)
-      E.push(E.lane == 0, a.src, __ldg(a.offs + a.src), __ldg(a.offs + a.src + 1), 0u);
+      E.push<true>(E.lane == 0, a.src, __ldg(a.offs + a.src), __ldg(a.offs + a.src + 1), 0u);
   } else {
     E.T = __ldcg(&a.ho->T);
     const uint32_t qc = __ldcg(&a.ho->qcount);
@@ -471,7 +487,7 @@ __global__ void __launch_bounds__(narrow::kBlock) sssp_narrow(Args a) {
       const uint32_t i = base + E.lane;
       const bool has = i < qc;
       const uint32_t v = has ? __ldcg(a.queue + i) : 0u;
-      E.push(has, v, has ? __ldg(a.offs + v) : 0u, has ? __ldg(a.offs + v + 1) : 0u,
+      E.push<true>(has, v, has ? __ldg(a.offs + v) : 0u, has ? __ldg(a.offs + v + 1) : 0u,
              has ? __ldcg(a.dist + v) : 0u);
     }
   }
@@ -562,7 +578,9 @@ int sssp_run(grus_graph *g, uint32_t src, uint32_t *dist, grus_stats *stats, cud
 
   a.ho = (Handover *)(w->ctrl + kOffHo);
   a.far = w->far;
-  a.low_degree = g->max_deg <= narrow::kLowDegree;
+  a.max_deg = g->max_deg;
+  a.lanes = narrow::lanes_per_entry(g->max_deg);
+  a.ahead = a.lanes && narrow::beyond_l2(g->n, g->m, 8);
   const int ncl = narrow_cluster();
   a.narrow_nf = tail ? kNarrowNf * (uint32_t)ncl : 0u;
   a.narrow_delta = std::max(1u, tune_or(g->tuning.sssp_delta, kNarrowDelta));

@@ -75,6 +75,27 @@ def test_sssp_narrow_shapes(grus, oracle_mod, name, n, pairs, weights, src):
     g.free()
 
 
+@pytest.mark.parametrize("name,n,pairs,weights,src", list(_cases()),
+                         ids=[c[0] for c in _cases()])
+def test_bfs_narrow_shapes(grus, oracle_mod, name, n, pairs, weights, src):
+    """The same shapes without weights: depths, reach counts and the level
+    count (one more than the largest depth), and the trace's vertices."""
+    offs, cols, _ = _csr(n, pairs, weights)
+    ref = oracle_mod.bfs(oracle_mod.CSR(offs, cols), src)
+    g = grus.Graph.from_csr(offs, cols, symmetric=True)
+    reached = ref != grus.INFINIT
+    for tail in (0, 2):
+        g.set_tuning(tail_cluster=tail)
+        got, st = grus.bfs(g, src, stats=True)
+        assert np.array_equal(got, ref), (name, tail)
+        assert st["levels"] == int(ref[reached].max()) + 1
+        assert st["vertices_reached"] == int(reached.sum())
+        assert st["edges_reached"] == int(np.diff(offs)[reached].sum())
+        for i, t in enumerate(grus.bfs_trace(g, 100)):
+            assert t["vertices"] == int((ref == i + 1).sum()), (name, tail, i)
+    g.free()
+
+
 @pytest.mark.parametrize("make", [
     lambda g: g.Graph.grid2d(400, 500, 5, weighted=True),    # handed over, 2^19 edges and more
     lambda g: g.Graph.grid2d(700, 31, 6, weighted=True),     # whole
@@ -82,7 +103,7 @@ def test_sssp_narrow_shapes(grus, oracle_mod, name, n, pairs, weights, src):
     lambda g: g.Graph.rmat(15, 8, 4, weighted=True),         # hubs, handed over near the end
     lambda g: g.Graph.rmat(13, 4, 4, weighted=True, symmetric=False),
 ])
-def test_sssp_narrow_matches_persistent(grus, make):
+def test_narrow_matches_persistent(grus, make):
     """The same distances with and without the cluster kernel, from several
     sources, synchronous and queued back to back on a stream."""
     torch = pytest.importorskip("torch")
@@ -103,4 +124,11 @@ def test_sssp_narrow_matches_persistent(grus, make):
         assert np.array_equal(got, ref)
         assert st["vertices_reached"] == rst["vertices_reached"]
         assert st["edges_reached"] == rst["edges_reached"]
+        b0, s0 = grus.bfs(g, s, stats=True)
+        g.set_tuning(tail_cluster=2)
+        b2, s2 = grus.bfs(g, s, stats=True)
+        g.set_tuning(tail_cluster=0)
+        assert np.array_equal(b0, b2)
+        for k in ("levels", "vertices_reached", "edges_reached"):
+            assert s0[k] == s2[k], k
     g.free()
