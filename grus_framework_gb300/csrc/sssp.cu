@@ -218,7 +218,7 @@ struct RelaxVisitor {
   const Args *a;
   uint32_t T;
   uint32_t *nnext;
-  unsigned long long visits;
+  uint32_t visits;  // of this thread in this level
 
   using aux_t = uint32_t;
 
@@ -389,16 +389,19 @@ __global__ void __launch_bounds__(kBlock, 8) sssp_persistent(Args a) {
       if (r == kHandedOver) return;
       if (threadIdx.x == 0) s_need = r;
     }
-    RelaxVisitor vis{&a, T, nnext, 0ull};
+    RelaxVisitor vis{&a, T, nnext, 0u};
     expand_binned<kBlock>(a.offs, a.queue, qc, a.chunks, cc, vis);
-    const unsigned long long bv = block_sum_u64<kBlock>(vis.visits);
-    if (threadIdx.x == 0 && bv) atomicAdd(&sl->visits, bv);
+    // counted for a caller that asked for statistics only
+    if (a.trace) {
+      const unsigned long long bv = block_sum_u64<kBlock>(vis.visits);
+      if (threadIdx.x == 0 && bv) atomicAdd(&sl->visits, bv);
+    }
     if (!grid_sync(a.bar, a.err, a.timeout_ns)) return;
-    const unsigned long long lv = __ldcg(&sl->visits);
     ++L;
-    if (gtid == 0) {
+    if (gtid == 0 && a.trace) {
+      const unsigned long long lv = __ldcg(&sl->visits);
       a.summary->visits += lv;
-      if (a.trace && L < (uint32_t)kMaxTrace)
+      if (L < (uint32_t)kMaxTrace)
         a.trace[L] = LevelTrace{global_timer_ns(), lv, qc + cc, splits};
     }
     if (L > 4u * a.n + 64u) {
