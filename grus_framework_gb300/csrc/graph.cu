@@ -873,7 +873,8 @@ namespace grus {
 // CTAs, with an L2 persisting access-policy window over [win_base, +win_bytes)
 // attached to this launch only (the caller's stream is left untouched).
 int launch_persistent(const void *fn, void **args, int block, int per_sm_req,
-                      int occupancy, cudaStream_t s, void *win_base, size_t win_bytes) {
+                      int occupancy, cudaStream_t s, void *win_base, size_t win_bytes,
+                      size_t smem, int ctas) {
   int per_sm = occupancy;
   if (per_sm_req > 0) per_sm = std::min(per_sm, per_sm_req);
   if (per_sm < 1) {
@@ -896,8 +897,10 @@ int launch_persistent(const void *fn, void **args, int block, int per_sm_req,
     ++nattr;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(device_sm_count() * per_sm));
+  const int most = device_sm_count() * per_sm;
+  cfg.gridDim = dim3((unsigned)(ctas > 0 ? std::min(ctas, most) : most));
   cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = attrs;
   cfg.numAttrs = nattr;

@@ -88,8 +88,10 @@ inline T tune_or(T v, T def) { return v ? v : def; }
 // Output buffers may be host or device memory; the call copies as needed.
 bool is_device_pointer(const void *p);
 
+// smem: dynamic shared memory per CTA; ctas: fewer CTAs than fit, if not 0.
 int launch_persistent(const void *fn, void **args, int block, int per_sm_req,
-                      int occupancy, cudaStream_t s, void *win_base, size_t win_bytes);
+                      int occupancy, cudaStream_t s, void *win_base, size_t win_bytes,
+                      size_t smem = 0, int ctas = 0);
 
 // Multi-source BFS (msbfs.cu): outs[i] (device memory, n entries) receives
 // the depths from hsrc[i] (host array), 1 <= k <= 64.  With stats the call

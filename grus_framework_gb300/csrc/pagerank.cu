@@ -13,15 +13,31 @@
 // Layout: in-edges (CSC) from grus_graph_build_csc; a contribution array
 // c(u) = r(u)/outdeg(u) double-buffered across iterations, so an iteration is
 // one fused pass: gather c over in-edges, form r, write c_next (and r on the
-// last iteration).  In-degree is binned:
-//   >= kCtaTh (1024) : cut into 2048-edge pieces, one CTA per piece, the
-//                      piece sums added in order afterwards
-//   >= kWarpTh (64) : one warp, loads four wide, shuffle reduction
-//   <  kWarpTh      : the warp's short lists laid end to end, one edge per
-//                      lane, segmented warp scan (every lane busy)
-// Per-thread partial sums over more than kKahanTh terms use compensated
-// (Kahan-Babuska) summation; reductions across lanes are pairwise trees.
-// The contribution arrays sit in an L2 persisting window.
+// last iteration).  Every warp takes an equal share of the edges and vertices
+// (an edge counts 1, a vertex kVertexCost), a contiguous range of the CSC that
+// may begin and end inside a vertex's list, whatever the degrees are; the
+// sums of a list that several warps share are added by the last of them to
+// finish, in order, so one grid barrier separates the iterations.
+//
+// Bound by the gathers.  L2 serves random 4-byte reads at 285 G/s at most,
+// whatever the array's size beyond a few MB, and far fewer where they meet on
+// few lines (148 G/s over 128 KB, 40 over 4 KB); shared memory serves several
+// times more.  So each SM keeps contributions in shared memory (kHot): all of
+// them on a small graph, else those of the kHotCap vertices of largest
+// out-degree, if they are the sources of a quarter of the edges.  For that the
+// graph's column ids are relabelled once (plan, kept with the workspace) to the
+// contributions' places: first the slots, then the other vertices with
+// out-edges, so that what L2 has to hold shrinks too.  With less L1 beside
+// them the gathers in flight no longer fit: RMAT-24 with 16,384 / 24,576 /
+// 32,768 / 40,960 slots 15.8 / 15.6 / 16.4 / 21 ms.
+//
+// 20 iterations, ms, before (a warp per 32 vertices, segmented scans, all
+// gathers from L2, two barriers an iteration) and now: RMAT-24 (263 M edges)
+// 23.0, 14.6 (360 G gathers/s); RMAT-20 1.70, 1.01; RMAT-16 0.588, 0.229;
+// uniform 3 M vertices of degree 16 (no plan) 5.33, 3.62 (265 G/s); 50,021 of
+// degree 12 0.567, 0.162.  Of that for RMAT-24: equal shares 23.0 -> 20.7, the
+// next batch's loads in flight during the sums -> 16.8, shorter chains between
+// them -> 15.6, no L2 window -> 15.0, compact places -> 14.6.
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -32,28 +48,35 @@ namespace grus {
 
 namespace {
 
-constexpr int kBlock = 256;
-constexpr uint32_t kCtaTh = 1024;   // in-degree from which a vertex is "heavy"
-constexpr uint32_t kHChunk = 2048;  // edges per heavy-vertex piece
-constexpr uint32_t kKahanTh = 16;
-constexpr uint32_t kWarpTh = 64;    // in-degree from which a list gets a warp of its own
-constexpr int kShortSteps = 2;      // short-list steps whose gathers are in flight together
+constexpr int kBlock = 1024;        // 1 CTA/SM
+constexpr int kBatch = 256;         // edges a warp gathers at once
+constexpr uint32_t kLongRun = 64;   // edges of one vertex in a batch that the warp adds
+constexpr uint32_t kCutMin = 64;    // lists below it are not shared by warps
+constexpr uint32_t kVertexCost = 4;  // in edges
+constexpr uint32_t kWarpCost = 128; // least work per warp before fewer CTAs are launched
+constexpr uint32_t kHotCap = 24576; // slots beside contributions gathered from L2
+constexpr uint32_t kHotAll = 48000; // vertices of a graph kept whole in shared memory
+constexpr uint32_t kNone = 0xFFFFFFFFu;  // no source: every id is smaller
+constexpr int kPlanIters = 3;       // fewer iterations do not repay a relabelling pass
 
 struct Args {
   const uint32_t *__restrict__ toffs;  // CSC offsets
   const uint32_t *__restrict__ tcols;  // CSC sources
   const uint32_t *__restrict__ offs;   // CSR offsets (out-degrees)
-  uint32_t n;
+  uint32_t n, m;
   float base, damping;
   int iters;
   float *c[2];
   float *rank;
-  // heavy vertices (in-degree >= kCtaTh): heavy[i] = (v, first piece, pieces),
-  // pieces[j] = (v, begin, end, i), partial[j] = sum over piece j
-  uint4 *heavy, *pieces;
-  float *partial;
-  uint32_t heavy_cap, piece_cap;
-  uint32_t *hcount;  // [0] heavy vertices, [1] pieces
+  // kHot: how many contributions shared memory holds; with a plan, that of
+  // vertex v is c[slot[v]], else (slot null) c[v]
+  uint32_t hot;
+  const uint32_t *__restrict__ slot;
+  // lists that several warps share: warp w's sum of its first one (head) and
+  // of its last one (tail), and the arrivals of the warps sharing w's last one
+  float *head, *tail;
+  uint32_t *arrived;
+  unsigned long long share;  // work per warp
   GridBarrier *bar;
   uint32_t *err;
   uint64_t timeout_ns;
@@ -76,232 +99,348 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-__device__ __forceinline__ float outdeg_inv(const Args &a, uint32_t v) {
-  const uint32_t d = __ldg(a.offs + v + 1) - __ldg(a.offs + v);
-  return d ? 1.0f / (float)d : 0.0f;
+// Where v's contribution goes; kNone: nowhere.
+template <bool kHot>
+__device__ __forceinline__ uint32_t place(const Args &a, uint32_t v) {
+  return kHot && a.slot ? __ldg(a.slot + v) : v;
 }
 
-__device__ __forceinline__ void finish(const Args &a, uint32_t v, float sum, float *cn, bool last) {
+// Writes to place p the contribution of a vertex of out-degree d for rank r.
+__device__ __forceinline__ void contribute(uint32_t p, uint32_t d, float r, float *cn) {
+  if (p != kNone) cn[p] = r * (d ? 1.0f / (float)d : 0.0f);
+}
+
+__device__ __forceinline__ uint32_t out_degree(const Args &a, uint32_t v) {
+  return __ldg(a.offs + v + 1) - __ldg(a.offs + v);
+}
+
+__device__ __forceinline__ void finish(const Args &a, uint32_t v, uint32_t p, uint32_t d, float sum,
+                                       float *cn, bool last) {
   const float r = a.base + a.damping * sum;
-  cn[v] = r * outdeg_inv(a, v);
+  contribute(p, d, r, cn);
   if (last) a.rank[v] = r;
 }
 
-// Strided gather of one list: four source ids, then their four
-// contributions, are loaded before they are added (four load chains in
-// flight per thread).
-__device__ __forceinline__ float gather_seq(const Args &a, const float *cs, uint32_t b,
-                                            uint32_t e, uint32_t step) {
-  if (b >= e) return 0.f;
-  const bool comp = (e - b) > kKahanTh * step;
-  KSum k;
-  float s = 0.f;
-  uint32_t x = b;
-  for (; x + 3 * step < e; x += 4 * step) {
-    const uint32_t u0 = __ldg(a.tcols + x), u1 = __ldg(a.tcols + x + step);
-    const uint32_t u2 = __ldg(a.tcols + x + 2 * step), u3 = __ldg(a.tcols + x + 3 * step);
-    const float f0 = __ldcg(cs + u0), f1 = __ldcg(cs + u1);
-    const float f2 = __ldcg(cs + u2), f3 = __ldcg(cs + u3);
-    if (comp) {
-      k.add(f0);
-      k.add(f1);
-      k.add(f2);
-      k.add(f3);
-    } else {
-      s += (f0 + f1) + (f2 + f3);
-    }
-  }
-  for (; x < e; x += step) {
-    const float f = __ldcg(cs + __ldg(a.tcols + x));
-    if (comp) k.add(f);
-    else s += f;
-  }
-  return comp ? k.value() : s;
+// A source id, read once per iteration: no line of L1 is kept for it.
+__device__ __forceinline__ uint32_t source_id(const uint32_t *p) {
+  uint32_t v;
+  asm("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
 }
 
-// The short lists (< kWarpTh in-edges) of a warp's vertices, laid end to end:
-// lane k of a step takes edge k of the concatenation (coalesced source-id
-// loads, every lane busy), a segmented warp scan sums each vertex's run
-// within the step (a fixed pairwise order), and the owning lane adds its
-// run's sum.  Steps go in rounds of kShortSteps: all their source ids, then
-// all their contributions, are loaded before any is summed (kShortSteps
-// gathers in flight per lane).  Returns the full sum for the calling lane's
-// vertex.
-__device__ __forceinline__ uint32_t short_owner(uint32_t incl, uint32_t k) {
-  int j = 0;
+template <bool kHot>
+__device__ __forceinline__ float fetch(const Args &a, const float *cs, const float *sc, uint32_t u) {
+  return kHot && u < a.hot ? sc[u] : __ldcg(cs + u);
+}
+
+// The work before vertex r, and the vertex whose work contains unit c: the
+// largest r with work_before(r) <= c (a 32-way search by the whole warp).
+__device__ __forceinline__ unsigned long long work_before(const Args &a, uint32_t r) {
+  return (unsigned long long)__ldg(a.toffs + r) + (unsigned long long)kVertexCost * r;
+}
+
+__device__ __forceinline__ uint32_t vertex_at(const Args &a, unsigned long long c) {
+  uint32_t lo = 0, hi = a.n + 1;
+  while (hi - lo > 1) {
+    const uint32_t step = (hi - lo + 31) / 32;
+    const uint32_t p = lo + lane_id() * step;
+    const bool below = p < hi && p >= lo && work_before(a, min(p, a.n)) <= c;
+    const uint32_t k = __popc(__ballot_sync(0xffffffffu, below));
+    lo += (k - 1) * step;
+    hi = min(hi, lo + step);
+  }
+  return lo;
+}
+
+// A warp's share: edges [e0, e1), vertices r0 .. r1 - 1 and, if its end cuts
+// r1's list (cut1), part of r1; cut0: its start cuts r0's list.
+struct Share {
+  uint32_t r0, r1, e0, e1;
+  bool cut0, cut1;
+};
+
+__device__ __forceinline__ void share_bound(const Args &a, unsigned long long c, uint32_t &r,
+                                            uint32_t &e, bool &cut) {
+  r = vertex_at(a, c);
+  e = a.m;
+  cut = false;
+  if (r >= a.n) return;
+  const uint32_t b = __ldg(a.toffs + r), end = __ldg(a.toffs + r + 1);
+  // a short list is not cut: the next warp takes all of it
+  e = end - b < kCutMin ? b
+                        : (uint32_t)min((unsigned long long)end, c - (unsigned long long)kVertexCost * r);
+  cut = e > b;
+}
+
+// The source ids of the batch from edge x on (up to edge e), and the
+// contributions of the sources; 0 past the end.
+__device__ __forceinline__ void load_ids(const Args &a, uint32_t x, uint32_t e,
+                                         uint32_t (&u)[kBatch / 32]) {
+  const uint32_t left = e > x ? e - x : 0u;
+  const uint32_t *p = a.tcols + x + lane_id();
 #pragma unroll
-  for (int step = 16; step >= 1; step >>= 1) {
-    const uint32_t pv = __shfl_sync(0xffffffffu, incl, j + step - 1);
-    if (pv <= k) j += step;
-  }
-  return (uint32_t)j;
+  for (int j = 0; j < kBatch / 32; ++j)
+    u[j] = lane_id() + 32 * j < left ? source_id(p + 32 * j) : kNone;
 }
 
-// Adds to acc the calling lane's run within the step starting at k0, whose
-// lane value is v (edge k0 + lane's contribution, 0 past the end).
-__device__ __forceinline__ void short_step(KSum &acc, uint32_t lane, uint32_t k0, uint32_t oe,
-                                           uint32_t excl, uint32_t incl, float v) {
-  bool head = lane == 0 || k0 + lane == oe;
+template <bool kHot>
+__device__ __forceinline__ void load_values(const Args &a, const float *cs, const float *sc,
+                                            const uint32_t (&u)[kBatch / 32],
+                                            float (&f)[kBatch / 32]) {
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const float tv = __shfl_up_sync(0xffffffffu, v, o);
-    const bool th = __shfl_up_sync(0xffffffffu, head, o);
-    if ((int)lane >= o && !head) {
-      v += tv;
-      head = th;
-    }
-  }
-  // this lane's run within the step ends at min(incl, k0 + 32) - 1
-  const uint32_t rs = max(excl, k0), re = min(incl, k0 + 32);
-  const float t = __shfl_sync(0xffffffffu, v, rs < re ? re - 1 - k0 : 0);
-  if (rs < re) acc.add(t);
+  for (int j = 0; j < kBatch / 32; ++j) f[j] = u[j] != kNone ? fetch<kHot>(a, cs, sc, u[j]) : 0.f;
 }
 
-__device__ __forceinline__ float gather_short(const Args &a, const float *cs, uint32_t beg,
-                                              uint32_t deg) {
+// One warp's share of an iteration.  The edges are taken in batches of kBatch:
+// all source ids, then all contributions of a batch are loaded (coalesced,
+// kBatch / 32 gathers in flight per lane) and put side by side in `sv`, from
+// where each lane adds the run of its vertex, four at a time, compensated; a
+// run of kLongRun or more is added by the whole warp.  Nothing has to find an
+// edge's owner: a search and a segmented scan over the lanes per 32 edges
+// cost more instructions than the rest.  u: the source ids of the first batch.
+template <bool kHot>
+__device__ __forceinline__ void run_share(const Args &a, const Share &sh, const float *cs,
+                                          const float *sc, float *sv, float *cn, bool last,
+                                          uint32_t gwarp, uint32_t (&u)[kBatch / 32]) {
   const uint32_t lane = lane_id();
-  uint32_t incl = deg;
+  const uint32_t rows = sh.r1 - sh.r0 + sh.cut1;  // vertices with work here
+  uint32_t x = sh.e0, lim = sh.e0;                // the batch [x, lim) is in sv
+  // in flight while a batch is summed: the contributions of the next one and
+  // the source ids of the one after it
+  float f[kBatch / 32];
+  load_values<kHot>(a, cs, sc, u, f);
+  load_ids(a, x + kBatch, sh.e1, u);
+  for (uint32_t w = 0; w < rows; w += 32) {
+    const uint32_t v = sh.r0 + w + lane;
+    const bool ok = w + lane < rows;
+    const uint32_t beg = ok ? max(__ldg(a.toffs + v), sh.e0) : sh.e1;
+    const uint32_t end = ok ? min(__ldg(a.toffs + v + 1), sh.e1) : sh.e1;
+    const uint32_t p = ok ? place<kHot>(a, v) : kNone;
+    const uint32_t od0 = ok ? __ldg(a.offs + v) : 0u, od1 = ok ? __ldg(a.offs + v + 1) : 0u;
+    const uint32_t stop = __shfl_sync(0xffffffffu, end, min(31u, rows - 1 - w));
+    KSum acc;
+    while (true) {
+      const uint32_t lo = max(beg, x), hi = min(end, lim);
+      uint32_t len = hi > lo ? hi - lo : 0u;
+      for (uint32_t lm = __ballot_sync(0xffffffffu, len >= kLongRun); lm; lm &= lm - 1) {
+        const int l = __ffs(lm) - 1;
+        const uint32_t at = __shfl_sync(0xffffffffu, lo, l) - x;
+        const uint32_t n = __shfl_sync(0xffffffffu, len, l);
+        KSum t;
+        for (uint32_t k = lane; k < n; k += 64)
+          t.add(sv[at + k] + (k + 32 < n ? sv[at + k + 32] : 0.f));
+        const float sum = warp_sum(t.value());
+        if ((int)lane == l) {
+          acc.add(sum);
+          len = 0u;
+        }
+      }
+      const float *run = sv + (lo - x);
+      for (uint32_t k = 0; k < len; k += 4) {
+        const float f0 = run[k], f1 = k + 1 < len ? run[k + 1] : 0.f;
+        const float f2 = k + 2 < len ? run[k + 2] : 0.f, f3 = k + 3 < len ? run[k + 3] : 0.f;
+        acc.add((f0 + f1) + (f2 + f3));
+      }
+      if (stop <= lim) break;  // these 32 vertices are complete
+      __syncwarp();
+      x = lim;
+      lim = min(sh.e1, x + kBatch);
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-    if ((int)lane >= o) incl += t;
-  }
-  const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-  const uint32_t excl = incl - deg;
-  KSum acc;
-  constexpr int P = kShortSteps;
-  for (uint32_t k0 = 0; k0 < total; k0 += 32 * P) {
-    uint32_t oe[P], u[P];
-    float v[P];
-#pragma unroll
-    for (int i = 0; i < P; ++i) {
-      const uint32_t k = k0 + 32 * i + lane;
-      const uint32_t j = short_owner(incl, k);
-      const uint32_t ob = __shfl_sync(0xffffffffu, beg, j);
-      oe[i] = __shfl_sync(0xffffffffu, excl, j);
-      u[i] = k < total ? __ldg(a.tcols + ob + (k - oe[i])) : 0u;
+      for (int j = 0; j < kBatch / 32; ++j) sv[lane + 32 * j] = f[j];
+      load_values<kHot>(a, cs, sc, u, f);
+      load_ids(a, x + 2 * kBatch, sh.e1, u);
+      __syncwarp();
     }
-#pragma unroll
-    for (int i = 0; i < P; ++i) v[i] = k0 + 32 * i + lane < total ? __ldcg(cs + u[i]) : 0.f;
-#pragma unroll
-    for (int i = 0; i < P; ++i)
-      if (k0 + 32 * i < total) short_step(acc, lane, k0 + 32 * i, oe[i], excl, incl, v[i]);
+    if (ok) {
+      const float sum = acc.value();
+      if (sh.cut0 && v == sh.r0) a.head[gwarp] = sum;
+      else if (sh.cut1 && v == sh.r1) a.tail[gwarp] = sum;
+      else finish(a, v, p, od1 - od0, sum, cn, last);
+    }
   }
-  return acc.value();
 }
 
-// One iteration is
-//   A. every warp, independently, takes groups of 32 consecutive vertices:
-//      in-lists of 32..kCtaTh-1 edges by the whole warp (four loads in
-//      flight), shorter ones laid end to end (gather_short); heavy vertices
-//      are skipped;
-//   B. every CTA takes pieces of kHChunk edges of the heavy vertices and
-//      writes each piece's sum;
-//   -- grid barrier --
-//   C. each heavy vertex adds its pieces in order (compensated) and finishes;
-//   -- grid barrier --
-// so no block barrier separates the warps of a light tile, and a heavy
-// vertex is spread over many CTAs.  The heavy lists are built once per call.
-__global__ void __launch_bounds__(kBlock, 8) pr_persistent(Args a) {
-  __shared__ float s_part[kBlock / 32];
+// This warp has written its sums of lists that it shares with others: its
+// first one (begun by warp f0, ended by l0) and its last one (ended by l1).
+// Of the warps sharing a list the last one to say so adds their sums in order.
+template <bool kHot>
+__device__ __forceinline__ void arrive(const Args &a, const Share &sh, uint32_t gwarp, uint32_t f0,
+                                       uint32_t l0, uint32_t l1, int it, float *cn, bool last) {
+  const uint32_t lane = lane_id();
+  const bool tail = sh.cut1 && !(sh.cut0 && sh.r0 == sh.r1);
+  __syncwarp();
+  bool all = false;  // lane 0: every sum of the first list is there; lane 1: of the last
+  if (lane < 2 && (lane ? tail : sh.cut0)) {
+    __threadfence();
+    const uint32_t sharers = lane ? l1 - gwarp + 1 : l0 - f0 + 1;
+    all = atomicAdd(a.arrived + (lane ? gwarp : f0), 1u) + 1u == sharers * (uint32_t)(it + 1);
+    __threadfence();
+  }
+  const uint32_t complete = __ballot_sync(0xffffffffu, all);
+  for (uint32_t which = 0; which < 2; ++which) {
+    if (!((complete >> which) & 1u)) continue;
+    const uint32_t f = which ? gwarp : f0, l = which ? l1 : l0;
+    KSum k;
+    for (uint32_t w = f + lane; w <= l; w += 32) k.add(__ldcg(w == f ? a.tail + w : a.head + w));
+    const float sum = warp_sum(k.value());
+    const uint32_t v = which ? sh.r1 : sh.r0;
+    if (lane == 0) finish(a, v, place<kHot>(a, v), out_degree(a, v), sum, cn, last);
+  }
+}
+
+template <bool kHot>
+__global__ void __launch_bounds__(kBlock, 1) pr_persistent(Args a) {
+  extern __shared__ __align__(16) float s_hot[];  // hot contributions, then batches
+  float *sv = s_hot + (kHot ? (a.hot + 31) / 32 * 32 : 0u) + (threadIdx.x >> 5) * kBatch;
   const uint32_t gtid = blockIdx.x * kBlock + threadIdx.x;
   const uint32_t nthreads = gridDim.x * kBlock;
-  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-  const uint32_t gwarp = gtid >> 5, nwarps = nthreads >> 5;
+  const uint32_t gwarp = gtid >> 5;
   const float r0 = 1.0f / (float)a.n;
-  for (uint32_t v = gtid; v < a.n; v += nthreads) {
-    a.c[0][v] = r0 * outdeg_inv(a, v);
-    const uint32_t b = __ldg(a.toffs + v), e = __ldg(a.toffs + v + 1);
-    if (e - b >= kCtaTh) {
-      const uint32_t np = (e - b + kHChunk - 1) / kHChunk;
-      const uint32_t hi = atomicAdd(&a.hcount[0], 1u);
-      const uint32_t p0 = atomicAdd(&a.hcount[1], np);
-      if (hi >= a.heavy_cap || p0 + np > a.piece_cap) {
-        atomicOr(a.err, kErrOverflow);
-        continue;
-      }
-      a.heavy[hi] = make_uint4(v, p0, np, 0u);
-      for (uint32_t k = 0; k < np; ++k)
-        a.pieces[p0 + k] = make_uint4(v, b + k * kHChunk, min(e, b + (k + 1) * kHChunk), hi);
-    }
+  for (uint32_t v = gtid; v < a.n; v += nthreads) 
+    contribute(place<kHot>(a, v), out_degree(a, v), r0, a.c[0]);
+  if (lane_id() == 0) a.arrived[gwarp] = 0u;
+  Share sh;
+  share_bound(a, gwarp * a.share, sh.r0, sh.e0, sh.cut0);
+  share_bound(a, (gwarp + 1) * a.share, sh.r1, sh.e1, sh.cut1);
+  // the warps sharing the first list and the last one
+  uint32_t f0 = 0, l0 = 0, l1 = 0;
+  if (sh.cut0) {
+    f0 = (uint32_t)(work_before(a, sh.r0) / a.share);
+    l0 = (uint32_t)((work_before(a, sh.r0 + 1) - 1) / a.share);
   }
+  if (sh.cut1) l1 = (uint32_t)((work_before(a, sh.r1 + 1) - 1) / a.share);
   if (!grid_sync(a.bar, a.err, a.timeout_ns)) return;
-  const uint32_t nheavy = min(__ldcg(&a.hcount[0]), a.heavy_cap);
-  const uint32_t npieces = min(__ldcg(&a.hcount[1]), a.piece_cap);
 
+  uint32_t u[kBatch / 32];
+  load_ids(a, sh.e0, sh.e1, u);
   for (int it = 0; it < a.iters; ++it) {
     const float *cs = a.c[it & 1];
     float *cn = a.c[(it + 1) & 1];
     const bool last = it + 1 == a.iters;
-    // A: light vertices, warp by warp
-    for (uint32_t g0 = gwarp * 32; g0 < a.n; g0 += nwarps * 32) {
-      const uint32_t v = g0 + lane;
-      uint32_t beg = 0, end = 0;
-      if (v < a.n) {
-        beg = __ldg(a.toffs + v);
-        end = __ldg(a.toffs + v + 1);
-      }
-      bool done = v >= a.n || end - beg >= kCtaTh;
-      while (true) {
-        const uint32_t ball = __ballot_sync(0xffffffffu, !done && end - beg >= kWarpTh);
-        if (!ball) break;
-        const int leader = __ffs(ball) - 1;
-        const uint32_t wv = __shfl_sync(0xffffffffu, v, leader);
-        const uint32_t wb = __shfl_sync(0xffffffffu, beg, leader);
-        const uint32_t we = __shfl_sync(0xffffffffu, end, leader);
-        if ((int)lane == leader) done = true;
-        const float tot = warp_sum(gather_seq(a, cs, wb + lane, we, 32));
-        if ((int)lane == leader) finish(a, wv, tot, cn, last);
-      }
-      const float sum = gather_short(a, cs, beg, done ? 0u : end - beg);
-      if (!done) finish(a, v, sum, cn, last);
-    }
-    // B: pieces of heavy vertices, CTA by CTA
-    for (uint32_t p = blockIdx.x; p < npieces; p += gridDim.x) {
-      const uint4 pc = __ldcg(a.pieces + p);
-      const float part = warp_sum(gather_seq(a, cs, pc.y + threadIdx.x, pc.z, kBlock));
-      if (lane == 0) s_part[warp] = part;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        float tot = 0.f;
-        for (int i = 0; i < kBlock / 32; ++i) tot += s_part[i];
-        a.partial[p] = tot;
-      }
+    if (kHot) {
+      const uint32_t quads = a.hot / 4;
+      for (uint32_t i = threadIdx.x; i < quads; i += kBlock)
+        reinterpret_cast<float4 *>(s_hot)[i] = __ldcg(reinterpret_cast<const float4 *>(cs) + i);
+      for (uint32_t i = 4 * quads + threadIdx.x; i < a.hot; i += kBlock) s_hot[i] = __ldcg(cs + i);
       __syncthreads();
     }
-    if (!grid_sync(a.bar, a.err, a.timeout_ns)) return;
-    // C: heavy vertices add their pieces in order
-    for (uint32_t h = gtid; h < nheavy; h += nthreads) {
-      const uint4 hv = __ldcg(a.heavy + h);
-      KSum k;
-      for (uint32_t j = 0; j < hv.z; ++j) k.add(__ldcg(a.partial + hv.y + j));
-      finish(a, hv.x, k.value(), cn, last);
-    }
-    if (!grid_sync(a.bar, a.err, a.timeout_ns)) return;
+    run_share<kHot>(a, sh, cs, s_hot, sv, cn, last, gwarp, u);
+    load_ids(a, sh.e0, sh.e1, u);  // of the next iteration, before the wait
+    if (sh.cut0 || sh.cut1) arrive<kHot>(a, sh, gwarp, f0, l0, l1, it, cn, last);
+    if (!last && !grid_sync(a.bar, a.err, a.timeout_ns)) return;
   }
 }
 
+// ---- plan: the vertices of largest out-degree and the relabelled columns ----
+constexpr uint32_t kBins = 1u << 16;  // out-degrees, the last bin open-ended
+
+__global__ void k_degree_bins(const uint32_t *__restrict__ offs, uint32_t n, uint32_t *bins) {
+  __shared__ uint32_t s_low[256];  // most vertices have few edges
+  s_low[threadIdx.x] = 0u;
+  __syncthreads();
+  for (uint32_t v = blockIdx.x * 256 + threadIdx.x; v < n; v += gridDim.x * 256) {
+    const uint32_t d = min(offs[v + 1] - offs[v], kBins - 1);
+    if (d < 256) atomicAdd(&s_low[d], 1u);
+    else atomicAdd(bins + d, 1u);
+  }
+  __syncthreads();
+  if (s_low[threadIdx.x]) atomicAdd(bins + threadIdx.x, s_low[threadIdx.x]);
+}
+
+struct PlanCtl {
+  uint32_t above, at, rest;     // slots given to degrees > cut, = cut, and to the others
+  uint32_t n_above, cut;
+  unsigned long long edges;     // at least this many edges leave the vertices with slots
+};
+
+// One CTA of 1024: the smallest degree that still gets slots.
+__global__ void k_plan_cut(const uint32_t *__restrict__ bins, PlanCtl *ctl) {
+  __shared__ unsigned long long s_cnt[1024], s_edges[1024];
+  constexpr uint32_t per = kBins / 1024;
+  const uint32_t t = threadIdx.x, hi = kBins - t * per;  // bins [hi - per, hi), from the top down
+  unsigned long long c = 0, e = 0;
+  for (uint32_t d = hi - per; d < hi; ++d) {
+    c += bins[d];
+    e += (unsigned long long)bins[d] * d;
+  }
+  s_cnt[t] = c;
+  s_edges[t] = e;
+  __syncthreads();
+  if (t == 0) {
+    unsigned long long above = 0, edges = 0;
+    uint32_t i = 0;
+    while (i < 1024 && above + s_cnt[i] <= kHotCap) {
+      above += s_cnt[i];
+      edges += s_edges[i];
+      ++i;
+    }
+    uint32_t d = kBins - i * per;  // the cut lies below d
+    while (d > 1 && above + bins[d - 1] <= kHotCap) {
+      --d;
+      above += bins[d];
+      edges += (unsigned long long)bins[d] * d;
+    }
+    // degree d - 1 fills what is left
+    ctl->n_above = (uint32_t)above;
+    ctl->cut = d - 1;
+    ctl->edges = edges + (kHotCap - above) * (unsigned long long)(d - 1);
+  }
+}
+
+// slot[v]: below kHotCap for the vertices of largest out-degree, from kHotCap
+// on for the others with out-edges (those of a block side by side, in order),
+// kNone for vertices without: nothing reads their contributions.
+__global__ void k_plan_slots(const uint32_t *__restrict__ offs, uint32_t n, PlanCtl *ctl,
+                             uint32_t *slot) {
+  __shared__ uint32_t s_base;
+  const uint32_t cut = ctl->cut, above = ctl->n_above;
+  for (uint32_t v0 = blockIdx.x * 256; v0 < n; v0 += gridDim.x * 256) {
+    const uint32_t v = v0 + threadIdx.x;
+    const uint32_t d = v < n ? offs[v + 1] - offs[v] : 0u;
+    uint32_t s = kNone;
+    if (min(d, kBins - 1) > cut) s = atomicAdd(&ctl->above, 1u);
+    else if (d && d == cut) s = above + atomicAdd(&ctl->at, 1u);
+    const bool rest = d && s >= kHotCap;
+    uint32_t total = 0;
+    const uint32_t at = block_exclusive_scan<256>(rest, &total);
+    if (threadIdx.x == 0) s_base = kHotCap + atomicAdd(&ctl->rest, total);
+    __syncthreads();
+    if (v < n) slot[v] = rest ? s_base + at : s;
+    __syncthreads();
+  }
+}
+
+__global__ void k_plan_cols(const uint32_t *__restrict__ tcols, uint64_t m,
+                            const uint32_t *__restrict__ slot, uint32_t *__restrict__ out) {
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m;
+       i += (uint64_t)gridDim.x * blockDim.x)
+    out[i] = __ldcg(slot + __ldcs(tcols + i));
+}
+
 struct Workspace {
-  float *c = nullptr;   // 2 * n contributions
+  float *c = nullptr;   // 2 * stride contributions
+  uint64_t stride = 0;
+  // plan (n > kHotAll): relabelled columns and slots, once asked for
+  bool planned = false;
+  uint32_t *cols = nullptr, *slot = nullptr;
   float *rank = nullptr;
-  uint4 *heavy = nullptr, *pieces = nullptr;
-  float *partial = nullptr;
-  uint32_t heavy_cap = 0, piece_cap = 0;
+  uint32_t *shared = nullptr;  // per warp: head, tail, arrivals
+  uint32_t warps = 0;
   char *ctrl = nullptr, *ctrl_host = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 };
 
-constexpr size_t kOffBar = 0, kOffErr = 256, kOffHeavy = 320, kCtrlBytes = 384;
+constexpr size_t kOffBar = 0, kOffErr = 256, kCtrlBytes = 384;
 static_assert(kOffBar + sizeof(GridBarrier) <= kOffErr, "barrier layout");
 
 void ws_free(void *p) {
   Workspace *w = (Workspace *)p;
   if (!w) return;
   cudaFree(w->c);
+  cudaFree(w->cols);
+  cudaFree(w->slot);
   cudaFree(w->rank);
-  cudaFree(w->heavy);
-  cudaFree(w->pieces);
-  cudaFree(w->partial);
+  cudaFree(w->shared);
   cudaFree(w->ctrl);
   if (w->ctrl_host) cudaFreeHost(w->ctrl_host);
   if (w->ev0) cudaEventDestroy(w->ev0);
@@ -316,12 +455,10 @@ int ws_get(grus_graph *g, Workspace **out) {
   }
   Workspace *w = new Workspace();
   const uint64_t n1 = std::max<uint64_t>(g->n, 1);
-  w->heavy_cap = (uint32_t)std::min<uint64_t>(n1, g->m / kCtaTh + 1);
-  w->piece_cap = (uint32_t)(g->m / kHChunk + w->heavy_cap + 1);
-  cudaError_t e = cudaMalloc(&w->c, 2 * n1 * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&w->heavy, (size_t)w->heavy_cap * sizeof(uint4));
-  if (e == cudaSuccess) e = cudaMalloc(&w->pieces, (size_t)w->piece_cap * sizeof(uint4));
-  if (e == cudaSuccess) e = cudaMalloc(&w->partial, (size_t)w->piece_cap * sizeof(float));
+  w->warps = (uint32_t)std::max(device_sm_count(), 1) * (kBlock / 32);
+  w->stride = (n1 + (n1 > kHotAll ? kHotCap : 0u) + 31) / 32 * 32;
+  cudaError_t e = cudaMalloc(&w->c, 2 * w->stride * 4);
+  if (e == cudaSuccess) e = cudaMalloc(&w->shared, (size_t)w->warps * 12);
   if (e == cudaSuccess) e = cudaMalloc(&w->ctrl, kCtrlBytes);
   if (e == cudaSuccess) e = cudaMemset(w->ctrl, 0, kCtrlBytes);
   if (e == cudaSuccess) e = cudaMallocHost(&w->ctrl_host, kCtrlBytes);
@@ -337,6 +474,76 @@ int ws_get(grus_graph *g, Workspace **out) {
   g->ws_free[kWsPr] = ws_free;
   *out = w;
   return GRUS_OK;
+}
+
+// The plan of a graph beyond kHotAll vertices, built on the first call with
+// enough iterations to repay it: a few passes over the vertices and one over
+// the columns (RMAT-24: 1.3 ms and 1.1 GB).  None on a managed graph, whose
+// columns may not fit the device, without room for it, or where the vertices
+// with slots would not be the sources of a quarter of the edges.
+void make_plan(grus_graph *g, Workspace *w, cudaStream_t s) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return;  // it waits for the stream: left to a call outside the capture
+  }
+  w->planned = true;
+  if (g->mem_mode == GRUS_MEM_MANAGED) return;
+  const uint32_t n = (uint32_t)g->n;
+  const int grid = std::max(device_sm_count(), 1) * 8;
+  uint32_t *bins = nullptr;
+  PlanCtl h{};
+  cudaError_t e = cudaMalloc(&bins, kBins * 4 + sizeof(PlanCtl));
+  PlanCtl *ctl = (PlanCtl *)(bins + kBins);
+  if (e == cudaSuccess) e = cudaMemsetAsync(bins, 0, kBins * 4 + sizeof(PlanCtl), s);
+  if (e == cudaSuccess) {
+    k_degree_bins<<<grid, 256, 0, s>>>(g->csr.offs, n, bins);
+    k_plan_cut<<<1, 1024, 0, s>>>(bins, ctl);
+    e = cudaMemcpyAsync(&h, ctl, sizeof(h), cudaMemcpyDeviceToHost, s);
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess && 4 * h.edges >= g->m) {
+    e = cudaMalloc(&w->slot, g->n * 4);
+    if (e == cudaSuccess) e = cudaMalloc(&w->cols, g->m * 4);
+    if (e == cudaSuccess) {
+      k_plan_slots<<<grid, 256, 0, s>>>(g->csr.offs, n, ctl, w->slot);
+      k_plan_cols<<<grid, 256, 0, s>>>(g->csc.cols, g->m, w->slot, w->cols);
+      e = cudaGetLastError();
+    }
+    // later calls may come on other streams
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  }
+  cudaFree(bins);
+  if (e != cudaSuccess) {  // no room: gather from L2
+    cudaGetLastError();
+    cudaFree(w->slot);
+    cudaFree(w->cols);
+    w->slot = w->cols = nullptr;
+  }
+}
+
+template <bool kHot>
+int launch(Workspace *w, Args &a, cudaStream_t s) {
+  static int occ = -1;
+  constexpr size_t batches = (size_t)(kBlock / 32) * kBatch * 4;
+  const size_t smem = batches + (kHot ? (size_t)(a.hot + 31) / 32 * 128 : 0);
+  if (occ < 0) {
+    constexpr size_t most = batches + (kHot ? (size_t)std::max(kHotAll, kHotCap) * 4 : 0);
+    GRUS_CUDA_TRY(cudaFuncSetAttribute(pr_persistent<kHot>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+    GRUS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pr_persistent<kHot>, kBlock, most));
+  }
+  // small graphs take fewer CTAs: the barrier of each iteration is cheaper
+  const uint64_t work = (uint64_t)a.m + (uint64_t)kVertexCost * a.n;
+  const int ctas = (int)std::min<uint64_t>(
+      (uint64_t)device_sm_count(), std::max<uint64_t>(1, work / (kWarpCost * (kBlock / 32))));
+  const uint64_t warps = (uint64_t)ctas * (kBlock / 32);
+  a.share = std::max<uint64_t>(1, (work + warps - 1) / warps);
+  void *args[] = {&a};
+  // no L2 persisting window on the contributions: RMAT-24 15.4 ms with one,
+  // 15.0 without
+  return launch_persistent((const void *)pr_persistent<kHot>, args, kBlock, 1, occ, s, nullptr, 0,
+                           smem, ctas);
 }
 
 }  // namespace
@@ -357,27 +564,31 @@ extern "C" int grus_pagerank(grus_graph *g, float damping, int iters, float *ran
   if (rc) return rc;
   const bool dev_out = is_device_pointer(rank);
   if (!dev_out && !w->rank) GRUS_CUDA_TRY(cudaMalloc(&w->rank, g->n * 4));
-  static int occ = -1;
-  if (occ < 0)
-    GRUS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pr_persistent, kBlock, 0));
+  if (g->n > kHotAll && iters >= kPlanIters && !w->planned) make_plan(g, w, s);
   Args a;
   std::memset(&a, 0, sizeof(a));
   a.toffs = g->csc.offs;
   a.tcols = g->csc.cols;
   a.offs = g->csr.offs;
   a.n = (uint32_t)g->n;
+  a.m = (uint32_t)g->m;
   a.base = (1.0f - damping) / (float)g->n;
   a.damping = damping;
   a.iters = iters;
   a.c[0] = w->c;
-  a.c[1] = w->c + g->n;
+  a.c[1] = w->c + w->stride;
+  const bool hot = g->n <= kHotAll || w->cols;
+  if (g->n <= kHotAll) {
+    a.hot = a.n;
+  } else if (w->cols) {
+    a.tcols = w->cols;
+    a.hot = kHotCap;
+    a.slot = w->slot;
+  }
   a.rank = dev_out ? rank : w->rank;
-  a.heavy = w->heavy;
-  a.pieces = w->pieces;
-  a.partial = w->partial;
-  a.heavy_cap = w->heavy_cap;
-  a.piece_cap = w->piece_cap;
-  a.hcount = (uint32_t *)(w->ctrl + kOffHeavy);
+  a.head = (float *)w->shared;
+  a.tail = a.head + w->warps;
+  a.arrived = w->shared + 2 * w->warps;
   a.bar = (GridBarrier *)(w->ctrl + kOffBar);
   a.err = (uint32_t *)(w->ctrl + kOffErr);
   a.timeout_ns = (uint64_t)tune_or(g->tuning.timeout_ms, 30000u) * 1000000ull;
@@ -388,13 +599,10 @@ extern "C" int grus_pagerank(grus_graph *g, float damping, int iters, float *ran
     GRUS_CUDA_TRY(cudaStreamSynchronize(s));
     return GRUS_OK;
   }
-  // barrier, error word and heavy-list counters: a timed-out launch leaves
-  // stale barrier state
-  GRUS_CUDA_TRY(cudaMemsetAsync(w->ctrl + kOffBar, 0, kOffHeavy + 8 - kOffBar, s));
+  // barrier and error word: a timed-out launch leaves stale barrier state
+  GRUS_CUDA_TRY(cudaMemsetAsync(w->ctrl + kOffBar, 0, kOffErr + 4 - kOffBar, s));
   if (stats) GRUS_CUDA_TRY(cudaEventRecord(w->ev0, s));
-  void *args[] = {&a};
-  rc = launch_persistent((const void *)pr_persistent, args, kBlock, (int)g->tuning.ctas_per_sm,
-                         occ, s, w->c, 2 * g->n * 4);
+  rc = hot ? launch<true>(w, a, s) : launch<false>(w, a, s);
   if (rc) return rc;
   if (stats) GRUS_CUDA_TRY(cudaEventRecord(w->ev1, s));
   if (!dev_out) GRUS_CUDA_TRY(cudaMemcpyAsync(rank, w->rank, g->n * 4, cudaMemcpyDeviceToHost, s));
