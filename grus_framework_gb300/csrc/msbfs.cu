@@ -33,6 +33,24 @@ namespace {
 
 constexpr int kBlock = 256;
 constexpr uint32_t kPullLane = 32;  // in-edges a lane scans alone in a pull level
+// A warp searching a long list has the gathers of kPullDeep 32-edge steps in
+// flight: one step at a time, a level waited for the warps with the longest
+// lists (RMAT-20, 16 sources: 832 us; 2 steps 592, 4 steps 565, 8 steps 553 but
+// 2 % slower at RMAT-16).
+constexpr int kPullDeep = 4;
+// Lists of kPullSplit edges or more are searched by one warp only as far as
+// kPullFirst; what has not found every live source by then is searched in
+// kChunk-edge pieces by all warps.  A hub that misses one source's bit is
+// searched to the end, and at RMAT-23 (64 sources) that took most of the level
+// after the sources' own: 8.6-13.0 ms whole for sources that such hubs miss,
+// 3.8-6.8 ms with pieces.  They cost a grid barrier and the hub's words again,
+// 20-30 us, so that shorter first searches lose on small graphs (kPullFirst of
+// 1 / 4 / 8 / 16 chunks, 64 sources: RMAT-16 284 / 262 / 251 / 250 us, RMAT-20
+// 684 / 708 / 726 / 725, RMAT-23 3,760 / 3,737 / 3,889 / 3,846).  A limit on
+// what a warp searches in all its lists together gains 1-3 % from RMAT-20 on
+// and loses 5-6 % at RMAT-16.
+constexpr uint32_t kPullFirst = 16 * kChunk;
+constexpr uint32_t kPullSplit = 2 * kPullFirst;
 constexpr uint32_t kDefHuge = 1024;
 // Pull once the frontier's out-edges exceed m / alpha.  A pull level scans
 // in-lists until every missing source bit is found, so it costs more the more
@@ -46,9 +64,9 @@ constexpr float kDefAlphaWide = 6.f;   // 33-64 sources
 struct Slot {
   uint32_t tcount;        // touched / frontier list length of the level
   uint32_t qcount, ccount;
-  uint32_t pad;
+  uint32_t dcount;        // pull: vertices whose long lists are searched in pieces
+  uint32_t pcount, pad;   // pull: the pieces
   unsigned long long mf;  // out-edges of the frontier
-  unsigned long long bits;
   unsigned long long live;  // sources present in the level's frontier words
 };
 
@@ -63,6 +81,7 @@ struct Args {
   const uint32_t *__restrict__ ioffs;
   const uint32_t *__restrict__ icols;
   bool allow_pull;
+  bool long_lists;  // some in-list may be searched in pieces
   uint32_t n;
   uint64_t m;
   int k;
@@ -173,6 +192,99 @@ struct PushVisitor {
   }
 };
 
+// The bits accumulated in acc for the `count` vertices of `list` enter visit,
+// the depths and the next frontier's lists; `tnext` (if given) takes the
+// vertices that have any.  The counts are this thread's share.
+__device__ __forceinline__ void apply_bits(const Args &a, const uint32_t *list, uint32_t count,
+                                           const unsigned long long *acc, uint32_t val,
+                                           uint32_t *tnext, uint32_t *qnext, uint4 *cnext, Slot *nx,
+                                           unsigned long long &mf,
+                                           unsigned long long &live) {
+  const uint32_t nthreads = gridDim.x * kBlock;
+  for (uint32_t i = blockIdx.x * kBlock + threadIdx.x; i < count; i += nthreads) {
+    const uint32_t u = __ldcg(list + i);
+    const unsigned long long bits = __ldcg(acc + u);
+    const unsigned long long had = __ldcg(a.visit + u);
+    if (!bits) continue;
+    a.visit[u] = had | bits;
+    record_depths(a, u, bits, had, val);
+    const uint32_t b = __ldg(a.offs + u), e = __ldg(a.offs + u + 1);
+    mf += e - b;
+    live |= bits;
+    if (tnext) {
+      const uint32_t pos = agg_reserve(&nx->tcount);
+      if (pos < a.cap) tnext[pos] = u;
+    }
+    if (!push_binned(u, b, e, a.huge, qnext, &nx->qcount, a.cap, cnext, &nx->ccount, a.chunk_cap))
+      atomicOr(a.err, kErrOverflow);
+  }
+}
+
+// The frontier bits among in-edges [b, e), by the whole warp, until `have` is
+// complete with them.
+__device__ __forceinline__ unsigned long long search_list(const Args &a,
+                                                          const unsigned long long *fcur, uint32_t b,
+                                                          uint32_t e, unsigned long long have) {
+  unsigned long long acc = 0;
+  const uint32_t lane = lane_id();
+  for (; b < e; b += 32 * kPullDeep) {
+    uint32_t c[kPullDeep];
+#pragma unroll
+    for (int j = 0; j < kPullDeep; ++j)
+      c[j] = b + 32 * j + lane < e ? __ldg(a.icols + b + 32 * j + lane) : 0xFFFFFFFFu;
+#pragma unroll
+    for (int j = 0; j < kPullDeep; ++j)
+      if (c[j] != 0xFFFFFFFFu) acc |= __ldcg(fcur + c[j]);
+    acc = warp_or64(acc);
+    if ((acc | have) == a.full) break;
+  }
+  return acc;
+}
+
+// A pull level's unfinished long lists.  Both functions are called by few
+// levels and stay out of line, away from the loop's 32 registers.
+//
+// In-edges [b, e) of u become pieces for any warp, in the level's own push
+// lists, which a pull level does not use.  More than a chunk of every such list
+// has been searched, so there are fewer than m / kChunk pieces.
+__device__ __noinline__ void put_pieces(const Args &a, uint32_t L, uint32_t u, uint32_t b, uint32_t e) {
+  Slot *nx = a.slots + ((L + 1) & 3u);
+  const uint32_t np = (e - b + kChunk - 1) / kChunk;
+  uint32_t pos = lane_id() == 0 ? atomicAdd(&nx->pcount, np) : 0u;
+  pos = __shfl_sync(0xffffffffu, pos, 0);
+  for (uint32_t k = lane_id(); k < np && pos + k < a.chunk_cap; k += 32)
+    a.chunks[L & 1u][pos + k] = make_uint4(u, b + k * kChunk, min(e, b + (k + 1) * kChunk), 0u);
+  if (lane_id() == 0) a.queue[L & 1u][atomicAdd(&nx->dcount, 1u)] = u;
+}
+
+// All warps search the pieces, then the vertices that have them enter the next
+// frontier.  False if the barrier gave up.
+__device__ __noinline__ bool pull_pieces(const Args &a, uint32_t L) {
+  const Slot *cur = a.slots + (L & 3u);
+  Slot *nx = a.slots + ((L + 1) & 3u);
+  const unsigned long long *fcur = a.front[L & 1u];
+  unsigned long long *acc = a.front[(L + 1) & 1u];
+  const uint4 *pieces = a.chunks[L & 1u];
+  const unsigned long long dead = a.full & ~__ldcg(&cur->live);
+  const uint32_t pc = min(__ldcg(&nx->pcount), a.chunk_cap);
+  const uint32_t nw = gridDim.x * kBlock / 32;
+  for (uint32_t i = (blockIdx.x * kBlock + threadIdx.x) / 32; i < pc; i += nw) {
+    const uint4 p = __ldcg(pieces + i);
+    const unsigned long long seen = __ldcg(a.visit + p.x);
+    const unsigned long long have = seen | dead | __ldcg(acc + p.x);
+    if (have == a.full) continue;
+    const unsigned long long found = search_list(a, fcur, p.y, p.z, have) & ~seen;
+    if (lane_id() == 0 && found) atomicOr(acc + p.x, found);
+  }
+  if (!grid_sync(a.bar, a.err, a.timeout_ns)) return false;
+  unsigned long long mf = 0, live = 0;
+  apply_bits(a, a.queue[L & 1u], min(__ldcg(&nx->dcount), a.cap), acc, L + 1, a.touched[(L + 1) & 1u],
+             a.queue[(L + 1) & 1u], a.chunks[(L + 1) & 1u], nx, mf, live);
+  if (mf) atomicAdd(&nx->mf, mf);
+  if (live) atomicOr(&nx->live, live);
+  return true;
+}
+
 __global__ void __launch_bounds__(kBlock, 8) msbfs_persistent(Args a) {
   const uint32_t gtid = blockIdx.x * kBlock + threadIdx.x;
   const uint32_t nthreads = gridDim.x * kBlock;
@@ -220,7 +332,7 @@ __global__ void __launch_bounds__(kBlock, 8) msbfs_persistent(Args a) {
     uint4 *cnext = a.chunks[(L + 1) & 1u];
     if (gtid < sizeof(Slot) / 4) ((uint32_t *)(a.slots + ((L + 2) & 3u)))[gtid] = 0u;
     const uint32_t val = L + 1;
-    unsigned long long mf = 0, nbits = 0, live = 0;
+    unsigned long long mf = 0, live = 0;
     if (!pull) {
       // phase A: push -- accumulate new bits of every touched vertex
       PushVisitor vis{&a, fcur, acc, tnext, &nx->tcount};
@@ -228,26 +340,8 @@ __global__ void __launch_bounds__(kBlock, 8) msbfs_persistent(Args a) {
                             a.chunks[L & 1u], min(__ldcg(&cur->ccount), a.chunk_cap), vis);
       if (!grid_sync(a.bar, a.err, a.timeout_ns)) return;
       // phase B: apply the accumulated bits (they exclude visit: exact)
-      const uint32_t tc = min(__ldcg(&nx->tcount), a.cap);
-      for (uint32_t base = gtid & ~31u; base < tc; base += nthreads) {
-        const uint32_t i = base + lane;
-        uint32_t u = 0;
-        unsigned long long bits = 0;
-        if (i < tc) {
-          u = __ldcg(tnext + i);
-          bits = __ldcg(acc + u);
-          const unsigned long long had = __ldcg(a.visit + u);
-          a.visit[u] = had | bits;
-          record_depths(a, u, bits, had, val);
-          const uint32_t b = __ldg(a.offs + u), e = __ldg(a.offs + u + 1);
-          mf += e - b;
-          nbits += __popcll(bits);
-          live |= bits;
-          if (!push_binned(u, b, e, a.huge, qnext, &nx->qcount, a.cap, cnext, &nx->ccount,
-                           a.chunk_cap))
-            atomicOr(a.err, kErrOverflow);
-        }
-      }
+      apply_bits(a, tnext, min(__ldcg(&nx->tcount), a.cap), acc, val, nullptr, qnext, cnext, nx, mf,
+                 live);
     } else {
       // phase A: pull -- every vertex missing bits ORs its in-neighbours'
       // frontier words.  Only sources present in those words can add a bit
@@ -255,9 +349,10 @@ __global__ void __launch_bounds__(kBlock, 8) msbfs_persistent(Args a) {
       // -- never will), so a vertex looks for the live sources it misses and
       // is skipped when it misses none.  A lane scans the first kPullLane in-edges of its
       // vertex (four gathers in flight) and stops once no bit is missing;
-      // longer lists still missing bits are finished by the whole warp, one
-      // vertex at a time, 32 edges per step, so a high-degree vertex costs
-      // its warp deg/32 steps instead of deg serial loads on one lane.
+      // longer lists still missing bits are searched by the whole warp, one
+      // vertex at a time, and the rest of very long ones by all warps in
+      // pieces, so a high-degree vertex costs neither its lane nor its warp
+      // its whole list.
       ++pull_levels;
       const unsigned long long lv = __ldcg(&cur->live);
       const uint32_t gw = gtid >> 5, nw = nthreads >> 5;
@@ -289,6 +384,7 @@ __global__ void __launch_bounds__(kBlock, 8) msbfs_persistent(Args a) {
             }
           }
         }
+        bool later = false;  // finished by pull_pieces
         unsigned dm = __ballot_sync(0xffffffffu, rest_e > rest_b);
         while (dm) {
           const int sl = __ffs(dm) - 1;
@@ -297,23 +393,25 @@ __global__ void __launch_bounds__(kBlock, 8) msbfs_persistent(Args a) {
           const uint32_t re = __shfl_sync(0xffffffffu, rest_e, sl);
           const unsigned long long have =
               __shfl_sync(0xffffffffu, accb | want, sl);
-          unsigned long long wacc = 0;
-          for (uint32_t base = rb; base < re; base += 32) {
-            const uint32_t x = base + lane;
-            if (x < re) wacc |= __ldcg(fcur + __ldg(a.icols + x));
-            if ((warp_or64(wacc) | have) == a.full) break;
-          }
-          wacc = warp_or64(wacc);
+          const bool split = re - rb >= kPullSplit;
+          const unsigned long long wacc =
+              search_list(a, fcur, rb, split ? rb + kPullFirst : re, have);
           if (lane == sl) accb |= wacc;
+          if (split && (wacc | have) != a.full) {
+            put_pieces(a, L, w * 32 + sl, rb + kPullFirst, re);
+            if (lane == sl) {
+              acc[u] = accb & ~vis;
+              later = true;
+            }
+          }
         }
-        if (u < a.n && want != a.full) {
+        if (u < a.n && want != a.full && !later) {
           bits = accb & ~vis;
           if (bits) {
             acc[u] = bits;
             a.visit[u] = vis | bits;
             const uint32_t ob = __ldg(a.offs + u), oe = __ldg(a.offs + u + 1);
             mf += oe - ob;
-            nbits += __popcll(bits);
             live |= bits;
             const uint32_t pos = agg_reserve(&nx->tcount);
             if (pos < a.cap) tnext[pos] = u;
@@ -329,20 +427,17 @@ __global__ void __launch_bounds__(kBlock, 8) msbfs_persistent(Args a) {
         }
       }
       if (!grid_sync(a.bar, a.err, a.timeout_ns)) return;
+      if (a.long_lists && __ldcg(&nx->pcount) && !pull_pieces(a, L)) return;
     }
     // phase B (both): retire the current frontier words so the array can
     // accumulate the level after next
     const uint32_t tcc = min(__ldcg(&cur->tcount), a.cap);
     for (uint32_t i = gtid; i < tcc; i += nthreads) fcur[__ldcg(tcur + i)] = 0ull;
     const unsigned long long bmf = block_sum_u64<kBlock>(mf);
-    const unsigned long long bnb = block_sum_u64<kBlock>(nbits);
     // OR of the bits that entered the next frontier: one reduction per warp
     for (int o = 16; o > 0; o >>= 1) live |= __shfl_xor_sync(0xffffffffu, live, o);
     if (lane == 0 && live) atomicOr(&nx->live, live);
-    if (threadIdx.x == 0 && (bmf || bnb)) {
-      atomicAdd(&nx->mf, bmf);
-      atomicAdd(&nx->bits, bnb);
-    }
+    if (threadIdx.x == 0 && bmf) atomicAdd(&nx->mf, bmf);
     if (!grid_sync(a.bar, a.err, a.timeout_ns)) return;
     ++L;
     const uint32_t T = __ldcg(&nx->tcount);
@@ -501,6 +596,7 @@ int msbfs_run(grus_graph *g, const uint32_t *hsrc, int k, uint32_t *const *outs,
   a.ioffs = (g->flags & GRUS_GRAPH_SYMMETRIC) ? g->csr.offs : g->csc.offs;
   a.icols = (g->flags & GRUS_GRAPH_SYMMETRIC) ? g->csr.cols : g->csc.cols;
   a.allow_pull = a.ioffs != nullptr;
+  a.long_lists = !(g->flags & GRUS_GRAPH_SYMMETRIC) || g->max_deg >= kPullLane + kPullSplit;
   a.n = (uint32_t)g->n;
   a.m = g->m;
   a.k = k;
