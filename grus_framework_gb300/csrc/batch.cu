@@ -323,6 +323,7 @@ __device__ void run_msssp(const Args &a, const Ctx &c, cg::cluster_group &cl, co
   v.minfar = ctl->far.minfar;
   v.err = &ctl->err;
   v.delta = a.delta;
+  v.lanes = ms::entry_lanes(g->n, g->m);
   ClusterSync sync{&cl};
   GroupOut out{a.out, a.moff + task.src};
   ms::Result r;

@@ -20,6 +20,9 @@ namespace {
 constexpr int kBlock = 256;
 constexpr uint32_t kDefDelta = 1024;
 constexpr int kMaxSources = 32;
+// CTAs an SM: what relax_pairs and relax_rows run best with.
+template <int KS>
+constexpr int kCtas = KS == 32 ? 8 : 6;
 using ms::kPiece;
 using ms::Slot;
 
@@ -49,7 +52,7 @@ struct OutTable {
 };
 
 template <int KS>
-__global__ void __launch_bounds__(kBlock, 8) msssp_persistent(Args a) {
+__global__ void __launch_bounds__(kBlock, kCtas<KS>) msssp_persistent(Args a) {
   const uint32_t gtid = blockIdx.x * kBlock + threadIdx.x;
   const uint32_t nthreads = gridDim.x * kBlock;
   GridSync sync{a.bar, a.v.err, a.timeout_ns};
@@ -58,14 +61,15 @@ __global__ void __launch_bounds__(kBlock, 8) msssp_persistent(Args a) {
   if (!ms::run<KS, kBlock>(a.v, gtid, nthreads, sync, out, r)) return;
   const unsigned long long bnr = block_sum_u64<kBlock>(r.nr);
   const unsigned long long bmr = block_sum_u64<kBlock>(r.mr);
+  const unsigned long long bv = block_sum_u64<kBlock>(r.visits);
   if (threadIdx.x == 0) {
+    atomicAdd(&a.summary->visits, bv);
     atomicAdd(&a.summary->nr, bnr);
     atomicAdd(&a.summary->mr, bmr);
   }
   if (gtid == 0) {
     a.summary->levels = r.levels;
     a.summary->splits = r.splits;
-    a.summary->visits = r.visits;
   }
 }
 
@@ -84,7 +88,7 @@ struct NoOut {
 };
 
 template <int KS>
-__global__ void __launch_bounds__(kBlock, 8) msssp_union(UnionArgs a) {
+__global__ void __launch_bounds__(kBlock, kCtas<KS>) msssp_union(UnionArgs a) {
   __shared__ uint32_t s_vb[ms::kMaxUnion + 1];
   for (uint32_t i = threadIdx.x; i <= a.v.ngraphs; i += kBlock)
     s_vb[i] = i < a.v.ngraphs ? a.v.ug[i].vbase : a.v.n;
@@ -96,14 +100,15 @@ __global__ void __launch_bounds__(kBlock, 8) msssp_union(UnionArgs a) {
   if (!ms::run<KS, kBlock, true>(a.v, gtid, nthreads, sync, NoOut{}, r, s_vb)) return;
   const unsigned long long bnr = block_sum_u64<kBlock>(r.nr);
   const unsigned long long bmr = block_sum_u64<kBlock>(r.mr);
+  const unsigned long long bv = block_sum_u64<kBlock>(r.visits);
   if (threadIdx.x == 0) {
+    atomicAdd(&a.summary->visits, bv);
     atomicAdd(&a.summary->nr, bnr);
     atomicAdd(&a.summary->mr, bmr);
   }
   if (gtid == 0) {
     a.summary->levels = r.levels;
     a.summary->splits = r.splits;
-    a.summary->visits = r.visits;
   }
 }
 
@@ -223,6 +228,8 @@ int msssp_run(grus_graph *g, const uint32_t *hsrc, int k, uint32_t *const *outs,
   a.v.minfar = (uint32_t *)(w->ctrl + kOffFar);
   a.v.err = (uint32_t *)(w->ctrl + kOffErr);
   a.v.delta = std::max(1u, tune_or(g->tuning.sssp_delta, kDefDelta));
+  a.v.lanes = ms::entry_lanes(g->n, g->m);
+  a.v.skewed = g->max_deg >= 4 * kPiece;
   for (int i = 0; i < k; ++i) a.out[i] = outs[i];
   a.bar = (GridBarrier *)(w->ctrl + kOffBar);
   a.summary = (Summary *)(w->ctrl + kOffSummary);
@@ -413,6 +420,8 @@ int msssp_union_run(void *wsp, int region, grus_graph *const *gs, int ng, const 
   a.v.minfar = (uint32_t *)(ctrl + kOffFar);
   a.v.err = (uint32_t *)(ctrl + kOffErr);
   a.v.delta = std::max(1u, delta ? delta : kDefDelta);
+  a.v.lanes = ms::entry_lanes(V, M);
+  for (int i = 0; i < ng; ++i) a.v.skewed |= gs[i]->max_deg >= 4 * kPiece;
   a.bar = (GridBarrier *)(ctrl + kOffBar);
   a.summary = (Summary *)(ctrl + kOffSummary);
   a.timeout_ns = 30000ull * 1000000ull;
