@@ -560,7 +560,8 @@ class Batch:
     `big_edges` edges run first as whole-GPU launches -- SSSP packs of up to
     32 sources per graph, several graphs' packs per launch while their
     distance rows total at most `launch_entries` entries -- and the rest on
-    cluster workers in one launch.  Zero arguments take the library
+    cluster workers in one launch; with the defaults, SSSP queries on smaller
+    graphs join the packs where that is estimated to be faster.  Zero arguments take the library
     defaults (grus_batch_config)."""
 
     def __init__(self, graphs, cluster_size=0, workers=0, huge_degree=0, sssp_delta=0,

@@ -18,7 +18,9 @@
 //          such groups.
 // Queries on graphs of at least big_edges edges do not go to the cluster
 // workers: a 16-CTA worker is a small slice of the GPU and such a query would
-// set the batch's critical path, so they run first as whole-GPU launches.
+// set the batch's critical path, so they run first as whole-GPU launches.  SSSP
+// queries on smaller graphs join them where that is estimated to be faster
+// (pack_small).
 // SSSP: up to 32 queries per graph form a pack, and the packs of up to 64
 // graphs share ONE multi-graph multi-source launch (msssp.cu), so the graphs'
 // levels overlap instead of following one another; BFS: up to 64 sources per
@@ -567,6 +569,7 @@ struct grus_batch {
   uint64_t big_edges = 1ull << 21;     // graphs served by whole-GPU launches
   uint64_t launch_entries = 1ull << 23;  // distance entries per multi-graph launch
   std::vector<uint8_t> big;            // per graph
+  bool adaptive = true;                // SSSP on small graphs may join the packs
   uint32_t *h_errs = nullptr;          // pinned error words of whole-GPU launches
   uint32_t err_cap = 0;
   void *uws = nullptr;                 // multi-graph SSSP launches' workspace
@@ -586,15 +589,21 @@ struct grus_batch {
 
 using namespace grus;
 
-// SSSP queries on big graphs (big_q sorted by graph), grouped into launches
-// by plan_union (union_plan.h): up to 32 per graph per pack, several graphs'
+// A launch of one small graph does not use the graph's own workspace, which
+// callers on other streams may be using: the batch's serves it too.
+static bool own_launch(const grus_batch *b, const std::vector<UnionPack> &l) {
+  return l.size() == 1 && b->big[l[0].graph];
+}
+
+// Plans the launches of big_q's SSSP queries (big_q sorted by graph) with
+// plan_union (union_plan.h): up to 32 per graph per pack, several graphs'
 // packs per multi-graph launch while their distance rows total at most
 // launch_entries.  The cap keeps a launch's distance rows in L2: 256 queries
 // over 32 RMAT graphs of scales 14-20 in one launch (368 MB of rows) took
-// 48.7 ms against 37 ms as one launch per graph.  Each launch's error word is
-// copied to h_errs.
-static int union_sssp(grus_batch *b, const grus_query *queries, const std::vector<int> &big_q,
-                      uint32_t *out, cudaStream_t s, uint32_t *nerr, uint32_t *nlaunch) {
+// 48.7 ms against 37 ms as one launch per graph.  Makes room for them.
+static int plan_sssp(grus_batch *b, const grus_query *queries, const std::vector<int> &big_q,
+                     UnionPlan *out) {
+  *out = UnionPlan();
   std::vector<int> sssp;
   for (int qi : big_q)
     if (queries[qi].algo == GRUS_ALGO_SSSP) sssp.push_back(qi);
@@ -606,18 +615,31 @@ static int union_sssp(grus_batch *b, const grus_query *queries, const std::vecto
     gn[g] = b->graphs[g]->n;
     gm[g] = b->graphs[g]->m;
   }
-  const UnionPlan plan =
+  UnionPlan plan =
       plan_union(sssp, qgraph, gn, gm, b->launch_entries, (size_t)ms::kMaxUnion, ms::kPiece);
+  for (const auto &l : plan.launches) {
+    if (l.size() > 1 || own_launch(b, l)) continue;
+    plan.max_v = std::max(plan.max_v, gn[l[0].graph]);
+    plan.max_m = std::max(plan.max_m, gm[l[0].graph]);
+    plan.max_ks = std::max(plan.max_ks, union_row_width(l[0].q.size()));
+    ++plan.unions;
+  }
   if (plan.unions) {
     int rc = msssp_union_reserve(&b->uws, plan.unions, plan.max_v, plan.max_m, plan.max_ks);
     if (rc) return rc;
   }
-  const auto &launches = plan.launches;
+  *out = std::move(plan);
+  return GRUS_OK;
+}
+
+// Queues the planned launches.  Each launch's error word is copied to h_errs.
+static int union_sssp(grus_batch *b, const grus_query *queries, const UnionPlan &plan,
+                      uint32_t *out, cudaStream_t s, uint32_t *nerr, uint32_t *nlaunch) {
   int region = 0;
-  for (const auto &l : launches) {
+  for (const auto &l : plan.launches) {
     CtrlView cv;
     int rc;
-    if (l.size() == 1) {
+    if (own_launch(b, l)) {
       const UnionPack &p = l[0];
       grus_graph *g = b->graphs[p.graph];
       if (p.q.size() == 1) {
@@ -685,6 +707,8 @@ int grus_batch_create(grus_graph *const *graphs, int ngraphs, const grus_batch_c
     b->max_m = std::max<uint64_t>(b->max_m, graphs[i]->m);
   }
   if (cfg) {
+    b->adaptive = !cfg->cluster_size && !cfg->workers && !cfg->sssp_delta && !cfg->group_sources &&
+                  !cfg->big_edges;
     if (cfg->cluster_size) b->cluster = (int)cfg->cluster_size;
     if (cfg->huge_degree) b->huge = cfg->huge_degree;
     if (cfg->sssp_delta) b->delta = cfg->sssp_delta;
@@ -862,6 +886,75 @@ static int stage_tasks(grus_batch *b, const grus_query *q, int nq) {
 }
 
 
+// Whether the SSSP queries on small graphs join the big graphs' multi-graph
+// launches, or form some, instead of going to the workers one by one.  A worker takes about
+// 200 us + 0.55 ns an edge for an SSSP query (RMAT-10 / 12 / 14 / 15 / 16: 240 /
+// 300 / 590 / 790 / 1,350 us) and some 0.6 of that for a BFS; a launch takes
+// about 250 us and, an edge, 0.02 ns + 0.01 ns for each source.  Both sides
+// measured, workers / launches: ten RMAT graphs of scales 10 to 14, a query
+// each 789 / 299 us, eight queries each 1,255 / 746; eight of scales 13 to 15,
+// eight queries each 1,437 / 529; but 16 uniform graphs of 2,000 vertices, two
+// queries each, 268 / 358, and 200 queries on one RMAT-12 2,205 / 2,455.  Graphs
+// without hubs stay with the workers, whose levels are cheaper (four 100 x 100
+// grids: 2,129 / 2,527).
+constexpr uint32_t kPackDeg = 9;
+
+static bool packable(const grus_batch *b, uint32_t gi) {
+  const grus_graph *g = b->graphs[gi];
+  return !b->big[gi] && g->max_deg >= kPackDeg && g->n * 8 <= b->launch_entries;
+}
+
+static bool pack_small(const grus_batch *b, const grus_query *q, int nq, cudaStream_t s) {
+  if (!b->adaptive) return false;
+  std::vector<uint32_t> k(b->graphs.size(), 0u);  // SSSP queries in packs, per graph
+  double all = 0.0, top = 0.0, rest = 0.0, rest_top = 0.0;  // the workers' time with and without
+  for (int i = 0; i < nq; ++i) {
+    const bool is_sssp = q[i].algo == GRUS_ALGO_SSSP, small = !b->big[q[i].graph];
+    const bool moves = is_sssp && packable(b, q[i].graph);
+    k[q[i].graph] += is_sssp && (!small || moves);
+    if (!small) continue;
+    const double c = (200.0 + 0.55e-3 * (double)b->graphs[q[i].graph]->m) * (is_sssp ? 1.0 : 0.6);
+    all += c;
+    top = std::max(top, c);
+    if (!moves) {
+      rest += c;
+      rest_top = std::max(rest_top, c);
+    }
+  }
+  // launches and edge work of the packs, of big graphs alone and of both
+  struct Load {
+    uint64_t rounds = 0, packs = 0, rows = 0;
+    double edges = 0.0;
+    void add(const grus_graph *g, uint32_t kq) {
+      const uint64_t p = (kq + kPackMax - 1) / kPackMax;
+      rounds = std::max(rounds, p);
+      packs += p;
+      rows += g->n * ((kq + 7) / 8 * 8);
+      edges += (double)g->m * (0.02e-3 * (double)p + 0.01e-3 * (double)kq);
+    }
+    double us(uint64_t cap) const {
+      if (!packs) return 0.0;
+      return 250.0 * (double)std::max({rounds, (packs + ms::kMaxUnion - 1) / ms::kMaxUnion,
+                                       rows / cap + 1}) + edges;
+    }
+  } bigs, both;
+  for (size_t g = 0; g < k.size(); ++g) {
+    if (!k[g]) continue;
+    if (b->big[g]) bigs.add(b->graphs[g], k[g]);
+    both.add(b->graphs[g], k[g]);
+  }
+  const double w = std::max(b->workers, 1);
+  if (both.packs == bigs.packs || both.us(b->launch_entries) - bigs.us(b->launch_entries) >=
+                                      std::max(top, all / w) - std::max(rest_top, rest / w))
+    return false;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return false;  // the launches' workspace may have to grow
+  }
+  return true;
+}
+
 int grus_batch_run(grus_batch *b, const grus_query *queries, int nq, uint32_t *out,
                    int use_graph, grus_stats *stats, void *stream) {
   if (!b || !queries || nq < 0 || !out) return GRUS_EINVAL;
@@ -885,9 +978,26 @@ int grus_batch_run(grus_batch *b, const grus_query *queries, int nq, uint32_t *o
   std::vector<grus_query> small_q;
   std::vector<int> big_q;
   small_q.reserve(nq);
-  for (int i = 0; i < nq; ++i) {
-    if (b->big[queries[i].graph]) big_q.push_back(i);
-    else small_q.push_back(queries[i]);
+  bool pack = pack_small(b, queries, nq, s);
+  UnionPlan plan;
+  while (true) {
+    for (int i = 0; i < nq; ++i) {
+      if (b->big[queries[i].graph] ||
+          (pack && queries[i].algo == GRUS_ALGO_SSSP && packable(b, queries[i].graph)))
+        big_q.push_back(i);
+      else
+        small_q.push_back(queries[i]);
+    }
+    std::stable_sort(big_q.begin(), big_q.end(), [&](int x, int y) {
+      if (queries[x].graph != queries[y].graph) return queries[x].graph < queries[y].graph;
+      return queries[x].algo < queries[y].algo;
+    });
+    const int prc = plan_sssp(b, queries, big_q, &plan);
+    if (!prc) break;
+    if (!pack) return prc;
+    pack = false;  // no room for the packs: the workers take them
+    big_q.clear();
+    small_q.clear();
   }
   int rc = GRUS_OK;
   if (!small_q.empty()) {
@@ -911,11 +1021,7 @@ int grus_batch_run(grus_batch *b, const grus_query *queries, int nq, uint32_t *o
       GRUS_CUDA_TRY(cudaMallocHost(&b->h_errs, big_q.size() * 4));
       b->err_cap = (uint32_t)big_q.size();
     }
-    std::stable_sort(big_q.begin(), big_q.end(), [&](int x, int y) {
-      if (queries[x].graph != queries[y].graph) return queries[x].graph < queries[y].graph;
-      return queries[x].algo < queries[y].algo;
-    });
-    rc = union_sssp(b, queries, big_q, out, s, &nerr, &nlaunch);
+    rc = union_sssp(b, queries, plan, out, s, &nerr, &nlaunch);
     if (rc) return rc;
     for (size_t i = 0; i < big_q.size();) {
       const grus_query &q0 = queries[big_q[i]];

@@ -330,7 +330,10 @@ typedef struct grus_batch_config {
                             workers start: SSSP packed up to 32 sources
                             per graph, BFS up to 64 per launch when enough
                             share a graph, else one launch each (default
-                            2^21; 0xFFFFFFFF: never) */
+                            2^21, where SSSP queries on smaller graphs are
+                            packed too if that is estimated to be faster
+                            and cluster_size, workers, sssp_delta and
+                            group_sources are 0; 0xFFFFFFFF: never) */
   uint32_t launch_entries;/* the SSSP packs of several of those graphs share
                             one launch while their distance rows (vertices
                             x 8/16/32 sources) total at most this many
