@@ -35,9 +35,10 @@ constexpr int kBlock = 256;
 constexpr uint32_t kPullLane = 32;  // in-edges a lane scans alone in a pull level
 // A warp searching a long list has the gathers of kPullDeep 32-edge steps in
 // flight: one step at a time, a level waited for the warps with the longest
-// lists (RMAT-20, 16 sources: 832 us; 2 steps 592, 4 steps 565, 8 steps 553 but
-// 2 % slower at RMAT-16).
-constexpr int kPullDeep = 4;
+// lists (RMAT-20, 16 sources: 832 us; 2 steps 592, 4 steps 565, 8 steps 553; at
+// four CTAs an SM 4 / 8 steps, 40 sources: RMAT-19 585 / 507, RMAT-22 2,451 /
+// 2,341).
+constexpr int kPullDeep = 8;
 // Lists of kPullSplit edges or more are searched by one warp only as far as
 // kPullFirst; what has not found every live source by then is searched in
 // kChunk-edge pieces by all warps.  A hub that misses one source's bit is
@@ -285,7 +286,10 @@ __device__ __noinline__ bool pull_pieces(const Args &a, uint32_t L) {
   return true;
 }
 
-__global__ void __launch_bounds__(kBlock, 8) msbfs_persistent(Args a) {
+// Four CTAs an SM: with eight the loop spills (32 registers) and every level
+// waits for twice the CTAs at its two barriers (64 sources: RMAT-23 3,858 ->
+// 3,682 us, RMAT-16 250 -> 176, uniform graph of 800 K vertices 750 -> 624).
+__global__ void __launch_bounds__(kBlock, 4) msbfs_persistent(Args a) {
   const uint32_t gtid = blockIdx.x * kBlock + threadIdx.x;
   const uint32_t nthreads = gridDim.x * kBlock;
   const uint32_t lane = lane_id();
@@ -563,6 +567,17 @@ int ws_get(grus_graph *g, Workspace **out) {
   return GRUS_OK;
 }
 
+// CTAs an SM, 0 for all that fit.  Small graphs' levels are mostly barrier: 16
+// sources at 1 / 2 / 3 / 4 CTAs, RMAT-13 102 / 106 / 114 / 116 us, uniform graph of
+// 150 K vertices 228 / 209 / 225 / 224, RMAT-18 238 / 224 / 220 / 236, uniform
+// graph of 800 K 610 / 444 / 443 / 463, RMAT-20 - / 545 / 490 / 496, RMAT-22 - /
+// 1,765 / 1,448 / 1,370.
+int grid_ctas(const grus_graph *g) {
+  if (g->tuning.ctas_per_sm) return (int)g->tuning.ctas_per_sm;
+  if (g->mem_mode == GRUS_MEM_MANAGED) return 0;
+  return g->n <= 1u << 15 ? 1 : (g->n <= 1u << 18 ? 2 : (g->n <= 1u << 20 ? 3 : 0));
+}
+
 }  // namespace
 
 int msbfs_run(grus_graph *g, const uint32_t *hsrc, int k, uint32_t *const *outs,
@@ -628,8 +643,7 @@ int msbfs_run(grus_graph *g, const uint32_t *hsrc, int k, uint32_t *const *outs,
   GRUS_CUDA_TRY(cudaMemsetAsync(w->ctrl + kOffBar, 0, kCtrlBytes - kOffBar, s));
   if (stats) GRUS_CUDA_TRY(cudaEventRecord(w->ev0, s));
   void *args[] = {&a};
-  rc = launch_persistent((const void *)msbfs_persistent, args, kBlock, (int)g->tuning.ctas_per_sm,
-                         occ, s, nullptr, 0);
+  rc = launch_persistent((const void *)msbfs_persistent, args, kBlock, grid_ctas(g), occ, s, nullptr, 0);
   if (rc) return rc;
   if (stats) GRUS_CUDA_TRY(cudaEventRecord(w->ev1, s));
   if (!stats) return GRUS_OK;
