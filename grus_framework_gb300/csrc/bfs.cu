@@ -64,7 +64,10 @@ constexpr float kDefAlpha = 15.f, kDefBeta = 18.f;
 // thread-block cluster of up to 16 CTAs.  The edge bound caps the work the
 // cluster may be left with.  (Handing over the last one or two levels of a
 // shorter traversal costs what it saves: RMAT scales 16-20 0.072 -> 0.078 and
-// 0.086 -> 0.092 ms.)
+// 0.086 -> 0.092 ms.)  The frontier must not be growing by more than an eighth:
+// a random graph of mean degree 2 still grows twofold at its 16th level, and the
+// cluster then ran its widest levels too (400 K vertices 713 us, 332 without;
+// 2 M vertices 1,004 / 529); a grid's grows by a sixteenth there, and less later.
 constexpr uint32_t kNarrowAfter = 16;
 constexpr uint32_t kNarrowNf = 1024;
 constexpr uint64_t kNarrowMu = 1ull << 26;
@@ -964,7 +967,8 @@ __global__ void __launch_bounds__(kBlock) bfs_persistent(Args a) {
       if ((double)NF * a.beta < (double)a.n && NF < prev_nf) nbu = false;
     }
     if (a.narrow_nf && !bu && !nbu && L + 1 >= kNarrowAfter && NF <= a.narrow_nf &&
-        MF <= 16ull * a.narrow_nf && mu <= kNarrowMu && __ldcg(&nx->ccount) == 0) {
+        8 * NF <= 9 * prev_nf && MF <= 16ull * a.narrow_nf && mu <= kNarrowMu &&
+        __ldcg(&nx->ccount) == 0) {
       // A long traversal down to a small push frontier: every further level
       // would be a grid barrier for a few thousand vertices.  Hand over to
       // bfs_narrow (launched after this kernel).  Vertices unreached so far
@@ -1121,6 +1125,23 @@ int narrow_cluster() {
   return c;
 }
 
+// CTAs an SM.  A level of a small graph is mostly its two barriers, which cost
+// more the more CTAs arrive (1 / 2 / 3 / 4 CTAs: RMAT-16 67 / 70 / 76 / 80 us,
+// uniform graph of 150 K vertices 137 / 150 / 159 / 170, RMAT-18 96 / 99 / 106 /
+// 113); larger ones need the gathers in flight, those without hubs earlier
+// (RMAT-20 129 / 115 / 117 / 122, RMAT-21 223 / 169 / 174 / 177; uniform graphs of
+// 400 K vertices 151 / 138 / 123 / 126, of 1.1 M 209 at 3 and 197 at 4, of 3 M
+// 735 / 486 / 431 / 408).  Without pull levels every edge is pushed, and the
+// smallest already need all (directed RMAT-17, 5 M edges: 434 at 1, 260 at 4).
+int grid_ctas(const grus_graph *g, bool pull, int occ) {
+  if (g->tuning.ctas_per_sm) return std::min<int>(occ, (int)g->tuning.ctas_per_sm);
+  if (!pull || g->mem_mode == GRUS_MEM_MANAGED) return occ;
+  if (g->n <= 1u << 17) return std::min(occ, 1);
+  if (g->n <= 1u << 18) return std::min(occ, 2);
+  if (g->max_deg >= kDefHuge) return g->n <= 1u << 21 ? std::min(occ, 2) : occ;
+  return g->n <= 3u << 18 ? std::min(occ, 3) : occ;
+}
+
 // Small graphs run in the cluster kernel altogether, unless the caller set a
 // knob of the persistent kernel.
 bool runs_whole(const grus_graph *g) {
@@ -1165,8 +1186,7 @@ int bfs_run(grus_graph *g, uint32_t src, uint32_t *depth, grus_stats *stats, cud
     GRUS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kBlock, 0));
   }
   const int sms = device_sm_count();
-  int per_sm = occ;
-  if (g->tuning.ctas_per_sm) per_sm = std::min<int>(per_sm, (int)g->tuning.ctas_per_sm);
+  const int per_sm = grid_ctas(g, (g->flags & GRUS_GRAPH_SYMMETRIC) || g->csc.offs, occ);
   if (per_sm < 1) {
     set_last_error("bfs kernel cannot be resident");
     return GRUS_ECUDA;

@@ -517,6 +517,19 @@ int narrow_cluster() {
   return c;
 }
 
+// CTAs an SM, 0 for all that fit (8).  Without hubs the levels are many and
+// small, and fewer CTAs pass their barriers sooner (uniform graphs, 2 / 4 / 5 / 6
+// / 8 CTAs: 1.2 M edges 472 / 479 / 494 / 511 / 538 us, 1.6 M 550 / 567 / 586 /
+// 616 / 681, 6.4 M 853 / 754 / 753 / 783 / 839, 9 M 835 / 769 / 761 / 804 / 858;
+// 32 M 3,144 / 2,103 / 1,922 / 1,839 / 1,782).  With hubs only the smallest gain
+// (RMAT-13 382 -> 364, 131 K vertices and 5.4 M edges 464 -> 444; RMAT-19 needs 8).
+int grid_ctas(const grus_graph *g) {
+  if (g->tuning.ctas_per_sm) return (int)g->tuning.ctas_per_sm;
+  if (g->mem_mode == GRUS_MEM_MANAGED) return 0;
+  if (g->max_deg >= 64) return g->n <= 1u << 17 ? 6 : 0;
+  return g->m <= 1u << 21 ? 2 : (g->m <= 5u << 22 ? 5 : 0);
+}
+
 bool runs_whole(const grus_graph *g) {
   return g->tuning.tail_cluster != 2 &&
          (g->m <= kWholeM || (g->m <= kWholeMLow && g->max_deg <= kWholeDegree));
@@ -600,7 +613,7 @@ int sssp_run(grus_graph *g, uint32_t src, uint32_t *dist, grus_stats *stats, cud
   // near/far bitmaps (small and hot enough to stay in L2 without it)
   if (!a.whole) {
     rc = launch_persistent((const void *)sssp_persistent, args, kBlock,
-                           (int)g->tuning.ctas_per_sm, occ, s, a.dist, (size_t)g->n * 4);
+                           grid_ctas(g), occ, s, a.dist, (size_t)g->n * 4);
     if (rc) return rc;
   }
   if (a.whole || a.narrow_nf) GRUS_CUDA_TRY(narrow::launch(sssp_narrow, ncl, a, s));
