@@ -199,9 +199,7 @@ void ws_free(void *p) {
   cudaFree(w->queues);
   cudaFree(w->chunks);
   cudaFree(w->ctrl);
-  cudaFree(w->trace);
   if (w->ctrl_host) cudaFreeHost(w->ctrl_host);
-  if (w->trace_host) cudaFreeHost(w->trace_host);
   if (w->ev0) cudaEventDestroy(w->ev0);
   if (w->ev1) cudaEventDestroy(w->ev1);
   delete w;
@@ -230,16 +228,24 @@ int ws_get(grus_graph *g, Workspace **out) {
   const uint64_t cap = g->m / kChunk + g->m / std::max(huge, 1u) + 2;
   w->chunk_cap = (uint32_t)std::min<uint64_t>(cap, 0x7FFFFFFFull);
   const size_t map_bytes = (5 + (with_planes ? (uint64_t)P : 0)) * Wp * 4;
-  cudaError_t e = cudaMalloc(&w->bitmaps, map_bytes + narrow::far_bytes(g->n));
+  cudaError_t e = cudaMalloc(&w->bitmaps, map_bytes + narrow::far_bytes(g->n, narrow::kFarCapUnit));
   if (e == cudaSuccess) w->far = (uint2 *)((char *)w->bitmaps + map_bytes);
   if (e == cudaSuccess && with_planes) w->planes = w->bitmaps + 5 * Wp;
   if (e == cudaSuccess) e = cudaMalloc(&w->queues, 2 * std::max<uint64_t>(g->n, 1) * 4);
   if (e == cudaSuccess) e = cudaMalloc(&w->chunks, 2ull * w->chunk_cap * sizeof(uint4));
-  if (e == cudaSuccess) e = cudaMalloc(&w->ctrl, kCtrlBytes);
+  // control block and trace, and their pinned mirrors, in one allocation each
+  // (a first call on a graph is mostly allocations)
+  static_assert(kCtrlBytes % alignof(LevelTrace) == 0, "the trace follows the control block");
+  constexpr size_t trace_bytes = kMaxTrace * sizeof(LevelTrace);
+  if (e == cudaSuccess) e = cudaMalloc(&w->ctrl, kCtrlBytes + trace_bytes);
   if (e == cudaSuccess) e = cudaMemset(w->ctrl, 0, kCtrlBytes);
-  if (e == cudaSuccess) e = cudaMallocHost(&w->ctrl_host, kCtrlBytes);
-  if (e == cudaSuccess) e = cudaMalloc(&w->trace, kMaxTrace * sizeof(LevelTrace));
-  if (e == cudaSuccess) e = cudaMallocHost(&w->trace_host, kMaxTrace * sizeof(LevelTrace));
+  if (e == cudaSuccess) e = cudaMallocHost(&w->ctrl_host, kCtrlBytes + trace_bytes);
+  if (e == cudaSuccess) {
+    w->trace = (LevelTrace *)(w->ctrl + kCtrlBytes);
+    w->trace_host = (LevelTrace *)(w->ctrl_host + kCtrlBytes);
+  }
+  // the clearing must be over before a launch on any stream
+  if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
   if (e == cudaSuccess) e = cudaEventCreate(&w->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&w->ev1);
   if (e != cudaSuccess) {
@@ -1056,7 +1062,7 @@ __global__ void __launch_bounds__(narrow::kBlock) bfs_narrow(Args a) {
   view.nearbm = a.front[0];
   view.farbm = a.front[1];
   view.far = a.far;
-  view.far_cap = narrow::far_cap(a.n);
+  view.far_cap = narrow::far_cap(a.n, narrow::kFarCapUnit);
   view.delta = narrow::kUnitDelta;
   view.adapt = false;
   view.lanes = a.lanes;

@@ -66,17 +66,21 @@ inline bool beyond_l2(uint64_t n, uint64_t m, uint32_t edge) {
 }
 constexpr int kRounds = 4;           // rounds between cluster barriers
 constexpr int kIlp = 2;              // 32-edge steps whose loads are in flight together
-constexpr uint32_t kFarCap = 4096;   // most far entries per CTA and buffer
+constexpr uint32_t kFarCap = 4096;   // most far entries per CTA and buffer, SSSP
+constexpr uint32_t kFarCapUnit = 1024;  // ... and BFS
 constexpr uint32_t kInf = 4294967294u;
 constexpr uint32_t kRing = 128;      // BFS: depth counts, by depth modulo kRing
 constexpr uint32_t kUnitDelta = 32;  // BFS: levels per threshold step (<= kRing / 2)
 
 // Far lists of one cluster (2 buffers per CTA) for a graph of n vertices;
-// small graphs get short ones, so that a first call's allocation stays small.
-__host__ __device__ inline uint32_t far_cap(uint64_t n) {
-  return n >= 8ull * kFarCap ? kFarCap : (n < 512 ? 64u : (uint32_t)(n / 8));
+// small graphs get short ones, so that a first call's allocation stays small,
+// and so does BFS, whose far vertices are those past one threshold's levels.
+__host__ __device__ inline uint32_t far_cap(uint64_t n, uint32_t most = kFarCap) {
+  return n >= 8ull * most ? most : (n < 512 ? 64u : (uint32_t)(n / 8));
 }
-inline size_t far_bytes(uint64_t n) { return (size_t)kMaxCluster * 2 * far_cap(n) * sizeof(uint2); }
+inline size_t far_bytes(uint64_t n, uint32_t most = kFarCap) {
+  return (size_t)kMaxCluster * 2 * far_cap(n, most) * sizeof(uint2);
+}
 
 // Per-step record (SSSP) or per-level record (BFS), the layout of the
 // persistent kernels' traces.

@@ -49,3 +49,37 @@ def test_packs(grus, kind, sssp, bfs):
     b.free()
     for g in gs:
         g.free()
+
+
+def test_big_bfs_side_by_side(grus):
+    """BFS queries on several big graphs, several on each, beside packs and
+    workers' tasks: two runs of one batch follow each other on the caller's
+    stream, and each output is complete when that stream reaches its copy."""
+    torch = pytest.importorskip("torch")
+    gs = [grus.Graph.rmat(17, 16, i, symmetric=True, weighted=True) for i in range(5)]
+    gs.append(grus.Graph.rmat(13, 8, 9, symmetric=True, weighted=True))
+    rng = np.random.default_rng(3)
+    b = grus.Batch(gs)
+    sets = []
+    for k in (1, 3):
+        q = [(i, grus.ALGO_BFS, int(rng.integers(g.n))) for i, g in enumerate(gs) for _ in range(k)]
+        q += [(i, grus.ALGO_SSSP, int(rng.integers(gs[i].n))) for i in (0, 5)]
+        sets.append([q[i] for i in rng.permutation(len(q))])
+    stream = torch.cuda.Stream()
+    copies = []
+    with torch.cuda.stream(stream):
+        for q in sets + sets:
+            offs, total = b.layout(q)
+            out = torch.full((total,), -7, dtype=torch.int32, device="cuda")
+            b.run(q, out, offs, use_graph=len(copies) % 2 == 1, stream=stream)
+            copies.append((q, offs, out.clone()))
+            out.fill_(-9)
+    stream.synchronize()
+    for q, offs, out in copies:
+        res = out.cpu().numpy().view(np.uint32)
+        for (gi, algo, src), o in zip(q, offs):
+            ref = (grus.sssp if algo == grus.ALGO_SSSP else grus.bfs)(gs[gi], src)
+            assert np.array_equal(res[o:o + len(ref)], ref), (gi, algo, src)
+    b.free()
+    for g in gs:
+        g.free()
