@@ -228,4 +228,43 @@ __device__ __forceinline__ void expand_binned(const uint32_t *__restrict__ offs,
   expand_binned<kBlock>(offs, qcur, qcount, ccur, ccount, vis, blockIdx.x, gridDim.x);
 }
 
+// expand_binned for a whole grid and large queues: the chunks are dealt, then
+// tiles are taken in turn from `taken` (zero at the start), the last two or so
+// per CTA in quarters with their entries spread over all warps.
+template <int kBlock, class Visitor>
+__device__ __forceinline__ void expand_taken(const uint32_t *__restrict__ offs,
+                                             const uint32_t *qcur, uint32_t qcount,
+                                             const uint4 *ccur, uint32_t ccount, Visitor &vis,
+                                             uint32_t *taken) {
+  if (qcount <= 2 * gridDim.x * kBlock) {
+    expand_binned<kBlock>(offs, qcur, qcount, ccur, ccount, vis);
+    return;
+  }
+  __shared__ uint32_t s_tile;
+  expand_chunks<kBlock>(ccur, ccount, vis, blockIdx.x, gridDim.x);
+  const uint32_t tiles = qcount / kBlock;
+  const uint32_t full = tiles > 2 * gridDim.x ? tiles - 2 * gridDim.x : 0u;
+  uint32_t next = 0;
+  if (threadIdx.x == 0) next = atomicAdd(taken, 1u);
+  while (true) {
+    if (threadIdx.x == 0) s_tile = next;
+    __syncthreads();
+    const uint32_t t = s_tile;
+    const uint32_t per = t < full ? 32u : 8u;  // entries a warp
+    const uint32_t base = t < full ? t * kBlock : full * kBlock + (t - full) * (kBlock / 4);
+    if (base >= qcount) break;
+    if (threadIdx.x == 0) next = atomicAdd(taken, 1u);  // on its way while the tile is expanded
+    const uint32_t i = base + threadIdx.x / 32 * per + lane_id();
+    uint32_t v = 0, beg = 0, end = 0;
+    typename Visitor::aux_t aux{};
+    if (lane_id() < per && i < qcount) {
+      v = __ldcg(qcur + i);
+      beg = __ldg(offs + v);
+      end = __ldg(offs + v + 1);
+      aux = vis.aux(v);
+    }
+    expand_tile<kBlock>(v, beg, end, aux, vis);  // a barrier of the CTA comes first in it
+  }
+}
+
 }  // namespace grus

@@ -69,7 +69,8 @@ constexpr uint32_t kWholeDegree = 64;
 struct Slot {
   uint32_t qcount, ccount;
   unsigned long long visits;  // edge relaxations attempted in the level
-  uint32_t pad[4];
+  uint32_t taken;             // tiles of the queue that CTAs have taken
+  uint32_t pad[3];
 };
 
 // Far-set control.  minfar is double-buffered by split parity so that the
@@ -285,6 +286,16 @@ __device__ __noinline__ uint32_t try_hand_over(const Args &a, uint32_t run, uint
   return kHandedOver;
 }
 
+// kTaken: the CTAs take large levels' tiles in turn.  Dealt in advance, the last
+// CTAs of a level with hubs finish 13-16 % after the mean (RMAT-22: 636 us
+// against 548 in the widest); taking costs barriers and registers, which graphs
+// with less work a level do not earn back (taken / dealt: RMAT-23 3,440 / 3,719
+// us, RMAT-22 1,701 / 1,785, RMAT-21 with 95 M edges 1,391 / 1,526, with 64 M
+// 1,348 / 1,325; uniform graph of 32 M edges 1,802 / 1,733, RMAT-18 481 / 473).
+constexpr uint64_t kTakenM = 1ull << 26;
+bool takes_tiles(const grus_graph *g) { return g->m >= kTakenM && g->max_deg >= kDefHuge; }
+
+template <bool kTaken>
 __global__ void __launch_bounds__(kBlock, 8) sssp_persistent(Args a) {
   // small levels in a row, and how many the next attempt to hand over needs
   // (in shared memory: the level loop has no register to spare at 8 CTAs/SM)
@@ -390,7 +401,8 @@ __global__ void __launch_bounds__(kBlock, 8) sssp_persistent(Args a) {
       if (threadIdx.x == 0) s_need = r;
     }
     RelaxVisitor vis{&a, T, nnext, 0u};
-    expand_binned<kBlock>(a.offs, a.queue, qc, a.chunks, cc, vis);
+    if constexpr (kTaken) expand_taken<kBlock>(a.offs, a.queue, qc, a.chunks, cc, vis, &sl->taken);
+    else expand_binned<kBlock>(a.offs, a.queue, qc, a.chunks, cc, vis);
     // counted for a caller that asked for statistics only
     if (a.trace) {
       const unsigned long long bv = block_sum_u64<kBlock>(vis.visits);
@@ -560,9 +572,11 @@ int sssp_run(grus_graph *g, uint32_t src, uint32_t *dist, grus_stats *stats, cud
   if (rc) return rc;
   const bool dev_out = is_device_pointer(dist);
   if (!dev_out && !w->dist) GRUS_CUDA_TRY(cudaMalloc(&w->dist, g->n * 4));
-  static int occ = -1;
-  if (occ < 0)
-    GRUS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sssp_persistent, kBlock, 0));
+  const bool taken = takes_tiles(g);
+  auto kern = taken ? sssp_persistent<true> : sssp_persistent<false>;
+  static int occ_tab[2] = {-1, -1};
+  int &occ = occ_tab[taken];
+  if (occ < 0) GRUS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kBlock, 0));
 
   Args a;
   std::memset(&a, 0, sizeof(a));
@@ -612,7 +626,7 @@ int sssp_run(grus_graph *g, uint32_t src, uint32_t *dist, grus_stats *stats, cud
   // with an atomic: RMAT-22 1.99 -> 1.80-1.83 ms against the window on the
   // near/far bitmaps (small and hot enough to stay in L2 without it)
   if (!a.whole) {
-    rc = launch_persistent((const void *)sssp_persistent, args, kBlock,
+    rc = launch_persistent((const void *)kern, args, kBlock,
                            grid_ctas(g), occ, s, a.dist, (size_t)g->n * 4);
     if (rc) return rc;
   }
