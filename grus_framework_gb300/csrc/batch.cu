@@ -959,13 +959,13 @@ static bool pack_small(const grus_batch *b, const grus_query *q, int nq, cudaStr
   return true;
 }
 
-// The streams of a run's BFS launches on big graphs: those of one graph, which
-// share its workspace, follow one another, those of different graphs run side
-// by side (a BFS of a mid-sized graph takes one or two CTAs an SM and waits at
+// The streams of a run's single BFS launches on mid-sized graphs (bfs_side_ok):
+// those of one graph, which share its workspace, follow one another, those of
+// different graphs run side by side with one CTA an SM each (such a BFS waits at
 // barriers most of its time; 8 graphs of scales 16 to 19, one query each: 667 us
-// one by one, 387 / 264 / 230 on 2 / 4 / 8 streams; the same with two queries each
-// in a batch 2,074 -> 1,021 us).  They start after what the caller's stream holds,
-// and it waits for all of them.  Under capture everything stays on that stream.
+// one by one, 387 / 264 on 2 / 4 streams).  They start after what the caller's
+// stream holds, and it waits for all of them.  Under capture everything stays on
+// that stream.
 struct Sides {
   grus_batch *b;
   cudaStream_t s;
@@ -974,19 +974,23 @@ struct Sides {
   uint32_t last = 0xFFFFFFFFu;
 
   Sides(grus_batch *batch, cudaStream_t stream) : b(batch), s(stream) {}
-  int begin(const grus_query *q, const std::vector<int> &big_q) {
+  // Whether the run has launches for them, given which queries are singles.
+  bool wanted(const grus_query *q, const std::vector<int> &singles) const {
     uint32_t graphs = 0, prev = 0xFFFFFFFFu;
-    for (int qi : big_q) {
-      if (q[qi].algo == GRUS_ALGO_SSSP || q[qi].graph == prev) continue;
+    for (int qi : singles) {
+      if (q[qi].graph == prev || !bfs_side_ok(b->graphs[q[qi].graph])) continue;
       prev = q[qi].graph;
       ++graphs;
     }
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (graphs < 2) return GRUS_OK;
+    if (graphs < 2) return false;
     if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
       cudaGetLastError();
-      return GRUS_OK;
+      return false;
     }
+    return true;
+  }
+  int begin() {
     if (!b->fork) GRUS_CUDA_TRY(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
     GRUS_CUDA_TRY(cudaEventRecord(b->fork, s));
     for (int i = 0; i < grus_batch::kSide; ++i) {
@@ -998,7 +1002,6 @@ struct Sides {
     return GRUS_OK;
   }
   cudaStream_t of(uint32_t graph) {
-    if (!on) return s;
     if (graph != last) next = (next + 1) % grus_batch::kSide;
     last = graph;
     return b->side[next];
@@ -1085,54 +1088,62 @@ int grus_batch_run(grus_batch *b, const grus_query *queries, int nq, uint32_t *o
     }
     rc = union_sssp(b, queries, plan, out, s, &nerr, &nlaunch);
     if (rc) return rc;
-    rc = sides.begin(queries, big_q);
-    if (rc) return rc;
+    // the error word of a launch, to its place in h_errs
+    auto save_err = [&](const CtrlView &cv, cudaStream_t ls) -> int {
+      if (!cv.ctrl) return GRUS_OK;
+      GRUS_CUDA_TRY(cudaMemcpyAsync(b->h_errs + nerr, cv.ctrl + cv.err_off, 4, cudaMemcpyDeviceToHost, ls));
+      GRUS_CUDA_TRY(cudaMemsetAsync(cv.ctrl + cv.err_off, 0, 4, ls));
+      ++nerr;
+      return GRUS_OK;
+    };
+    // BFS queries of a graph run alone unless enough share the graph
+    std::vector<int> singles;
     for (size_t i = 0; i < big_q.size();) {
       const grus_query &q0 = queries[big_q[i]];
+      size_t j = i + 1;
       if (q0.algo == GRUS_ALGO_SSSP) {  // launched by union_sssp
-        ++i;
+        i = j;
         continue;
       }
       grus_graph *g = b->graphs[q0.graph];
-      const cudaStream_t ls = sides.of(q0.graph);
-      size_t j = i + 1;
-      const size_t cap = q0.algo == GRUS_ALGO_SSSP ? 32 : 64;
-      while (j < big_q.size() && j - i < cap && queries[big_q[j]].graph == q0.graph &&
+      while (j < big_q.size() && j - i < 64 && queries[big_q[j]].graph == q0.graph &&
              queries[big_q[j]].algo == q0.algo)
         ++j;
-      // BFS queries of a graph run alone unless enough share the graph
-      if (q0.algo != GRUS_ALGO_SSSP && j - i < bfs_pack_min(g->m)) j = i + 1;
-      CtrlView cv;
-      if (j - i == 1) {
-        rc = q0.algo == GRUS_ALGO_SSSP ? grus_sssp(g, q0.src, out + q0.out_offset, nullptr, ls)
-                                       : bfs_run(g, q0.src, out + q0.out_offset, nullptr, ls, false);
-        // a single BFS is the persistent kernel and its narrow-tail kernel
-        nlaunch += q0.algo == GRUS_ALGO_SSSP ? 1 : 2;
-        cv = q0.algo == GRUS_ALGO_SSSP ? sssp_ctrl(g) : bfs_ctrl(g);
-      } else {
-        uint32_t srcs[64];
-        uint32_t *outs[64];
-        for (size_t k = i; k < j; ++k) {
-          srcs[k - i] = queries[big_q[k]].src;
-          outs[k - i] = out + queries[big_q[k]].out_offset;
-        }
-        ++nlaunch;
-        if (q0.algo == GRUS_ALGO_SSSP) {
-          rc = msssp_run(g, srcs, (int)(j - i), outs, nullptr, ls);
-          cv = msssp_ctrl(g);
-        } else {
-          rc = msbfs_run(g, srcs, (int)(j - i), outs, nullptr, ls);
-          cv = msbfs_ctrl(g);
-        }
+      if (j - i == 1 || j - i < bfs_pack_min(g->m)) {
+        singles.push_back(big_q[i]);
+        ++i;
+        continue;
       }
+      uint32_t srcs[64];
+      uint32_t *outs[64];
+      for (size_t k = i; k < j; ++k) {
+        srcs[k - i] = queries[big_q[k]].src;
+        outs[k - i] = out + queries[big_q[k]].out_offset;
+      }
+      ++nlaunch;
+      rc = msbfs_run(g, srcs, (int)(j - i), outs, nullptr, s);
+      if (!rc) rc = save_err(msbfs_ctrl(g), s);
       if (rc) return rc;
-      if (cv.ctrl) {
-        GRUS_CUDA_TRY(cudaMemcpyAsync(b->h_errs + nerr, cv.ctrl + cv.err_off, 4,
-                                      cudaMemcpyDeviceToHost, ls));
-        GRUS_CUDA_TRY(cudaMemsetAsync(cv.ctrl + cv.err_off, 0, 4, ls));
-        ++nerr;
-      }
       i = j;
+    }
+    // the singles: whole-GPU launches first, then those that run side by side
+    const bool beside = sides.wanted(queries, singles);
+    for (int pass = 0; pass < 2; ++pass) {
+      if (pass == 1) {
+        if (!beside) break;
+        rc = sides.begin();
+        if (rc) return rc;
+      }
+      for (int qi : singles) {
+        grus_graph *g = b->graphs[queries[qi].graph];
+        const bool side = beside && bfs_side_ok(g);
+        if (side != (pass == 1)) continue;
+        const cudaStream_t ls = side ? sides.of(queries[qi].graph) : s;
+        nlaunch += 2;  // the persistent kernel and its narrow-tail kernel
+        rc = bfs_run(g, queries[qi].src, out + queries[qi].out_offset, nullptr, ls, false, side);
+        if (!rc) rc = save_err(bfs_ctrl(g), ls);
+        if (rc) return rc;
+      }
     }
   }
   if (nt == 0) {

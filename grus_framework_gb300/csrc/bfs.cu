@@ -1164,8 +1164,13 @@ using namespace grus;
 
 namespace grus {
 
+bool bfs_side_ok(const grus_graph *g) {
+  return !g->tuning.ctas_per_sm && g->mem_mode != GRUS_MEM_MANAGED && g->n <= 1u << 21 &&
+         ((g->flags & GRUS_GRAPH_SYMMETRIC) || g->csc.offs);
+}
+
 int bfs_run(grus_graph *g, uint32_t src, uint32_t *depth, grus_stats *stats, cudaStream_t s,
-            bool whole_ok) {
+            bool whole_ok, bool side) {
   if (!g || !depth) return GRUS_EINVAL;
   if (g->n == 0 || src >= g->n) {
     set_last_error("source vertex out of range");
@@ -1192,7 +1197,8 @@ int bfs_run(grus_graph *g, uint32_t src, uint32_t *depth, grus_stats *stats, cud
     GRUS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kBlock, 0));
   }
   const int sms = device_sm_count();
-  const int per_sm = grid_ctas(g, (g->flags & GRUS_GRAPH_SYMMETRIC) || g->csc.offs, occ);
+  int per_sm = grid_ctas(g, (g->flags & GRUS_GRAPH_SYMMETRIC) || g->csc.offs, occ);
+  if (side) per_sm = std::min(per_sm, 1);
   if (per_sm < 1) {
     set_last_error("bfs kernel cannot be resident");
     return GRUS_ECUDA;

@@ -104,9 +104,13 @@ int msssp_run(grus_graph *g, const uint32_t *hsrc, int k, uint32_t *const *outs,
 
 // Single-source BFS (bfs.cu): two kernels, or one where whole_ok and the graph
 // is small.  grus_bfs allows it; the batch and the server, whose small graphs
-// run on cluster workers anyway, keep the two.
+// run on cluster workers anyway, keep the two.  side: with one CTA an SM, to run
+// beside up to three like it; four of them fit the GPU whatever the order in
+// which their CTAs start, so none waits at a barrier for CTAs that find no room.
 int bfs_run(grus_graph *g, uint32_t src, uint32_t *depth, grus_stats *stats, cudaStream_t s,
-            bool whole_ok);
+            bool whole_ok, bool side = false);
+// Graphs whose BFS loses little by a side launch.
+bool bfs_side_ok(const grus_graph *g);
 // Single-source SSSP (sssp.cu).  tail: launch the cluster kernel behind the
 // persistent one (2 kernels, else 1); grus_sssp does where sssp_tail says so.
 // The batch and the server, whose lanes queue launches back to back, do on
