@@ -384,15 +384,6 @@ struct PushVisitor {
   }
 };
 
-__device__ __forceinline__ void enqueue_binned(const Args &a, uint32_t v,
-                                               uint32_t *qnext, uint4 *cnext,
-                                               LevelSlot *nx) {
-  const uint32_t b = __ldg(a.offs + v), e = __ldg(a.offs + v + 1);
-  if (!push_binned(v, b, e, a.huge, qnext, &nx->qcount, a.queue_cap, cnext, &nx->ccount,
-                   a.chunk_cap))
-    atomicOr(a.err, kErrOverflow);
-}
-
 // ---------------------------------------------------------------------------
 // pull level
 // ---------------------------------------------------------------------------
