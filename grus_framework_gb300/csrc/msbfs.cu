@@ -255,7 +255,11 @@ __device__ __noinline__ void put_pieces(const Args &a, uint32_t L, uint32_t u, u
   pos = __shfl_sync(0xffffffffu, pos, 0);
   for (uint32_t k = lane_id(); k < np && pos + k < a.chunk_cap; k += 32)
     a.chunks[L & 1u][pos + k] = make_uint4(u, b + k * kChunk, min(e, b + (k + 1) * kChunk), 0u);
-  if (lane_id() == 0) a.queue[L & 1u][atomicAdd(&nx->dcount, 1u)] = u;
+  if (lane_id() == 0) {
+    if (pos + np > a.chunk_cap) atomicOr(a.err, kErrOverflow);
+    const uint32_t at = atomicAdd(&nx->dcount, 1u);
+    if (at < a.cap) a.queue[L & 1u][at] = u;
+  }
 }
 
 // All warps search the pieces, then the vertices that have them enter the next
