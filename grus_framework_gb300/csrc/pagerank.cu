@@ -58,6 +58,11 @@ constexpr uint32_t kHotCap = 24576; // slots beside contributions gathered from 
 constexpr uint32_t kHotAll = 48000; // vertices of a graph kept whole in shared memory
 constexpr uint32_t kNone = 0xFFFFFFFFu;  // no source: every id is smaller
 constexpr int kPlanIters = 3;       // fewer iterations do not repay a relabelling pass
+// Edges from which the first call makes the plan; below, the second one does: the
+// plan takes 100-200 us, which 20 iterations on a smaller graph do not repay
+// (first / later calls with it 744 / 403 us at RMAT-18, without 643 / 527; RMAT-19
+// 1,026 / 621 and 985 / 828; RMAT-20 1,511 / 1,045 and 1,624 / 1,446).
+constexpr uint64_t kPlanNow = 3ull << 22;
 
 struct Args {
   const uint32_t *__restrict__ toffs;  // CSC offsets
@@ -422,6 +427,7 @@ struct Workspace {
   uint64_t stride = 0;
   // plan (n > kHotAll): relabelled columns and slots, once asked for
   bool planned = false;
+  bool ranked = false;  // a call that the plan is for has been made
   uint32_t *cols = nullptr, *slot = nullptr;
   float *rank = nullptr;
   uint32_t *shared = nullptr;  // per warp: head, tail, arrivals
@@ -476,8 +482,8 @@ int ws_get(grus_graph *g, Workspace **out) {
   return GRUS_OK;
 }
 
-// The plan of a graph beyond kHotAll vertices, built on the first call with
-// enough iterations to repay it: a few passes over the vertices and one over
+// The plan of a graph beyond kHotAll vertices, built on the first call (kPlanNow
+// edges and more) or the second with enough iterations to repay it: a few passes over the vertices and one over
 // the columns (RMAT-24: 1.3 ms and 1.1 GB).  None on a managed graph, whose
 // columns may not fit the device, without room for it, or where the vertices
 // with slots would not be the sources of a quarter of the edges.
@@ -564,7 +570,12 @@ extern "C" int grus_pagerank(grus_graph *g, float damping, int iters, float *ran
   if (rc) return rc;
   const bool dev_out = is_device_pointer(rank);
   if (!dev_out && !w->rank) GRUS_CUDA_TRY(cudaMalloc(&w->rank, g->n * 4));
-  if (g->n > kHotAll && iters >= kPlanIters && !w->planned) make_plan(g, w, s);
+  // a plan needs a quarter of the edges at kHotCap sources
+  if (g->n > kHotAll && iters >= kPlanIters && !w->planned &&
+      4ull * kHotCap * g->max_deg >= g->m) {
+    if (w->ranked || g->m >= kPlanNow) make_plan(g, w, s);
+    w->ranked = true;
+  }
   Args a;
   std::memset(&a, 0, sizeof(a));
   a.toffs = g->csc.offs;
