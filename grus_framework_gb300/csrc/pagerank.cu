@@ -112,7 +112,7 @@ __device__ __forceinline__ uint32_t place(const Args &a, uint32_t v) {
 
 // Writes to place p the contribution of a vertex of out-degree d for rank r.
 __device__ __forceinline__ void contribute(uint32_t p, uint32_t d, float r, float *cn) {
-  if (p != kNone) cn[p] = r * (d ? 1.0f / (float)d : 0.0f);
+  if (p != kNone) cn[p] = d ? r / (float)d : 0.0f;  // one rounding
 }
 
 __device__ __forceinline__ uint32_t out_degree(const Args &a, uint32_t v) {
