@@ -69,7 +69,7 @@ def build(verbose: bool = False, extra_flags: list[str] | None = None) -> Path:
     OUT.mkdir(exist_ok=True)
     OBJ.mkdir(exist_ok=True)
     cc = nvcc()
-    headers = list(CSRC.glob("*.cuh")) + list((ROOT / "include").glob("*.h"))
+    headers = list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + list((ROOT / "include").glob("*.h"))
     jobs = []
     objs = []
     for src in SOURCES:

@@ -40,6 +40,7 @@
 #include <cooperative_groups.h>
 
 #include "device_util.cuh"
+#include "narrow_steps.h"
 
 namespace grus {
 namespace narrow {
@@ -129,11 +130,11 @@ struct Shared {
   // the last step in which this CTA pushed to an inbox, spilled to the near
   // bitmap, put bits in the far bitmap (0: never), ...
   uint32_t pushed, spilled, farbm;
-  // ... and rank 0: the last step in which any CTA had work left or spilled,
-  // and the last that put bits in the far bitmap
-  uint32_t g_farbm;
-  uint2 g_work;
-  uint32_t g_far;                       // ... and had far vertices
+  // ... and rank 0: what the cluster found, by step parity, the last step that
+  // put bits in the far bitmap and the last that had far vertices (both read
+  // where no CTA can be past the step that wrote them)
+  StepWords found[2];
+  uint32_t g_farbm, g_far;
   // this CTA's copies: far bitmap bits up to this step have been taken; the
   // last threshold step and its size
   uint32_t scanned, last_split, delta;
@@ -180,7 +181,7 @@ struct Engine {
     if (threadIdx.x < kRing) s->ring[threadIdx.x] = s->ring_sum[threadIdx.x] = 0;
     if (threadIdx.x == 0) {
       s->pushed = s->spilled = s->farbm = s->g_farbm = 0u;
-      s->g_work = make_uint2(0u, 0u);
+      s->found[0] = s->found[1] = StepWords{0u, 0u};
       s->g_far = 0u;
       s->scanned = s->last_split = 0u;
       s->delta = a.delta;
@@ -561,21 +562,19 @@ struct Engine {
   // readers; true if any CTA has near work.
   __device__ __forceinline__ bool end_step(bool &spilled) {
     if (threadIdx.x == 0) {
-      // stamps only grow, so nobody clears them: a CTA already in the next
-      // step got there because this step had work, which every CTA saw
       Shared *r = cl.map_shared_rank(s, 0);
-      if (s->cnt[cq] || s->pushed == step) *(volatile uint32_t *)&r->g_work.x = step;
-      if (s->spilled == step) *(volatile uint32_t *)&r->g_work.y = step;
+      volatile StepWords *w = &words_of(r->found, step);
+      if (s->cnt[cq] || s->pushed == step) w->work = step;
+      if (s->spilled == step) w->spilled = step;
       if (s->farbm == step) *(volatile uint32_t *)&r->g_farbm = step;
       if (s->farcnt[fb]) *(volatile uint32_t *)&r->g_far = step;
     }
     cl.sync();
-    const Shared *r = cl.map_shared_rank(s, 0);
-    const uint32_t gw = *(const volatile uint32_t *)&r->g_work.x;
-    const uint32_t gs = *(const volatile uint32_t *)&r->g_work.y;
-    spilled = gs >= step;
+    const volatile StepWords *w = &words_of(cl.map_shared_rank(s, 0)->found, step);
+    spilled = found(w->spilled, step);
+    const bool work = found(w->work, step);
     ++step;
-    return gw >= step - 1 || spilled;
+    return work || spilled;
   }
 
   __device__ __forceinline__ void next_round() {

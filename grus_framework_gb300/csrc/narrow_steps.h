@@ -1,0 +1,37 @@
+// narrow_steps.h -- the words by which the CTAs of narrow.cuh's cluster agree
+// on what a step found.  Plain code without CUDA types, so that the host can
+// run it too.
+//
+// Every thread of the cluster decides for itself from these words which
+// barrier it goes to next, so a word must read the same to all of them, however
+// late a thread comes to read it.
+#pragma once
+
+#include <stdint.h>
+
+#ifdef __CUDACC__
+#define GRUS_HD __host__ __device__ __forceinline__
+#else
+#define GRUS_HD inline
+#endif
+
+namespace grus {
+namespace narrow {
+
+// What a step found, kept by step parity.  Before the cluster barrier that ends
+// a step, CTAs write the step's number into its words; after the barrier every
+// thread reads them.  A CTA that has read them may run ahead and write the next
+// step's before another thread reads this step's -- which are others -- but not
+// those of the step after that: its barrier in between waits for that thread.
+// A word holds an older step's number until it is written, so nobody clears it.
+struct StepWords {
+  uint32_t work;     // some CTA has near work left
+  uint32_t spilled;  // some list was full: vertices wait in the near bitmap
+};
+
+GRUS_HD bool found(uint32_t word, uint32_t step) { return word == step; }
+
+GRUS_HD StepWords &words_of(StepWords (&w)[2], uint32_t step) { return w[step & 1u]; }
+
+}  // namespace narrow
+}  // namespace grus

@@ -1,0 +1,62 @@
+"""CPU: the words by which the one-cluster kernel's threads agree on what comes
+next (grus_framework_gb300/csrc/narrow_steps.h), compiled with g++.  A thread
+may read them late, when other CTAs are already a step ahead or other warps are
+already pushing: what it reads must not depend on that, or threads of one block
+go to different barriers."""
+import subprocess
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parents[1]
+DRIVER = r"""
+#include <cstdio>
+#include <cstring>
+#include <initializer_list>
+#include "narrow_steps.h"
+using namespace grus::narrow;
+static int fail(const char *what, unsigned step) {
+  printf("%s at step %u\n", what, step);
+  return 1;
+}
+// A fast CTA is past step `step` and has written the words of step + 1 (which
+// it may do before a slow thread reads those of `step`).
+int late_reads() {
+  for (unsigned history = 0; history < 64; ++history) {
+    StepWords w[2] = {{0u, 0u}, {0u, 0u}};
+    for (unsigned step = 1; step <= 6; ++step) {
+      const bool sp = history >> (step - 1) & 1u, work = step % 3 != 0;
+      if (sp) words_of(w, step).spilled = step;
+      if (work) words_of(w, step).work = step;
+      StepWords ahead[2];
+      memcpy(ahead, w, sizeof(w));
+      words_of(ahead, step + 1).spilled = step + 1;
+      words_of(ahead, step + 1).work = step + 1;
+      for (const StepWords *v : {&words_of(w, step), &words_of(ahead, step)}) {
+        if (found(v->spilled, step) != sp) return fail("spilled", step);
+        if (found(v->work, step) != work) return fail("work", step);
+      }
+    }
+  }
+  return 0;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def driver(tmp_path_factory):
+    d = tmp_path_factory.mktemp("steps")
+    (d / "steps.cpp").write_text(DRIVER + """
+int main(int argc, char **argv) {
+  return argc > 1 && !strcmp(argv[1], "late_reads") ? late_reads() : 2;
+}
+""")
+    exe = d / "steps"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", str(ROOT / "grus_framework_gb300" / "csrc"),
+                    str(d / "steps.cpp"), "-o", str(exe)], check=True)
+    return exe
+
+
+def test_step_words_read_late(driver):
+    r = subprocess.run([str(driver), "late_reads"], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
