@@ -65,7 +65,6 @@ inline uint32_t lanes_per_entry(uint32_t max_degree) {
 inline bool beyond_l2(uint64_t n, uint64_t m, uint32_t edge) {
   return 8 * n + edge * m > (96ull << 20);
 }
-constexpr int kRounds = 4;           // rounds between cluster barriers
 constexpr int kIlp = 2;              // 32-edge steps whose loads are in flight together
 constexpr uint32_t kFarCap = 4096;   // most far entries per CTA and buffer, SSSP
 constexpr uint32_t kFarCapUnit = 1024;  // ... and BFS
@@ -126,7 +125,7 @@ struct Shared {
   uint4 inb[2][kCap];
   uint32_t cnt[3];                      // local list lengths, rotating by round
   uint32_t incnt[2], farcnt[2];
-  uint32_t away[2];                     // entries pushed to other CTAs, by step parity
+  AwayCounts away;                      // entries pushed to other CTAs
   // the last step in which this CTA pushed to an inbox, spilled to the near
   // bitmap, put bits in the far bitmap (0: never), ...
   uint32_t pushed, spilled, farbm;
@@ -161,6 +160,7 @@ struct Engine {
   uint32_t scale;             // home of v: umulhi(v, scale)
   uint32_t T, step;           // steps count from 1 (0 = never)
   uint32_t cq, lb, fb;        // read: cnt[cq], loc[lb], far buffer fb
+  int round;                  // of the step, 0 before its first
   Result res;
 
   __device__ __forceinline__ Engine(const View &view, Shared *sh)
@@ -175,9 +175,10 @@ struct Engine {
     T = 0;
     step = 1;
     cq = lb = fb = 0;
+    round = 0;
     if (threadIdx.x < 3) s->cnt[threadIdx.x] = 0u;
-    if (threadIdx.x < 2)
-      s->incnt[threadIdx.x] = s->farcnt[threadIdx.x] = s->away[threadIdx.x] = 0u;
+    if (threadIdx.x < 2) s->incnt[threadIdx.x] = s->farcnt[threadIdx.x] = 0u;
+    if (threadIdx.x < kRounds) s->away.n[0][threadIdx.x] = s->away.n[1][threadIdx.x] = 0u;
     if (threadIdx.x < kRing) s->ring[threadIdx.x] = s->ring_sum[threadIdx.x] = 0;
     if (threadIdx.x == 0) {
       s->pushed = s->spilled = s->farbm = s->g_farbm = 0u;
@@ -222,7 +223,7 @@ struct Engine {
       uint32_t base = 0;
       if ((int)lane == leader) {
         base = atomicAdd(&r->incnt[ip() ^ 1u], __popc(peers));
-        atomicAdd(&s->away[ip()], __popc(peers));
+        atomicAdd(&away_in(s->away, step, round), __popc(peers));
       }
       base = __shfl_sync(peers, base, leader);
       const uint32_t pos = base + __popc(peers & ((1u << lane) - 1u));
@@ -245,7 +246,7 @@ struct Engine {
       if ((int)lane >= o2) incl += t;
     }
     const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-    if (lane == 0) atomicAdd(&s->away[ip()], total - total / C);
+    if (lane == 0) atomicAdd(&away_in(s->away, step, round), total - total / C);
     for (uint32_t k0 = 0; k0 < total; k0 += 32) {
       const uint32_t k = k0 + lane;
       int j = 0;
@@ -569,6 +570,10 @@ struct Engine {
       if (s->farbm == step) *(volatile uint32_t *)&r->g_farbm = step;
       if (s->farcnt[fb]) *(volatile uint32_t *)&r->g_far = step;
     }
+    // the counts that the next step's rounds start from: the last ones to read
+    // them were the step before's
+    if (threadIdx.x >= 32 && threadIdx.x < 32 + kRounds)
+      away_in(s->away, step + 1, threadIdx.x - 32) = 0u;
     cl.sync();
     const volatile StepWords *w = &words_of(cl.map_shared_rank(s, 0)->found, step);
     spilled = found(w->spilled, step);
@@ -596,17 +601,17 @@ struct Engine {
         next_round();
       }
       const uint32_t v0 = res.visits;
-      uint32_t taken = 0;
+      uint32_t taken = 0, sent = 0;
 #pragma unroll 1
-      for (int r = 0; r < kRounds; ++r) {
+      for (round = 0; round < kRounds; ++round) {
         const uint32_t nc = min(s->cnt[cq], kCap);
-        const uint32_t ni = r == 0 ? min(s->incnt[ip()], kCap) : 0u;
+        const uint32_t ni = round == 0 ? min(s->incnt[ip()], kCap) : 0u;
         const uint32_t total = nc + ni;
-        const bool scan = r == 0 && spilled;
+        const bool scan = round == 0 && spilled;
         if (total == 0 && !scan) break;
         // ids that jump between homes: most of this step's pushes wait in
         // other CTAs' inboxes, and further rounds over the rest only delay them
-        if (r && 4 * nc <= s->away[ip()]) break;
+        if (!goes_on(s->away, step, round, nc, sent)) break;
         // the list after next was read in the round before this one
         if (threadIdx.x == 0) s->cnt[cq == 0 ? 2 : cq - 1] = 0u;
         taken += total;
@@ -630,11 +635,9 @@ struct Engine {
         }
         if (scan) take_spilled();
         next_round();
-        if (r == 0 && threadIdx.x == 0) {
-          s->incnt[ip()] = 0u;
-          s->away[ip() ^ 1u] = 0u;
-        }
+        if (round == 0 && threadIdx.x == 0) s->incnt[ip()] = 0u;
       }
+      round = 0;
       ++res.steps;
       if (!kUnit && a.trace && res.steps < a.trace_cap) {
         Trace *t = a.trace + res.steps;

@@ -33,5 +33,25 @@ GRUS_HD bool found(uint32_t word, uint32_t step) { return word == step; }
 
 GRUS_HD StepWords &words_of(StepWords (&w)[2], uint32_t step) { return w[step & 1u]; }
 
+constexpr int kRounds = 4;  // rounds between cluster barriers
+
+// A CTA's pushes to other CTAs, by step parity and by the round that makes them.
+// Warps decide before a round, each when it gets there, whether the block goes
+// on; faster warps may already push in that round, so the decision counts the
+// rounds before it only, which a block barrier has ended.
+struct AwayCounts {
+  uint32_t n[2][kRounds];
+};
+
+GRUS_HD uint32_t &away_in(AwayCounts &a, uint32_t step, int round) { return a.n[step & 1u][round]; }
+
+// Whether the block goes on to `round` over its `own` entries.  `sum`: the
+// pushes of the rounds before, which this call keeps up to date.
+GRUS_HD bool goes_on(AwayCounts &a, uint32_t step, int round, uint32_t own, uint32_t &sum) {
+  if (round == 0) return true;
+  sum += away_in(a, step, round - 1);
+  return 4u * own > sum;
+}
+
 }  // namespace narrow
 }  // namespace grus

@@ -40,6 +40,32 @@ int late_reads() {
   }
   return 0;
 }
+// Warps that reach the decision before a round at different times: the fastest
+// has pushed `extra` entries in that round already, the slowest none.  Counts
+// start anew in every step.
+int late_warps() {
+  for (unsigned own : {0u, 1u, 7u, 64u, 2048u})
+    for (unsigned before : {0u, 3u, 29u, 300u, 9000u})
+      for (unsigned extra : {1u, 30u, 100000u})
+        for (unsigned step = 1; step <= 4; ++step)
+          for (int round = 0; round < kRounds; ++round) {
+            AwayCounts slow{}, fast{};
+            for (int r = 0; r < round; ++r)
+              away_in(slow, step, r) = away_in(fast, step, r) = before + r;
+            away_in(fast, step, round) += extra;
+            unsigned sum[2] = {0u, 0u};
+            bool go[2] = {true, true};
+            for (int r = 0; r <= round; ++r) {
+              go[0] = goes_on(slow, step, r, own, sum[0]);
+              go[1] = goes_on(fast, step, r, own, sum[1]);
+            }
+            if (go[0] != go[1]) return fail("go on", step);
+            if (round == 0 && !go[0]) return fail("first round", step);
+            if (&away_in(fast, step, round) == &away_in(fast, step + 1, round))
+              return fail("neighbouring steps share a count", step);
+          }
+  return 0;
+}
 """
 
 
@@ -48,7 +74,8 @@ def driver(tmp_path_factory):
     d = tmp_path_factory.mktemp("steps")
     (d / "steps.cpp").write_text(DRIVER + """
 int main(int argc, char **argv) {
-  return argc > 1 && !strcmp(argv[1], "late_reads") ? late_reads() : 2;
+  if (argc > 1 && !strcmp(argv[1], "late_reads")) return late_reads();
+  return argc > 1 && !strcmp(argv[1], "late_warps") ? late_warps() : 2;
 }
 """)
     exe = d / "steps"
@@ -59,4 +86,9 @@ int main(int argc, char **argv) {
 
 def test_step_words_read_late(driver):
     r = subprocess.run([str(driver), "late_reads"], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
+
+
+def test_rounds_decided_late(driver):
+    r = subprocess.run([str(driver), "late_warps"], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout
