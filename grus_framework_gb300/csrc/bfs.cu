@@ -1059,6 +1059,7 @@ __global__ void __launch_bounds__(narrow::kBlock) bfs_narrow(Args a) {
   view.lanes = a.lanes;
   view.ahead = a.ahead;
   view.err = a.err;
+  view.timeout_ns = a.timeout_ns;
   view.trace = (narrow::Trace *)a.trace;
   view.trace_cap = a.trace ? kMaxTrace : 0u;
   view.tag = 0u;

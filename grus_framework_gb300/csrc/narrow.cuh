@@ -24,7 +24,10 @@
 //     when no CTA has near work, T advances to the smallest far distance plus
 //     Delta (one cluster barrier), so all distances below the old T are final.
 // A full list never loses work: its overflow goes to the near or far bitmap,
-// which the next step (split) scans.
+// which the next step (split) scans.  A vertex of several entries in the near
+// bitmap is then relaxed where it stands, by the whole cluster: queued again it
+// might get no further than its first entries every time (one of more than
+// 2,097,152 out-edges, or several smaller ones at once, fill all lists).
 //
 // Bound by latency: a round with one entry takes 1.4-1.6 us (a path of 4,001
 // vertices), of which the atomic's round trip is about a third, and a cluster
@@ -52,6 +55,7 @@ constexpr int kWarps = kBlock / 32;
 constexpr int kMaxCluster = 16;
 constexpr uint32_t kCap = 2048;      // entries of one list
 constexpr uint32_t kPiece = 64;      // edges per entry
+constexpr uint32_t kWide = 64;       // spilled vertices of more edges taken in a step
 // Low-degree graphs, few entries: 4 or 8 lanes per entry instead of a scan
 // over the entries' degrees (a path's round 1.57 -> 1.04 us with 512 threads;
 // entries of up to 64 edges would take 8 serial steps instead: RMAT-12 0.19
@@ -104,6 +108,7 @@ struct View {
   uint32_t lanes;    // lanes_per_entry of the graph
   bool ahead;        // low degrees, and beyond_l2
   uint32_t *err;
+  uint64_t timeout_ns;  // a step that takes longer ends the traversal
   // null: none.  SSSP: record i is the i-th step's (from 1); BFS: record d
   // counts the vertices of depth d.  Records to be written start out zero.
   Trace *trace;
@@ -133,6 +138,10 @@ struct Shared {
   // put bits in the far bitmap and the last that had far vertices (both read
   // where no CTA can be past the step that wrote them)
   StepWords found[2];
+  // rank 0, by step parity: spilled vertices that all CTAs relax together
+  uint4 wide[2][kWide];
+  uint32_t nwide[2];
+  unsigned long long t_step;            // rank 0: when the last step ended
   uint32_t g_farbm, g_far;
   // this CTA's copies: far bitmap bits up to this step have been taken; the
   // last threshold step and its size
@@ -182,7 +191,9 @@ struct Engine {
     if (threadIdx.x < kRing) s->ring[threadIdx.x] = s->ring_sum[threadIdx.x] = 0;
     if (threadIdx.x == 0) {
       s->pushed = s->spilled = s->farbm = s->g_farbm = 0u;
-      s->found[0] = s->found[1] = StepWords{0u, 0u};
+      s->found[0] = s->found[1] = StepWords{0u, 0u, 0u};
+      s->nwide[0] = s->nwide[1] = 0u;
+      s->t_step = global_timer_ns();
       s->g_far = 0u;
       s->scanned = s->last_split = 0u;
       s->delta = a.delta;
@@ -446,8 +457,10 @@ struct Engine {
     }
   }
 
-  // Vertices spilled to the near bitmap in the previous step: this CTA's
-  // share of the words goes back to the lists (what does not fit spills again).
+  // Vertices spilled to the near bitmap in the previous step, this CTA's share
+  // of the words: those of one entry go back to the lists, the others to the
+  // cluster's wide list.  What does not fit spills again: at least a full list
+  // of vertices is out of the way by then.
   __device__ __forceinline__ void take_spilled() {
     const uint32_t per = (a.W + C - 1) / C;
     const uint32_t w0 = min(a.W, rank * per), w1 = min(a.W, w0 + per);
@@ -458,9 +471,40 @@ struct Engine {
       if (!bits) continue;
       const bool has = (bits >> lane) & 1u;
       const uint32_t v = w * 32 + lane;
-      push<true>(has, v, has ? __ldg(a.offs + v) : 0u, has ? __ldg(a.offs + v + 1) : 0u,
-                 has ? __ldcg(a.dist + v) : 0u);
+      const uint32_t b = has ? __ldg(a.offs + v) : 0u, e = has ? __ldg(a.offs + v + 1) : 0u;
+      const uint32_t d = has ? __ldcg(a.dist + v) : 0u;
+      const bool wide = e - b > kPiece;
+      push<false>(has && !wide, v, b, e, d);
+      if (wide) {
+        Shared *r = cl.map_shared_rank(s, 0);
+        const uint32_t pos = atomicAdd(&r->nwide[step & 1u], 1u);
+        if (pos < kWide) r->wide[step & 1u][pos] = make_uint4(v, b, e, d);
+        else spill(v);
+      }
     }
+  }
+
+  // The wide list's entries are dealt to the CTAs one by one: the next ones of
+  // this CTA's share, `at` of which it has had, into the list of this round,
+  // which has been read.  Returns how many; called by the whole block.
+  __device__ __forceinline__ uint32_t take_wide(uint32_t at) {
+    const Shared *r = cl.map_shared_rank(s, 0);
+    const uint4 *wide = r->wide[step & 1u];
+    const uint32_t nw = min(r->nwide[step & 1u], kWide);
+    uint32_t all = 0;
+    for (uint32_t j = 0; j < nw; ++j) all += (wide[j].z - wide[j].y + kPiece - 1) / kPiece;
+    const uint32_t mine = all > rank ? (all - rank + C - 1) / C : 0u;
+    const uint32_t count = min(mine - at, kCap);
+    for (uint32_t k = threadIdx.x; k < count; k += kBlock) {
+      uint32_t i = (at + k) * C + rank, j = 0;
+      uint4 en = wide[0];
+      for (uint32_t np; i >= (np = (en.z - en.y + kPiece - 1) / kPiece); en = wide[++j]) i -= np;
+      en.y += i * kPiece;
+      en.z = min(en.z, en.y + kPiece);
+      s->loc[lb][k] = en;
+    }
+    __syncthreads();
+    return count;
   }
 
   __device__ __forceinline__ uint32_t block_min(uint32_t x) {
@@ -561,7 +605,7 @@ struct Engine {
 
   // After a round: the pushes made before the call become readable by their
   // readers; true if any CTA has near work.
-  __device__ __forceinline__ bool end_step(bool &spilled) {
+  __device__ __forceinline__ bool end_step(bool &spilled, bool &late) {
     if (threadIdx.x == 0) {
       Shared *r = cl.map_shared_rank(s, 0);
       volatile StepWords *w = &words_of(r->found, step);
@@ -570,13 +614,20 @@ struct Engine {
       if (s->farbm == step) *(volatile uint32_t *)&r->g_farbm = step;
       if (s->farcnt[fb]) *(volatile uint32_t *)&r->g_far = step;
     }
-    // the counts that the next step's rounds start from: the last ones to read
-    // them were the step before's
+    // the counts that the next step starts from: the last to read them was the
+    // step before this one
     if (threadIdx.x >= 32 && threadIdx.x < 32 + kRounds)
       away_in(s->away, step + 1, threadIdx.x - 32) = 0u;
+    if (rank == 0 && threadIdx.x == 64) {
+      s->nwide[(step + 1) & 1u] = 0u;
+      const unsigned long long t = global_timer_ns();
+      if (t - s->t_step > a.timeout_ns) words_of(s->found, step).late = step;
+      s->t_step = t;
+    }
     cl.sync();
     const volatile StepWords *w = &words_of(cl.map_shared_rank(s, 0)->found, step);
     spilled = found(w->spilled, step);
+    late = found(w->late, step);
     const bool work = found(w->work, step);
     ++step;
     return work || spilled;
@@ -594,46 +645,61 @@ struct Engine {
   __device__ __forceinline__ void run() {
     next_round();
     while (true) {
-      bool spilled = false;
-      const bool work = end_step(spilled);
+      bool spilled = false, late = false;
+      const bool work = end_step(spilled, late);
+      if (late) {
+        if (rank == 0 && threadIdx.x == 0) atomicOr(a.err, kErrTimeout);
+        break;
+      }
       if (!work) {
         if (!split()) break;
         next_round();
       }
       const uint32_t v0 = res.visits;
-      uint32_t taken = 0, sent = 0;
+      uint32_t taken = 0;
 #pragma unroll 1
       for (round = 0; round < kRounds; ++round) {
-        const uint32_t nc = min(s->cnt[cq], kCap);
-        const uint32_t ni = round == 0 ? min(s->incnt[ip()], kCap) : 0u;
-        const uint32_t total = nc + ni;
+        uint32_t nc = min(s->cnt[cq], kCap);
+        uint32_t total = nc + (round == 0 ? min(s->incnt[ip()], kCap) : 0u);
         const bool scan = round == 0 && spilled;
         if (total == 0 && !scan) break;
         // ids that jump between homes: most of this step's pushes wait in
         // other CTAs' inboxes, and further rounds over the rest only delay them
-        if (!goes_on(s->away, step, round, nc, sent)) break;
+        if (!goes_on(s->away, step, round, nc)) break;
         // the list after next was read in the round before this one
         if (threadIdx.x == 0) s->cnt[cq == 0 ? 2 : cq - 1] = 0u;
-        taken += total;
-        if (a.lanes && total * a.lanes <= 2 * kBlock) {
-          for (uint32_t base = threadIdx.x; base < total * a.lanes + lane; base += kBlock) {
-            const uint32_t i = base >> lane_shift;
-            const bool has = i < total;
-            uint4 en = make_uint4(0u, 0u, 0u, 0u);
-            if (has) en = i < nc ? s->loc[lb][i] : s->inb[ip()][i - nc];
-            relax_few(en, has);
+        // once over the lists; after a spill, then over the wide list's entries
+        for (uint32_t wide = 0;;) {
+          taken += total;
+          if (a.lanes && total * a.lanes <= 2 * kBlock) {
+            for (uint32_t base = threadIdx.x; base < total * a.lanes + lane; base += kBlock) {
+              const uint32_t i = base >> lane_shift;
+              const bool has = i < total;
+              uint4 en = make_uint4(0u, 0u, 0u, 0u);
+              if (has) en = i < nc ? s->loc[lb][i] : s->inb[ip()][i - nc];
+              relax_few(en, has);
+            }
+          } else {
+            const uint32_t epw = min(32u, (total + kWarps - 1) / kWarps);
+            for (uint32_t base = warp * epw; base < total; base += kWarps * epw) {
+              const uint32_t i = base + lane;
+              const bool has = lane < epw && i < total;
+              uint4 en = make_uint4(0u, 0u, 0u, 0u);
+              if (has) en = i < nc ? s->loc[lb][i] : s->inb[ip()][i - nc];
+              relax(en, has);
+            }
           }
-        } else {
-          const uint32_t epw = min(32u, (total + kWarps - 1) / kWarps);
-          for (uint32_t base = warp * epw; base < total; base += kWarps * epw) {
-            const uint32_t i = base + lane;
-            const bool has = lane < epw && i < total;
-            uint4 en = make_uint4(0u, 0u, 0u, 0u);
-            if (has) en = i < nc ? s->loc[lb][i] : s->inb[ip()][i - nc];
-            relax(en, has);
+          if (!scan) break;
+          if (wide == 0) {
+            take_spilled();
+            cl.sync();
+          } else {
+            __syncthreads();
           }
+          nc = total = take_wide(wide);
+          if (total == 0) break;
+          wide += total;
         }
-        if (scan) take_spilled();
         next_round();
         if (round == 0 && threadIdx.x == 0) s->incnt[ip()] = 0u;
       }

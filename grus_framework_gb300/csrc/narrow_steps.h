@@ -27,6 +27,7 @@ namespace narrow {
 struct StepWords {
   uint32_t work;     // some CTA has near work left
   uint32_t spilled;  // some list was full: vertices wait in the near bitmap
+  uint32_t late;     // the step took longer than the time limit
 };
 
 GRUS_HD bool found(uint32_t word, uint32_t step) { return word == step; }
@@ -45,12 +46,11 @@ struct AwayCounts {
 
 GRUS_HD uint32_t &away_in(AwayCounts &a, uint32_t step, int round) { return a.n[step & 1u][round]; }
 
-// Whether the block goes on to `round` over its `own` entries.  `sum`: the
-// pushes of the rounds before, which this call keeps up to date.
-GRUS_HD bool goes_on(AwayCounts &a, uint32_t step, int round, uint32_t own, uint32_t &sum) {
-  if (round == 0) return true;
-  sum += away_in(a, step, round - 1);
-  return 4u * own > sum;
+// Whether the block goes on to `round` over its `own` entries.
+GRUS_HD bool goes_on(AwayCounts &a, uint32_t step, int round, uint32_t own) {
+  uint32_t sum = 0;
+  for (int r = 0; r < round; ++r) sum += away_in(a, step, r);
+  return round == 0 || 4u * own > sum;
 }
 
 }  // namespace narrow

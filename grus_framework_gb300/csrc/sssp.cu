@@ -465,6 +465,7 @@ __global__ void __launch_bounds__(narrow::kBlock) sssp_narrow(Args a) {
   view.lanes = a.lanes;
   view.ahead = a.ahead;
   view.err = a.err;
+  view.timeout_ns = a.timeout_ns;
   const uint32_t L0 = a.whole ? 0u : __ldcg(&a.summary->levels);
   view.tag = a.whole ? 0u : __ldcg(&a.summary->splits);
   view.nearbm = a.near[a.whole ? 0u : __ldcg(&a.ho->sel)];

@@ -23,18 +23,21 @@ static int fail(const char *what, unsigned step) {
 // it may do before a slow thread reads those of `step`).
 int late_reads() {
   for (unsigned history = 0; history < 64; ++history) {
-    StepWords w[2] = {{0u, 0u}, {0u, 0u}};
+    StepWords w[2] = {};
     for (unsigned step = 1; step <= 6; ++step) {
       const bool sp = history >> (step - 1) & 1u, work = step % 3 != 0;
       if (sp) words_of(w, step).spilled = step;
       if (work) words_of(w, step).work = step;
+      if (sp && work) words_of(w, step).late = step;
       StepWords ahead[2];
       memcpy(ahead, w, sizeof(w));
       words_of(ahead, step + 1).spilled = step + 1;
       words_of(ahead, step + 1).work = step + 1;
+      words_of(ahead, step + 1).late = step + 1;
       for (const StepWords *v : {&words_of(w, step), &words_of(ahead, step)}) {
         if (found(v->spilled, step) != sp) return fail("spilled", step);
         if (found(v->work, step) != work) return fail("work", step);
+        if (found(v->late, step) != (sp && work)) return fail("late", step);
       }
     }
   }
@@ -53,12 +56,7 @@ int late_warps() {
             for (int r = 0; r < round; ++r)
               away_in(slow, step, r) = away_in(fast, step, r) = before + r;
             away_in(fast, step, round) += extra;
-            unsigned sum[2] = {0u, 0u};
-            bool go[2] = {true, true};
-            for (int r = 0; r <= round; ++r) {
-              go[0] = goes_on(slow, step, r, own, sum[0]);
-              go[1] = goes_on(fast, step, r, own, sum[1]);
-            }
+            const bool go[2] = {goes_on(slow, step, round, own), goes_on(fast, step, round, own)};
             if (go[0] != go[1]) return fail("go on", step);
             if (round == 0 && !go[0]) return fail("first round", step);
             if (&away_in(fast, step, round) == &away_in(fast, step + 1, round))
