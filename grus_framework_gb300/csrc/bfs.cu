@@ -1051,7 +1051,8 @@ __global__ void __launch_bounds__(narrow::kBlock) bfs_narrow(Args a) {
   view.m = (uint32_t)a.m;
   view.dist = a.depth;
   view.nearbm = a.front[0];
-  view.farbm = a.front[1];
+  view.near_odd = (uint32_t)(a.front[1] - a.front[0]);
+  view.farbm = a.front[2];
   view.far = a.far;
   view.far_cap = narrow::far_cap(a.n, narrow::kFarCapUnit);
   view.delta = narrow::kUnitDelta;
@@ -1069,7 +1070,7 @@ __global__ void __launch_bounds__(narrow::kBlock) bfs_narrow(Args a) {
   for (uint32_t d = d0 + 1 + tid; d < view.trace_cap; d += nt)
     view.trace[d] = narrow::Trace{0ull, 0ull, 0u, 0u};
   for (uint32_t i = tid; i < a.W; i += nt) {
-    view.nearbm[i] = 0u;
+    a.front[0][i] = a.front[1][i] = 0u;
     view.farbm[i] = 0u;
   }
   if (a.whole) {

@@ -23,11 +23,14 @@
 //   * Distances of T and above wait in a far list per CTA (global memory);
 //     when no CTA has near work, T advances to the smallest far distance plus
 //     Delta (one cluster barrier), so all distances below the old T are final.
-// A full list never loses work: its overflow goes to the near or far bitmap,
-// which the next step (split) scans.  A vertex of several entries in the near
-// bitmap is then relaxed where it stands, by the whole cluster: queued again it
-// might get no further than its first entries every time (one of more than
-// 2,097,152 out-edges, or several smaller ones at once, fill all lists).
+// A full list never loses work: its overflow goes to the near or far bitmap.
+// The next step relaxes what is in the near bitmap where it stands, all of it
+// (the far bitmap waits for the split).  Queued again instead, a vertex of
+// several entries might get no further than its first ones every time (one of
+// more than 2,097,152 out-edges, or several smaller ones, fill all lists), and a
+// frontier wider than the lists would take many steps, each at another depth:
+// BFS along a path of 24 vertices into a random graph of 4 M vertices, degree
+// 16, 49.8 ms with queueing, 10.1 without.
 //
 // Bound by latency: a round with one entry takes 1.4-1.6 us (a path of 4,001
 // vertices), of which the atomic's round trip is about a third, and a cluster
@@ -55,7 +58,9 @@ constexpr int kWarps = kBlock / 32;
 constexpr int kMaxCluster = 16;
 constexpr uint32_t kCap = 2048;      // entries of one list
 constexpr uint32_t kPiece = 64;      // edges per entry
-constexpr uint32_t kWide = 64;       // spilled vertices of more edges taken in a step
+// Spilled vertices: up to kWideEdges edges go to one CTA, those of more to the
+// whole cluster, kWide of them in a step.
+constexpr uint32_t kWideEdges = 1024, kWide = 128;
 // Low-degree graphs, few entries: 4 or 8 lanes per entry instead of a scan
 // over the entries' degrees (a path's round 1.57 -> 1.04 us with 512 threads;
 // entries of up to 64 edges would take 8 serial steps instead: RMAT-12 0.19
@@ -99,7 +104,8 @@ struct View {
   const uint32_t *__restrict__ wts;  // unused by BFS
   uint32_t n, W, m;
   uint32_t *dist;
-  uint32_t *nearbm;  // W words, all zero at the start
+  uint32_t *nearbm;  // W words by step parity, all zero at the start ...
+  uint32_t near_odd;  // ... the odd steps' this far behind
   uint32_t *farbm;   // W words, zero but for what farbm_used announces
   uint2 *far;        // far_bytes(n)
   uint32_t far_cap;
@@ -138,6 +144,10 @@ struct Shared {
   // put bits in the far bitmap and the last that had far vertices (both read
   // where no CTA can be past the step that wrote them)
   StepWords found[2];
+  // taking spilled vertices: entries claimed in the list, the place of the first
+  // claim that found no room, each warp's next words, and how many entries of
+  // the wide list this CTA has had
+  uint32_t claimed, refused, cur[kWarps], had;
   // rank 0, by step parity: spilled vertices that all CTAs relax together
   uint4 wide[2][kWide];
   uint32_t nwide[2];
@@ -204,8 +214,13 @@ struct Engine {
   __device__ __forceinline__ uint32_t ip() const { return (step & 1u) ^ 1u; }
   __device__ __forceinline__ uint32_t home(uint32_t v) const { return __umulhi(v, scale); }
 
+  // The near bitmap that this step's pushes spill to.
+  __device__ __forceinline__ uint32_t *near_of(uint32_t st) const {
+    return a.nearbm + (st & 1u ? a.near_odd : 0u);
+  }
+
   __device__ __forceinline__ void spill(uint32_t v) {
-    atomicOr(a.nearbm + (v >> 5), 1u << (v & 31u));
+    atomicOr(near_of(step) + (v >> 5), 1u << (v & 31u));
     s->spilled = step;
   }
 
@@ -217,7 +232,11 @@ struct Engine {
     want = want && e > b;
     const uint32_t nq = cq == 2 ? 0 : cq + 1;
     const uint32_t o = home(u);
-    const bool big = kBig && want && e - b > kPiece;
+    bool big = kBig && want && e - b > kPiece;
+    if (big && *(volatile uint32_t *)&s->cnt[nq] >= kCap) {  // no pieces into full lists
+      spill(u);
+      want = big = false;
+    }
     const bool here = want && !big && o == rank;
     if (here) {
       const uint32_t pos = atomicAdd(&s->cnt[nq], 1u);
@@ -457,46 +476,85 @@ struct Engine {
     }
   }
 
-  // Vertices spilled to the near bitmap in the previous step, this CTA's share
-  // of the words: those of one entry go back to the lists, the others to the
-  // cluster's wide list.  What does not fit spills again: at least a full list
-  // of vertices is out of the way by then.
-  __device__ __forceinline__ void take_spilled() {
-    const uint32_t per = (a.W + C - 1) / C;
-    const uint32_t w0 = min(a.W, rank * per), w1 = min(a.W, w0 + per);
-    for (uint32_t w = w0 + warp; w < w1; w += kWarps) {
-      uint32_t bits = 0;
-      if (lane == 0 && __ldcg(a.nearbm + w)) bits = atomicExch(a.nearbm + w, 0u);
-      bits = __shfl_sync(0xffffffffu, bits, 0);
-      if (!bits) continue;
-      const bool has = (bits >> lane) & 1u;
-      const uint32_t v = w * 32 + lane;
-      const uint32_t b = has ? __ldg(a.offs + v) : 0u, e = has ? __ldg(a.offs + v + 1) : 0u;
-      const uint32_t d = has ? __ldcg(a.dist + v) : 0u;
-      const bool wide = e - b > kPiece;
-      push<false>(has && !wide, v, b, e, d);
-      if (wide) {
-        Shared *r = cl.map_shared_rank(s, 0);
-        const uint32_t pos = atomicAdd(&r->nwide[step & 1u], 1u);
-        if (pos < kWide) r->wide[step & 1u][pos] = make_uint4(v, b, e, d);
-        else spill(v);
-      }
+  // The next entries of what the step before spilled, in place of this round's
+  // list, which has been read: first the vertices in this CTA's share of the
+  // near bitmap's words, then its share of the wide list.  Returns how many,
+  // 0 when all are done.  Called by the whole block.
+  __device__ __forceinline__ uint32_t next_spilled() {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      s->claimed = 0u;
+      s->refused = kCap;
     }
+    __syncthreads();
+    if (!s->had) {
+      take_words();
+      __syncthreads();
+      if (s->claimed) return min(s->claimed, s->refused);
+      cl.sync();  // the wide list is complete
+    }
+    return take_wide();
   }
 
-  // The wide list's entries are dealt to the CTAs one by one: the next ones of
-  // this CTA's share, `at` of which it has had, into the list of this round,
-  // which has been read.  Returns how many; called by the whole block.
-  __device__ __forceinline__ uint32_t take_wide(uint32_t at) {
+  // A warp takes 32 words at a time and of those one after another, until the
+  // list has no room for a word's entries.  The words are dealt to the CTAs by
+  // 32: neighbouring ids are often of the same depth.
+  __device__ __forceinline__ void take_words() {
+    uint32_t *bm = near_of(step - 1);
+    uint32_t w = s->cur[warp];
+    bool room = true;
+    for (; room && w < a.W; w += room ? 32 * kWarps * C : 0) {
+      const uint32_t at = w + lane;
+      const uint32_t word = at < a.W ? __ldcg(bm + at) : 0u;
+      for (uint32_t left = __ballot_sync(0xffffffffu, word != 0u); left; left &= left - 1) {
+        const int src = __ffs(left) - 1;
+        const bool has = (__shfl_sync(0xffffffffu, word, src) >> lane) & 1u;
+        const uint32_t v = (w + src) * 32 + lane;
+        const uint32_t b = has ? __ldg(a.offs + v) : 0u, e = has ? __ldg(a.offs + v + 1) : 0u;
+        const uint32_t d = has ? __ldcg(a.dist + v) : 0u;
+        const bool wide = e - b > kWideEdges;
+        uint32_t np = wide ? 0u : (e - b + kPiece - 1) / kPiece, incl = np;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+          if ((int)lane >= o) incl += t;
+        }
+        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+        uint32_t pos = lane == 0 ? atomicAdd(&s->claimed, total) : 0u;
+        pos = __shfl_sync(0xffffffffu, pos, 0);
+        // once one claim finds no room none does, so the first one's place is
+        // where the entries end
+        if (pos + total > kCap) {
+          if (lane == 0) atomicMin(&s->refused, pos);
+          room = false;
+          break;
+        }
+        pos += incl - np;
+        for (uint32_t x = b; np; --np, x += kPiece)
+          s->loc[lb][pos++] = make_uint4(v, x, min(e, x + kPiece), d);
+        if (wide) {
+          Shared *r = cl.map_shared_rank(s, 0);
+          const uint32_t i = atomicAdd(&r->nwide[step & 1u], 1u);
+          if (i < kWide) r->wide[step & 1u][i] = make_uint4(v, b, e, d);
+          else spill(v);
+        }
+        if ((int)lane == src) __stcg(bm + at, 0u);
+      }
+    }
+    if (lane == 0) s->cur[warp] = w;
+  }
+
+  // The wide list's entries are dealt to the CTAs one by one.
+  __device__ __forceinline__ uint32_t take_wide() {
     const Shared *r = cl.map_shared_rank(s, 0);
     const uint4 *wide = r->wide[step & 1u];
-    const uint32_t nw = min(r->nwide[step & 1u], kWide);
+    const uint32_t nw = min(r->nwide[step & 1u], kWide), had = s->had;
     uint32_t all = 0;
     for (uint32_t j = 0; j < nw; ++j) all += (wide[j].z - wide[j].y + kPiece - 1) / kPiece;
     const uint32_t mine = all > rank ? (all - rank + C - 1) / C : 0u;
-    const uint32_t count = min(mine - at, kCap);
+    const uint32_t count = min(mine - had, kCap);
     for (uint32_t k = threadIdx.x; k < count; k += kBlock) {
-      uint32_t i = (at + k) * C + rank, j = 0;
+      uint32_t i = (had + k) * C + rank, j = 0;
       uint4 en = wide[0];
       for (uint32_t np; i >= (np = (en.z - en.y + kPiece - 1) / kPiece); en = wide[++j]) i -= np;
       en.y += i * kPiece;
@@ -504,6 +562,7 @@ struct Engine {
       s->loc[lb][k] = en;
     }
     __syncthreads();
+    if (threadIdx.x == 0) s->had = had + count;
     return count;
   }
 
@@ -667,9 +726,13 @@ struct Engine {
         // other CTAs' inboxes, and further rounds over the rest only delay them
         if (!goes_on(s->away, step, round, nc)) break;
         // the list after next was read in the round before this one
-        if (threadIdx.x == 0) s->cnt[cq == 0 ? 2 : cq - 1] = 0u;
-        // once over the lists; after a spill, then over the wide list's entries
-        for (uint32_t wide = 0;;) {
+        if (threadIdx.x == 0) {
+          s->cnt[cq == 0 ? 2 : cq - 1] = 0u;
+          s->had = 0u;
+        }
+        if (scan && lane == 0) s->cur[warp] = 32u * (warp * C + rank);
+        // once over the lists, then over what the step before spilled
+        while (true) {
           taken += total;
           if (a.lanes && total * a.lanes <= 2 * kBlock) {
             for (uint32_t base = threadIdx.x; base < total * a.lanes + lane; base += kBlock) {
@@ -690,15 +753,8 @@ struct Engine {
             }
           }
           if (!scan) break;
-          if (wide == 0) {
-            take_spilled();
-            cl.sync();
-          } else {
-            __syncthreads();
-          }
-          nc = total = take_wide(wide);
+          nc = total = next_spilled();
           if (total == 0) break;
-          wide += total;
         }
         next_round();
         if (round == 0 && threadIdx.x == 0) s->incnt[ip()] = 0u;

@@ -99,7 +99,7 @@ constexpr int kMaxTries = 4;
 struct Handover {
   uint32_t flag;                     // 1: sssp_narrow continues the traversal
   uint32_t qcount;                   // vertices of the near set (Args::queue)
-  uint32_t T, sel;                   // threshold; near[sel] is all zero
+  uint32_t T, pad;                   // threshold; near[0] and near[1] are all zero
   // by attempt: out-edges of the vertices that are not below the threshold,
   // and the unreached vertices with their out-edges
   unsigned long long left[kMaxTries], mu[kMaxTries];
@@ -276,7 +276,6 @@ __device__ __noinline__ uint32_t try_hand_over(const Args &a, uint32_t run, uint
   if (gtid == 0) {
     a.ho->qcount = qc;
     a.ho->T = T;
-    a.ho->sel = (L + 1) & 1u;
     a.summary->levels = L;
     a.summary->splits = splits;
     a.summary->nr = a.n - __ldcg(&a.ho->nu[k]);
@@ -468,7 +467,8 @@ __global__ void __launch_bounds__(narrow::kBlock) sssp_narrow(Args a) {
   view.timeout_ns = a.timeout_ns;
   const uint32_t L0 = a.whole ? 0u : __ldcg(&a.summary->levels);
   view.tag = a.whole ? 0u : __ldcg(&a.summary->splits);
-  view.nearbm = a.near[a.whole ? 0u : __ldcg(&a.ho->sel)];
+  view.nearbm = a.near[0];
+  view.near_odd = (uint32_t)(a.near[1] - a.near[0]);
   view.trace = a.trace && L0 < (uint32_t)kMaxTrace ? (narrow::Trace *)a.trace + L0 : nullptr;
   view.trace_cap = L0 < (uint32_t)kMaxTrace ? kMaxTrace - L0 : 0u;
   narrow::Engine<false> E(view, (narrow::Shared *)smem);
@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(narrow::kBlock) sssp_narrow(Args a) {
   if (a.whole) {
     for (uint32_t i = tid; i < a.n; i += nt) a.dist[i] = i == a.src ? 0u : kInfinit;
     for (uint32_t i = tid; i < a.W; i += nt) {
-      view.nearbm[i] = 0u;
+      a.near[0][i] = a.near[1][i] = 0u;
       a.farbm[i] = 0u;
     }
     if (tid == 0) {

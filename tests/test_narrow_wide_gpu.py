@@ -73,3 +73,45 @@ def test_sssp_settled_hubs_improved_in_the_cluster(grus, count, leaves):
     assert st["vertices_reached"] == n and st["edges_reached"] == len(cols)
     assert st["levels"] < st2["levels"]  # the cluster's steps are several levels each
     g.free()
+
+
+def _tree(path, depth):
+    """A path into the root of a binary tree numbered in preorder: few
+    neighbours, near by id, and a frontier that doubles."""
+    size = (1 << depth) - 1
+    left, right, stack = [], [], [(0, depth)]
+    while stack:
+        v, d = stack.pop()
+        if d == 1:
+            continue
+        half = (1 << (d - 1)) - 1
+        left += [v, v]
+        right += [v + 1, v + 1 + half]
+        stack += [(v + 1, d - 1), (v + 1 + half, d - 1)]
+    u = np.concatenate([np.arange(path), np.array(left) + path])
+    v = np.concatenate([np.arange(1, path + 1), np.array(right) + path])
+    n = path + size
+    src, dst = np.concatenate([u, v]), np.concatenate([v, u])
+    order = np.lexsort((dst, src))
+    w = (np.minimum(u, v) * 40503 + np.maximum(u, v) * 9973) % 255 + 1
+    offs = np.zeros(n + 1, np.uint32)
+    offs[1:] = np.cumsum(np.bincount(src, minlength=n))
+    return offs, dst[order].astype(np.uint32), np.concatenate([w, w])[order].astype(np.uint32)
+
+
+@pytest.mark.parametrize("path,depth", [(40, 18), (100, 19)])
+def test_frontier_wider_than_the_lists(grus, oracle_mod, path, depth):
+    offs, cols, wts = _tree(path, depth)
+    csr = oracle_mod.CSR(offs, cols, wts)
+    g = grus.Graph.from_csr(offs, cols, wts, symmetric=True)
+    for call, ref in ((grus.bfs, oracle_mod.bfs(csr, 0)), (grus.sssp, oracle_mod.sssp(csr, 0))):
+        for tail in (0, 2):
+            g.set_tuning(tail_cluster=tail)
+            got, st = call(g, 0, stats=True)
+            assert np.array_equal(got, ref), (call.__name__, tail)
+            assert st["vertices_reached"] == int(g.n) and st["edges_reached"] == int(g.m)
+            if call is grus.bfs:
+                assert st["levels"] == path + depth
+                for i, t in enumerate(grus.bfs_trace(g, 200)):
+                    assert t["vertices"] == int((ref == i + 1).sum()), (tail, i)
+    g.free()
