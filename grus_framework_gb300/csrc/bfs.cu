@@ -35,8 +35,10 @@
 //     the first push level after a pull level turns the frontier bitmap into
 //     the queue with one atomic per CTA per 256 words.
 //   * narrow tail: a long traversal (16+ levels) whose push frontier and
-//     remaining edges have become small is handed to bfs_narrow, one cluster
-//     of up to 16 CTAs launched after the persistent kernel (narrow.cuh); it
+//     remaining edges have become small is handed to one cluster of up to 16
+//     CTAs, launched after the persistent kernel: bfs_tail, level by level with
+//     one cluster barrier each, or bfs_narrow (narrow.cuh), several levels a
+//     barrier, where a graph's ids follow its geometry (near_ids).  bfs_narrow
 //     also runs small graphs from the start.
 // Depths are order-independent (every writer stores level+1), so results are
 // bit-exact against the serial oracle whatever the schedule.
@@ -50,6 +52,8 @@
 namespace grus {
 namespace {
 
+namespace cg = cooperative_groups;
+
 constexpr int kBlock = 256;
 constexpr uint32_t kDefHuge = 8192;   // chunking threshold
 constexpr uint32_t kDefBuScan = 4;    // pull: neighbours a lane checks alone (one round)
@@ -59,8 +63,8 @@ constexpr uint32_t kDefBuScanManaged = 8;
 constexpr uint32_t kDefBuWords = 4;   // pull: bitmap words per warp step
 constexpr float kDefAlpha = 15.f, kDefBeta = 18.f;
 // Narrow tail: a traversal still running after kNarrowAfter levels, with a
-// push frontier of at most kNarrowNf vertices per tail CTA and at most
-// kNarrowMu edges left whose source is undiscovered, is finished by one
+// push frontier of at most kNarrowNf (bfs_tail: kTailNf) vertices per CTA and at
+// most kNarrowMu edges left whose source is undiscovered, is finished by one
 // thread-block cluster of up to 16 CTAs.  The edge bound caps the work the
 // cluster may be left with.  (Handing over the last one or two levels of a
 // shorter traversal costs what it saves: RMAT scales 16-20 0.072 -> 0.078 and
@@ -69,8 +73,10 @@ constexpr float kDefAlpha = 15.f, kDefBeta = 18.f;
 // cluster then ran its widest levels too (400 K vertices 713 us, 332 without;
 // 2 M vertices 1,004 / 529); a grid's grows by a sixteenth there, and less later.
 constexpr uint32_t kNarrowAfter = 16;
-constexpr uint32_t kNarrowNf = 1024;
+constexpr uint32_t kNarrowNf = 1024, kTailNf = 4096;
 constexpr uint64_t kNarrowMu = 1ull << 26;
+constexpr int kTailBlock = 1024;
+constexpr uint32_t kTailCap = 4096;   // shared-memory frontier entries per buffer per CTA
 // Graphs whose whole traversal runs in the cluster kernel, one launch without
 // grid barriers: up to 2^17 edges, or 2^18 when no vertex has more than 64
 // out-edges.  Times against the grid kernels: RMAT-10 0.036 / 0.059 ms,
@@ -102,6 +108,7 @@ struct Handover {
   uint32_t qsel;
   unsigned long long nr, mr;  // reach counts so far
   uint32_t bu_levels, switches;
+  uint32_t spill[3];          // bfs_tail: spilled frontier entries, by depth mod 3
 };
 
 // Per-level record written by one thread after each level's barrier:
@@ -1032,6 +1039,276 @@ __global__ void __launch_bounds__(kBlock) bfs_persistent(Args a) {
   }
 }
 
+// Per-level state of the tail cluster.  Every frontier vertex has an owner
+// CTA (a hash of its id); the owner keeps it as the (begin, end) range of its
+// out-edges in shared memory, or -- beyond kTailCap entries -- the vertex id
+// goes to a global spill list shared by the cluster.
+struct Tail {
+  cg::cluster_group cl;
+  uint32_t rank, C;
+  uint2 *q;            // this CTA's 2 * kTailCap entries
+  uint32_t *cnt;       // this CTA's 2 entry counters
+  uint32_t *found;     // this CTA's flag: it found a vertex at this level
+};
+
+__device__ __forceinline__ uint32_t tail_owner(uint32_t v, uint32_t C) {
+  return __umulhi(v * 2654435761u, C);
+}
+
+// Claims up to kTailBatch targets at once.  The chain per batch is short:
+// the column ids come from L1 (their lines were prefetched), the claiming
+// atomicOr goes to L2 while the targets' offsets are prefetched, and a new
+// vertex's offsets then come from L1.  A new vertex gets depth d and, if it
+// has out-edges, a place in its owner's next frontier and a prefetch of its
+// first out-edges.
+constexpr int kTailBatch = 4;
+
+__device__ __forceinline__ void tail_batch(const Args &a, Tail &t,
+                                             const uint32_t (&xs)[kTailBatch], int cnt,
+                                             uint32_t d, uint32_t nxt, unsigned long long &nr,
+                                             unsigned long long &mr) {
+  uint32_t c[kTailBatch], old[kTailBatch];
+#pragma unroll
+  for (int r = 0; r < kTailBatch; ++r) c[r] = r < cnt ? __ldg(a.cols + xs[r]) : 0u;
+#pragma unroll
+  for (int r = 0; r < kTailBatch; ++r)
+    if (r < cnt) narrow::prefetch_l1(a.offs + c[r]);
+#pragma unroll
+  for (int r = 0; r < kTailBatch; ++r) {
+    const uint32_t bit = 1u << (c[r] & 31u);
+    old[r] = r < cnt ? atomicOr(a.visited + (c[r] >> 5), bit) : bit;
+  }
+#pragma unroll
+  for (int r = 0; r < kTailBatch; ++r) {
+    if (old[r] & (1u << (c[r] & 31u))) continue;
+    const uint32_t v = c[r];
+    a.depth[v] = d;
+    const uint32_t cb = __ldg(a.offs + v), ce = __ldg(a.offs + v + 1);
+    ++nr;
+    mr += ce - cb;
+    *t.found = 1u;
+    if (ce == cb) continue;
+    const uint32_t o = tail_owner(v, t.C);
+    if (o == t.rank) {
+      narrow::prefetch_l1(a.cols + cb);
+      narrow::prefetch_l1(a.cols + ce - 1);
+    } else {
+      narrow::prefetch_l2(a.cols + cb);
+      narrow::prefetch_l2(a.cols + ce - 1);
+    }
+    // one reservation per owner among the lanes pushing together
+    cg::coalesced_group pg = cg::coalesced_threads();
+    cg::coalesced_group peers = cg::labeled_partition(pg, o);
+    uint32_t base = 0;
+    if (peers.thread_rank() == 0) base = atomicAdd(t.cl.map_shared_rank(t.cnt + nxt, o), peers.size());
+    const uint32_t pos = peers.shfl(base, 0) + peers.thread_rank();
+    if (pos < kTailCap) {
+      t.cl.map_shared_rank(t.q, o)[nxt * kTailCap + pos] = make_uint2(cb, ce);
+    } else {
+      const uint32_t g = atomicAdd(&a.ho->spill[d % 3], 1u);
+      if (g < a.queue_cap) a.queue[d & 1u][g] = v;
+      else atomicOr(a.err, kErrOverflow);  // cannot happen: spilled vertices are distinct
+    }
+  }
+}
+
+// The narrow tail of a long traversal: one cluster of C CTAs (1 <= C <= 16)
+// of 1024 threads takes the small frontier the persistent kernel handed over
+// and runs the remaining levels with one hardware cluster barrier per level.
+// Each CTA deals the edges of the frontier vertices it owns evenly to its
+// threads (a block scan of the degrees and a binary search for each thread's
+// first entry), so a wide vertex is shared by many threads, and each thread
+// claims its edges in batches; spilled entries are dealt over the whole
+// cluster one vertex per thread.  A CTA that found a vertex writes the new
+// depth into every CTA's stamp before the level's barrier, so after it each
+// CTA reads its own stamp; stamps only grow, so no CTA has to clear them.
+// Returns at once when the persistent kernel finished the traversal itself.
+__global__ void __launch_bounds__(kTailBlock) bfs_tail(Args a) {
+  extern __shared__ uint2 s_q[];  // 2 * kTailCap entries
+  __shared__ uint32_t s_pref[kTailCap + 1];
+  __shared__ uint32_t s_cnt[2], s_found, s_stamp;
+  __shared__ unsigned long long s_red[kTailBlock / 32];
+  Handover *ho = a.ho;
+  if (__ldcg(&ho->flag) != 1u) return;  // the same answer in every CTA
+  Tail t{cg::this_cluster(), 0, 1, s_q, s_cnt, &s_found};
+  t.rank = t.cl.block_rank();
+  t.C = t.cl.num_blocks();
+  const uint32_t tid = threadIdx.x;
+  uint32_t d = __ldcg(&ho->level);  // depth of the current frontier
+  const uint32_t d0 = d;
+  const uint32_t nf0 = __ldcg(&ho->nf);
+  const uint32_t *q0 = a.queue[__ldcg(&ho->qsel)];
+  if (tid == 0) {
+    s_cnt[0] = 0;
+    s_cnt[1] = 0;
+    s_found = 0;
+    s_stamp = d;
+    if (t.rank == 0) {
+      ho->spill[d % 3] = 0u;  // the counters of depths d0 and d0 + 1
+      ho->spill[(d + 1) % 3] = 0u;
+      a.summary->nr = __ldcg(&ho->nr);
+      a.summary->mr = __ldcg(&ho->mr);
+      if (a.trace && d + 1 < (uint32_t)kMaxTrace) a.trace[d + 1] = LevelTrace{0ull, 0ull, 0u, 0u};
+    }
+  }
+  __syncthreads();
+  // this CTA's share of the handed-over queue (vertex ids) becomes ranges in
+  // buffer 0; vertices without out-edges are left out, so every entry has at
+  // least one edge, which the edge dealing relies on
+  for (uint32_t i = t.rank + t.C * tid; i < nf0; i += t.C * kTailBlock) {
+    const uint32_t v = __ldcg(q0 + i);
+    const uint2 r = make_uint2(__ldg(a.offs + v), __ldg(a.offs + v + 1));
+    if (r.x == r.y) continue;
+    const uint32_t pos = atomicAdd(&s_cnt[0], 1u);
+    if (pos < kTailCap) s_q[pos] = r;
+    else atomicOr(a.err, kErrOverflow);  // cannot happen: nf0 <= C * kTailCap
+  }
+  t.cl.sync();  // every CTA's counters are set before any remote push
+  unsigned long long nr = 0, mr = 0;
+  uint32_t cur = 0, levels = 0;
+  constexpr uint32_t kPer = (kTailCap + kTailBlock - 1) / kTailBlock;
+  while (true) {
+    const uint32_t nxt = cur ^ 1u;
+    const uint32_t in_smem = min(s_cnt[cur], kTailCap);
+    // entries spilled into the frontier at depth d
+    const uint32_t spilled = min(__ldcg(&ho->spill[d % 3]), a.queue_cap);
+    const uint2 *qc = s_q + cur * kTailCap;
+    // exclusive prefix of the entries' degrees; the first line of each
+    // entry's adjacency is pulled into L1 meanwhile
+    const uint32_t e0 = tid * kPer;
+    uint32_t sum = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; ++k)
+      if (e0 + k < in_smem) {
+        const uint2 r = qc[e0 + k];
+        narrow::prefetch_l1(a.cols + r.x);
+        sum += r.y - r.x;
+      }
+    uint32_t E = 0;
+    uint32_t run = block_exclusive_scan<kTailBlock>(sum, &E);
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; ++k)
+      if (e0 + k < in_smem) {
+        s_pref[e0 + k] = run;
+        run += qc[e0 + k].y - qc[e0 + k].x;
+      }
+    if (tid == 0) {
+      s_pref[in_smem] = E;
+      // the spill counter for depth d + 2 is reused: its last readers
+      // finished before the previous cluster barrier
+      if (t.rank == 0) {
+        ho->spill[(d + 2) % 3] = 0u;
+        if (a.trace && d + 2 < (uint32_t)kMaxTrace) a.trace[d + 2] = LevelTrace{0ull, 0ull, 0u, 0u};
+      }
+    }
+    __syncthreads();
+    const unsigned long long nr0 = nr, mr0 = mr;
+    if (tid == 0) s_cnt[cur] = 0;  // read by every thread above; refilled next level
+    // this thread's edges [lo, hi) of the E in shared-memory entries
+    const uint32_t lo = (uint32_t)((unsigned long long)tid * E / kTailBlock);
+    const uint32_t hi = (uint32_t)((unsigned long long)(tid + 1) * E / kTailBlock);
+    if (lo < hi) {
+      uint32_t j = 0, span = in_smem;  // largest j with s_pref[j] <= lo
+      while (span > 1) {
+        const uint32_t half = span / 2;
+        if (s_pref[j + half] <= lo) j += half;
+        span -= half;
+      }
+      uint32_t x = qc[j].x + (lo - s_pref[j]);
+      uint32_t xe = qc[j].y;
+      for (uint32_t k = lo; k < hi; k += kTailBatch) {
+        const int cnt = (int)min(hi - k, (uint32_t)kTailBatch);
+        uint32_t xs[kTailBatch];
+#pragma unroll
+        for (int r = 0; r < kTailBatch; ++r) {
+          xs[r] = x;
+          if (r < cnt && ++x == xe && k + r + 1 < hi) {
+            ++j;
+            x = qc[j].x;
+            xe = qc[j].y;
+          }
+        }
+        tail_batch(a, t, xs, cnt, d + 1, nxt, nr, mr);
+      }
+    }
+    // spilled entries (rare: a frontier beyond C * kTailCap), one vertex
+    // per thread over the whole cluster
+    if (spilled) {
+      const uint32_t *sp = a.queue[d & 1u];
+      for (uint32_t i = t.rank * kTailBlock + tid; i < spilled; i += t.C * kTailBlock) {
+        const uint32_t v = __ldcg(sp + i);
+        const uint32_t b = __ldg(a.offs + v), e = __ldg(a.offs + v + 1);
+        for (uint32_t x = b; x < e; x += kTailBatch) {
+          const int cnt = (int)min(e - x, (uint32_t)kTailBatch);
+          uint32_t xs[kTailBatch];
+#pragma unroll
+          for (int r = 0; r < kTailBatch; ++r) xs[r] = x + r;
+          tail_batch(a, t, xs, cnt, d + 1, nxt, nr, mr);
+        }
+      }
+    }
+    // the record of the level: the vertices found, as the persistent kernel has it
+    if (a.trace && d + 1 < (uint32_t)kMaxTrace) {
+      const uint32_t found = __reduce_add_sync(0xffffffffu, (uint32_t)(nr - nr0));
+      const uint32_t edges = __reduce_add_sync(0xffffffffu, (uint32_t)(mr - mr0));
+      if (lane_id() == 0 && found) {
+        atomicAdd(&a.trace[d + 1].nf, found);
+        atomicAdd(&a.trace[d + 1].mf, (unsigned long long)edges);
+      }
+    }
+    __syncthreads();
+    if (tid < t.C && s_found) *t.cl.map_shared_rank(&s_stamp, tid) = d + 1;
+    // every push and stamp of this level is visible after the barrier
+    t.cl.sync();
+    if (tid == 0) s_found = 0;  // set again at the next level, after its scan barriers
+    const bool found = s_stamp > d;  // stamps only grow: a faster CTA may already write d + 2
+    if (t.rank == 0 && tid == 0 && a.trace && d + 1 < (uint32_t)kMaxTrace)
+      a.trace[d + 1].t_ns = global_timer_ns();
+    if (!found) {
+      levels = d + 1;  // nothing at depth d + 1
+      break;
+    }
+    ++d;
+    cur = nxt;
+    if (d > a.n + 1) {
+      if (t.rank == 0 && tid == 0) atomicOr(a.err, kErrLevels);
+      levels = d;
+      break;
+    }
+  }
+  // reach counts: the persistent kernel's share (set above) plus each CTA's
+  for (int o = 16; o > 0; o >>= 1) {
+    nr += __shfl_down_sync(0xffffffffu, nr, o);
+    mr += __shfl_down_sync(0xffffffffu, mr, o);
+  }
+  if ((tid & 31u) == 0) s_red[tid >> 5] = nr;
+  __syncthreads();
+  if (tid == 0) {
+    unsigned long long v = 0;
+    for (int i = 0; i < kTailBlock / 32; ++i) v += s_red[i];
+    atomicAdd(&a.summary->nr, v);
+  }
+  __syncthreads();
+  if ((tid & 31u) == 0) s_red[tid >> 5] = mr;
+  __syncthreads();
+  if (tid == 0) {
+    unsigned long long v = 0;
+    for (int i = 0; i < kTailBlock / 32; ++i) v += s_red[i];
+    atomicAdd(&a.summary->mr, v);
+    if (t.rank == 0) {
+      a.summary->levels = levels;
+      a.summary->bu_levels = __ldcg(&ho->bu_levels);
+      a.summary->switches = __ldcg(&ho->switches);
+      a.summary->pad = d0;  // level of the hand-over
+    }
+  }
+  // no CTA leaves while another may still write its shared memory
+  t.cl.sync();
+  if (t.rank == 0 && tid == 0) ho->flag = 0u;
+}
+
+constexpr size_t kTailSmem = 2 * kTailCap * sizeof(uint2);
+
 // One cluster (narrow.cuh): the rest of a traversal whose frontier has become
 // small, handed over by bfs_persistent (returns at once otherwise), or all of
 // a traversal of a small graph.  Depths are lowered in place, so a vertex may
@@ -1120,8 +1397,32 @@ __global__ void __launch_bounds__(narrow::kBlock) bfs_narrow(Args a) {
 }
 
 int narrow_cluster() {
-  static const int c = narrow::cluster_size(bfs_narrow);
+  static const int c = narrow::cluster_size(bfs_narrow, sizeof(narrow::Shared));
   return c;
+}
+
+int tail_cluster() {
+  static const int c = narrow::cluster_size(bfs_tail, kTailSmem);
+  return c;
+}
+
+// Graphs whose tail bfs_narrow runs: few neighbours, near by id.  Its rounds
+// without a cluster barrier and its home ranges only help there (ms, bfs_tail /
+// bfs_narrow: 4,096 x 4,096 grid 34.0 / 27.3, 1,500 x 1,500 grid with a quarter
+// of the edges gone 10.2 / 8.3, path of 4,001 9.6 / 7.5); with shuffled ids, more
+// neighbours or a tree's frontier levels are unevenly spread over the homes and
+// run again (shuffled 1,000 x 1,000 grid 5.0 / 6.7, 1,000 x 1,000 mesh of 6
+// neighbours 4.2 / 6.5, of 12 3.1 / 5.2, 3,000 x 3,000 of 8 26 / 85, binary tree
+// of 4 M 1.9 / 5.8).
+constexpr uint32_t kNearDegree = 4;
+bool near_ids(const grus_graph *g) { return g->near_ids && g->max_deg <= kNearDegree; }
+
+// Regular graphs whose ids do not follow their geometry: long traversals of
+// which bfs_narrow gains nothing (path of 4,001 with shuffled ids: grid kernels
+// 8.4 ms, cluster 12.1; shuffled 150 x 140 mesh of 6 neighbours 0.59 / 0.74).
+// A random graph's largest degree is further from its mean.
+bool regular_far_ids(const grus_graph *g) {
+  return !g->near_ids && g->max_deg <= 8 && (uint64_t)g->max_deg * g->n <= 2 * g->m;
 }
 
 // CTAs an SM.  A level of a small graph is mostly its two barriers, which cost
@@ -1146,7 +1447,7 @@ int grid_ctas(const grus_graph *g, bool pull, int occ) {
 bool runs_whole(const grus_graph *g) {
   const grus_tuning &t = g->tuning;
   return t.tail_cluster != 2 && t.alpha == 0.f && t.beta == 0.f && !t.ctas_per_sm &&
-         !t.huge_degree && !t.bu_scan && !t.bu_words && !t.depth_planes &&
+         !t.huge_degree && !t.bu_scan && !t.bu_words && !t.depth_planes && !regular_far_ids(g) &&
          (g->m <= kWholeM || (g->m <= kWholeMLow && g->max_deg <= kWholeDegree));
 }
 
@@ -1250,8 +1551,9 @@ int bfs_run(grus_graph *g, uint32_t src, uint32_t *depth, grus_stats *stats, cud
   a.huge = tune_or(g->tuning.huge_degree, kDefHuge);
   a.bu_scan = tune_or(g->tuning.bu_scan,
                       g->mem_mode == GRUS_MEM_MANAGED ? kDefBuScanManaged : kDefBuScan);
-  const int ncl = narrow_cluster();
-  a.narrow_nf = g->tuning.tail_cluster == 2 ? 0u : kNarrowNf * (uint32_t)ncl;
+  const bool narrow_tail = whole || near_ids(g);
+  const int ncl = narrow_tail ? narrow_cluster() : tail_cluster();
+  a.narrow_nf = g->tuning.tail_cluster == 2 ? 0u : (narrow_tail ? kNarrowNf : kTailNf) * (uint32_t)ncl;
   a.far = w->far;
   a.whole = whole;
   a.lanes = narrow::lanes_per_entry(g->max_deg);
@@ -1289,7 +1591,8 @@ int bfs_run(grus_graph *g, uint32_t src, uint32_t *depth, grus_stats *stats, cud
   if (!whole) GRUS_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, a));
   // runs a small graph, or continues a traversal the persistent kernel handed
   // over; returns at once otherwise
-  GRUS_CUDA_TRY(narrow::launch(bfs_narrow, ncl, a, s));
+  if (narrow_tail) GRUS_CUDA_TRY(narrow::launch(bfs_narrow, ncl, sizeof(narrow::Shared), a, s));
+  else GRUS_CUDA_TRY(narrow::launch(bfs_tail, ncl, kTailSmem, a, s));
   if (stats) GRUS_CUDA_TRY(cudaEventRecord(w->ev1, s));
   if (!dev_out) GRUS_CUDA_TRY(cudaMemcpyAsync(depth, w->depth, g->n * 4, cudaMemcpyDeviceToHost, s));
   if (!sync) return GRUS_OK;

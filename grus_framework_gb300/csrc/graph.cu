@@ -196,17 +196,45 @@ static int grid_for(uint64_t work, int block = 256) {
   return (int)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)sms * 16));
 }
 
+// Edges of kNearSample vertices spread over the ids (their first kNearEdges
+// each), and how many of them end less than n / 64 (at least kNearMin) ids away: count[1],
+// count[0].
+constexpr uint32_t kNearSample = 4096, kNearEdges = 4, kNearMin = 16;
+
+static __global__ void k_near_ids(const uint32_t *__restrict__ offs,
+                                  const uint32_t *__restrict__ cols, uint64_t n, uint64_t m,
+                                  uint32_t *count) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint64_t v = (uint64_t)i * n / kNearSample;
+  const uint64_t b = offs[v], e = min(min((uint64_t)offs[v + 1], b + kNearEdges), m);
+  const uint64_t reach = max(n / 64, (uint64_t)kNearMin);
+  uint32_t near = 0;
+  for (uint64_t x = b; x < e; ++x) {
+    const uint64_t u = cols[x];
+    near += (u > v ? u - v : v - u) < reach;
+  }
+  if (near) atomicAdd(count, near);
+  if (e > b) atomicAdd(count + 1, (uint32_t)(e - b));
+}
+
 int finalize_graph(grus_graph *g) {
-  unsigned long long *d_best = nullptr, best = 0;
-  GRUS_CUDA_TRY(cudaMalloc(&d_best, sizeof(unsigned long long)));
-  cudaMemset(d_best, 0, sizeof(unsigned long long));
-  if (g->n) k_max_degree<<<grid_for(g->n), 256>>>(g->csr.offs, g->n, d_best);
-  cudaError_t e = cudaMemcpy(&best, d_best, sizeof(best), cudaMemcpyDeviceToHost);
-  cudaFree(d_best);
+  struct {
+    unsigned long long best;
+    uint32_t near, edges;
+  } h{}, *d = nullptr;
+  GRUS_CUDA_TRY(cudaMalloc(&d, sizeof(h)));
+  cudaMemset(d, 0, sizeof(h));
+  if (g->n) k_max_degree<<<grid_for(g->n), 256>>>(g->csr.offs, g->n, &d->best);
+  // (not a managed graph's columns, which would be faulted in before their advice)
+  if (g->m && g->mem_mode != GRUS_MEM_MANAGED)
+    k_near_ids<<<kNearSample / 256, 256>>>(g->csr.offs, g->csr.cols, g->n, g->m, &d->near);
+  cudaError_t e = cudaMemcpy(&h, d, sizeof(h), cudaMemcpyDeviceToHost);
+  cudaFree(d);
   GRUS_CUDA_TRY(e);
-  g->max_deg = (uint32_t)(best >> 32);
-  g->max_deg_vertex = g->n ? (uint32_t)(0xFFFFFFFFull - (best & 0xFFFFFFFFull)) : 0;
+  g->max_deg = (uint32_t)(h.best >> 32);
+  g->max_deg_vertex = g->n ? (uint32_t)(0xFFFFFFFFull - (h.best & 0xFFFFFFFFull)) : 0;
   if (g->max_deg == 0) g->max_deg_vertex = 0;
+  g->near_ids = h.edges && 10ull * h.near >= 9ull * h.edges;
   return GRUS_OK;
 }
 

@@ -54,6 +54,7 @@ struct grus_graph {
   grus::Csr csr;              // out-edges
   grus::Csr csc;              // in-edges (built on demand; aliases csr if symmetric)
   uint32_t max_deg_vertex = 0, max_deg = 0;
+  bool near_ids = false;  // most edges join ids less than n / 64 apart (sampled)
   // BFS pull index: per vertex {an in-neighbour of high out-degree (kNoRep
   // without in-edges), the vertex's out-degree}, built on demand
   // (grus::build_rep_locked)

@@ -806,11 +806,11 @@ struct Engine {
   }
 };
 
-// Launch attributes of a one-cluster kernel using Engine: the largest cluster
+// Launches of a one-cluster kernel of kBlock threads a CTA: the largest cluster
 // (16, 8, 4, 2 or 1 CTAs) the device can co-schedule.
 template <class Kernel>
-int cluster_size(Kernel kern) {
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Shared));
+int cluster_size(Kernel kern, size_t smem) {
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   for (int k = kMaxCluster; k > 1; k /= 2) {
     cudaLaunchAttribute attr;
@@ -821,7 +821,7 @@ int cluster_size(Kernel kern) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)k);
     cfg.blockDim = dim3(kBlock);
-    cfg.dynamicSmemBytes = sizeof(Shared);
+    cfg.dynamicSmemBytes = smem;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     int nc = 0;
@@ -832,7 +832,7 @@ int cluster_size(Kernel kern) {
 }
 
 template <class Kernel, class Args>
-cudaError_t launch(Kernel kern, int cluster, const Args &a, cudaStream_t s) {
+cudaError_t launch(Kernel kern, int cluster, size_t smem, const Args &a, cudaStream_t s) {
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeClusterDimension;
   attr.val.clusterDim.x = (unsigned)cluster;
@@ -841,7 +841,7 @@ cudaError_t launch(Kernel kern, int cluster, const Args &a, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)cluster);
   cfg.blockDim = dim3(kBlock);
-  cfg.dynamicSmemBytes = sizeof(Shared);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;

@@ -526,7 +526,7 @@ __global__ void __launch_bounds__(narrow::kBlock) sssp_narrow(Args a) {
 }
 
 int narrow_cluster() {
-  static const int c = narrow::cluster_size(sssp_narrow);
+  static const int c = narrow::cluster_size(sssp_narrow, sizeof(narrow::Shared));
   return c;
 }
 
@@ -631,7 +631,7 @@ int sssp_run(grus_graph *g, uint32_t src, uint32_t *dist, grus_stats *stats, cud
                            grid_ctas(g), occ, s, a.dist, (size_t)g->n * 4);
     if (rc) return rc;
   }
-  if (a.whole || a.narrow_nf) GRUS_CUDA_TRY(narrow::launch(sssp_narrow, ncl, a, s));
+  if (a.whole || a.narrow_nf) GRUS_CUDA_TRY(narrow::launch(sssp_narrow, ncl, sizeof(narrow::Shared), a, s));
   if (stats) GRUS_CUDA_TRY(cudaEventRecord(w->ev1, s));
   if (!dev_out) GRUS_CUDA_TRY(cudaMemcpyAsync(dist, w->dist, g->n * 4, cudaMemcpyDeviceToHost, s));
   if (!sync) return GRUS_OK;
