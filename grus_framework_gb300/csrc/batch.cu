@@ -649,7 +649,7 @@ static int union_sssp(grus_batch *b, const grus_query *queries, const UnionPlan 
       if (p.q.size() == 1) {
         const grus_query &q = queries[p.q[0]];
         rc = sssp_run(g, q.src, out + q.out_offset, nullptr, s, sssp_lane_tail(g));
-        *nlaunch += sssp_lane_tail(g);
+        *nlaunch += sssp_kernels(g, sssp_lane_tail(g)) - 1;
         cv = sssp_ctrl(g);
       } else {
         uint32_t srcs[32];

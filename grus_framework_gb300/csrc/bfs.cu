@@ -1336,6 +1336,7 @@ __global__ void __launch_bounds__(narrow::kBlock) bfs_narrow(Args a) {
   view.adapt = false;
   view.lanes = a.lanes;
   view.ahead = a.ahead;
+  view.hand_back = false;
   view.err = a.err;
   view.timeout_ns = a.timeout_ns;
   view.trace = (narrow::Trace *)a.trace;

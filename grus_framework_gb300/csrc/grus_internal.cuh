@@ -113,12 +113,14 @@ int bfs_run(grus_graph *g, uint32_t src, uint32_t *depth, grus_stats *stats, cud
 // Graphs whose BFS loses little by a side launch.
 bool bfs_side_ok(const grus_graph *g);
 // Single-source SSSP (sssp.cu).  tail: launch the cluster kernel behind the
-// persistent one (2 kernels, else 1); grus_sssp does where sssp_tail says so.
+// persistent one, and that one again where the traversal may come back
+// (sssp_kernels: how many kernels); grus_sssp does where sssp_tail says so.
 // The batch and the server, whose lanes queue launches back to back, do on
 // graphs without hubs (sssp_lane_tail): on scale-free graphs the cluster
 // takes over the last few levels only (0-9 % of a query).
 int sssp_run(grus_graph *g, uint32_t src, uint32_t *dist, grus_stats *stats, cudaStream_t s,
              bool tail);
+int sssp_kernels(const grus_graph *g, bool tail);
 bool sssp_tail(const grus_graph *g);
 bool sssp_lane_tail(const grus_graph *g);
 

@@ -61,6 +61,11 @@ constexpr uint32_t kPiece = 64;      // edges per entry
 // Spilled vertices: up to kWideEdges edges go to one CTA, those of more to the
 // whole cluster, kWide of them in a step.
 constexpr uint32_t kWideEdges = 1024, kWide = 128;
+// SSSP: a step that relaxes this many spilled vertices is the grid's work; the
+// traversal is handed back.  (A path of 24 vertices into a binary tree of 4 M, ids
+// in level order / shuffled: grid kernel alone 1.75 / 1.44 ms, cluster 3.4 / 5.1,
+// handed back 1.68 / 2.14.)
+constexpr uint32_t kHandBack = 1u << 17;
 // Low-degree graphs, few entries: 4 or 8 lanes per entry instead of a scan
 // over the entries' degrees (a path's round 1.57 -> 1.04 us with 512 threads;
 // entries of up to 64 edges would take 8 serial steps instead: RMAT-12 0.19
@@ -113,6 +118,7 @@ struct View {
   bool adapt;        // SSSP: delta may grow while threshold steps do little
   uint32_t lanes;    // lanes_per_entry of the graph
   bool ahead;        // low degrees, and beyond_l2
+  bool hand_back;    // SSSP: stop at a step of kHandBack spilled vertices
   uint32_t *err;
   uint64_t timeout_ns;  // a step that takes longer ends the traversal
   // null: none.  SSSP: record i is the i-th step's (from 1); BFS: record d
@@ -150,7 +156,7 @@ struct Shared {
   uint32_t claimed, refused, cur[kWarps], had;
   // rank 0, by step parity: spilled vertices that all CTAs relax together
   uint4 wide[2][kWide];
-  uint32_t nwide[2];
+  uint32_t nwide[2], nspilled[2];
   unsigned long long t_step;            // rank 0: when the last step ended
   uint32_t g_farbm, g_far;
   // this CTA's copies: far bitmap bits up to this step have been taken; the
@@ -181,6 +187,7 @@ struct Engine {
   uint32_t cq, lb, fb;        // read: cnt[cq], loc[lb], far buffer fb
   int round;                  // of the step, 0 before its first
   Result res;
+  bool handed_back = false;
 
   __device__ __forceinline__ Engine(const View &view, Shared *sh)
       : a(view), s(sh), cl(cg::this_cluster()) {
@@ -201,8 +208,8 @@ struct Engine {
     if (threadIdx.x < kRing) s->ring[threadIdx.x] = s->ring_sum[threadIdx.x] = 0;
     if (threadIdx.x == 0) {
       s->pushed = s->spilled = s->farbm = s->g_farbm = 0u;
-      s->found[0] = s->found[1] = StepWords{0u, 0u, 0u};
-      s->nwide[0] = s->nwide[1] = 0u;
+      s->found[0] = s->found[1] = StepWords{0u, 0u, 0u, 0u};
+      s->nwide[0] = s->nwide[1] = s->nspilled[0] = s->nspilled[1] = 0u;
       s->t_step = global_timer_ns();
       s->g_far = 0u;
       s->scanned = s->last_split = 0u;
@@ -490,7 +497,15 @@ struct Engine {
     if (!s->had) {
       take_words();
       __syncthreads();
-      if (s->claimed) return min(s->claimed, s->refused);
+      if (s->claimed) {
+        const uint32_t count = min(s->claimed, s->refused);
+        if (!kUnit && a.hand_back && threadIdx.x == 0) {
+          Shared *r = cl.map_shared_rank(s, 0);
+          if (atomicAdd(&r->nspilled[step & 1u], count) + count >= kHandBack)
+            *(volatile uint32_t *)&words_of(r->found, step).many = step;
+        }
+        return count;
+      }
       cl.sync();  // the wide list is complete
     }
     return take_wide();
@@ -662,9 +677,31 @@ struct Engine {
     return true;
   }
 
+  // SSSP: what waits in the lists goes to the bitmaps: near vertices to those of
+  // the step that ended, far ones to the far bitmap.
+  __device__ __forceinline__ void give_back() {
+    uint32_t *near = near_of(step - 1);
+    const uint32_t nc = min(s->cnt[cq], kCap), ni = min(s->incnt[ip()], kCap);
+    for (uint32_t i = threadIdx.x; i < nc + ni; i += kBlock) {
+      const uint32_t v = (i < nc ? s->loc[lb][i] : s->inb[ip()][i - nc]).x;
+      atomicOr(near + (v >> 5), 1u << (v & 31u));
+    }
+    const uint2 *far = a.far + (size_t)(rank * 2 + fb) * a.far_cap;
+    const uint32_t nf = min(s->farcnt[fb], a.far_cap);
+    for (uint32_t i = threadIdx.x; i < nf; i += kBlock) {
+      const uint32_t v = __ldcg(far + i).x;
+      atomicOr(a.farbm + (v >> 5), 1u << (v & 31u));
+    }
+  }
+
+  // What the cluster found in a step.
+  struct Found {
+    bool work, spilled, late, many;
+  };
+
   // After a round: the pushes made before the call become readable by their
-  // readers; true if any CTA has near work.
-  __device__ __forceinline__ bool end_step(bool &spilled, bool &late) {
+  // readers.
+  __device__ __forceinline__ Found end_step() {
     if (threadIdx.x == 0) {
       Shared *r = cl.map_shared_rank(s, 0);
       volatile StepWords *w = &words_of(r->found, step);
@@ -678,18 +715,17 @@ struct Engine {
     if (threadIdx.x >= 32 && threadIdx.x < 32 + kRounds)
       away_in(s->away, step + 1, threadIdx.x - 32) = 0u;
     if (rank == 0 && threadIdx.x == 64) {
-      s->nwide[(step + 1) & 1u] = 0u;
+      s->nwide[(step + 1) & 1u] = s->nspilled[(step + 1) & 1u] = 0u;
       const unsigned long long t = global_timer_ns();
       if (t - s->t_step > a.timeout_ns) words_of(s->found, step).late = step;
       s->t_step = t;
     }
     cl.sync();
-    const volatile StepWords *w = &words_of(cl.map_shared_rank(s, 0)->found, step);
-    spilled = found(w->spilled, step);
-    late = found(w->late, step);
-    const bool work = found(w->work, step);
+    const StepWords w = words_of(cl.map_shared_rank(s, 0)->found, step);  // one load
+    const Found f{found(w.work, step), found(w.spilled, step), found(w.late, step),
+                  !kUnit && found(w.many, step)};
     ++step;
-    return work || spilled;
+    return f;
   }
 
   __device__ __forceinline__ void next_round() {
@@ -704,13 +740,17 @@ struct Engine {
   __device__ __forceinline__ void run() {
     next_round();
     while (true) {
-      bool spilled = false, late = false;
-      const bool work = end_step(spilled, late);
-      if (late) {
+      const Found f = end_step();
+      if (f.late) {
         if (rank == 0 && threadIdx.x == 0) atomicOr(a.err, kErrTimeout);
         break;
       }
-      if (!work) {
+      if (f.many) {
+        give_back();
+        handed_back = true;
+        break;
+      }
+      if (!f.work && !f.spilled) {
         if (!split()) break;
         next_round();
       }
@@ -720,7 +760,7 @@ struct Engine {
       for (round = 0; round < kRounds; ++round) {
         uint32_t nc = min(s->cnt[cq], kCap);
         uint32_t total = nc + (round == 0 ? min(s->incnt[ip()], kCap) : 0u);
-        const bool scan = round == 0 && spilled;
+        const bool scan = round == 0 && f.spilled;
         if (total == 0 && !scan) break;
         // ids that jump between homes: most of this step's pushes wait in
         // other CTAs' inboxes, and further rounds over the rest only delay them

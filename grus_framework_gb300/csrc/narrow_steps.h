@@ -24,10 +24,11 @@ namespace narrow {
 // step's before another thread reads this step's -- which are others -- but not
 // those of the step after that: its barrier in between waits for that thread.
 // A word holds an older step's number until it is written, so nobody clears it.
-struct StepWords {
+struct alignas(16) StepWords {
   uint32_t work;     // some CTA has near work left
   uint32_t spilled;  // some list was full: vertices wait in the near bitmap
   uint32_t late;     // the step took longer than the time limit
+  uint32_t many;     // it relaxed so many spilled vertices that the grid should
 };
 
 GRUS_HD bool found(uint32_t word, uint32_t step) { return word == step; }

@@ -287,9 +287,10 @@ int big_launch(grus_server *s, BigJob &j) {
              : msbfs_run(g, srcs, (int)j.group.size(), outs, nullptr, s->big_stream);
   }
   if (rc) return rc;
-  // a single query is one kernel and, for BFS and where sssp_lane_tail says
-  // so, the narrow one behind it; a pack is one kernel
-  s->kernel_launches += !multi && (r.algo != GRUS_ALGO_SSSP || sssp_lane_tail(g)) ? 2 : 1;
+  // a single BFS is the persistent kernel and the narrow one behind it; a pack is
+  // one kernel
+  s->kernel_launches +=
+      multi ? 1 : (r.algo == GRUS_ALGO_SSSP ? sssp_kernels(g, sssp_lane_tail(g)) : 2);
   j.ctrl = r.algo == GRUS_ALGO_SSSP ? (multi ? msssp_ctrl(g) : sssp_ctrl(g))
                                     : (multi ? msbfs_ctrl(g) : bfs_ctrl(g));
   *j.h_err = 0;

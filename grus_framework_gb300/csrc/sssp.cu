@@ -94,10 +94,10 @@ struct LevelTrace {
   uint32_t frontier, splits;
 };
 
-// Hand-over from the persistent kernel to sssp_narrow.
+// Hand-over from the persistent kernel to sssp_narrow, and back.
 constexpr int kMaxTries = 4;
 struct Handover {
-  uint32_t flag;                     // 1: sssp_narrow continues the traversal
+  uint32_t flag;                     // 1: sssp_narrow continues the traversal, 2: the grid again
   uint32_t qcount;                   // vertices of the near set (Args::queue)
   uint32_t T, pad;                   // threshold; near[0] and near[1] are all zero
   // by attempt: out-edges of the vertices that are not below the threshold,
@@ -133,6 +133,8 @@ struct Args {
   bool narrow_adapt;      // no Delta set by the caller
   uint2 *far;             // its far lists
   bool whole;             // sssp_narrow runs the whole traversal
+  bool hand_back;         // the grid may have to go on after sssp_narrow ...
+  bool resume;            // ... and does in this launch, if flag is 2
   uint32_t max_deg;       // of the graph
   uint32_t lanes;         // narrow::lanes_per_entry
   bool ahead;             // narrow::View::ahead
@@ -305,29 +307,36 @@ __global__ void __launch_bounds__(kBlock, 8) sssp_persistent(Args a) {
   }
   const uint32_t gtid = blockIdx.x * kBlock + threadIdx.x;
   const uint32_t nthreads = gridDim.x * kBlock;
+  if (a.resume && __ldcg(&a.ho->flag) != 2u) return;  // the same answer in every CTA
   // prologue: distances to INFINIT, bitmaps and control words to zero
-  for (uint32_t i = gtid; i < a.n; i += nthreads) a.dist[i] = kInfinit;
-  for (uint32_t i = gtid; i < a.W; i += nthreads) {
-    a.near[0][i] = 0u;
-    a.near[1][i] = 0u;
-    a.farbm[i] = 0u;
+  if (!a.resume) {
+    for (uint32_t i = gtid; i < a.n; i += nthreads) a.dist[i] = kInfinit;
+    for (uint32_t i = gtid; i < a.W; i += nthreads) {
+      a.near[0][i] = 0u;
+      a.near[1][i] = 0u;
+      a.farbm[i] = 0u;
+    }
+    if (gtid < 4 * sizeof(Slot) / 4) ((uint32_t *)a.slots)[gtid] = 0u;
+    if (gtid < sizeof(FarCtl) / 4) ((uint32_t *)a.farctl)[gtid] = 0u;
+    if (gtid < sizeof(Handover) / 4) ((uint32_t *)a.ho)[gtid] = 0u;
+    if (gtid == 0) {
+      a.farctl->minfar[0] = 0xFFFFFFFFu;
+      a.farctl->minfar[1] = 0xFFFFFFFFu;
+    }
+    if (!grid_sync(a.bar, a.err, a.timeout_ns)) return;
+    if (gtid == 0) {
+      a.dist[a.src] = 0;
+      a.near[0][a.src >> 5] = 1u << (a.src & 31u);
+    }
+    if (!grid_sync(a.bar, a.err, a.timeout_ns)) return;
   }
-  if (gtid < 4 * sizeof(Slot) / 4) ((uint32_t *)a.slots)[gtid] = 0u;
-  if (gtid < sizeof(FarCtl) / 4) ((uint32_t *)a.farctl)[gtid] = 0u;
-  if (gtid < sizeof(Handover) / 4) ((uint32_t *)a.ho)[gtid] = 0u;
-  if (gtid == 0) {
-    a.farctl->minfar[0] = 0xFFFFFFFFu;
-    a.farctl->minfar[1] = 0xFFFFFFFFu;
-  }
-  if (!grid_sync(a.bar, a.err, a.timeout_ns)) return;
-  if (gtid == 0) {
-    a.dist[a.src] = 0;
-    a.near[0][a.src >> 5] = 1u << (a.src & 31u);
-  }
-  if (!grid_sync(a.bar, a.err, a.timeout_ns)) return;
 
   uint32_t L = 0, T = a.delta, splits = 0;
-  if (gtid == 0 && a.trace) a.trace[0] = LevelTrace{global_timer_ns(), 0ull, 1u, 0u};
+  if (a.resume) {
+    L = __ldcg(&a.summary->levels);
+    T = __ldcg(&a.ho->T);
+    splits = __ldcg(&a.summary->splits);
+  } else if (gtid == 0 && a.trace) a.trace[0] = LevelTrace{global_timer_ns(), 0ull, 1u, 0u};
   while (true) {
     Slot *sl = a.slots + (L & 3u);
     if (gtid < sizeof(Slot) / 4) ((uint32_t *)(a.slots + ((L + 2) & 3u)))[gtid] = 0u;
@@ -463,6 +472,7 @@ __global__ void __launch_bounds__(narrow::kBlock) sssp_narrow(Args a) {
   view.adapt = a.narrow_adapt;
   view.lanes = a.lanes;
   view.ahead = a.ahead;
+  view.hand_back = a.hand_back;
   view.err = a.err;
   view.timeout_ns = a.timeout_ns;
   const uint32_t L0 = a.whole ? 0u : __ldcg(&a.summary->levels);
@@ -508,15 +518,31 @@ __global__ void __launch_bounds__(narrow::kBlock) sssp_narrow(Args a) {
     }
   }
   E.run();
+  if (E.handed_back) {
+    // level L's near set is near[L & 1]; the last step's is near[(step - 1) & 1]
+    uint32_t L = L0 + E.res.steps;
+    L += (L ^ (E.step - 1)) & 1u;
+    if (tid < 4 * sizeof(Slot) / 4) ((uint32_t *)a.slots)[tid] = 0u;
+    if (tid == 0) {
+      a.farctl->moved = a.farctl->remaining = 0u;
+      a.farctl->minfar[0] = a.farctl->minfar[1] = 0xFFFFFFFFu;
+      a.summary->levels = L;
+      a.summary->splits = view.tag + E.res.splits;
+      a.summary->nr = a.summary->mr = 0ull;  // counted at the end
+      a.ho->T = E.T;
+      a.ho->flag = 2u;
+    }
+  }
   if (!a.trace) return;
   const unsigned long long bv = E.block_sum(E.res.visits);
   if (threadIdx.x == 0) {
     atomicAdd(&a.summary->visits, bv);
-    if (E.rank == 0) {
+    if (E.rank == 0 && !E.handed_back) {
       a.summary->levels = L0 + E.res.steps;
       a.summary->splits = view.tag + E.res.splits;
     }
   }
+  if (E.handed_back) return;
   const unsigned long long bnr = E.block_sum(E.res.nr);
   const unsigned long long bmr = E.block_sum(E.res.mr);
   if (threadIdx.x == 0) {
@@ -553,6 +579,11 @@ bool runs_whole(const grus_graph *g) {
 bool sssp_tail(const grus_graph *g) {
   return !runs_whole(g) && g->tuning.tail_cluster != 2;
 }
+
+// Whether the cluster may be left with more than it should finish.
+static bool may_return(const grus_graph *g) { return g->max_deg <= kLongDegree; }
+
+int sssp_kernels(const grus_graph *g, bool tail) { return tail ? (may_return(g) ? 3 : 2) : 1; }
 
 bool sssp_lane_tail(const grus_graph *g) { return sssp_tail(g) && g->max_deg <= kWholeDegree; }
 
@@ -617,6 +648,7 @@ int sssp_run(grus_graph *g, uint32_t src, uint32_t *dist, grus_stats *stats, cud
   a.narrow_delta = std::max(1u, tune_or(g->tuning.sssp_delta, kNarrowDelta));
   a.narrow_adapt = g->tuning.sssp_delta == 0;
   a.whole = runs_whole(g);
+  a.hand_back = tail && may_return(g);
 
   const bool sync = stats != nullptr || !dev_out;
   // barrier, error word and summary: a timed-out launch leaves stale barrier state
@@ -632,6 +664,13 @@ int sssp_run(grus_graph *g, uint32_t src, uint32_t *dist, grus_stats *stats, cud
     if (rc) return rc;
   }
   if (a.whole || a.narrow_nf) GRUS_CUDA_TRY(narrow::launch(sssp_narrow, ncl, sizeof(narrow::Shared), a, s));
+  if (a.hand_back) {
+    a.resume = true;
+    a.narrow_nf = 0u;
+    rc = launch_persistent((const void *)kern, args, kBlock,
+                           grid_ctas(g), occ, s, a.dist, (size_t)g->n * 4);
+    if (rc) return rc;
+  }
   if (stats) GRUS_CUDA_TRY(cudaEventRecord(w->ev1, s));
   if (!dev_out) GRUS_CUDA_TRY(cudaMemcpyAsync(dist, w->dist, g->n * 4, cudaMemcpyDeviceToHost, s));
   if (!sync) return GRUS_OK;
@@ -651,7 +690,7 @@ int sssp_run(grus_graph *g, uint32_t src, uint32_t *dist, grus_stats *stats, cud
     std::memset(stats, 0, sizeof(*stats));
     stats->levels = sm->levels;
     stats->direction_switches = sm->splits;  // threshold advances
-    stats->kernel_launches = tail ? 2 : 1;
+    stats->kernel_launches = sssp_kernels(g, tail);
     stats->vertices_reached = sm->nr;
     stats->edges_reached = sm->mr;
     stats->edges_relaxed = sm->visits;
