@@ -382,14 +382,15 @@ __global__ void __launch_bounds__(kBatchBlock, 4) batch_kernel(Args a) {
 using namespace batch;
 
 // Clusters of up to 16 CTAs: sizes above the portable 8 need an opt-in per
-// kernel (set once per process).
+// kernel (set once per device).
 static int allow_wide_clusters() {
-  static int done = 0;
-  if (!done) {
+  static PerDevice<int> set;
+  int done = 0;
+  return set.get(current_device(), &done, [](int &v) -> int {
     GRUS_CUDA_TRY(cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    done = 1;
-  }
-  return GRUS_OK;
+    v = 1;
+    return GRUS_OK;
+  });
 }
 
 int batch_occupancy(int cluster, int *workers) {

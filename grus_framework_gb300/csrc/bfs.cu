@@ -1398,12 +1398,22 @@ __global__ void __launch_bounds__(narrow::kBlock) bfs_narrow(Args a) {
 }
 
 int narrow_cluster() {
-  static const int c = narrow::cluster_size(bfs_narrow, sizeof(narrow::Shared));
+  static PerDevice<int> sizes;
+  int c = 1;
+  sizes.get(current_device(), &c, [](int &v) {
+    v = narrow::cluster_size(bfs_narrow, sizeof(narrow::Shared));
+    return 0;
+  });
   return c;
 }
 
 int tail_cluster() {
-  static const int c = narrow::cluster_size(bfs_tail, kTailSmem);
+  static PerDevice<int> sizes;
+  int c = 1;
+  sizes.get(current_device(), &c, [](int &v) {
+    v = narrow::cluster_size(bfs_tail, kTailSmem);
+    return 0;
+  });
   return c;
 }
 

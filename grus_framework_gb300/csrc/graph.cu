@@ -48,6 +48,11 @@ int status_from_device_error(uint32_t bits) {
   return GRUS_OK;
 }
 
+int current_device() {
+  int dev = -1;
+  return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;
+}
+
 int device_sm_count() {
   static int cached[64] = {0};
   int dev = 0;

@@ -12,6 +12,7 @@
 
 #include "device_util.cuh"
 #include "grus.h"
+#include "per_device.h"
 
 namespace grus {
 
@@ -71,6 +72,7 @@ namespace grus {
 int graph_alloc_array(grus_graph *g, void **p, size_t bytes);
 void graph_free_array(grus_graph *g, void *p);
 int device_sm_count();
+int current_device();  // -1: none
 int l2_window(cudaStream_t s, void *base, size_t bytes);
 // Share of a window of `bytes` that may persist: 1, or the persisting L2
 // set-aside over the window when the window is larger (persisting lines

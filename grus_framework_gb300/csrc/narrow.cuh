@@ -847,7 +847,8 @@ struct Engine {
 };
 
 // Launches of a one-cluster kernel of kBlock threads a CTA: the largest cluster
-// (16, 8, 4, 2 or 1 CTAs) the device can co-schedule.
+// (16, 8, 4, 2 or 1 CTAs) the current device can co-schedule.  Sets the kernel's
+// attributes on that device.
 template <class Kernel>
 int cluster_size(Kernel kern, size_t smem) {
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

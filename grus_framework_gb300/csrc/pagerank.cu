@@ -530,15 +530,18 @@ void make_plan(grus_graph *g, Workspace *w, cudaStream_t s) {
 
 template <bool kHot>
 int launch(Workspace *w, Args &a, cudaStream_t s) {
-  static int occ = -1;
+  static PerDevice<int> fits;
   constexpr size_t batches = (size_t)(kBlock / 32) * kBatch * 4;
   const size_t smem = batches + (kHot ? (size_t)(a.hot + 31) / 32 * 128 : 0);
-  if (occ < 0) {
+  int occ = 0;
+  const int rc = fits.get(current_device(), &occ, [](int &v) -> int {
     constexpr size_t most = batches + (kHot ? (size_t)std::max(kHotAll, kHotCap) * 4 : 0);
     GRUS_CUDA_TRY(cudaFuncSetAttribute(pr_persistent<kHot>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
-    GRUS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pr_persistent<kHot>, kBlock, most));
-  }
+    GRUS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, pr_persistent<kHot>, kBlock, most));
+    return GRUS_OK;
+  });
+  if (rc) return rc;
   // small graphs take fewer CTAs: the barrier of each iteration is cheaper
   const uint64_t work = (uint64_t)a.m + (uint64_t)kVertexCost * a.n;
   const int ctas = (int)std::min<uint64_t>(

@@ -552,7 +552,12 @@ __global__ void __launch_bounds__(narrow::kBlock) sssp_narrow(Args a) {
 }
 
 int narrow_cluster() {
-  static const int c = narrow::cluster_size(sssp_narrow, sizeof(narrow::Shared));
+  static PerDevice<int> sizes;
+  int c = 1;
+  sizes.get(current_device(), &c, [](int &v) {
+    v = narrow::cluster_size(sssp_narrow, sizeof(narrow::Shared));
+    return 0;
+  });
   return c;
 }
 
