@@ -41,6 +41,7 @@
 #include "expand.cuh"
 #include "grus_internal.cuh"
 #include "msssp_core.cuh"
+#include "side_streams.h"
 #include "union_plan.h"
 
 namespace cg = cooperative_groups;
@@ -971,20 +972,15 @@ struct Sides {
   grus_batch *b;
   cudaStream_t s;
   bool on = false;
-  int next = 0;
-  uint32_t last = 0xFFFFFFFFu;
+  SideStreams streams{grus_batch::kSide};
 
   Sides(grus_batch *batch, cudaStream_t stream) : b(batch), s(stream) {}
   // Whether the run has launches for them, given which queries are singles.
-  bool wanted(const grus_query *q, const std::vector<int> &singles) const {
-    uint32_t graphs = 0, prev = 0xFFFFFFFFu;
-    for (int qi : singles) {
-      if (q[qi].graph == prev || !bfs_side_ok(b->graphs[q[qi].graph])) continue;
-      prev = q[qi].graph;
-      ++graphs;
-    }
+  bool wanted(const grus_query *q, const std::vector<int> &singles) {
+    for (int qi : singles)
+      if (bfs_side_ok(b->graphs[q[qi].graph])) streams.of(b->graphs[q[qi].graph]);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (graphs < 2) return false;
+    if (streams.graphs() < 2) return false;
     if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
       cudaGetLastError();
       return false;
@@ -1002,11 +998,7 @@ struct Sides {
     on = true;
     return GRUS_OK;
   }
-  cudaStream_t of(uint32_t graph) {
-    if (graph != last) next = (next + 1) % grus_batch::kSide;
-    last = graph;
-    return b->side[next];
-  }
+  cudaStream_t of(uint32_t graph) { return b->side[streams.of(b->graphs[graph])]; }
   int join() {
     if (!on) return GRUS_OK;
     on = false;
