@@ -583,11 +583,13 @@ struct grus_batch {
   cudaGraphExec_t exec = nullptr;
   uint32_t graph_ntasks = 0, graph_nmembers = 0;
   uint32_t *graph_out = nullptr;
+  int graph_workers = 0;
   cudaStream_t graph_stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaEvent_t done = nullptr;  // last run's work (staging may be rewritten after it)
   // big graphs' BFS launches, side by side
   static constexpr int kSide = 4;
+  int slots = 0;  // CTAs of such launches and of the workers, in any mix, that fit an SM
   cudaStream_t side[kSide] = {};
   cudaEvent_t fork = nullptr, join[kSide] = {};
   bool in_flight = false;
@@ -740,6 +742,10 @@ int grus_batch_create(grus_graph *const *graphs, int ngraphs, const grus_batch_c
   }
   if (!rc) {
     b->workers = b->workers ? std::min(b->workers, maxw) : maxw;
+    int occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_kernel, kBatchBlock, 0) != cudaSuccess)
+      cudaGetLastError();
+    b->slots = std::min(occ, bfs_side_fit());
     rc = b->state.reserve(b->workers, b->max_n, b->max_m, b->huge);
   }
   cudaError_t e = cudaSuccess;
@@ -966,17 +972,24 @@ static bool pack_small(const grus_batch *b, const grus_query *q, int nq, cudaStr
 // different graphs run side by side with one CTA an SM each (such a BFS waits at
 // barriers most of its time; 8 graphs of scales 16 to 19, one query each: 667 us
 // one by one, 387 / 264 on 2 / 4 streams).  They start after what the caller's
-// stream holds, and it waits for all of them.  Under capture everything stays on
+// stream holds, and it waits for all of them: before the workers' kernel, or
+// after it where plan_sides finds room for both (12 graphs of scales 14 to 19, 6
+// SSSP and 2 BFS queries each: 5.1-5.5 ms, 4.8-5.1 beside the workers; 3 BFS queries
+// each on scales 13 to 18: 1.27-1.33, 0.91-1.25).  Under capture everything stays on
 // that stream.
 struct Sides {
   grus_batch *b;
   cudaStream_t s;
   bool on = false;
   SideStreams streams{grus_batch::kSide};
+  SidePlan plan{};
 
   Sides(grus_batch *batch, cudaStream_t stream) : b(batch), s(stream) {}
   // Whether the run has launches for them, given which queries are singles.
-  bool wanted(const grus_query *q, const std::vector<int> &singles) {
+  bool wanted(const grus_query *q, const std::vector<int> &singles, int tasks) {
+    plan = plan_sides(grus_batch::kSide, b->slots, device_sm_count(), b->cluster, b->workers, tasks);
+    if (plan.streams < 2) return false;
+    streams.limit(plan.streams);
     for (int qi : singles)
       if (bfs_side_ok(b->graphs[q[qi].graph])) streams.of(b->graphs[q[qi].graph]);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -1066,8 +1079,8 @@ int grus_batch_run(grus_batch *b, const grus_query *queries, int nq, uint32_t *o
   const uint32_t *msrc = nm ? b->d_msrc : nullptr;
   const unsigned long long *moff = nm ? b->d_moff : nullptr;
   if (stats) GRUS_CUDA_TRY(cudaEventRecord(b->ev0, s));
-  // queries on big graphs: whole-GPU launches queued first on the stream, and
-  // BFS launches beside it, which the workers' tasks need not wait for
+  // queries on big graphs: whole-GPU launches queued first on the stream, then BFS
+  // launches beside one another and, where there is room, beside the workers' kernel
   Sides sides(b, s);
   uint32_t nerr = 0;
   uint32_t nlaunch = 0;  // kernels launched by the big-graph lane
@@ -1120,7 +1133,7 @@ int grus_batch_run(grus_batch *b, const grus_query *queries, int nq, uint32_t *o
       i = j;
     }
     // the singles: whole-GPU launches first, then those that run side by side
-    const bool beside = sides.wanted(queries, singles);
+    const bool beside = sides.wanted(queries, singles, (int)nt);
     for (int pass = 0; pass < 2; ++pass) {
       if (pass == 1) {
         if (!beside) break;
@@ -1138,10 +1151,13 @@ int grus_batch_run(grus_batch *b, const grus_query *queries, int nq, uint32_t *o
         if (rc) return rc;
       }
     }
+    if (!sides.plan.beside) {
+      rc = sides.join();
+      if (rc) return rc;
+    }
   }
+  const int workers = sides.on ? sides.plan.workers : b->workers;
   if (nt == 0) {
-    rc = sides.join();
-    if (rc) return rc;
     // every query was on a big graph
     if (stats) GRUS_CUDA_TRY(cudaEventRecord(b->ev1, s));
     GRUS_CUDA_TRY(cudaEventRecord(b->done, s));
@@ -1165,7 +1181,7 @@ int grus_batch_run(grus_batch *b, const grus_query *queries, int nq, uint32_t *o
     // one captured graph per (task count, output buffer): H2D copy of the
     // staged tasks, counter reset, batch kernel
     if (b->exec && (b->graph_ntasks != nt || b->graph_nmembers != nm || b->graph_out != out ||
-                    b->graph_stream != s))
+                    b->graph_stream != s || b->graph_workers != workers))
       drop_graph(b);
     if (!b->exec) {
       cudaStream_t cap_s = nullptr;
@@ -1178,7 +1194,7 @@ int grus_batch_run(grus_batch *b, const grus_query *queries, int nq, uint32_t *o
           cudaMemcpyAsync(b->d_moff, b->h_moff, nm * 8, cudaMemcpyHostToDevice, cap_s);
         }
         cudaMemsetAsync(b->state.counter, 0, 4, cap_s);
-        rc = batch_launch(b->state, 0, b->workers, b->cluster, b->d_graphs, b->d_tasks, nt, out,
+        rc = batch_launch(b->state, 0, workers, b->cluster, b->d_graphs, b->d_tasks, nt, out,
                           b->huge, b->delta, b->state.counter, cap_s, msrc, moff);
         e = cudaStreamEndCapture(cap_s, &b->graph);
       }
@@ -1190,6 +1206,7 @@ int grus_batch_run(grus_batch *b, const grus_query *queries, int nq, uint32_t *o
       b->graph_nmembers = nm;
       b->graph_out = out;
       b->graph_stream = s;
+      b->graph_workers = workers;
     }
     GRUS_CUDA_TRY(cudaGraphLaunch(b->exec, s));
   } else {
@@ -1199,7 +1216,7 @@ int grus_batch_run(grus_batch *b, const grus_query *queries, int nq, uint32_t *o
       GRUS_CUDA_TRY(cudaMemcpyAsync(b->d_moff, b->h_moff, nm * 8, cudaMemcpyHostToDevice, s));
     }
     GRUS_CUDA_TRY(cudaMemsetAsync(b->state.counter, 0, 4, s));
-    rc = batch_launch(b->state, 0, b->workers, b->cluster, b->d_graphs, b->d_tasks, nt, out, b->huge,
+    rc = batch_launch(b->state, 0, workers, b->cluster, b->d_graphs, b->d_tasks, nt, out, b->huge,
                       b->delta, b->state.counter, s, msrc, moff);
     if (rc) return rc;
   }

@@ -1474,6 +1474,21 @@ bool bfs_side_ok(const grus_graph *g) {
          ((g->flags & GRUS_GRAPH_SYMMETRIC) || g->csc.offs);
 }
 
+int bfs_side_fit() {
+  int fit = 8;
+  auto least = [&](auto kern) {
+    int occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kBlock, 0) != cudaSuccess)
+      cudaGetLastError();
+    fit = std::min(fit, occ);
+  };
+  least(bfs_persistent<2, false>);
+  least(bfs_persistent<2, true>);
+  least(bfs_persistent<4, false>);
+  least(bfs_persistent<4, true>);
+  return fit;
+}
+
 int bfs_run(grus_graph *g, uint32_t src, uint32_t *depth, grus_stats *stats, cudaStream_t s,
             bool whole_ok, bool side) {
   if (!g || !depth) return GRUS_EINVAL;

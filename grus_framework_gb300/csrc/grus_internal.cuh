@@ -108,10 +108,12 @@ int msssp_run(grus_graph *g, const uint32_t *hsrc, int k, uint32_t *const *outs,
 // Single-source BFS (bfs.cu): two kernels, or one where whole_ok and the graph
 // is small.  grus_bfs allows it; the batch and the server, whose small graphs
 // run on cluster workers anyway, keep the two.  side: with one CTA an SM, to run
-// beside up to three like it; four of them fit the GPU whatever the order in
-// which their CTAs start, so none waits at a barrier for CTAs that find no room.
+// beside others like it: as many as bfs_side_fit fit the GPU whatever the order
+// in which their CTAs start, so none waits at a barrier for CTAs that find no room.
 int bfs_run(grus_graph *g, uint32_t src, uint32_t *depth, grus_stats *stats, cudaStream_t s,
             bool whole_ok, bool side = false);
+// CTAs of a side launch that fit an SM by themselves.
+int bfs_side_fit();
 // Graphs whose BFS loses little by a side launch.
 bool bfs_side_ok(const grus_graph *g);
 // Single-source SSSP (sssp.cu).  tail: launch the cluster kernel behind the

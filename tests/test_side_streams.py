@@ -33,3 +33,43 @@ def test_one_stream_per_handle(tmp_path):
         assert streams.setdefault(graph, stream) == stream
     assert [streams[i] for i in range(7)] == [0, 1, 2, 3, 0, 1, 2]
     assert int(count) == 7
+
+
+PLAN = r"""
+#include <cstdio>
+#include "side_streams.h"
+int main() {
+  int a[6];
+  while (std::scanf("%d %d %d %d %d %d", a, a + 1, a + 2, a + 3, a + 4, a + 5) == 6) {
+    const grus::SidePlan p = grus::plan_sides(a[0], a[1], a[2], a[3], a[4], a[5]);
+    std::printf("%d %d %d\n", p.streams, p.workers, (int)p.beside);
+  }
+  return 0;
+}
+"""
+
+
+def test_side_launches_fit_beside_the_workers(tmp_path):
+    """Side launches of one CTA an SM and the workers' CTAs never need more slots
+    than there are, whatever the order in which they start."""
+    (tmp_path / "p.cpp").write_text(PLAN)
+    exe = tmp_path / "p"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", str(ROOT / "grus_framework_gb300" / "csrc"),
+                    str(tmp_path / "p.cpp"), "-o", str(exe)], check=True)
+    cases = [(4, per_sm, 152, cluster, per_sm * 152 // cluster, tasks)
+             for per_sm in (0, 1, 2, 3, 4, 8) for cluster in (1, 3, 8, 16)
+             for tasks in (0, 1, 5, 9, 10, 19, 20, 38, 39, 500)]
+    out = subprocess.run([str(exe)], input="\n".join(" ".join(map(str, c)) for c in cases),
+                         capture_output=True, text=True, check=True).stdout.splitlines()
+    assert len(out) == len(cases)
+    seen = set()
+    for (most, per_sm, sms, cluster, workers, tasks), line in zip(cases, out):
+        k, w, beside = map(int, line.split())
+        assert 0 <= k <= min(most, per_sm)
+        if beside:
+            assert k >= 2 and 1 <= w <= workers and tasks <= 2 * w
+            assert k * sms + w * cluster <= per_sm * sms
+        else:
+            assert w == workers
+        seen.add((k, beside))
+    assert {(4, 0), (3, 1), (2, 1)} <= seen
