@@ -158,22 +158,46 @@ __global__ void k_fill_u32(uint32_t *__restrict__ a, uint64_t m, uint32_t v) {
     a[i] = v;
 }
 
+// What finalize_graph finds out about a graph.
+struct Shape {
+  unsigned long long best;        // packed key of the max out-degree vertex
+  unsigned long long edges[32];   // as grus_graph::deg_edges and deg_count
+  uint32_t count[32];
+  uint32_t near, sampled;         // k_near_ids
+};
+
 // Max out-degree vertex, first index on ties (include/graph_loader.cuh:132-137):
-// packed key (degree << 32) | ~index, reduced with atomicMax.
-__global__ void k_max_degree(const uint32_t *__restrict__ offs, uint64_t n,
-                             unsigned long long *__restrict__ best) {
+// packed key (degree << 32) | ~index, reduced with atomicMax.  And the vertices
+// and edges by the degree's power of two.
+__global__ void k_degrees(const uint32_t *__restrict__ offs, uint64_t n, Shape *shape) {
+  __shared__ unsigned long long s_edges[32];
+  __shared__ uint32_t s_count[32];
+  if (threadIdx.x < 32) {
+    s_edges[threadIdx.x] = 0ull;
+    s_count[threadIdx.x] = 0u;
+  }
+  __syncthreads();
   unsigned long long local = 0;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x) {
-    const unsigned long long d = offs[i + 1] - offs[i];
-    const unsigned long long key = (d << 32) | (0xFFFFFFFFull - i);
+    const uint32_t d = offs[i + 1] - offs[i];
+    const unsigned long long key = ((unsigned long long)d << 32) | (0xFFFFFFFFull - i);
     local = key > local ? key : local;
+    if (d) {
+      atomicAdd(&s_count[31 - __clz(d)], 1u);
+      atomicAdd(&s_edges[31 - __clz(d)], (unsigned long long)d);
+    }
   }
   for (int o = 16; o > 0; o >>= 1) {
     const unsigned long long t = __shfl_down_sync(0xffffffffu, local, o);
     local = t > local ? t : local;
   }
-  if ((threadIdx.x & 31) == 0) atomicMax(best, local);
+  if ((threadIdx.x & 31) == 0) atomicMax(&shape->best, local);
+  __syncthreads();
+  if (threadIdx.x < 32 && s_count[threadIdx.x]) {
+    atomicAdd(&shape->count[threadIdx.x], s_count[threadIdx.x]);
+    atomicAdd(&shape->edges[threadIdx.x], s_edges[threadIdx.x]);
+  }
 }
 
 // One CTA enters the persistent kernels' grid barrier; the host presets its
@@ -223,23 +247,22 @@ static __global__ void k_near_ids(const uint32_t *__restrict__ offs,
 }
 
 int finalize_graph(grus_graph *g) {
-  struct {
-    unsigned long long best;
-    uint32_t near, edges;
-  } h{}, *d = nullptr;
+  Shape h{}, *d = nullptr;
   GRUS_CUDA_TRY(cudaMalloc(&d, sizeof(h)));
   cudaMemset(d, 0, sizeof(h));
-  if (g->n) k_max_degree<<<grid_for(g->n), 256>>>(g->csr.offs, g->n, &d->best);
+  if (g->n) k_degrees<<<grid_for(g->n), 256>>>(g->csr.offs, g->n, d);
   // (not a managed graph's columns, which would be faulted in before their advice)
   if (g->m && g->mem_mode != GRUS_MEM_MANAGED)
     k_near_ids<<<kNearSample / 256, 256>>>(g->csr.offs, g->csr.cols, g->n, g->m, &d->near);
   cudaError_t e = cudaMemcpy(&h, d, sizeof(h), cudaMemcpyDeviceToHost);
   cudaFree(d);
   GRUS_CUDA_TRY(e);
+  std::copy(h.count, h.count + 32, g->deg_count);
+  std::copy(h.edges, h.edges + 32, g->deg_edges);
   g->max_deg = (uint32_t)(h.best >> 32);
   g->max_deg_vertex = g->n ? (uint32_t)(0xFFFFFFFFull - (h.best & 0xFFFFFFFFull)) : 0;
   if (g->max_deg == 0) g->max_deg_vertex = 0;
-  g->near_ids = h.edges && 10ull * h.near >= 9ull * h.edges;
+  g->near_ids = h.sampled && 10ull * h.near >= 9ull * h.sampled;
   return GRUS_OK;
 }
 

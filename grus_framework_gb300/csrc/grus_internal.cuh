@@ -55,6 +55,9 @@ struct grus_graph {
   grus::Csr csr;              // out-edges
   grus::Csr csc;              // in-edges (built on demand; aliases csr if symmetric)
   uint32_t max_deg_vertex = 0, max_deg = 0;
+  // vertices of out-degree 2^i to 2^(i + 1) - 1, and their out-edges
+  uint32_t deg_count[32] = {};
+  unsigned long long deg_edges[32] = {};
   bool near_ids = false;  // most edges join ids less than n / 64 apart (sampled)
   // BFS pull index: per vertex {an in-neighbour of high out-degree (kNoRep
   // without in-edges), the vertex's out-degree}, built on demand

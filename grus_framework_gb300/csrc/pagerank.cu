@@ -57,12 +57,6 @@ constexpr uint32_t kWarpCost = 128; // least work per warp before fewer CTAs are
 constexpr uint32_t kHotCap = 24576; // slots beside contributions gathered from L2
 constexpr uint32_t kHotAll = 48000; // vertices of a graph kept whole in shared memory
 constexpr uint32_t kNone = 0xFFFFFFFFu;  // no source: every id is smaller
-constexpr int kPlanIters = 3;       // fewer iterations do not repay a relabelling pass
-// Edges from which the first call makes the plan; below, the second one does: the
-// plan takes 100-200 us, which 20 iterations on a smaller graph do not repay
-// (first / later calls with it 744 / 403 us at RMAT-18, without 643 / 527; RMAT-19
-// 1,026 / 621 and 985 / 828; RMAT-20 1,511 / 1,045 and 1,624 / 1,446).
-constexpr uint64_t kPlanNow = 3ull << 22;
 
 struct Args {
   const uint32_t *__restrict__ toffs;  // CSC offsets
@@ -353,43 +347,29 @@ __global__ void k_degree_bins(const uint32_t *__restrict__ offs, uint32_t n, uin
 }
 
 struct PlanCtl {
-  uint32_t above, at, rest;     // slots given to degrees > cut, = cut, and to the others
+  uint32_t above, at, rest;  // slots given to degrees > cut, = cut, and to the others
   uint32_t n_above, cut;
-  unsigned long long edges;     // at least this many edges leave the vertices with slots
+  uint32_t made;
 };
 
-// One CTA of 1024: the smallest degree that still gets slots.
-__global__ void k_plan_cut(const uint32_t *__restrict__ bins, PlanCtl *ctl) {
-  __shared__ unsigned long long s_cnt[1024], s_edges[1024];
+// One CTA of 1024: the largest degree of which not all vertices get slots.
+__global__ void __launch_bounds__(1024) k_plan_cut(const uint32_t *__restrict__ bins, PlanCtl *ctl) {
   constexpr uint32_t per = kBins / 1024;
-  const uint32_t t = threadIdx.x, hi = kBins - t * per;  // bins [hi - per, hi), from the top down
-  unsigned long long c = 0, e = 0;
-  for (uint32_t d = hi - per; d < hi; ++d) {
-    c += bins[d];
-    e += (unsigned long long)bins[d] * d;
+  const uint32_t hi = kBins - threadIdx.x * per;  // bins [hi - per, hi), from the top down
+  const uint4 *mine = reinterpret_cast<const uint4 *>(bins + hi - per);
+  uint32_t count = 0, total = 0;
+#pragma unroll
+  for (uint32_t i = 0; i < per / 4; ++i) {
+    const uint4 x = mine[i];
+    count += x.x + x.y + x.z + x.w;
   }
-  s_cnt[t] = c;
-  s_edges[t] = e;
-  __syncthreads();
-  if (t == 0) {
-    unsigned long long above = 0, edges = 0;
-    uint32_t i = 0;
-    while (i < 1024 && above + s_cnt[i] <= kHotCap) {
-      above += s_cnt[i];
-      edges += s_edges[i];
-      ++i;
-    }
-    uint32_t d = kBins - i * per;  // the cut lies below d
-    while (d > 1 && above + bins[d - 1] <= kHotCap) {
-      --d;
-      above += bins[d];
-      edges += (unsigned long long)bins[d] * d;
-    }
-    // degree d - 1 fills what is left
-    ctl->n_above = (uint32_t)above;
-    ctl->cut = d - 1;
-    ctl->edges = edges + (kHotCap - above) * (unsigned long long)(d - 1);
-  }
+  uint32_t above = block_exclusive_scan<1024>(count, &total);
+  if (above > kHotCap || above + count <= kHotCap) return;  // (more vertices than slots: one thread stays)
+  uint32_t d = hi - 1;
+  for (; above + bins[d] <= kHotCap; --d) above += bins[d];
+  ctl->n_above = above;
+  ctl->cut = d;
+  ctl->made = 1u;
 }
 
 // slot[v]: below kHotCap for the vertices of largest out-degree, from kHotCap
@@ -425,10 +405,9 @@ __global__ void k_plan_cols(const uint32_t *__restrict__ tcols, uint64_t m,
 struct Workspace {
   float *c = nullptr;   // 2 * stride contributions
   uint64_t stride = 0;
-  // plan (n > kHotAll): relabelled columns and slots, once asked for
-  bool planned = false;
-  bool ranked = false;  // a call that the plan is for has been made
-  uint32_t *cols = nullptr, *slot = nullptr;
+  // plan (n > kHotAll): slots and relabelled columns behind the contributions
+  bool planned = false;  // queued
+  uint32_t *slot = nullptr, *cols = nullptr;
   float *rank = nullptr;
   uint32_t *shared = nullptr;  // per warp: head, tail, arrivals
   uint32_t warps = 0;
@@ -436,15 +415,14 @@ struct Workspace {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 };
 
-constexpr size_t kOffBar = 0, kOffErr = 256, kCtrlBytes = 384;
+// (the pinned mirror has one more word: not 0 once the plan is made)
+constexpr size_t kOffBar = 0, kOffErr = 256, kCtrlBytes = 384, kOffPlanned = kCtrlBytes;
 static_assert(kOffBar + sizeof(GridBarrier) <= kOffErr, "barrier layout");
 
 void ws_free(void *p) {
   Workspace *w = (Workspace *)p;
   if (!w) return;
   cudaFree(w->c);
-  cudaFree(w->cols);
-  cudaFree(w->slot);
   cudaFree(w->rank);
   cudaFree(w->shared);
   cudaFree(w->ctrl);
@@ -453,6 +431,29 @@ void ws_free(void *p) {
   if (w->ev1) cudaEventDestroy(w->ev1);
   delete w;
 }
+
+// Whether a graph beyond kHotAll vertices gets a plan: where the kHotCap vertices
+// of largest out-degree are the sources of a quarter of the edges (by the
+// graph's degree counts, the edges of the last range in proportion), from
+// kPlanEdges on.  Not a managed graph, whose columns may not fit the device.
+// Below kPlanEdges it gains nothing (20 iterations without / with it: RMAT-16 of 8
+// edges a vertex 219 / 224 us, 60,021 vertices of degree 12 165 / 174; RMAT-16 of
+// 16 258 / 239, of 24 307 / 268, RMAT-18 524 / 403) and costs the first call
+// 110 us, most of it the larger allocation.
+constexpr uint64_t kPlanEdges = 3ull << 18;
+bool wants_plan(const grus_graph *g) {
+  if (g->n <= kHotAll || g->m < kPlanEdges || g->mem_mode == GRUS_MEM_MANAGED) return false;
+  double edges = 0.0;
+  uint64_t left = kHotCap;
+  for (int i = 31; i >= 0 && left; --i) {
+    const uint64_t take = std::min<uint64_t>(left, g->deg_count[i]);
+    if (take) edges += (double)g->deg_edges[i] * ((double)take / (double)g->deg_count[i]);
+    left -= take;
+  }
+  return 4.0 * edges >= (double)g->m;
+}
+
+constexpr uint64_t kPlanSmall = 64ull << 20;
 
 int ws_get(grus_graph *g, Workspace **out) {
   if (g->ws[kWsPr]) {
@@ -463,11 +464,27 @@ int ws_get(grus_graph *g, Workspace **out) {
   const uint64_t n1 = std::max<uint64_t>(g->n, 1);
   w->warps = (uint32_t)std::max(device_sm_count(), 1) * (kBlock / 32);
   w->stride = (n1 + (n1 > kHotAll ? kHotCap : 0u) + 31) / 32 * 32;
-  cudaError_t e = cudaMalloc(&w->c, 2 * w->stride * 4);
+  // the plan's part is kept as long as the graph: not more than a sixteenth of
+  // the free memory, which is asked for where it is more than any GPU's small change
+  const uint64_t slots = (n1 + 31) / 32 * 32, plan = wants_plan(g) ? (slots + g->m) * 4 : 0;
+  size_t free_bytes = 0, all_bytes = 0;
+  bool room = plan && (plan <= kPlanSmall || (cudaMemGetInfo(&free_bytes, &all_bytes) == cudaSuccess &&
+                                              plan <= free_bytes / 16));
+  cudaError_t e = cudaMalloc(&w->c, 2 * w->stride * 4 + (room ? plan : 0));
+  if (e != cudaSuccess && room) {
+    room = false;
+    e = cudaMalloc(&w->c, 2 * w->stride * 4);
+  }
+  cudaGetLastError();
+  if (e == cudaSuccess && room) {
+    w->slot = (uint32_t *)(w->c + 2 * w->stride);
+    w->cols = w->slot + slots;
+  }
   if (e == cudaSuccess) e = cudaMalloc(&w->shared, (size_t)w->warps * 12);
   if (e == cudaSuccess) e = cudaMalloc(&w->ctrl, kCtrlBytes);
   if (e == cudaSuccess) e = cudaMemset(w->ctrl, 0, kCtrlBytes);
-  if (e == cudaSuccess) e = cudaMallocHost(&w->ctrl_host, kCtrlBytes);
+  if (e == cudaSuccess) e = cudaMallocHost(&w->ctrl_host, kCtrlBytes + 8);
+  if (e == cudaSuccess) std::memset(w->ctrl_host + kOffPlanned, 0, 8);
   if (e == cudaSuccess) e = cudaEventCreate(&w->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&w->ev1);
   if (e != cudaSuccess) {
@@ -482,50 +499,34 @@ int ws_get(grus_graph *g, Workspace **out) {
   return GRUS_OK;
 }
 
-// The plan of a graph beyond kHotAll vertices, built on the first call (kPlanNow
-// edges and more) or the second with enough iterations to repay it: a few passes over the vertices and one over
-// the columns (RMAT-24: 1.3 ms and 1.1 GB).  None on a managed graph, whose
-// columns may not fit the device, without room for it, or where the vertices
-// with slots would not be the sources of a quarter of the edges.
+// Queues the making of the plan: a few passes over the vertices and one over the
+// columns (RMAT-24: 1.3 ms and 1.1 GB).  It belongs to the first
+// call, like the workspace: later ones only queue their kernel, also under
+// capture.  Nothing waits; a later call uses the plan once its mark has arrived
+// in pinned memory.  Bins and counters stand in the contributions.
 void make_plan(grus_graph *g, Workspace *w, cudaStream_t s) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
     cudaGetLastError();
-    return;  // it waits for the stream: left to a call outside the capture
+    return;  // left to a call outside the capture
   }
-  w->planned = true;
-  if (g->mem_mode == GRUS_MEM_MANAGED) return;
   const uint32_t n = (uint32_t)g->n;
   const int grid = std::max(device_sm_count(), 1) * 8;
-  uint32_t *bins = nullptr;
-  PlanCtl h{};
-  cudaError_t e = cudaMalloc(&bins, kBins * 4 + sizeof(PlanCtl));
+  static_assert(2ull * (kHotAll + kHotCap) >= kBins + sizeof(PlanCtl) / 4, "they fit the contributions");
+  uint32_t *bins = (uint32_t *)w->c;
   PlanCtl *ctl = (PlanCtl *)(bins + kBins);
-  if (e == cudaSuccess) e = cudaMemsetAsync(bins, 0, kBins * 4 + sizeof(PlanCtl), s);
+  cudaError_t e = cudaMemsetAsync(bins, 0, kBins * 4 + sizeof(PlanCtl), s);
   if (e == cudaSuccess) {
     k_degree_bins<<<grid, 256, 0, s>>>(g->csr.offs, n, bins);
     k_plan_cut<<<1, 1024, 0, s>>>(bins, ctl);
-    e = cudaMemcpyAsync(&h, ctl, sizeof(h), cudaMemcpyDeviceToHost, s);
+    k_plan_slots<<<grid, 256, 0, s>>>(g->csr.offs, n, ctl, w->slot);
+    k_plan_cols<<<grid, 256, 0, s>>>(g->csc.cols, g->m, w->slot, w->cols);
+    e = cudaGetLastError();
   }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e == cudaSuccess && 4 * h.edges >= g->m) {
-    e = cudaMalloc(&w->slot, g->n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&w->cols, g->m * 4);
-    if (e == cudaSuccess) {
-      k_plan_slots<<<grid, 256, 0, s>>>(g->csr.offs, n, ctl, w->slot);
-      k_plan_cols<<<grid, 256, 0, s>>>(g->csc.cols, g->m, w->slot, w->cols);
-      e = cudaGetLastError();
-    }
-    // later calls may come on other streams
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  }
-  cudaFree(bins);
-  if (e != cudaSuccess) {  // no room: gather from L2
-    cudaGetLastError();
-    cudaFree(w->slot);
-    cudaFree(w->cols);
-    w->slot = w->cols = nullptr;
-  }
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(w->ctrl_host + kOffPlanned, &ctl->made, 4, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) w->planned = true;
+  else cudaGetLastError();
 }
 
 template <bool kHot>
@@ -573,11 +574,10 @@ extern "C" int grus_pagerank(grus_graph *g, float damping, int iters, float *ran
   if (rc) return rc;
   const bool dev_out = is_device_pointer(rank);
   if (!dev_out && !w->rank) GRUS_CUDA_TRY(cudaMalloc(&w->rank, g->n * 4));
-  // a plan needs a quarter of the edges at kHotCap sources
-  if (g->n > kHotAll && iters >= kPlanIters && !w->planned &&
-      4ull * kHotCap * g->max_deg >= g->m) {
-    if (w->ranked || g->m >= kPlanNow) make_plan(g, w, s);
-    w->ranked = true;
+  bool plan = w->planned && *(volatile uint32_t *)(w->ctrl_host + kOffPlanned);
+  if (iters > 0 && w->slot && !w->planned) {
+    make_plan(g, w, s);
+    plan = w->planned;  // this call's kernel follows it on the stream
   }
   Args a;
   std::memset(&a, 0, sizeof(a));
@@ -591,10 +591,10 @@ extern "C" int grus_pagerank(grus_graph *g, float damping, int iters, float *ran
   a.iters = iters;
   a.c[0] = w->c;
   a.c[1] = w->c + w->stride;
-  const bool hot = g->n <= kHotAll || w->cols;
+  const bool hot = g->n <= kHotAll || plan;
   if (g->n <= kHotAll) {
     a.hot = a.n;
-  } else if (w->cols) {
+  } else if (plan) {
     a.tcols = w->cols;
     a.hot = kHotCap;
     a.slot = w->slot;

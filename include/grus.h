@@ -19,6 +19,10 @@
  *     Calls with host outputs or a non-NULL stats pointer return after the
  *     work has finished; calls with device outputs and no stats are
  *     asynchronous on `stream`.
+ *   - An algorithm's first call on a graph allocates its workspace, which is
+ *     kept with the graph; later calls only queue work and can be captured.
+ *     PageRank's may hold a copy of the column ids, of at most a sixteenth of
+ *     the device memory that is free at that time.
  *   - Vertex ids and CSR arrays are uint32 (vtx_t, include/common.cuh:48);
  *     unreached vertices read GRUS_INFINIT (INFINIT, include/common.cuh:52).
  */
