@@ -795,7 +795,6 @@ static int ensure_members(grus_batch *b, uint32_t n) {
   drop_graph(b);
   cudaFree(b->d_msrc);
   cudaFree(b->d_moff);
-  if (b->h_errs) cudaFreeHost(b->h_errs);
   cudaFreeHost(b->h_msrc);
   cudaFreeHost(b->h_moff);
   b->d_msrc = b->h_msrc = nullptr;
