@@ -603,14 +603,49 @@ static bool own_launch(const grus_batch *b, const std::vector<UnionPack> &l) {
   return l.size() == 1 && b->big[l[0].graph];
 }
 
+constexpr uint32_t kPackDeg = 9;
+
+static bool packable(const grus_batch *b, uint32_t gi) {
+  const grus_graph *g = b->graphs[gi];
+  return !b->big[gi] && g->max_deg >= kPackDeg && g->n * 8 <= b->launch_entries;
+}
+
+// The packs' workspace is made with the batch, for what any of its runs may pack in
+// kPackLaunches launches: a run that had to allocate would wait for the device.
+// It is kept with the batch: not more than a sixteenth of the free memory.
+// Without it, or beyond it, small graphs' queries stay with the workers.
+constexpr int kPackLaunches = 16;
+constexpr uint32_t kErrWords = 256;
+
+static void reserve_packs(grus_batch *b) {
+  if (!b->adaptive) return;
+  std::vector<uint64_t> gn, gm;
+  std::vector<bool> alone;
+  for (size_t i = 0; i < b->graphs.size(); ++i) {
+    const grus_graph *g = b->graphs[i];
+    if (!g->csr.wts || !(b->big[i] || packable(b, (uint32_t)i))) continue;
+    gn.push_back(g->n);
+    gm.push_back(g->m);
+    alone.push_back(!b->big[i]);
+  }
+  if (std::find(alone.begin(), alone.end(), true) == alone.end()) return;
+  const UnionNeed need = union_need(gn, gm, alone, b->launch_entries);
+  size_t free_bytes = 0, total = 0;
+  if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess ||
+      msssp_union_bytes(kPackLaunches, need.max_v, need.max_m, need.entries) > free_bytes / 16 ||
+      msssp_union_reserve(&b->uws, kPackLaunches, need.max_v, need.max_m, need.entries) != GRUS_OK)
+    cudaGetLastError();
+}
+
 // Plans the launches of big_q's SSSP queries (big_q sorted by graph) with
 // plan_union (union_plan.h): up to 32 per graph per pack, several graphs'
 // packs per multi-graph launch while their distance rows total at most
 // launch_entries.  The cap keeps a launch's distance rows in L2: 256 queries
 // over 32 RMAT graphs of scales 14-20 in one launch (368 MB of rows) took
-// 48.7 ms against 37 ms as one launch per graph.  Makes room for them.
+// 48.7 ms against 37 ms as one launch per graph.  Makes room for them, or, with
+// `grow` false, fails where there is none.
 static int plan_sssp(grus_batch *b, const grus_query *queries, const std::vector<int> &big_q,
-                     UnionPlan *out) {
+                     bool grow, UnionPlan *out) {
   *out = UnionPlan();
   std::vector<int> sssp;
   for (int qi : big_q)
@@ -629,11 +664,13 @@ static int plan_sssp(grus_batch *b, const grus_query *queries, const std::vector
     if (l.size() > 1 || own_launch(b, l)) continue;
     plan.max_v = std::max(plan.max_v, gn[l[0].graph]);
     plan.max_m = std::max(plan.max_m, gm[l[0].graph]);
-    plan.max_ks = std::max(plan.max_ks, union_row_width(l[0].q.size()));
+    plan.entries = std::max(plan.entries, gn[l[0].graph] * union_row_width(l[0].q.size()));
     ++plan.unions;
   }
   if (plan.unions) {
-    int rc = msssp_union_reserve(&b->uws, plan.unions, plan.max_v, plan.max_m, plan.max_ks);
+    if (!grow && !msssp_union_fits(b->uws, plan.unions, plan.max_v, plan.max_m, plan.entries))
+      return GRUS_ENOMEM;
+    int rc = msssp_union_reserve(&b->uws, plan.unions, plan.max_v, plan.max_m, plan.entries);
     if (rc) return rc;
   }
   *out = std::move(plan);
@@ -748,8 +785,11 @@ int grus_batch_create(grus_graph *const *graphs, int ngraphs, const grus_batch_c
     b->slots = std::min(occ, bfs_side_fit());
     rc = b->state.reserve(b->workers, b->max_n, b->max_m, b->huge);
   }
+  if (!rc) reserve_packs(b);
   cudaError_t e = cudaSuccess;
-  if (!rc) e = cudaMalloc(&b->d_graphs, ngraphs * sizeof(GraphDesc));
+  if (!rc) e = cudaMallocHost(&b->h_errs, kErrWords * 4);
+  if (!rc && e == cudaSuccess) b->err_cap = kErrWords;
+  if (!rc && e == cudaSuccess) e = cudaMalloc(&b->d_graphs, ngraphs * sizeof(GraphDesc));
   if (!rc && e == cudaSuccess)
     e = cudaMemcpy(b->d_graphs, descs.data(), ngraphs * sizeof(GraphDesc), cudaMemcpyHostToDevice);
   if (!rc && e == cudaSuccess) e = cudaEventCreate(&b->ev0);
@@ -908,13 +948,6 @@ static int stage_tasks(grus_batch *b, const grus_query *q, int nq) {
 // queries each, 268 / 358, and 200 queries on one RMAT-12 2,205 / 2,455.  Graphs
 // without hubs stay with the workers, whose levels are cheaper (four 100 x 100
 // grids: 2,129 / 2,527).
-constexpr uint32_t kPackDeg = 9;
-
-static bool packable(const grus_batch *b, uint32_t gi) {
-  const grus_graph *g = b->graphs[gi];
-  return !b->big[gi] && g->max_deg >= kPackDeg && g->n * 8 <= b->launch_entries;
-}
-
 static bool pack_small(const grus_batch *b, const grus_query *q, int nq, cudaStream_t s) {
   if (!b->adaptive) return false;
   std::vector<uint32_t> k(b->graphs.size(), 0u);  // SSSP queries in packs, per graph
@@ -961,7 +994,7 @@ static bool pack_small(const grus_batch *b, const grus_query *q, int nq, cudaStr
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
     cudaGetLastError();
-    return false;  // the launches' workspace may have to grow
+    return false;  // a captured run is the workers'
   }
   return true;
 }
@@ -1060,7 +1093,7 @@ int grus_batch_run(grus_batch *b, const grus_query *queries, int nq, uint32_t *o
       if (queries[x].graph != queries[y].graph) return queries[x].graph < queries[y].graph;
       return queries[x].algo < queries[y].algo;
     });
-    const int prc = plan_sssp(b, queries, big_q, &plan);
+    const int prc = plan_sssp(b, queries, big_q, !pack, &plan);
     if (!prc) break;
     if (!pack) return prc;
     pack = false;  // no room for the packs: the workers take them
@@ -1084,12 +1117,15 @@ int grus_batch_run(grus_batch *b, const grus_query *queries, int nq, uint32_t *o
   uint32_t nerr = 0;
   uint32_t nlaunch = 0;  // kernels launched by the big-graph lane
   if (!big_q.empty()) {
-    if (b->err_cap < big_q.size()) {
+    // a word per launch
+    size_t words = plan.launches.size();
+    for (int qi : big_q) words += queries[qi].algo != GRUS_ALGO_SSSP;
+    if (b->err_cap < words) {
       if (b->h_errs) cudaFreeHost(b->h_errs);
       b->h_errs = nullptr;
       b->err_cap = 0;
-      GRUS_CUDA_TRY(cudaMallocHost(&b->h_errs, big_q.size() * 4));
-      b->err_cap = (uint32_t)big_q.size();
+      GRUS_CUDA_TRY(cudaMallocHost(&b->h_errs, words * 4));
+      b->err_cap = (uint32_t)words;
     }
     rc = union_sssp(b, queries, plan, out, s, &nerr, &nlaunch);
     if (rc) return rc;

@@ -163,7 +163,9 @@ CtrlView pr_ctrl(grus_graph *g);
 // at most max_v vertices, max_m edges and ks (8/16/32) sources per graph
 // before the first launch of a run; launch i of a run uses region i.  *cv
 // receives the launch's control block (error word).
-int msssp_union_reserve(void **ws, int regions, uint64_t max_v, uint64_t max_m, uint32_t ks);
+int msssp_union_reserve(void **ws, int regions, uint64_t max_v, uint64_t max_m, uint64_t entries);
+bool msssp_union_fits(const void *ws, int regions, uint64_t max_v, uint64_t max_m, uint64_t entries);
+uint64_t msssp_union_bytes(int regions, uint64_t max_v, uint64_t max_m, uint64_t entries);
 int msssp_union_run(void *ws, int region, grus_graph *const *gs, int ng, const uint32_t *kq,
                     const uint32_t *srcs, uint32_t *const *outs, uint32_t delta, cudaStream_t s,
                     CtrlView *cv);

@@ -308,7 +308,18 @@ void msssp_union_reset(void *p) {
   if (w && w->ctrl) cudaMemset(w->ctrl, 0, (size_t)w->regions * kCtrlBytes);
 }
 
-int msssp_union_reserve(void **wsp, int regions, uint64_t max_v, uint64_t max_m, uint32_t ks) {
+bool msssp_union_fits(const void *wsp, int regions, uint64_t max_v, uint64_t max_m, uint64_t entries) {
+  const UnionWs *w = (const UnionWs *)wsp;
+  return w && w->regions >= regions && w->vcap >= max_v && w->d_entries >= entries &&
+         w->ent_cap >= max_v + max_m / kPiece + 1024;
+}
+
+uint64_t msssp_union_bytes(int regions, uint64_t max_v, uint64_t max_m, uint64_t entries) {
+  return entries * 4 + max_v * 12 + (max_v + max_m / kPiece + 1024) * sizeof(uint4) +
+         (uint64_t)regions * (ms::kMaxUnion * sizeof(ms::UnionGraph) + 2 * kSeedCap * 4 + kCtrlBytes);
+}
+
+int msssp_union_reserve(void **wsp, int regions, uint64_t max_v, uint64_t max_m, uint64_t entries) {
   UnionWs *w = (UnionWs *)*wsp;
   const uint64_t v1 = std::max<uint64_t>(max_v, 1);
   const uint64_t ecap = v1 + max_m / kPiece + 1024;
@@ -316,13 +327,12 @@ int msssp_union_reserve(void **wsp, int regions, uint64_t max_v, uint64_t max_m,
     set_last_error("multi-graph sssp launch too large");
     return GRUS_EINVAL;
   }
-  if (w && w->regions >= regions && w->vcap >= v1 && w->d_entries >= v1 * ks && w->ent_cap >= ecap)
-    return GRUS_OK;
+  if (msssp_union_fits(w, regions, v1, max_m, entries)) return GRUS_OK;
   if (w) cudaDeviceSynchronize();  // launches of an earlier run may still use it
   UnionWs *nw = new UnionWs();
   nw->regions = std::max(regions, w ? w->regions : 0);
   nw->vcap = std::max(v1, w ? w->vcap : 0);
-  nw->d_entries = std::max(v1 * ks, w ? w->d_entries : 0);
+  nw->d_entries = std::max(entries, w ? w->d_entries : 0);
   nw->ent_cap = std::max(ecap, w ? w->ent_cap : 0);
   msssp_union_free(w);
   *wsp = nullptr;

@@ -29,8 +29,34 @@ struct UnionPlan {
   // sizes the multi-graph launches need (launches of one graph excluded)
   uint64_t max_v = 0, max_m = 0;
   uint32_t max_ks = 8;
+  uint64_t entries = 0;  // distance entries of the largest of them
   int unions = 0;  // launches of more than one graph
 };
+
+// What the launches of graphs of gn vertices and gm edges need at most, whatever
+// the queries: launches of several graphs keep to the cap, and one of `alone`'s
+// graphs alone may have rows of 32.
+struct UnionNeed {
+  uint64_t max_v = 0, max_m = 0, entries = 0;
+};
+
+inline UnionNeed union_need(const std::vector<uint64_t> &gn, const std::vector<uint64_t> &gm,
+                            const std::vector<bool> &alone, uint64_t cap) {
+  UnionNeed need;
+  uint64_t v = 0, top = 0;
+  for (size_t g = 0; g < gn.size(); ++g) {
+    if (gn[g] * 8 <= cap) {  // else it joins no launch of several
+      v += gn[g];
+      need.max_m += gm[g];
+    }
+    if (!alone[g]) continue;
+    top = std::max(top, gn[g]);
+    need.max_m = std::max(need.max_m, gm[g]);
+  }
+  need.max_v = std::max(std::min(v, cap / 8), top);
+  need.entries = std::max(std::min(v * 32, cap), top * 32);
+  return need;
+}
 
 inline uint32_t union_row_width(size_t k) { return k <= 8 ? 8u : (k <= 16 ? 16u : 32u); }
 
@@ -66,6 +92,7 @@ inline UnionPlan plan_union(const std::vector<int> &sssp, const std::vector<uint
         plan.max_v = std::max(plan.max_v, v);
         plan.max_m = std::max(plan.max_m, m);
         plan.max_ks = std::max(plan.max_ks, union_row_width(kmax));
+        plan.entries = std::max(plan.entries, v * union_row_width(kmax));
         ++plan.unions;
       }
       plan.launches.push_back(std::move(cur));
