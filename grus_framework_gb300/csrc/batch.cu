@@ -752,8 +752,8 @@ int grus_batch_create(grus_graph *const *graphs, int ngraphs, const grus_batch_c
     b->max_m = std::max<uint64_t>(b->max_m, graphs[i]->m);
   }
   if (cfg) {
-    b->adaptive = !cfg->cluster_size && !cfg->workers && !cfg->sssp_delta && !cfg->group_sources &&
-                  !cfg->big_edges;
+    b->adaptive = !cfg->cluster_size && !cfg->workers && !cfg->huge_degree && !cfg->sssp_delta &&
+                  !cfg->group_sources && !cfg->big_edges;
     if (cfg->cluster_size) b->cluster = (int)cfg->cluster_size;
     if (cfg->huge_degree) b->huge = cfg->huge_degree;
     if (cfg->sssp_delta) b->delta = cfg->sssp_delta;

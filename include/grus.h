@@ -336,8 +336,9 @@ typedef struct grus_batch_config {
                             share a graph, else one launch each (default
                             2^21, where SSSP queries on smaller graphs are
                             packed too if that is estimated to be faster
-                            and cluster_size, workers, sssp_delta and
-                            group_sources are 0; 0xFFFFFFFF: never) */
+                            and cluster_size, workers, huge_degree,
+                            sssp_delta and group_sources are 0;
+                            0xFFFFFFFF: never) */
   uint32_t launch_entries;/* the SSSP packs of several of those graphs share
                             one launch while their distance rows (vertices
                             x 8/16/32 sources) total at most this many
