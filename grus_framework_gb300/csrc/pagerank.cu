@@ -42,6 +42,7 @@
 #include <cstring>
 #include <vector>
 
+#include "edge_batches.h"
 #include "grus_internal.cuh"
 
 namespace grus {
@@ -171,15 +172,14 @@ __device__ __forceinline__ void share_bound(const Args &a, unsigned long long c,
   cut = e > b;
 }
 
-// The source ids of the batch from edge x on (up to edge e), and the
-// contributions of the sources; 0 past the end.
-__device__ __forceinline__ void load_ids(const Args &a, uint32_t x, uint32_t e,
+// The source ids of the batch from edge x on, of which `left` are in the range,
+// and the contributions of the sources; 0 past the end.
+__device__ __forceinline__ void load_ids(const Args &a, uint32_t x, int left,
                                          uint32_t (&u)[kBatch / 32]) {
-  const uint32_t left = e > x ? e - x : 0u;
   const uint32_t *p = a.tcols + x + lane_id();
 #pragma unroll
   for (int j = 0; j < kBatch / 32; ++j)
-    u[j] = lane_id() + 32 * j < left ? source_id(p + 32 * j) : kNone;
+    u[j] = (int)lane_id() + 32 * j < left ? source_id(p + 32 * j) : kNone;
 }
 
 template <bool kHot>
@@ -208,7 +208,7 @@ __device__ __forceinline__ void run_share(const Args &a, const Share &sh, const 
   // the source ids of the one after it
   float f[kBatch / 32];
   load_values<kHot>(a, cs, sc, u, f);
-  load_ids(a, x + kBatch, sh.e1, u);
+  load_ids(a, x + kBatch, edges_left(x, sh.e1) - kBatch, u);
   for (uint32_t w = 0; w < rows; w += 32) {
     const uint32_t v = sh.r0 + w + lane;
     const bool ok = w + lane < rows;
@@ -243,11 +243,12 @@ __device__ __forceinline__ void run_share(const Args &a, const Share &sh, const 
       if (stop <= lim) break;  // these 32 vertices are complete
       __syncwarp();
       x = lim;
-      lim = min(sh.e1, x + kBatch);
+      const int left = edges_left(x, sh.e1);
+      lim = batch_end(x, left, kBatch);
 #pragma unroll
       for (int j = 0; j < kBatch / 32; ++j) sv[lane + 32 * j] = f[j];
       load_values<kHot>(a, cs, sc, u, f);
-      load_ids(a, x + 2 * kBatch, sh.e1, u);
+      load_ids(a, x + 2 * kBatch, left - 2 * kBatch, u);
       __syncwarp();
     }
     if (ok) {
@@ -311,7 +312,7 @@ __global__ void __launch_bounds__(kBlock, 1) pr_persistent(Args a) {
   if (!grid_sync(a.bar, a.err, a.timeout_ns)) return;
 
   uint32_t u[kBatch / 32];
-  load_ids(a, sh.e0, sh.e1, u);
+  load_ids(a, sh.e0, edges_left(sh.e0, sh.e1), u);
   for (int it = 0; it < a.iters; ++it) {
     const float *cs = a.c[it & 1];
     float *cn = a.c[(it + 1) & 1];
@@ -324,7 +325,7 @@ __global__ void __launch_bounds__(kBlock, 1) pr_persistent(Args a) {
       __syncthreads();
     }
     run_share<kHot>(a, sh, cs, s_hot, sv, cn, last, gwarp, u);
-    load_ids(a, sh.e0, sh.e1, u);  // of the next iteration, before the wait
+    load_ids(a, sh.e0, edges_left(sh.e0, sh.e1), u);  // of the next iteration, before the wait
     if (sh.cut0 || sh.cut1) arrive<kHot>(a, sh, gwarp, f0, l0, l1, it, cn, last);
     if (!last && !grid_sync(a.bar, a.err, a.timeout_ns)) return;
   }
