@@ -476,7 +476,7 @@ int BatchState::reserve(int nworkers, uint64_t max_n, uint64_t max_m, uint32_t h
   if (e == cudaSuccess) e = cudaMalloc(&ctl, (uint64_t)nworkers * sizeof(WorkerCtl));
   if (e == cudaSuccess) e = cudaMalloc(&counter, 4);
   if (e == cudaSuccess) e = cudaMalloc(&err, 4);
-  if (e == cudaSuccess) e = cudaMemset(err, 0, 4);  // read back after every run
+  if (e == cudaSuccess) e = clear_now(err, 4);  // read back after every run
   if (e != cudaSuccess) {
     cudaGetLastError();
     release();
@@ -1266,7 +1266,7 @@ int grus_batch_run(grus_batch *b, const grus_query *queries, int nq, uint32_t *o
   GRUS_CUDA_TRY(cudaStreamSynchronize(s));
   for (uint32_t i = 0; i < nerr; ++i) err |= b->h_errs[i];
   if (err) {
-    cudaMemset(b->state.err, 0, 4);
+    clear_now(b->state.err, 4);
     msssp_union_reset(b->uws);
     return status_from_device_error(err);
   }

@@ -245,14 +245,12 @@ int ws_get(grus_graph *g, Workspace **out) {
   static_assert(kCtrlBytes % alignof(LevelTrace) == 0, "the trace follows the control block");
   constexpr size_t trace_bytes = kMaxTrace * sizeof(LevelTrace);
   if (e == cudaSuccess) e = cudaMalloc(&w->ctrl, kCtrlBytes + trace_bytes);
-  if (e == cudaSuccess) e = cudaMemset(w->ctrl, 0, kCtrlBytes);
+  if (e == cudaSuccess) e = clear_now(w->ctrl, kCtrlBytes);
   if (e == cudaSuccess) e = cudaMallocHost(&w->ctrl_host, kCtrlBytes + trace_bytes);
   if (e == cudaSuccess) {
     w->trace = (LevelTrace *)(w->ctrl + kCtrlBytes);
     w->trace_host = (LevelTrace *)(w->ctrl_host + kCtrlBytes);
   }
-  // the clearing must be over before a launch on any stream
-  if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
   if (e == cudaSuccess) e = cudaEventCreate(&w->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&w->ev1);
   if (e != cudaSuccess) {

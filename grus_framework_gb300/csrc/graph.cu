@@ -53,6 +53,17 @@ int current_device() {
   return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;
 }
 
+cudaError_t clear_now(void *p, size_t bytes) {
+  static PerDevice<cudaStream_t> streams;
+  cudaStream_t s = nullptr;
+  const int rc = streams.get(current_device(), &s, [](cudaStream_t &v) {
+    return (int)cudaStreamCreateWithFlags(&v, cudaStreamNonBlocking);
+  });
+  if (rc) return (cudaError_t)rc;
+  const cudaError_t e = cudaMemsetAsync(p, 0, bytes, s);
+  return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+}
+
 int device_sm_count() {
   static int cached[64] = {0};
   int dev = 0;

@@ -76,6 +76,9 @@ int graph_alloc_array(grus_graph *g, void **p, size_t bytes);
 void graph_free_array(grus_graph *g, void *p);
 int device_sm_count();
 int current_device();  // -1: none
+// Sets device memory to zero and returns when that is done, so that it precedes
+// a launch on any stream.  Waits for nothing else.
+cudaError_t clear_now(void *p, size_t bytes);
 int l2_window(cudaStream_t s, void *base, size_t bytes);
 // Share of a window of `bytes` that may persist: 1, or the persisting L2
 // set-aside over the window when the window is larger (persisting lines

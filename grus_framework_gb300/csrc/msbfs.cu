@@ -555,10 +555,8 @@ int ws_get(grus_graph *g, Workspace **out) {
   if (e == cudaSuccess) e = cudaMalloc(&w->chunks, 2ull * w->chunk_cap * sizeof(uint4));
   if (e == cudaSuccess) e = cudaMalloc(&w->srcs, 64 * 4);
   if (e == cudaSuccess) e = cudaMalloc(&w->ctrl, kCtrlBytes);
-  if (e == cudaSuccess) e = cudaMemset(w->ctrl, 0, kCtrlBytes);
+  if (e == cudaSuccess) e = clear_now(w->ctrl, kCtrlBytes);
   if (e == cudaSuccess) e = cudaMallocHost(&w->ctrl_host, kCtrlBytes);
-  // the clearing must be over before a launch on any stream
-  if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
   if (e == cudaSuccess) e = cudaEventCreate(&w->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&w->ev1);
   if (e != cudaSuccess) {

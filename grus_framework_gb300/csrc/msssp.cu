@@ -162,7 +162,7 @@ int ws_get(grus_graph *g, uint32_t ks, Workspace **out) {
   if (e == cudaSuccess) e = cudaMalloc(&w->ent, (size_t)w->ent_cap * sizeof(uint4));
   if (e == cudaSuccess) e = cudaMalloc(&w->srcs, kMaxSources * 4);
   if (e == cudaSuccess) e = cudaMalloc(&w->ctrl, kCtrlBytes);
-  if (e == cudaSuccess) e = cudaMemset(w->ctrl, 0, kCtrlBytes);
+  if (e == cudaSuccess) e = clear_now(w->ctrl, kCtrlBytes);
   if (e == cudaSuccess) e = cudaMallocHost(&w->ctrl_host, kCtrlBytes);
   if (e == cudaSuccess) e = cudaEventCreate(&w->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&w->ev1);
@@ -305,7 +305,7 @@ void msssp_union_free(void *p) {
 // clear every region's control block (the stream has been synchronised).
 void msssp_union_reset(void *p) {
   UnionWs *w = (UnionWs *)p;
-  if (w && w->ctrl) cudaMemset(w->ctrl, 0, (size_t)w->regions * kCtrlBytes);
+  if (w && w->ctrl) clear_now(w->ctrl, (size_t)w->regions * kCtrlBytes);
 }
 
 bool msssp_union_fits(const void *wsp, int regions, uint64_t max_v, uint64_t max_m, uint64_t entries) {
@@ -342,7 +342,7 @@ int msssp_union_reserve(void **wsp, int regions, uint64_t max_v, uint64_t max_m,
   if (e == cudaSuccess) e = cudaMalloc(&nw->ug, (size_t)nw->regions * ms::kMaxUnion * sizeof(ms::UnionGraph));
   if (e == cudaSuccess) e = cudaMalloc(&nw->seeds, (size_t)nw->regions * 2 * kSeedCap * 4);
   if (e == cudaSuccess) e = cudaMalloc(&nw->ctrl, (size_t)nw->regions * kCtrlBytes);
-  if (e == cudaSuccess) e = cudaMemset(nw->ctrl, 0, (size_t)nw->regions * kCtrlBytes);
+  if (e == cudaSuccess) e = clear_now(nw->ctrl, (size_t)nw->regions * kCtrlBytes);
   if (e == cudaSuccess)
     e = cudaMallocHost(&nw->ug_host, (size_t)nw->regions * ms::kMaxUnion * sizeof(ms::UnionGraph));
   if (e == cudaSuccess) e = cudaMallocHost(&nw->seeds_host, (size_t)nw->regions * 2 * kSeedCap * 4);

@@ -483,7 +483,7 @@ int ws_get(grus_graph *g, Workspace **out) {
   }
   if (e == cudaSuccess) e = cudaMalloc(&w->shared, (size_t)w->warps * 12);
   if (e == cudaSuccess) e = cudaMalloc(&w->ctrl, kCtrlBytes);
-  if (e == cudaSuccess) e = cudaMemset(w->ctrl, 0, kCtrlBytes);
+  if (e == cudaSuccess) e = clear_now(w->ctrl, kCtrlBytes);
   if (e == cudaSuccess) e = cudaMallocHost(&w->ctrl_host, kCtrlBytes + 8);
   if (e == cudaSuccess) std::memset(w->ctrl_host + kOffPlanned, 0, 8);
   if (e == cudaSuccess) e = cudaEventCreate(&w->ev0);

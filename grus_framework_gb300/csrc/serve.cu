@@ -110,7 +110,7 @@ int slot_prepare(grus_server *s, Slot &sl) {
   GRUS_CUDA_TRY(cudaMallocHost(&sl.h_task, sizeof(Task)));
   GRUS_CUDA_TRY(cudaMallocHost(&sl.h_err, 4));
   GRUS_CUDA_TRY(cudaMalloc(&sl.counter, 4));
-  GRUS_CUDA_TRY(cudaMemset(sl.state.err, 0, 4));
+  GRUS_CUDA_TRY(clear_now(sl.state.err, 4));
   sl.ready = true;
   ++s->slots_ready;
   return GRUS_OK;
@@ -356,7 +356,7 @@ void big_scheduler(grus_server *s) {
         // the failed launch may have left its barrier state behind: drain the
         // lane and clear the control block before the next launch on it
         cudaStreamSynchronize(s->big_stream);
-        if (j.ctrl.ctrl) cudaMemset(j.ctrl.ctrl, 0, j.ctrl.bytes);
+        if (j.ctrl.ctrl) clear_now(j.ctrl.ctrl, j.ctrl.bytes);
       }
       big_finish(s, j.group, rc);
       spare.push_back(inflight.front());

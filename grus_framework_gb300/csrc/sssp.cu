@@ -199,7 +199,7 @@ int ws_get(grus_graph *g, Workspace **out) {
   if (e == cudaSuccess) e = cudaMalloc(&w->queues, n1 * 4);
   if (e == cudaSuccess) e = cudaMalloc(&w->chunks, (uint64_t)w->chunk_cap * sizeof(uint4));
   if (e == cudaSuccess) e = cudaMalloc(&w->ctrl, kCtrlBytes);
-  if (e == cudaSuccess) e = cudaMemset(w->ctrl, 0, kCtrlBytes);
+  if (e == cudaSuccess) e = clear_now(w->ctrl, kCtrlBytes);
   if (e == cudaSuccess) e = cudaMallocHost(&w->ctrl_host, kCtrlBytes);
   if (e == cudaSuccess) e = cudaMalloc(&w->trace, kMaxTrace * sizeof(LevelTrace));
   if (e == cudaSuccess) e = cudaMallocHost(&w->trace_host, kMaxTrace * sizeof(LevelTrace));
