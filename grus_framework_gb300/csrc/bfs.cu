@@ -1325,8 +1325,8 @@ __global__ void __launch_bounds__(narrow::kBlock) bfs_narrow(Args a) {
   view.W = a.W;
   view.m = (uint32_t)a.m;
   view.dist = a.depth;
-  view.nearbm = a.front[0];
-  view.near_odd = (uint32_t)(a.front[1] - a.front[0]);
+  view.near0 = a.front[0];
+  view.near1 = a.front[1];
   view.farbm = a.front[2];
   view.far = a.far;
   view.far_cap = narrow::far_cap(a.n, narrow::kFarCapUnit);

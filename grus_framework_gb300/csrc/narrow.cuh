@@ -60,7 +60,9 @@ constexpr uint32_t kCap = 2048;      // entries of one list
 constexpr uint32_t kPiece = 64;      // edges per entry
 // Spilled vertices: up to kWideEdges edges go to one CTA, those of more to the
 // whole cluster, kWide of them in a step.
-constexpr uint32_t kWideEdges = 1024, kWide = 128;
+constexpr uint32_t kWideEdges = 1024, kWide = 32;
+// (Shared has to stay within 131 KB: past it the SM's L1 loses another 32 KB,
+// 4,096 x 4,096 grid 25.9 -> 26.6 ms.)
 // SSSP: a step that relaxes this many spilled vertices is the grid's work; the
 // traversal is handed back.  (A path of 24 vertices into a binary tree of 4 M, ids
 // in level order / shuffled: grid kernel alone 1.75 / 1.44 ms, cluster 3.4 / 5.1,
@@ -109,8 +111,7 @@ struct View {
   const uint32_t *__restrict__ wts;  // unused by BFS
   uint32_t n, W, m;
   uint32_t *dist;
-  uint32_t *nearbm;  // W words by step parity, all zero at the start ...
-  uint32_t near_odd;  // ... the odd steps' this far behind
+  uint32_t *near0, *near1;  // even and odd steps' near bitmaps, W words, all zero at the start
   uint32_t *farbm;   // W words, zero but for what farbm_used announces
   uint2 *far;        // far_bytes(n)
   uint32_t far_cap;
@@ -175,6 +176,8 @@ struct Result {
   uint32_t visits = 0, nr = 0, mr = 0;  // this thread's share (m < 2^32 bounds the last two)
 };
 
+static_assert(sizeof(Shared) <= 131 * 1024, "with 1 KB of the system's, 132 KB");
+
 template <bool kUnit>
 struct Engine {
   const View &a;
@@ -223,7 +226,7 @@ struct Engine {
 
   // The near bitmap that this step's pushes spill to.
   __device__ __forceinline__ uint32_t *near_of(uint32_t st) const {
-    return a.nearbm + (st & 1u ? a.near_odd : 0u);
+    return st & 1u ? a.near1 : a.near0;
   }
 
   __device__ __forceinline__ void spill(uint32_t v) {
@@ -792,7 +795,7 @@ struct Engine {
               relax(en, has);
             }
           }
-          if (!scan) break;
+          if (__builtin_expect(!scan, 1)) break;  // away from the rounds' code
           nc = total = next_spilled();
           if (total == 0) break;
         }

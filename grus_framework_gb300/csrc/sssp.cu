@@ -477,8 +477,8 @@ __global__ void __launch_bounds__(narrow::kBlock) sssp_narrow(Args a) {
   view.timeout_ns = a.timeout_ns;
   const uint32_t L0 = a.whole ? 0u : __ldcg(&a.summary->levels);
   view.tag = a.whole ? 0u : __ldcg(&a.summary->splits);
-  view.nearbm = a.near[0];
-  view.near_odd = (uint32_t)(a.near[1] - a.near[0]);
+  view.near0 = a.near[0];
+  view.near1 = a.near[1];
   view.trace = a.trace && L0 < (uint32_t)kMaxTrace ? (narrow::Trace *)a.trace + L0 : nullptr;
   view.trace_cap = L0 < (uint32_t)kMaxTrace ? kMaxTrace - L0 : 0u;
   narrow::Engine<false> E(view, (narrow::Shared *)smem);
