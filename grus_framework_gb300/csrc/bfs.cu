@@ -1438,7 +1438,8 @@ bool regular_far_ids(const grus_graph *g) {
 // more the more CTAs arrive (1 / 2 / 3 / 4 CTAs: RMAT-16 67 / 70 / 76 / 80 us,
 // uniform graph of 150 K vertices 137 / 150 / 159 / 170, RMAT-18 96 / 99 / 106 /
 // 113); larger ones need the gathers in flight, those without hubs earlier
-// (RMAT-20 129 / 115 / 117 / 122, RMAT-21 223 / 169 / 174 / 177; uniform graphs of
+// (RMAT-20 129 / 115 / 117 / 122, RMAT-21 223 / 169 / 174 / 177, directed RMAT-21
+// of 17 M edges 168 / 131 / 124 / 127; uniform graphs of
 // 400 K vertices 151 / 138 / 123 / 126, of 1.1 M 209 at 3 and 197 at 4, of 3 M
 // 735 / 486 / 431 / 408).  Without pull levels every edge is pushed, and the
 // smallest already need all (directed RMAT-17, 5 M edges: 434 at 1, 260 at 4).
@@ -1447,7 +1448,8 @@ int grid_ctas(const grus_graph *g, bool pull, int occ) {
   if (!pull || g->mem_mode == GRUS_MEM_MANAGED) return occ;
   if (g->n <= 1u << 17) return std::min(occ, 1);
   if (g->n <= 1u << 18) return std::min(occ, 2);
-  if (g->max_deg >= kDefHuge) return g->n <= 1u << 21 ? std::min(occ, 2) : occ;
+  if (g->max_deg >= kDefHuge)
+    return g->n <= 1u << 21 ? std::min(occ, g->flags & GRUS_GRAPH_SYMMETRIC ? 2 : 3) : occ;
   return g->n <= 3u << 18 ? std::min(occ, 3) : occ;
 }
 
