@@ -243,7 +243,7 @@ __device__ __forceinline__ unsigned long long search_list(const Args &a,
 }
 
 // A pull level's unfinished long lists.  Both functions are called by few
-// levels and stay out of line, away from the loop's 32 registers.
+// levels and stay out of line, away from the level loop's registers.
 //
 // In-edges [b, e) of u become pieces for any warp, in the level's own push
 // lists, which a pull level does not use.  More than a chunk of every such list

@@ -32,15 +32,18 @@
 // BFS along a path of 24 vertices into a random graph of 4 M vertices, degree
 // 16, 49.8 ms with queueing, 10.1 without.
 //
-// Bound by latency: a round with one entry takes 1.4-1.6 us (a path of 4,001
-// vertices), of which the atomic's round trip is about a third, and a cluster
-// barrier with its stamp about 0.8 us more.  Measured for SSSP (a 1,021 x
-// 1,531 grid / a 40 x 3,000 grid / RMAT-12, ms; the grid kernel 81 / 88 /
-// 0.29): 512 threads 13.5 / 11.4 / 0.17, 768 threads 10.9 / 11.7 / 0.14,
-// 1,024 threads 10.8 / 13.0 / 0.14.  1,024 are kept for the widest frontiers
-// (BFS on a 4,096 x 4,096 grid: 32.2, 30.2, 25.4 ms).  Rounds per step, with
-// an earlier form at 512 threads: 2 14.2 / 14.8, 4 12.7 / 14.8, 8 13.6 /
-// 18.5, 16 16.7 / 20.8.
+// Which barrier a thread goes to next depends on words that other warps and
+// other CTAs write; narrow_steps.h keeps them so that all threads read the same.
+//
+// Bound by latency: a level of a path of 4,001 vertices takes 1.7 us in BFS and
+// 1.8 in SSSP, of which the atomic's round trip is about a third and its quarter
+// of a cluster barrier with the words of the step 0.2.  Measured for SSSP with an
+// earlier form (a 1,021 x 1,531 grid / a 40 x 3,000 grid / RMAT-12, ms; the grid
+// kernel 81 / 88 / 0.29): 512 threads 13.5 / 11.4 / 0.17, 768 threads 10.9 /
+// 11.7 / 0.14, 1,024 threads 10.8 / 13.0 / 0.14.  1,024 are kept for the widest
+// frontiers (BFS on a 4,096 x 4,096 grid: 32.2, 30.2, 25.4 ms; 25.9 now).  Rounds
+// per step, at 512 threads: 2 14.2 / 14.8, 4 12.7 / 14.8, 8 13.6 / 18.5, 16 16.7 /
+// 20.8.
 #pragma once
 
 #include <cooperative_groups.h>

@@ -33,11 +33,11 @@
 //
 // 20 iterations, ms, before (a warp per 32 vertices, segmented scans, all
 // gathers from L2, two barriers an iteration) and now: RMAT-24 (263 M edges)
-// 23.0, 14.6 (360 G gathers/s); RMAT-20 1.70, 1.01; RMAT-16 0.588, 0.229;
+// 23.0, 14.8 (355 G gathers/s); RMAT-20 1.70, 1.05; RMAT-16 0.62, 0.235;
 // uniform 3 M vertices of degree 16 (no plan) 5.33, 3.62 (265 G/s); 50,021 of
-// degree 12 0.567, 0.162.  Of that for RMAT-24: equal shares 23.0 -> 20.7, the
+// degree 12 0.567, 0.165.  Of that for RMAT-24: equal shares 23.0 -> 20.7, the
 // next batch's loads in flight during the sums -> 16.8, shorter chains between
-// them -> 15.6, no L2 window -> 15.0, compact places -> 14.6.
+// them -> 15.6, no L2 window -> 15.0, compact places -> 14.8.
 #include <algorithm>
 #include <cstring>
 #include <vector>

@@ -229,7 +229,7 @@ size_t big_workspace_bytes(const grus_graph *g, uint32_t algo, bool multi) {
   const size_t n = g->n, m = g->m;
   if (algo == GRUS_ALGO_SSSP && multi) return 128 * n + 16 * n + m / 8 + (1u << 20);
   // a BFS pack also keeps 64 depth bytes per vertex
-  // ... and a single query 2 MB of far lists
+  // ... and a single query up to 1 MB of far lists
   return (algo == GRUS_ALGO_SSSP ? 20 * n : (multi ? 104 * n : 40 * n)) + m / 32 + (4u << 20);
 }
 

@@ -27,7 +27,7 @@
 //
 // A level costs the grid at least 13 us, so levels that stay small are handed
 // to one thread-block cluster (sssp_narrow, narrow.cuh), which also runs small
-// graphs from the start.
+// graphs from the start and may hand back.
 #include <algorithm>
 #include <cstring>
 
@@ -49,7 +49,9 @@ constexpr uint32_t kDefDelta = 640;
 // than kLongDegree out-edges (grids, road networks).
 // The bounds cap what the cluster, a tenth of the chip, can be left with when
 // a long thin stretch ends in a dense part: uniform graphs of 2-9 M edges that
-// were handed over at 2^20 took 1.1-3.2 times the grid kernel's time.
+// were handed over at 2^20 took 1.1-3.2 times the grid kernel's time.  Under the
+// wider bound the cluster hands a frontier that gets too wide for it back
+// (narrow::kHandBack) to a second launch of the persistent kernel.
 constexpr uint32_t kNarrowNf = 128;
 constexpr uint32_t kSteady = 8;
 constexpr uint32_t kSteadyBits = 19, kLongBits = 26;

@@ -110,7 +110,8 @@ typedef struct grus_tuning {
   uint32_t ctas_per_sm;   /* persistent grid = SMs x ctas_per_sm (<= occupancy) */
   uint32_t huge_degree;   /* degree at/above which a vertex is split into chunks */
   uint32_t bu_scan;       /* neighbours a pull thread checks before deferring */
-  uint32_t timeout_ms;    /* bound on every device-side wait */
+  uint32_t timeout_ms;    /* bound on every device-side wait, and on a step of
+                             the cluster kernel */
   uint32_t sssp_delta;    /* SSSP near/far bucket width (distance units) */
   uint32_t bu_words;      /* BFS pull levels: bitmap words per warp step (2 or 4) */
   float multi_alpha;      /* multi-source BFS: push->pull when the union frontier's
@@ -121,10 +122,11 @@ typedef struct grus_tuning {
                              depth as its vertex is found (2); 0: planes from
                              2^22 vertices on */
   uint32_t tail_cluster;  /* BFS and SSSP: hand a traversal whose frontier has
-                             become small to the thread-block-cluster kernel,
-                             and SSSP on a small graph to it altogether (0 or
-                             1), or run every level in the persistent kernel
-                             (2) */
+                             become small to a thread-block-cluster kernel,
+                             and small graphs to it altogether (BFS: unless a
+                             field that only the persistent kernel has is
+                             set) (0 or 1), or run every level in the
+                             persistent kernel (2) */
 } grus_tuning;
 
 /* ---- library ------------------------------------------------------------- */
