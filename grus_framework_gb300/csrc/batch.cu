@@ -603,6 +603,7 @@ static bool own_launch(const grus_batch *b, const std::vector<UnionPack> &l) {
   return l.size() == 1 && b->big[l[0].graph];
 }
 
+// Graphs below big_edges whose SSSP queries may join the packs (pack_small).
 constexpr uint32_t kPackDeg = 9;
 
 static bool packable(const grus_batch *b, uint32_t gi) {
